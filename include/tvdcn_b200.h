@@ -230,6 +230,11 @@ const int *tvdcn_b200_device_status_address(void);
  * after every operator call and raises at the next one.  No counterpart in the reference. */
 int tvdcn_b200_publish_status(int *host_word_device_ptr, void *cuda_stream);
 
+/* Registers such an int for the current device (NULL: none): from then on the tensor-core kernels of every call store
+ * their codes there themselves, and each call's first kernel stores what an earlier one left.  A publish_status for the
+ * same int right behind such a call (same thread) then launches nothing. */
+int tvdcn_b200_watch_status(int *host_word_device_ptr);
+
 /* Self test of the bounded waits: launches, on `cuda_stream`, one small kernel that waits (at most `max_polls`
  * polls of about 20 microseconds, 1 <= max_polls <= 4096) on a barrier nothing ever arrives on, gives up and
  * records code 900 in the status word -- the path a real kernel takes when a wait runs out.  No counterpart in

@@ -154,108 +154,106 @@ int *device_status_word() {
     return cached[dev];
 }
 
-// The channels-last copy of the sampled image is shared by every tensor-core kernel of one call; the entry
-// points reset this marker, the first user stages the image.
-static thread_local const void *t_staged_image = nullptr;
+// Host words that mirror the status word, one per device (tvdcn_b200_watch_status); and whether this thread's latest
+// call has a kernel that publishes an earlier call's code there.
+static std::atomic<int *> g_host_word[64];
+static thread_local bool t_published = false;
 
-static cudaError_t stage_image(const tvdcn_problem *p, const GeoHost &g, const Plan &pl, const void *img, char *ws,
-                               cudaStream_t stream) {
-    if (t_staged_image == img) return cudaSuccess;
-    const int es = p->dtype == TVDCN_F32 ? 4 : 2;
-    cudaError_t e = launch_to_channels_last(img, ws + pl.img_cl, g.B, g.Cs, g.S, es, stream);
-    // Row B*S of the staged image is all zeros: corners that fall outside the image (and the positions past the
-    // end of the last tile) read it, so that an Inf or NaN elsewhere in the image cannot leak into results that
-    // the reference computes without touching that pixel (0 x Inf = NaN).
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(ws + pl.img_cl + (size_t)g.B * g.S * g.Cs * es, 0, (size_t)g.Cs * es, stream);
-    if (e == cudaSuccess) t_staged_image = img;
-    return e;
+static cudaError_t current_status(Status *st) {
+    int dev = 0;
+    st->device = device_status_word();
+    if (st->device == nullptr || cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;
+    st->host = g_host_word[dev].load(std::memory_order_acquire);
+    return cudaSuccess;
 }
 
-// sample -> GEMM on the tensor cores: stage the image channels-last, pack the weights per tap, run.
-static cudaError_t run_sample_gemm_tc(const tvdcn_problem *p, const GeoHost &g, const Plan &pl, const void *img,
-                                      const void *weight, const void *offset, const void *mask, const void *bias,
-                                      void *out, char *ws, cudaStream_t stream) {
-    const int mode = tc_mode_of(p->dtype);
-    int *status = device_status_word();
-    if (status == nullptr) return cudaErrorInvalidDevice;
-    void *w_hi = ws + pl.w_pack;
-    void *w_lo = pl.w_pack_lo != NO_BUF ? (void *)(ws + pl.w_pack_lo) : nullptr;
-    cudaError_t e = stage_image(p, g, pl, img, ws, stream);
-    if (e != cudaSuccess) return e;
-    e = launch_pack_weight_ks(weight, p->dtype, mode, g.groups, g.Cd / g.groups, g.Cs / g.groups, g.K, w_hi, w_lo,
-                              stream);
-    if (e != cudaSuccess) return e;
-    return launch_sample_gemm_tc(g, mode, ws + pl.img_cl, w_hi, w_lo, (const float *)offset, (const float *)mask,
-                                 (const float *)bias, out, status, stream);
-}
+// One call on the tensor-core kernels: pointers into the workspace, and the preparations, which all go into one
+// launch in front of the kernels.
+struct TcCall {
+    const tvdcn_problem *p;
+    GeoHost g;              // padded geometry
+    const Plan &pl;
+    char *ws;
+    Status status{};
+    Stager stage;
+    const float *offset = nullptr, *mask = nullptr, *bias = nullptr;
 
-// GEMM -> scatter / coordinate gradients on the tensor cores.  `img` (the sampled image) is needed only for
-// goff / gmask; `scatter_out` (data type of the problem, [B, Cs, *img]) receives the scattered image plus
-// `bias`; goff / gmask are f32 outputs that the caller has zeroed.
-static cudaError_t run_gemm_scatter_tc(const tvdcn_problem *p, const GeoHost &g, const Plan &pl, const void *dense,
-                                       const void *weight, const void *offset, const void *mask, const void *img,
-                                       void *scatter_out, const void *bias, void *goff, void *gmask, char *ws,
-                                       cudaStream_t stream) {
-    const int mode = tc_mode_of(p->dtype);
-    int *status = device_status_word();
-    if (status == nullptr) return cudaErrorInvalidDevice;
-    void *w_hi = ws + pl.w_pack_kd;
-    void *w_lo = pl.w_pack_kd_lo != NO_BUF ? (void *)(ws + pl.w_pack_kd_lo) : nullptr;
-    cudaError_t e = launch_pack_weight_kd(weight, p->dtype, mode, g.groups, g.Cd / g.groups, g.Cs / g.groups, g.K, w_hi, w_lo,
-                              stream);
-    if (e != cudaSuccess) return e;
-    const bool want_coord = goff != nullptr || gmask != nullptr;
-    if (want_coord) {
-        e = stage_image(p, g, pl, img, ws, stream);
-        if (e != cudaSuccess) return e;
+    TcCall(const tvdcn_problem *p_, const GeoHost &real, const Plan &pl_, char *ws_)
+        : p(p_), g(tc_geometry(real)), pl(pl_), ws(ws_) {}
+    void *at(size_t buf) const { return buf == NO_BUF ? nullptr : ws + buf; }
+    void parts(const size_t (&buf)[3], void *(&out)[3]) const {
+        for (int q = 0; q < 3; ++q) out[q] = at(buf[q]);
     }
-    float *acc = nullptr;
-    if (scatter_out != nullptr) {
-        acc = (float *)(ws + pl.img_grad_cl);
-        e = cudaMemsetAsync(acc, 0, (size_t)g.B * g.S * g.Cs * sizeof(float), stream);
-        if (e != cudaSuccess) return e;
+    void stage_image(const void *img) { stage.image(img, at(pl.img_cl), g, p->dtype == TVDCN_F32 ? 4 : 2); }
+    void stage_weight(const void *weight, bool kd) {
+        void *w[3];
+        parts(kd ? pl.w_pack_kd : pl.w_pack, w);
+        stage.pack(weight, w, g, p->dtype, mode_mat_parts(pl.mode), kd);
     }
-    e = launch_gemm_scatter_tc(g, mode, dense, w_hi, w_lo, want_coord ? ws + pl.img_cl : nullptr,
-                               (const float *)offset, (const float *)mask, acc, (float *)goff, (float *)gmask, status,
-                               stream);
-    if (e != cudaSuccess) return e;
-    if (scatter_out != nullptr)
-        e = launch_from_channels_last_bias(acc, (const float *)bias, scatter_out, p->dtype, g.B, g.Cs, g.S, stream);
-    return e;
-}
-
-// sampled weight gradient on the tensor cores; `gw_acc` is zero-initialised f32.  `dense_channel_sum` (f32, Cd
-// values, may be NULL): wanted sum of the dense tensor over batch and space -- where the dense tensor is split into
-// bf16 parts anyway (f32 data) the same pass takes it and `*summed` says so, else the caller runs channel_sum.
-static cudaError_t run_sample_wgrad_tc(const tvdcn_problem *p, const GeoHost &g, const Plan &pl, const void *dense,
-                                       const void *img, const void *offset, const void *mask, void *gw_acc, char *ws,
-                                       cudaStream_t stream, float *dense_channel_sum = nullptr,
-                                       bool *summed = nullptr) {
-    const int mode = tc_mode_of(p->dtype);
-    int *status = device_status_word();
-    if (status == nullptr) return cudaErrorInvalidDevice;
-    cudaError_t e = stage_image(p, g, pl, img, ws, stream);
-    if (e != cudaSuccess) return e;
-    const void *d_hi = dense, *d_lo = nullptr;
-    if (summed) *summed = false;
-    if (p->dtype == TVDCN_F32) {
-        if (dense_channel_sum != nullptr &&
-            can_split_f32_with_channel_sum((const float *)dense, ws + pl.dense_hi, ws + pl.dense_lo, g.P)) {
-            e = launch_split_f32_channel_sum((const float *)dense, ws + pl.dense_hi, ws + pl.dense_lo, g.B, g.Cd, g.P,
-                                             dense_channel_sum, stream);
-            if (summed) *summed = true;
-        } else {
-            e = launch_split_f32((const float *)dense, ws + pl.dense_hi, ws + pl.dense_lo,
-                                 (int64_t)g.B * g.Cd * g.P, stream);
+    void stage_aux(const void *off, const void *msk, const void *bia) {
+        const int64_t points = (int64_t)g.B * g.K * g.P;
+        auto widen = [&](const void *src, size_t buf, int64_t n) -> const float * {
+            if (src == nullptr || buf == NO_BUF) return static_cast<const float *>(src);
+            stage.widen(src, at(buf), p->aux_dtype, n);
+            return static_cast<const float *>(at(buf));
+        };
+        offset = widen(off, pl.off32, points * g.og * g.dim);
+        mask = widen(msk, pl.mask32, points * g.mg);
+        bias = widen(bia, pl.bias32, p->out_channels);
+    }
+    cudaError_t prepare(cudaStream_t stream) {
+        cudaError_t e = current_status(&status);
+        if (e == cudaSuccess) e = stage.launch(status, stream);
+        t_published = !stage.empty();
+        return e;
+    }
+    cudaError_t sample_gemm(void *out, cudaStream_t stream) const {
+        void *w[3];
+        parts(pl.w_pack, w);
+        return launch_sample_gemm_tc(g, pl.mode, at(pl.img_cl), w, offset, mask, bias, out, status, stream);
+    }
+    // scatter_out (data type of the problem, [B, Cs, *img], may be null) receives the scattered image plus bias;
+    // goff / gmask are zeroed f32 accumulators, may be null
+    cudaError_t gemm_scatter(const void *dense, void *scatter_out, void *goff, void *gmask, cudaStream_t stream) const {
+        void *w[3];
+        parts(pl.w_pack_kd, w);
+        float *acc = scatter_out != nullptr ? static_cast<float *>(at(pl.img_grad_cl)) : nullptr;
+        const bool want_coord = goff != nullptr || gmask != nullptr;
+        cudaError_t e = launch_gemm_scatter_tc(g, pl.mode, dense, w, want_coord ? at(pl.img_cl) : nullptr, offset, mask, acc,
+                                               (float *)goff, (float *)gmask, status, stream);
+        if (e == cudaSuccess && scatter_out != nullptr)
+            e = launch_from_channels_last_bias(acc, bias, scatter_out, p->dtype, g, stream);
+        return e;
+    }
+    cudaError_t channel_sum(const void *x, int C, int S, void *out, cudaStream_t stream) const {
+        return launch_dense_pass(x, p->dtype, 0, nullptr, g.B, C, S, 0, (float *)at(pl.sum_partial),
+                                 (unsigned *)at(pl.sum_done), out, p->aux_dtype, stream);
+    }
+    // Weight gradient into the staged accumulator and from there to grad_weight.  f32 data: the dense tensor is split
+    // into bf16 parts first; the same pass takes its channel sums (bias gradient of the conv) where `sum_out` is given
+    // and the pointer allows 16-byte loads, which *summed reports.
+    cudaError_t sample_wgrad(const void *dense, void *grad_weight, void *sum_out, bool *summed, cudaStream_t stream) const {
+        void *d[3] = {const_cast<void *>(dense), nullptr, nullptr};
+        int pitch = g.P;
+        cudaError_t e = cudaSuccess;
+        *summed = false;
+        if (pl.dense[0] != NO_BUF) {
+            parts(pl.dense, d);
+            pitch = pl.dense_pitch;
+            if (p->dtype == TVDCN_F32) {
+                *summed = sum_out != nullptr && reinterpret_cast<uintptr_t>(dense) % 16 == 0;
+                e = launch_dense_pass(dense, p->dtype, mode_mat_parts(pl.mode_sw), d, g.B, g.Cd_r, g.P, pitch,
+                                      (float *)at(pl.sum_partial), (unsigned *)at(pl.sum_done),
+                                      *summed ? sum_out : nullptr, p->aux_dtype, stream);
+            }
         }
-        if (e != cudaSuccess) return e;
-        d_hi = ws + pl.dense_hi;
-        d_lo = ws + pl.dense_lo;
+        float *acc = static_cast<float *>(at(pl.gw_acc));
+        if (e == cudaSuccess)
+            e = launch_sample_wgrad_tc(g, pl.mode_sw, d, pitch, at(pl.img_cl), offset, mask, acc, status, stream);
+        if (e == cudaSuccess) e = launch_unpack_weight_grad(acc, grad_weight, p->dtype, g, stream);
+        return e;
     }
-    return launch_sample_wgrad_tc(g, mode, d_hi, d_lo, ws + pl.img_cl, (const float *)offset, (const float *)mask,
-                                  (float *)gw_acc, status, stream);
-}
+};
 
 // Waits on a barrier that nothing arrives on, with a small poll limit, and reports the time-out the way the
 // tensor-core kernels do.
@@ -271,12 +269,8 @@ __global__ void bounded_wait_selftest_kernel(int *status, uint32_t max_polls) {
     if (!done && threadIdx.x == 0) atomicExch(status, 900);
 }
 
-// Copies a non-zero status word to host memory the device can write (mapped pinned memory): a store from a
-// kernel, so the copy engines, which may be busy with a caller's own large transfers, are not involved.
-__global__ void publish_status_kernel(const int *status, int *host_word) {
-    const int v = *status;
-    if (v != 0) *host_word = v;
-}
+// What a call's first tensor-core kernel does in passing, for calls that launch none.
+__global__ void publish_status_kernel(const Status status) { ptx::publish(status); }
 
 }  // namespace tvdcn_b200
 
@@ -287,6 +281,19 @@ using namespace tvdcn_b200;
         cudaError_t e__ = (expr);                        \
         if (e__ != cudaSuccess) return cuda_fail(e__, #expr); \
     } while (0)
+
+// The plan of a call.  Shapes that the tensor-core kernels take only with padding also run on the SIMT kernels, which
+// need less workspace or none: a caller that brings no more than that gets those.
+template <typename F>
+static Plan plan_for(const tvdcn_problem *p, size_t workspace_bytes, F &&plan) {
+    Plan pl = plan(p);
+    if (pl.tensor && pl.wide && pl.total > workspace_bytes && p->engine == TVDCN_ENGINE_AUTO) {
+        tvdcn_problem simt = *p;
+        simt.engine = TVDCN_ENGINE_SIMT;
+        pl = plan(&simt);
+    }
+    return pl;
+}
 
 extern "C" {
 
@@ -348,28 +355,32 @@ int tvdcn_b200_deform_conv_forward(const tvdcn_problem *p, const void *input, co
     if ((p->mask_groups > 0) != (mask != nullptr))
         return fail(TVDCN_ERR_INVALID, "mask pointer and mask_groups disagree");
     cudaStream_t stream = (cudaStream_t)cuda_stream;
-    const Plan pl = plan_forward(p);
+    const Plan pl = plan_for(p, workspace_bytes, [](const tvdcn_problem *q) { return plan_forward(q); });
     if (p->engine == TVDCN_ENGINE_TENSOR && !pl.tensor)
         return fail(TVDCN_ERR_UNSUPPORTED, "shape not covered by the tensor-core kernels: %s", pl.why_not);
     rc = check_ws(pl, workspace, workspace_bytes);
     if (rc) return rc;
     char *ws = (char *)workspace;
-    t_staged_image = nullptr;
     const GeoHost g = make_geo_host(p);
     const int dt = p->dtype, aux = p->aux_dtype;
+    t_published = false;
 
-    if (pl.tc_sg) {
-        CUDA_TRY(run_sample_gemm_tc(p, g, pl, input, weight, offset, mask, bias, output, ws, stream));
+    if (pl.tensor) {
+        TcCall tc(p, g, pl, ws);
+        if (pl.tc_sg) tc.stage_image(input);
+        tc.stage_weight(weight, pl.tc_gs);
+        tc.stage_aux(offset, mask, bias);
+        if (pl.tc_gs) tc.stage.zero(ws + pl.img_grad_cl, (int64_t)g.B * g.S * tc.g.Cs * (int64_t)sizeof(float));
+        CUDA_TRY(tc.prepare(stream));
+        if (pl.tc_sg)
+            CUDA_TRY(tc.sample_gemm(output, stream));
+        else
+            CUDA_TRY(tc.gemm_scatter(input, output, nullptr, nullptr, stream));
         return TVDCN_OK;
     }
 
     if (!p->transposed) {
         CUDA_TRY(launch_sample_gemm(g, dt, aux, input, weight, offset, mask, bias, output, stream));
-        return TVDCN_OK;
-    }
-    if (pl.tc_gs) {
-        CUDA_TRY(run_gemm_scatter_tc(p, g, pl, input, weight, offset, mask, nullptr, output, bias, nullptr, nullptr, ws,
-                                     stream));
         return TVDCN_OK;
     }
     // transposed: output (= sampled image) starts as the bias and receives the scatter
@@ -381,9 +392,10 @@ int tvdcn_b200_deform_conv_forward(const tvdcn_problem *p, const void *input, co
     return TVDCN_OK;
 }
 
-// Side stream of the backward pass: the weight-gradient kernel and the bias sum do not depend on the scatter
-// kernel, so they run beside it and fill the SMs that the scatter kernel's last, partial wave of CTAs leaves
-// idle.  One stream and two events per host thread and device, created on first use and kept; fork and join are
+// Side stream of the backward pass: the scatter kernel does not depend on the weight-gradient kernel and the bias sum,
+// so it is queued beside them and its CTAs fill the SMs that their last, partial wave leaves idle.  The weight gradient
+// keeps the caller's stream and goes first: it is final early in the call, so its all-reduce can run under the rest of
+// the scatter (the other way round its CTAs had to wait for whole waves of scatter CTAs to retire).  One stream and two events per host thread and device, created on first use and kept; fork and join are
 // event waits, so the caller's stream still orders the whole call (and a capture of it picks both streams up).
 // TVDCN_B200_OVERLAP=0 keeps everything on the caller's stream, and so does tvdcn_b200_timing_enable(1).
 struct SideStream {
@@ -404,11 +416,7 @@ static SideStream *side_stream() {
     SideStream &s = per_device[dev];
     if (!s.tried) {
         s.tried = true;
-        // highest priority: the weight-gradient CTAs take the SMs the scatter kernel frees first, so the weight
-        // gradient is complete early in the call and its all-reduce can run under the rest of the scatter
-        int least = 0, greatest = 0;
-        (void)cudaDeviceGetStreamPriorityRange(&least, &greatest);
-        if (cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, greatest) != cudaSuccess ||
+        if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess) {
             s.stream = nullptr;
@@ -444,7 +452,6 @@ int tvdcn_b200_deform_conv_backward_ex(const tvdcn_problem *p, const void *grad_
     const int64_t n_off = (int64_t)g.B * g.og * g.K * g.dim * g.P;
     const int64_t n_mask = (int64_t)g.B * g.mg * g.K * g.P;
     const int64_t n_img = (int64_t)g.B * g.Cs * g.S;
-    const int64_t n_dense = (int64_t)g.B * g.Cd * g.P;
     if (p->batch == 0) {
         if (grad_weight) CUDA_TRY(cudaMemsetAsync(grad_weight, 0, n_w * es, stream));
         if (grad_bias) CUDA_TRY(cudaMemsetAsync(grad_bias, 0, (size_t)p->out_channels * as, stream));
@@ -460,120 +467,103 @@ int tvdcn_b200_deform_conv_backward_ex(const tvdcn_problem *p, const void *grad_
     if (grad_offset != nullptr && offset == nullptr)
         return fail(TVDCN_ERR_INVALID, "grad_offset requested without offset");
     if (grad_mask != nullptr && mask == nullptr) return fail(TVDCN_ERR_INVALID, "grad_mask requested without mask");
-    const Plan pl = plan_backward(p, grad_input != nullptr, grad_weight != nullptr, grad_offset != nullptr,
-                                  grad_mask != nullptr);
+    const Plan pl = plan_for(p, workspace_bytes, [&](const tvdcn_problem *q) {
+        return plan_backward(q, grad_input != nullptr, grad_weight != nullptr, grad_offset != nullptr, grad_mask != nullptr);
+    });
     if (p->engine == TVDCN_ENGINE_TENSOR && !pl.tensor)
         return fail(TVDCN_ERR_UNSUPPORTED, "shape not covered by the tensor-core kernels: %s", pl.why_not);
     rc = check_ws(pl, workspace, workspace_bytes);
     if (rc) return rc;
     char *ws = (char *)workspace;
-    // the caller may vouch that the forward call's staging of `input` is still at the start of this workspace
-    // (only where the forward call for this problem stages the image at all, and at the same offset)
-    t_staged_image = nullptr;
-    if ((p->flags & TVDCN_FLAG_REUSE_STAGED_INPUT) && !p->transposed && pl.tensor) {
-        const Plan fwd = plan_forward(p);
-        if (fwd.img_cl != NO_BUF && fwd.img_cl == pl.img_cl) t_staged_image = input;
-    }
-
+    t_published = false;
     const size_t acs = dtype_size(acc_dtype(dt));
     // accumulation targets: the outputs themselves when they already have the accumulation type
     void *gw_acc = grad_weight ? (pl.gw_acc != NO_BUF ? (void *)(ws + pl.gw_acc) : grad_weight) : nullptr;
     void *goff_acc = grad_offset ? (pl.goff_acc != NO_BUF ? (void *)(ws + pl.goff_acc) : grad_offset) : nullptr;
     void *gmask_acc = grad_mask ? (pl.gmask_acc != NO_BUF ? (void *)(ws + pl.gmask_acc) : grad_mask) : nullptr;
-    if (gw_acc) CUDA_TRY(cudaMemsetAsync(gw_acc, 0, n_w * acs, stream));
-    if (goff_acc) CUDA_TRY(cudaMemsetAsync(goff_acc, 0, n_off * acs, stream));
-    if (gmask_acc) CUDA_TRY(cudaMemsetAsync(gmask_acc, 0, n_mask * acs, stream));
+    // sampled image and dense tensor: conv: input and grad_output, transposed: grad_output and input
+    const void *img = p->transposed ? grad_output : input, *dense = p->transposed ? input : grad_output;
+    void *gi_acc = nullptr;   // conv on the SIMT kernels: where grad_input is accumulated
+    if (!p->transposed && grad_input && !pl.tc_gs) gi_acc = pl.img_acc != NO_BUF ? (void *)(ws + pl.img_acc) : grad_input;
 
     // The weight-gradient kernel reads 16-bit dense tensors by TMA straight from the caller's pointer, which must
     // then sit on a 16-byte boundary (a tensor view with a storage offset may not): the SIMT kernel takes over.
-    const void *dense_for_w = p->transposed ? input : grad_output;
-    const bool tc_sw = pl.tc_sw && (p->dtype == TVDCN_F32 || (reinterpret_cast<uintptr_t>(dense_for_w) & 15) == 0);
+    const bool tc_sw = pl.tc_sw && (pl.dense[0] != NO_BUF || (reinterpret_cast<uintptr_t>(dense) & 15) == 0);
 
-    // the tensor-core weight-gradient kernel accumulates in a staged layout: convert right behind it
-    // (for conv with f32 data and f32 bias the split of grad_output also takes grad_bias)
-    bool bias_summed = false;
-    auto wgrad_tc = [&](const void *dense, const void *img, cudaStream_t st) -> cudaError_t {
-        float *sum_out = (!p->transposed && grad_bias != nullptr && aux == TVDCN_F32) ? (float *)grad_bias : nullptr;
-        cudaError_t e = run_sample_wgrad_tc(p, g, pl, dense, img, offset, mask, gw_acc, ws, st, sum_out, &bias_summed);
-        if (e != cudaSuccess) return e;
-        return launch_unpack_weight_grad((const float *)gw_acc, grad_weight, dt, g.groups, g.Cd / g.groups,
-                                         g.Cs / g.groups, g.K, st);
-    };
-
-    // fork: weight gradient + bias sum on the side stream when both sides run on the tensor cores
+    TcCall tc(p, g, pl, ws);
+    if (pl.tensor) {
+        // The caller may vouch that the forward call's staging of `input` is still at the start of this workspace
+        // (only where the forward call for this problem stages the image at all, and at the same offset).
+        bool staged = false;
+        if ((p->flags & TVDCN_FLAG_REUSE_STAGED_INPUT) && !p->transposed) {
+            const Plan fwd = plan_forward(p);
+            staged = fwd.img_cl != NO_BUF && fwd.img_cl == pl.img_cl;
+        }
+        if (!staged && (pl.tc_sg || tc_sw || goff_acc || gmask_acc)) tc.stage_image(img);
+        if (pl.tc_gs) tc.stage_weight(weight, true);
+        if (pl.tc_sg) tc.stage_weight(weight, false);
+        tc.stage_aux(offset, mask, nullptr);
+        if (tc_sw && p->dtype != TVDCN_F32 && pl.dense[0] != NO_BUF)
+            tc.stage.pitch(dense, ws + pl.dense[0], (int64_t)g.B * g.Cd, g.P, pl.dense_pitch);
+        if (grad_bias) tc.stage.zero(ws + pl.sum_done, (int64_t)p->out_channels * (int64_t)sizeof(unsigned));
+    }
+    auto zero = [&](void *ptr, int64_t bytes) { if (ptr != nullptr) tc.stage.zero(ptr, bytes); };
+    zero(gw_acc, pl.tc_sw ? (int64_t)g.Cd * (tc.g.Cs / g.groups) * g.K * 4 : n_w * (int64_t)acs);
+    zero(goff_acc, n_off * (int64_t)acs);
+    zero(gmask_acc, n_mask * (int64_t)acs);
+    zero(gi_acc, n_img * (int64_t)acs);
+    // Fork: the scatter kernel on the side stream when both sides run on the tensor cores.
     SideStream *side = (tc_sw && gw_acc && (pl.tc_gs || pl.tc_sg)) ? side_stream() : nullptr;
-    cudaStream_t wstream = stream;
+    cudaStream_t sstream = side != nullptr ? side->stream : stream;
+    // A large scatter accumulator is zeroed under the weight gradient; below 32 MB (5 us) the launch costs more.
+    const int64_t acc_bytes = pl.img_grad_cl != NO_BUF ? (int64_t)g.B * g.S * tc.g.Cs * 4 : 0;
+    const bool zero_later = side != nullptr && acc_bytes > (32 << 20);
+    if (acc_bytes > 0 && !zero_later) tc.stage.zero(ws + pl.img_grad_cl, acc_bytes);
+    CUDA_TRY(tc.prepare(stream));
     if (side != nullptr) {
-        CUDA_TRY(stage_image(p, g, pl, p->transposed ? grad_output : input, ws, stream));
         CUDA_TRY(cudaEventRecord(side->fork, stream));
-        CUDA_TRY(cudaStreamWaitEvent(side->stream, side->fork, 0));
-        wstream = side->stream;
+        CUDA_TRY(cudaStreamWaitEvent(sstream, side->fork, 0));
     }
-
-    if (!p->transposed) {
-        // sampled image = input, dense = grad_output
-        void *gi_acc = grad_input ? (pl.img_acc != NO_BUF ? (void *)(ws + pl.img_acc) : grad_input) : nullptr;
-        if (side != nullptr) {
-            CUDA_TRY(wgrad_tc(grad_output, input, wstream));
-            if (grad_bias && !bias_summed)
-                CUDA_TRY(launch_channel_sum(dt, aux, grad_output, g.B, g.Cd, g.P, grad_bias, wstream));
-        }
-        if (pl.tc_gs) {
-            CUDA_TRY(run_gemm_scatter_tc(p, g, pl, grad_output, weight, offset, mask, input, grad_input, nullptr,
-                                         goff_acc, gmask_acc, ws, stream));
-            gi_acc = nullptr;
-        } else {
-            if (gi_acc) CUDA_TRY(cudaMemsetAsync(gi_acc, 0, n_img * acs, stream));
-            if (gi_acc || goff_acc || gmask_acc)
-                CUDA_TRY(launch_gemm_scatter(g, dt, aux, grad_output, weight, offset, mask, input, gi_acc, goff_acc,
-                                             gmask_acc, stream));
-        }
-        if (side != nullptr) {
-            // already queued beside the scatter kernel
-        } else if (gw_acc && tc_sw)
-            CUDA_TRY(wgrad_tc(grad_output, input, stream));
+    auto weight_and_bias = [&]() -> int {
+        bool summed = false;
+        if (gw_acc && tc_sw)
+            CUDA_TRY(tc.sample_wgrad(dense, grad_weight, p->transposed ? nullptr : grad_bias, &summed, stream));
         else if (gw_acc)
-            CUDA_TRY(launch_sample_wgrad(g, dt, aux, grad_output, input, offset, mask, gw_acc, stream));
-        if (grad_bias && side == nullptr && !bias_summed)
-            CUDA_TRY(launch_channel_sum(dt, aux, grad_output, g.B, g.Cd, g.P, grad_bias, stream));
-        if (gi_acc && pl.img_acc != NO_BUF) CUDA_TRY(launch_cast_from_acc(dt, gi_acc, grad_input, n_img, stream));
-    } else {
-        // sampled image = grad_output, dense = input
-        if (side != nullptr) {
-            CUDA_TRY(wgrad_tc(input, grad_output, wstream));
-            if (grad_bias) CUDA_TRY(launch_channel_sum(dt, aux, grad_output, g.B, g.Cs, g.S, grad_bias, wstream));
+            CUDA_TRY(launch_sample_wgrad(g, dt, aux, dense, img, offset, mask, gw_acc, stream));
+        if (grad_bias && !summed) {
+            const int c = (int)p->out_channels, n = p->transposed ? g.S : g.P;
+            if (pl.tensor)
+                CUDA_TRY(tc.channel_sum(grad_output, c, n, grad_bias, stream));
+            else
+                CUDA_TRY(launch_channel_sum(dt, aux, grad_output, g.B, c, n, grad_bias, stream));
         }
-        if ((goff_acc || gmask_acc) && pl.tc_gs)
-            CUDA_TRY(run_gemm_scatter_tc(p, g, pl, input, weight, offset, mask, grad_output, nullptr, nullptr, goff_acc,
-                                         gmask_acc, ws, stream));
-        else if (goff_acc || gmask_acc)
-            CUDA_TRY(launch_gemm_scatter(g, dt, aux, input, weight, offset, mask, grad_output, nullptr, goff_acc,
-                                         gmask_acc, stream));
-        if (grad_input && pl.tc_sg)
-            CUDA_TRY(run_sample_gemm_tc(p, g, pl, grad_output, weight, offset, mask, nullptr, grad_input, ws, stream));
-        else if (grad_input)
-            CUDA_TRY(launch_sample_gemm(g, dt, aux, grad_output, weight, offset, mask, nullptr, grad_input, stream));
-        if (side != nullptr) {
-            // already queued beside the other kernels
-        } else if (gw_acc && tc_sw)
-            CUDA_TRY(wgrad_tc(input, grad_output, stream));
-        else if (gw_acc)
-            CUDA_TRY(launch_sample_wgrad(g, dt, aux, input, grad_output, offset, mask, gw_acc, stream));
-        if (grad_bias && side == nullptr)
-            CUDA_TRY(launch_channel_sum(dt, aux, grad_output, g.B, g.Cs, g.S, grad_bias, stream));
-        (void)n_dense;
+        if (gw_acc && pl.gw_acc != NO_BUF && !tc_sw)
+            CUDA_TRY(launch_cast_from_acc(dt, gw_acc, grad_weight, n_w, stream));
+        if (weight_grad_ready) CUDA_TRY(cudaEventRecord((cudaEvent_t)weight_grad_ready, stream));
+        return TVDCN_OK;
+    };
+    if ((rc = weight_and_bias()) != TVDCN_OK) return rc;
+    // scatter and coordinate gradients; the transposed conv's grad_input is a sample -> GEMM
+    if (zero_later) {
+        Stager later;
+        later.zero(ws + pl.img_grad_cl, acc_bytes);
+        CUDA_TRY(later.launch(tc.status, sstream));
     }
-    // grad_weight / grad_bias are final on the side stream: the tensor-core kernel's staged sum is converted there
-    const bool gw_in_place = true;
+    if (pl.tc_gs)
+        CUDA_TRY(tc.gemm_scatter(dense, p->transposed ? nullptr : grad_input, goff_acc, gmask_acc, sstream));
+    else if (gi_acc || goff_acc || gmask_acc)
+        CUDA_TRY(launch_gemm_scatter(g, dt, aux, dense, weight, offset, mask, img, gi_acc, goff_acc, gmask_acc, sstream));
+    if (p->transposed && grad_input) {
+        if (pl.tc_sg)
+            CUDA_TRY(tc.sample_gemm(grad_input, sstream));
+        else
+            CUDA_TRY(launch_sample_gemm(g, dt, aux, img, weight, offset, mask, nullptr, grad_input, sstream));
+    }
     if (side != nullptr) {  // join
-        if (weight_grad_ready && gw_in_place)
-            CUDA_TRY(cudaEventRecord((cudaEvent_t)weight_grad_ready, side->stream));
-        CUDA_TRY(cudaEventRecord(side->join, side->stream));
+        CUDA_TRY(cudaEventRecord(side->join, sstream));
         CUDA_TRY(cudaStreamWaitEvent(stream, side->join, 0));
     }
-    if (gw_acc && pl.gw_acc != NO_BUF && !tc_sw) CUDA_TRY(launch_cast_from_acc(dt, gw_acc, grad_weight, n_w, stream));
-    if (weight_grad_ready && !(side != nullptr && gw_in_place))
-        CUDA_TRY(cudaEventRecord((cudaEvent_t)weight_grad_ready, stream));
+    if (gi_acc && pl.img_acc != NO_BUF) CUDA_TRY(launch_cast_from_acc(dt, gi_acc, grad_input, n_img, stream));
     if (goff_acc && pl.goff_acc != NO_BUF) CUDA_TRY(launch_cast_from_acc(aux, goff_acc, grad_offset, n_off, stream));
     if (gmask_acc && pl.gmask_acc != NO_BUF)
         CUDA_TRY(launch_cast_from_acc(aux, gmask_acc, grad_mask, n_mask, stream));
@@ -670,10 +660,22 @@ const int *tvdcn_b200_device_status_address(void) { return device_status_word();
 
 int tvdcn_b200_publish_status(int *host_word_device_ptr, void *cuda_stream) {
     if (host_word_device_ptr == nullptr) return fail(TVDCN_ERR_INVALID, "host_word_device_ptr is NULL");
-    const int *status = device_status_word();
-    if (status == nullptr) return fail(TVDCN_ERR_CUDA, "status word not found");
-    publish_status_kernel<<<1, 1, 0, (cudaStream_t)cuda_stream>>>(status, host_word_device_ptr);
+    Status status;
+    CUDA_TRY(current_status(&status));
+    const bool published = t_published;
+    t_published = false;
+    if (published && status.host == host_word_device_ptr) return TVDCN_OK;   // the call's own kernels did it
+    status.host = host_word_device_ptr;
+    publish_status_kernel<<<1, 1, 0, (cudaStream_t)cuda_stream>>>(status);
     CUDA_TRY(cudaGetLastError());
+    return TVDCN_OK;
+}
+
+int tvdcn_b200_watch_status(int *host_word_device_ptr) {
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(TVDCN_ERR_UNSUPPORTED, "device index %d", dev);
+    g_host_word[dev].store(host_word_device_ptr, std::memory_order_release);
     return TVDCN_OK;
 }
 

@@ -47,6 +47,7 @@ struct Geo {
     int K;          // kernel taps
     int S, P;       // spatial elements per image: sampled image, offset grid
     int csg, cdg;   // channels per convolution group
+    int Cd_r, cdg_r; // tensor-core kernels: dense channels of the caller's tensor where Cd, cdg are padded to tiles
     int cs_per_og, cs_per_mg;
     long long BP;   // B * P
     int img[DIM], grid[DIM], ker[DIM], stride[DIM], pad[DIM], dil[DIM];

@@ -12,6 +12,11 @@ struct GeoHost {
     int dim;
     int B, Cs, Cd, groups, og, mg, K, S, P;
     int img[3], grid[3], ker[3], stride[3], pad[3], dil[3];
+    // Only the tensor-core kernels look at these: their chunks of 64 channels must not straddle a convolution,
+    // offset or mask group, so tc_geometry() pads every run of `gran` sampled channels that share their groups to
+    // gran_pad (in the staged image and weights) and the dense channels of a group to a multiple of 64.  Cs and Cd
+    // then count padded channels, Cs_r and Cd_r those of the caller's tensors.
+    int Cs_r, Cd_r, gran, gran_pad;
 };
 
 enum : int { DT_F32 = 0, DT_F64 = 1, DT_F16 = 2, DT_BF16 = 3 };
@@ -19,6 +24,28 @@ enum : int { DT_F32 = 0, DT_F64 = 1, DT_F16 = 2, DT_BF16 = 3 };
 inline size_t dtype_size(int dt) { return dt == DT_F64 ? 8 : (dt == DT_F32 ? 4 : 2); }
 // accumulation type that goes with a data type: double for f64, float otherwise
 inline int acc_dtype(int dt) { return dt == DT_F64 ? DT_F64 : DT_F32; }
+
+// How the 16-bit tensor-core operands are derived from the user's data type.  A sampled column or a matrix operand
+// (weights, dense tensor) travels as one or more 16-bit parts of decreasing magnitude whose sum is the value:
+//   TC_BF16, TC_F16   16-bit data; columns blended and rounded in that type: one part, one MMA per K step
+//   TC_SPLIT          f32 data as bf16 hi + lo (about 16 bits): three MMAs (hi*hi, lo*hi, hi*lo)
+//   TC_*_WIDE         the precision of the SIMT kernels, for the shapes and types that only those used to take:
+//                     16-bit data with columns blended in f32 and kept in two parts (the matrix operand is exact in
+//                     one): two MMAs; f32 data in three bf16 parts (all 24 bits): the six products above 2^-24
+// For f32 data the products of the leading parts have accumulators of their own: the tensor core's f32 accumulation
+// rounds toward zero, by half an ulp of the accumulator per MMA on average, so the small products must not touch the
+// large sum (16-bit results do not see it).
+enum : int { TC_BF16 = 0, TC_F16 = 1, TC_SPLIT = 2, TC_BF16_WIDE = 3, TC_F16_WIDE = 4, TC_F32_WIDE = 5 };
+inline int mode_col_parts(int mode) { return mode == TC_F32_WIDE ? 3 : (mode >= TC_SPLIT ? 2 : 1); }
+inline int mode_mat_parts(int mode) { return mode == TC_F32_WIDE ? 3 : (mode == TC_SPLIT ? 2 : 1); }
+inline bool mode_f32(int mode) { return mode == TC_SPLIT || mode == TC_F32_WIDE; }
+
+// Where a kernel whose bounded wait ran out leaves a code: the device word, and the host word (mapped pinned memory,
+// may be null) that the PyTorch front end looks at.
+struct Status {
+    int *device;
+    int *host;
+};
 
 void count_launch(int n = 1);
 

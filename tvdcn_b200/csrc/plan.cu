@@ -14,77 +14,113 @@ struct Bump {
         return at;
     }
 };
+// A granule of channels padded by more than this runs on the SIMT kernels.
+constexpr int MAX_CHANNEL_PADDING = 8;
 bool is16(int dt) { return dt == DT_F16 || dt == DT_BF16; }
 
-// Shape conditions shared by all tensor-core kernels: K chunks of 64 channels of one tap must not
-// straddle a convolution, offset or mask group, and rows of the channels-last image are indexed in 32 bits.
+int gcd(int a, int b) { return b == 0 ? a : gcd(b, a % b); }
+int round_up(int v, int m) { return (v + m - 1) / m * m; }
+
+// Shape conditions shared by all tensor-core kernels, on the padded geometry: rows of the channels-last image are
+// indexed in 32 bits, and padding must not outweigh what the tensor cores gain.
 const char *tc_common(const tvdcn_problem *p, const GeoHost &g) {
     if (p->engine == TVDCN_ENGINE_SIMT) return "SIMT engine requested";
     if (p->dtype == TVDCN_F64) return "f64 has no tensor-core kind";
-    if (p->aux_dtype != TVDCN_F32) return "offset / mask / bias must be f32 for the tensor-core kernels";
-    const int csg = g.Cs / g.groups, cdg = g.Cd / g.groups;
-    if (csg % 64 != 0) return "sampled channels per group must be a multiple of 64";
-    if (cdg % 64 != 0) return "dense channels per group must be a multiple of 64";
+    const int csg = g.Cs / g.groups;
     if (g.K > 512) return "more than 512 kernel taps (the tensor-core kernels tabulate tap coordinates)";
-    if (g.B > 65535) return "batch above 65535 (the layout staging kernels put the batch in gridDim.z)";
-    if (g.og > 0 && (g.Cs / g.og) % 64 != 0) return "channels per offset group must be a multiple of 64";
-    if (g.mg > 0 && (g.Cs / g.mg) % 64 != 0) return "channels per mask group must be a multiple of 64";
+    if (g.gran_pad > MAX_CHANNEL_PADDING * g.gran) return "too few sampled channels share their groups";
     if (((long long)g.B * g.S + 1) * g.Cs >= (1LL << 31) || (long long)g.B * g.P >= (1LL << 31))
         return "sampled image has 2^31 elements or more (32-bit element offsets)";
-    if ((long long)g.Cd * csg * g.K >= (1LL << 31)) return "weight has 2^31 elements or more (32-bit packing indices)";
+    if ((long long)g.Cd * csg * g.K >= (1LL << 31)) return "weight has 2^31 elements or more";
     return nullptr;
 }
 
+// The shapes whose 16-bit columns and two-part f32 operands the tolerances of these data types were set for: no
+// padding, f32 offsets.  Everything else used to run on the SIMT kernels and keeps their precision (wide modes).
+bool unpadded(const tvdcn_problem *p, const GeoHost &g) {
+    return g.gran_pad == g.gran && g.Cd == g.Cd_r && p->aux_dtype == TVDCN_F32;
+}
+int mode_of(int dtype, bool wide) {
+    if (dtype == DT_F32) return wide ? TC_F32_WIDE : TC_SPLIT;
+    if (dtype == DT_F16) return wide ? TC_F16_WIDE : TC_F16;
+    return wide ? TC_BF16_WIDE : TC_BF16;
+}
+
 // f32 data on the tensor cores: one accumulator may take about 2400 MMAs before the round-toward-zero error of
-// the f32 accumulation (~2e-8 of the result per MMA) eats half of the 1e-4 budget.  The sample -> GEMM kernel adds
-// 12 MMAs per (tap, 64-channel chunk), spread over min(4, 512 / bn) accumulators.
+// the f32 accumulation (~2e-8 of the result per MMA) eats half of the 1e-4 budget.  Longer reductions stay on the
+// SIMT kernel.
 bool chain_ok(int mode, const GeoHost &g, int bn) {
-    if (mode != 2) return true;
+    if (!mode_f32(mode)) return true;
     const int nacc = std::min(4, 512 / std::max(bn, 1));
     const long long chain = (long long)g.K * (g.Cs / g.groups / 64) * 12 / nacc;
     return chain <= 2400;
 }
 
+void take_parts(size_t (&at)[3], Bump &b, int parts, size_t elems) {
+    for (int q = 0; q < parts; ++q) at[q] = b.take(elems * 2);
+}
+size_t packed_elems(const GeoHost &g) { return (size_t)g.Cd * (g.Cs / g.groups) * g.K; }
+
+// 16-bit offset / mask / bias reach the tensor-core kernels as f32
+void take_aux(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool bias) {
+    if (!is16(p->aux_dtype)) return;
+    if (g.og > 0) pl.off32 = b.take((size_t)g.B * g.og * g.K * g.dim * g.P * sizeof(float));
+    if (g.mg > 0) pl.mask32 = b.take((size_t)g.B * g.mg * g.K * g.P * sizeof(float));
+    if (bias) pl.bias32 = b.take((size_t)p->out_channels * sizeof(float));
+}
+
 // buffers of the GEMM -> scatter kernel
-void take_scatter_buffers(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool scatter) {
-    const size_t nw = (size_t)g.Cd * (g.Cs / g.groups) * g.K;
-    pl.w_pack_kd = b.take(nw * 2);
-    if (p->dtype == TVDCN_F32) pl.w_pack_kd_lo = b.take(nw * 2);
+void take_scatter_buffers(Plan &pl, Bump &b, const GeoHost &g, bool scatter) {
+    take_parts(pl.w_pack_kd, b, mode_mat_parts(pl.mode), packed_elems(g));
     if (scatter) pl.img_grad_cl = b.take((size_t)g.B * g.S * g.Cs * sizeof(float));
 }
 }  // namespace
 
-int tc_mode_of(int dtype) { return dtype == DT_F32 ? 2 : (dtype == DT_F16 ? 1 : 0); }
+GeoHost tc_geometry(const GeoHost &g) {
+    GeoHost t = g;
+    int gran = gcd(g.Cs, g.Cs / g.groups);
+    if (g.og > 0) gran = gcd(gran, g.Cs / g.og);
+    if (g.mg > 0) gran = gcd(gran, g.Cs / g.mg);
+    t.gran = gran;
+    t.gran_pad = round_up(gran, 64);
+    t.Cs_r = g.Cs;
+    t.Cd_r = g.Cd;
+    const long long cs = (long long)g.Cs / gran * t.gran_pad, cd = (long long)g.groups * round_up(g.Cd / g.groups, 64);
+    t.Cs = (int)std::min<long long>(cs, 0x7fffffff);
+    t.Cd = (int)std::min<long long>(cd, 0x7fffffff);
+    return t;
+}
 
 Plan plan_forward(const tvdcn_problem *p) {
     Plan pl;
-    const GeoHost g = make_geo_host(p);
+    const GeoHost g = tc_geometry(make_geo_host(p));
     Bump b;
     const char *why = tc_common(p, g);
-    const int mode = tc_mode_of(p->dtype);
+    pl.wide = !unpadded(p, g);
+    pl.mode = mode_of(p->dtype, pl.wide);
     const size_t es = p->dtype == TVDCN_F32 ? 4 : 2;
-    const size_t nw = (size_t)g.Cd * (g.Cs / g.groups) * g.K;
     int bn = 0, st = 0, gbufs = 0;
     if (why == nullptr && !p->transposed) {
-        if (fwd_tc_config(g.dim, mode, g.Cd / g.groups, &bn, &st) && chain_ok(mode, g, bn)) {
+        if (fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &bn, &st) && chain_ok(pl.mode, g, bn)) {
             pl.tensor = pl.tc_sg = true;
-            pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);   // + one row of zeros, see stage_image
-            pl.w_pack = b.take(nw * 2);
-            if (p->dtype == TVDCN_F32) pl.w_pack_lo = b.take(nw * 2);
+            pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);   // + one row of zeros
+            take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
+            take_aux(pl, b, p, g, true);
         } else {
             why = "no tile configuration fits (or the f32 accumulation chain would be too long)";
         }
     } else if (why == nullptr) {
-        if (dgrad_tc_config(g.dim, mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st)) {
+        if (dgrad_tc_config(g.dim, pl.mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st)) {
             pl.tensor = pl.tc_gs = true;
-            take_scatter_buffers(pl, b, p, g, true);
+            take_scatter_buffers(pl, b, g, true);
+            take_aux(pl, b, p, g, true);
         } else {
             why = "no tile configuration fits";
         }
     }
     if (why != nullptr) {
         pl.why_not = why;
-        if (p->transposed && is16(p->dtype)) pl.img_acc = b.take((size_t)g.B * g.Cs * g.S * sizeof(float));
+        if (p->transposed && is16(p->dtype)) pl.img_acc = b.take((size_t)g.B * g.Cs_r * g.S * sizeof(float));
     }
     pl.total = b.off;
     return pl;
@@ -92,51 +128,61 @@ Plan plan_forward(const tvdcn_problem *p) {
 
 Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bool want_offset, bool want_mask) {
     Plan pl;
-    const GeoHost g = make_geo_host(p);
+    const GeoHost g = tc_geometry(make_geo_host(p));
     Bump b;
     const char *why = tc_common(p, g);
-    const int mode = tc_mode_of(p->dtype);
+    pl.wide = !unpadded(p, g);
+    pl.mode = mode_of(p->dtype, pl.wide);
+    pl.mode_sw = mode_of(p->dtype, pl.wide || g.P % 8 != 0);
     const size_t es = p->dtype == TVDCN_F32 ? 4 : 2;
-    const size_t nw = (size_t)g.Cd * (g.Cs / g.groups) * g.K;
     want_offset = want_offset && g.og > 0;
     want_mask = want_mask && g.mg > 0;
     if (why == nullptr) {
         int bn = 0, st = 0, ns = 0, mt = 0, gbufs = 0;
         // which primitives run on the tensor cores
         // transposed backward: grad_input is a sample -> GEMM over grad_output
-        pl.tc_sg = p->transposed && want_input && fwd_tc_config(g.dim, mode, g.Cd / g.groups, &bn, &st) &&
-                   chain_ok(mode, g, bn);
-        pl.tc_sw = want_weight && wgrad_tc_config(g.dim, mode, g.Cd / g.groups, g.P, &ns, &mt, &st);
+        pl.tc_sg = p->transposed && want_input && fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &bn, &st) &&
+                   chain_ok(pl.mode, g, bn);
+        pl.tc_sw = want_weight && wgrad_tc_config(g.dim, pl.mode_sw, g.Cd_r / g.groups, &ns, &mt, &st);
         // conv: scatter into grad_input + coordinate gradients; transposed: coordinate gradients only
         const bool scatter = !p->transposed && want_input;
         pl.tc_gs = (scatter || want_offset || want_mask) &&
-                   dgrad_tc_config(g.dim, mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st);
+                   dgrad_tc_config(g.dim, pl.mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st);
         pl.tensor = pl.tc_sg || pl.tc_sw || pl.tc_gs;
         // The staged image comes first, as in the forward plan: a backward call that is told to reuse the
         // forward call's staging (TVDCN_FLAG_REUSE_STAGED_INPUT) finds it at the same offset of the same workspace.
-        if (pl.tensor) pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);
-        if (pl.tc_sg) {
-            pl.w_pack = b.take(nw * 2);
-            if (p->dtype == TVDCN_F32) pl.w_pack_lo = b.take(nw * 2);
+        if (pl.tensor) {
+            pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);
+            take_aux(pl, b, p, g, false);
         }
-        if (pl.tc_sw && p->dtype == TVDCN_F32) {
-            pl.dense_hi = b.take((size_t)g.B * g.Cd * g.P * 2);
-            pl.dense_lo = b.take((size_t)g.B * g.Cd * g.P * 2);
+        if (pl.tc_sg) take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
+        if (pl.tc_sw) {
+            // f32 data is split into 16-bit parts; 16-bit rows are copied only where TMA cannot read them
+            pl.dense_pitch = round_up(g.P, 8);
+            const int parts = p->dtype == TVDCN_F32 ? mode_mat_parts(pl.mode_sw) : (g.P % 8 != 0 ? 1 : 0);
+            take_parts(pl.dense, b, parts, (size_t)g.B * g.Cd_r * pl.dense_pitch);
         }
-        if (pl.tc_gs) take_scatter_buffers(pl, b, p, g, scatter);
+        if (pl.tc_gs) take_scatter_buffers(pl, b, g, scatter);
         if (!pl.tensor) pl.why_not = "no tensor-core kernel covers the requested gradients for this shape";
     } else {
         pl.why_not = why;
     }
     if (is16(p->dtype)) {
-        if (!p->transposed && want_input && !pl.tc_gs) pl.img_acc = b.take((size_t)g.B * g.Cs * g.S * sizeof(float));
+        if (!p->transposed && want_input && !pl.tc_gs) pl.img_acc = b.take((size_t)g.B * g.Cs_r * g.S * sizeof(float));
     }
     // 16-bit data accumulates the weight gradient in f32; the tensor-core kernel accumulates (any data type) into
     // a staged layout that a small kernel turns into the caller's afterwards
-    if (want_weight && (is16(p->dtype) || pl.tc_sw)) pl.gw_acc = b.take(nw * sizeof(float));
+    if (want_weight && (is16(p->dtype) || pl.tc_sw))
+        pl.gw_acc = b.take((size_t)g.Cd_r * ((pl.tc_sw ? g.Cs : g.Cs_r) / g.groups) * g.K * sizeof(float));
     if (is16(p->aux_dtype)) {
         if (want_offset) pl.goff_acc = b.take((size_t)g.B * g.og * g.K * g.dim * g.P * sizeof(float));
         if (want_mask) pl.gmask_acc = b.take((size_t)g.B * g.mg * g.K * g.P * sizeof(float));
+    }
+    // bias gradient: the sum of grad_output (the dense tensor of the conv, the sampled image of the transposed conv)
+    if (pl.tensor) {
+        const int c = p->transposed ? g.Cs_r : g.Cd_r, n = p->transposed ? g.S : g.P;
+        pl.sum_partial = b.take((size_t)dense_sum_scratch_floats(g.B, c, n) * sizeof(float));
+        pl.sum_done = b.take((size_t)c * sizeof(unsigned));
     }
     pl.total = b.off;
     return pl;

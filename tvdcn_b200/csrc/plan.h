@@ -16,22 +16,24 @@ struct Plan {
     bool tc_sg = false;            // sample -> GEMM on tensor cores
     bool tc_gs = false;            // GEMM -> scatter / coordinate gradients on tensor cores
     bool tc_sw = false;            // sampled weight gradient on tensor cores
+    bool wide = false;             // a shape or type that needs padding or widening (see the modes)
+    int mode = 0, mode_sw = 0;     // TC_* mode of tc_sg and tc_gs, and of tc_sw
     const char *why_not = "";      // reason the tensor-core kernels were not chosen
     size_t total = 0;              // workspace bytes
-    // SIMT path: accumulation buffers for 16-bit outputs (byte offsets into the workspace)
-    size_t img_acc = NO_BUF;       // sampled-image-shaped accumulator (grad_input / transposed output)
+    // accumulation buffers for 16-bit outputs (byte offsets into the workspace)
+    size_t img_acc = NO_BUF;       // SIMT path: sampled-image-shaped accumulator (grad_input / transposed output)
     size_t gw_acc = NO_BUF;        // f32 weight gradient: [Cd, csg, K] for the SIMT kernel, [g][tap][d'][s'] for the tensor-core one
     size_t goff_acc = NO_BUF;
     size_t gmask_acc = NO_BUF;
-    // tensor path: staged copies
-    size_t img_cl = NO_BUF;        // sampled image, channels-last (16-bit, or f32 in split mode)
-    size_t w_pack = NO_BUF;        // weights packed [g][tap][d'][s'], 16-bit (hi part in split mode)
-    size_t w_pack_lo = NO_BUF;     // low part of the split
-    size_t w_pack_kd = NO_BUF;     // weights packed [g][tap][s'][d']
-    size_t w_pack_kd_lo = NO_BUF;
-    size_t dense_hi = NO_BUF;      // dense tensor, original layout, 16-bit hi / lo (split mode)
-    size_t dense_lo = NO_BUF;
+    // tensor path: staged copies; weights and dense tensor in as many 16-bit parts as the mode has
+    size_t img_cl = NO_BUF;        // sampled image, channels-last, data type of the problem
+    size_t w_pack[3] = {NO_BUF, NO_BUF, NO_BUF};      // weights packed [g][tap][d'][s']
+    size_t w_pack_kd[3] = {NO_BUF, NO_BUF, NO_BUF};   // weights packed [g][tap][s'][d']
+    size_t dense[3] = {NO_BUF, NO_BUF, NO_BUF};       // dense tensor, rows dense_pitch apart (absent: the caller's own)
+    int dense_pitch = 0;
     size_t img_grad_cl = NO_BUF;   // f32 channels-last accumulator of the scatter
+    size_t off32 = NO_BUF, mask32 = NO_BUF, bias32 = NO_BUF;   // 16-bit offset / mask / bias widened to f32
+    size_t sum_partial = NO_BUF, sum_done = NO_BUF;   // partial sums of the bias gradient and their arrival counters
 };
 
 inline size_t align_up(size_t v, size_t a = 256) { return (v + a - 1) / a * a; }
@@ -43,39 +45,65 @@ GeoHost make_geo_host(const tvdcn_problem *p);
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t e, const char *what);
 
-// 0: bf16, 1: f16, 2: f32 split into bf16 hi + lo (the TC_* modes of the tensor-core kernels)
-int tc_mode_of(int dtype);
+// The geometry the tensor-core kernels work on: channels padded as GeoHost describes.
+GeoHost tc_geometry(const GeoHost &g);
 
-// ---- tensor-core kernels (sm100_*.cu) -----------------------------------------------------------------
-bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages);
-cudaError_t launch_sample_gemm_tc(const GeoHost &g, int mode, const void *img_cl, const void *w_hi, const void *w_lo,
-                                  const float *offset, const float *mask, const float *bias, void *out, int *status,
-                                  cudaStream_t stream);
-bool wgrad_tc_config(int dim, int mode, int cdg, int P, int *n_sub, int *m_tiles, int *stages);
-cudaError_t launch_sample_wgrad_tc(const GeoHost &g, int mode, const void *dense_hi, const void *dense_lo,
-                                   const void *img_cl, const float *offset, const float *mask, float *gw,
-                                   int *status, cudaStream_t stream);
-bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int *b_stages);
-cudaError_t launch_gemm_scatter_tc(const GeoHost &g, int mode, const void *dense, const void *w_kd_hi,
-                                   const void *w_kd_lo, const void *img_cl, const float *offset, const float *mask,
-                                   float *img_grad_cl, float *goff, float *gmask, int *status, cudaStream_t stream);
-cudaError_t launch_from_channels_last_bias(const float *src, const float *bias, void *dst, int dst_dtype, int B, int C,
-                                           int S, cudaStream_t stream);
-cudaError_t launch_pack_weight_kd(const void *w, int dtype, int mode, int groups, int cdg, int csg, int K, void *hi,
-                                  void *lo, cudaStream_t stream);
+// ---- staging (sm100_staging.cu) ------------------------------------------------------------------------
+enum : int { STAGE_IMAGE, STAGE_PACK, STAGE_ZERO, STAGE_WIDEN, STAGE_PITCH };
+struct StageJob {
+    const void *src;
+    void *dst, *part[3];
+    int64_t n;
+    int kind, end_block;           // the job's blocks end before this one
+    int dtype, elem_bytes, wide, kd;
+    int C, c_pad, gran, gran_pad, S, K, cdg, cdg_pad;
+};
+struct StageList {
+    static constexpr int MAX = 14;
+    int n;
+    Status status;
+    StageJob job[MAX];
+};
+// Collects the preparations of one call and runs them as one launch.
+class Stager {
+   public:
+    void image(const void *src, void *dst, const GeoHost &h, int elem_bytes);   // + the row of zeros behind it
+    void pack(const void *weight, void *const *parts, const GeoHost &h, int dtype, int n_parts, bool kd);
+    void zero(void *dst, int64_t bytes);                                        // bytes: a multiple of 4
+    void widen(const void *src, void *dst, int dtype, int64_t n);               // 16-bit -> f32
+    void pitch(const void *src, void *dst, int64_t rows, int P, int pitch);     // 16-bit rows, `pitch` apart
+    cudaError_t launch(const Status &status, cudaStream_t stream);
+    bool empty() const { return list_.n == 0; }
+
+   private:
+    StageJob *add(int kind, int64_t blocks);
+    StageList list_{};
+    int64_t blocks_ = 0;
+    cudaError_t error_ = cudaSuccess;
+};
+cudaError_t launch_from_channels_last_bias(const float *src, const float *bias, void *dst, int dst_dtype, const GeoHost &h,
+                                           cudaStream_t stream);
 // staged weight gradient of the tensor-core kernel, [g][tap][d'][s'] f32 -> [Cd, csg, K] in the data type `dtype`
-cudaError_t launch_unpack_weight_grad(const float *staged, void *gw, int dtype, int groups, int cdg, int csg, int K,
-                                      cudaStream_t stream);
-cudaError_t launch_split_f32(const float *src, void *hi, void *lo, int64_t n, cudaStream_t stream);
-// the same split of a [B, C, S] tensor plus sum_out[c] = sum over batch and space, in one pass; only where
-// can_split_f32_with_channel_sum says so (S a multiple of 4, pointers aligned for 16- / 8-byte accesses)
-bool can_split_f32_with_channel_sum(const float *src, const void *hi, const void *lo, int S);
-cudaError_t launch_split_f32_channel_sum(const float *src, void *hi, void *lo, int B, int C, int S, float *sum_out,
-                                         cudaStream_t stream);
-cudaError_t launch_to_channels_last(const void *src, void *dst, int B, int C, int S, int elem_bytes,
-                                    cudaStream_t stream);
-cudaError_t launch_pack_weight_ks(const void *w, int dtype, int mode, int groups, int cdg, int csg, int K, void *hi,
-                                  void *lo, cudaStream_t stream);
+cudaError_t launch_unpack_weight_grad(const float *staged, void *gw, int dtype, const GeoHost &h, cudaStream_t stream);
+// One read of a [B, C, P] tensor (f32, f16 or bf16): its bf16 parts (f32 data; n_parts 0: none) and / or the sum over
+// batch and space per channel (sum_out, may be null).  partial: dense_sum_scratch_floats values; done: C zeroed counters.
+int64_t dense_sum_scratch_floats(int B, int C, int P);
+cudaError_t launch_dense_pass(const void *src, int dtype, int n_parts, void *const *parts, int B, int C, int P, int pitch,
+                              float *partial, unsigned *done, void *sum_out, int sum_dtype, cudaStream_t stream);
+
+// ---- tensor-core kernels (sm100_*.cu); all take the padded geometry ---------------------------------------
+bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages);
+cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
+                                  const float *offset, const float *mask, const float *bias, void *out,
+                                  const Status &status, cudaStream_t stream);
+bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages);
+cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch, const void *img_cl,
+                                   const float *offset, const float *mask, float *gw, const Status &status,
+                                   cudaStream_t stream);
+bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int *b_stages);
+cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense, void *const *w_parts,
+                                   const void *img_cl, const float *offset, const float *mask, float *img_grad_cl,
+                                   float *goff, float *gmask, const Status &status, cudaStream_t stream);
 
 int tuning_int(const char *name, int fallback);
 

@@ -24,6 +24,8 @@ inline Geo<DIM> geo_from_host(const GeoHost &h) {
     g.cdg = h.Cd / h.groups;
     g.cs_per_og = h.og > 0 ? h.Cs / h.og : h.Cs;
     g.cs_per_mg = h.mg > 0 ? h.Cs / h.mg : h.Cs;
+    g.Cd_r = h.Cd_r;
+    g.cdg_r = h.Cd_r / h.groups;
     g.BP = (long long)h.B * h.P;
     for (int a = 0; a < DIM; ++a) {
         g.img[a] = h.img[a]; g.grid[a] = h.grid[a]; g.ker[a] = h.ker[a];
@@ -32,13 +34,16 @@ inline Geo<DIM> geo_from_host(const GeoHost &h) {
     return g;
 }
 
-// How the 16-bit tensor-core operands are derived from the user's data type.
-enum : int {
-    TC_BF16 = 0,   // bf16 data, one MMA pass
-    TC_F16 = 1,    // f16 data, one MMA pass
-    TC_SPLIT = 2   // f32 data, each operand split into bf16 hi + lo, three MMA passes (hi*hi + lo*hi + hi*lo)
+template <int MODE>
+struct Mode {
+    static constexpr bool F32 = MODE == TC_SPLIT || MODE == TC_F32_WIDE;       // type of image, weight and dense tensor
+    static constexpr bool HALF = MODE == TC_F16 || MODE == TC_F16_WIDE;
+    static constexpr bool BLEND_F32 = MODE >= TC_SPLIT;                        // corners are blended in f32
+    static constexpr int COL_PARTS = MODE == TC_F32_WIDE ? 3 : (MODE >= TC_SPLIT ? 2 : 1);
+    static constexpr int MAT_PARTS = MODE == TC_F32_WIDE ? 3 : (MODE == TC_SPLIT ? 2 : 1);
+    static constexpr bool LOW_ACC = F32;                                       // the small products have accumulators
+    using T16 = typename std::conditional<HALF, __half, __nv_bfloat16>::type;  // type of the operands
 };
-
 constexpr int TILE_POS = 128;       // grid positions per tile = TMEM lanes
 constexpr int CHUNK_C = 64;         // channels per K chunk = one 128-byte swizzle row of 16-bit values
 constexpr int A_TILE_BYTES = TILE_POS * 128;
@@ -78,14 +83,34 @@ __device__ __forceinline__ PosInfo<DIM> decode_position(const Geo<DIM> &g, long 
 }
 
 // ---- sampling plan ------------------------------------------------------------------------------------
-// One entry per (position, corner of the 2^DIM cell): where the corner's 64-channel row starts in the
-// channels-last image, in 16-byte units, and the corner's interpolation weight times the mask -- as a packed
-// 16-bit pair (w, w) for 16-bit data, as f32 bits for f32 data.  Unused / out-of-bounds corners point at row 0
-// with weight 0, so the producers can load unconditionally.
-struct PlanEntry {
-    uint32_t row16;
-    uint32_t w;
-};
+// One slot per (position, tap): for each of the NC = 2^DIM corners of the cell where the corner's 64-channel row
+// starts in the channels-last image, in 16-byte units, then for each corner its interpolation weight times the mask
+// -- as a packed 16-bit pair (w, w) where the corners are blended in 16 bits, else as f32 bits.  Rows and weights are
+// apart so that a producer reads the weights only when it blends: they would hold NC registers per position in flight.
+// Out-of-image corners point at the row of zeros behind the image with weight 0, so the producers load
+// unconditionally.
+template <int NC>
+__device__ __forceinline__ void load_slot_half(uint32_t (&out)[NC], const uint32_t *p) {
+    if constexpr (NC == 2) {
+        const uint2 x = *reinterpret_cast<const uint2 *>(p);
+        out[0] = x.x; out[1] = x.y;
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; c += 4) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(p + c);
+            out[c] = x.x; out[c + 1] = x.y; out[c + 2] = x.z; out[c + 3] = x.w;
+        }
+    }
+}
+template <int NC>
+__device__ __forceinline__ void store_slot_half(uint32_t *p, const uint32_t (&v)[NC]) {
+    if constexpr (NC == 2) {
+        *reinterpret_cast<uint2 *>(p) = make_uint2(v[0], v[1]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; c += 4) *reinterpret_cast<uint4 *>(p + c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+    }
+}
 
 // Offsets and mask of one (position, tap, groups): loaded early, turned into plan entries later, so that the
 // global-memory latency overlaps the sampling of the previous chunk.
@@ -113,7 +138,7 @@ __device__ __forceinline__ RawCoords<DIM> load_coords(const Geo<DIM> &g, const P
 
 template <int MODE>
 __device__ __forceinline__ uint32_t encode_weight(float w) {
-    if constexpr (MODE == TC_SPLIT) {
+    if constexpr (Mode<MODE>::BLEND_F32) {
         return __float_as_uint(w);
     } else if constexpr (MODE == TC_F16) {
         const __half2 h = __float2half2_rn(w);
@@ -138,12 +163,12 @@ __device__ __forceinline__ void tap_coords(const Geo<DIM> &g, int tap, int (&tc)
 template <int DIM, int MODE>
 __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
                                               bool deformable, const int (&tc)[DIM], uint32_t row_scale,
-                                              PlanEntry *slot);
+                                              uint32_t *slot);
 
-// Writes the NC plan entries of one position.  row_scale = Cs * element size / 16.
+// Writes the plan slot of one position.  row_scale = Cs * element size / 16.
 template <int DIM, int MODE>
 __device__ __forceinline__ void build_plan(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
-                                           bool deformable, int tap, uint32_t row_scale, PlanEntry *slot) {
+                                           bool deformable, int tap, uint32_t row_scale, uint32_t *slot) {
     int tc[DIM];
     tap_coords<DIM>(g, tap, tc);
     build_plan_at<DIM, MODE>(g, pi, rc, deformable, tc, row_scale, slot);
@@ -154,7 +179,7 @@ __device__ __forceinline__ void build_plan(const Geo<DIM> &g, const PosInfo<DIM>
 template <int DIM, int MODE>
 __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
                                               bool deformable, const int (&tc)[DIM], uint32_t row_scale,
-                                              PlanEntry *slot) {
+                                              uint32_t *slot) {
     constexpr int NC = 1 << DIM;
     int fl[DIM];
     float fr[DIM];
@@ -171,6 +196,7 @@ __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<D
             fr[a] = 0.f;
         }
     }
+    uint32_t rows[NC], ws[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         bool ok = pi.valid && (deformable || c == 0);
@@ -184,12 +210,12 @@ __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<D
             flat = flat * g.img[a] + i;
             w *= bit ? fr[a] : (1.f - fr[a]);
         }
-        PlanEntry e;
         // out-of-image corners read the row of zeros that follows the staged image
-        e.row16 = (uint32_t)(ok ? pi.b * g.S + flat : g.B * g.S) * row_scale;
-        e.w = encode_weight<MODE>(ok ? w : 0.f);
-        slot[c] = e;
+        rows[c] = (uint32_t)(ok ? pi.b * g.S + flat : g.B * g.S) * row_scale;
+        ws[c] = encode_weight<MODE>(ok ? w : 0.f);
     }
+    store_slot_half<NC>(slot, rows);
+    store_slot_half<NC>(slot + NC, ws);
 }
 
 __device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8], __nv_bfloat16) {
@@ -245,83 +271,109 @@ __device__ __forceinline__ uint32_t mul2(uint32_t w, uint32_t v) {
     }
 }
 
+// A value as PARTS 16-bit parts of decreasing magnitude: part k is what rounding leaves of the first k.
+template <int PARTS, typename T16>
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t (&out)[PARTS]) {
+#pragma unroll
+    for (int k = 0; k < PARTS; ++k) {
+        out[k] = pack2(a, b, T16());
+        if (k + 1 < PARTS) {
+            if constexpr (std::is_same<T16, __half>::value) {
+                const float2 r = __half22float2(*reinterpret_cast<const __half2 *>(&out[k]));
+                a -= r.x;
+                b -= r.y;
+            } else {
+                a -= __uint_as_float(out[k] << 16);
+                b -= __uint_as_float(out[k] & 0xffff0000u);
+            }
+        }
+    }
+}
+
 // Samples `nvpos` virtual positions x 64 channels into 128-byte-swizzled tiles (row = position).  Virtual
 // position v belongs to sub-tile v / pos_per_sub (tiles `sub_bytes` apart, each with its own first channel
-// chan16[sub], in 16-byte units) and is row v % pos_per_sub of it.  plan[v * NC + c] is the entry of corner c.
+// chan16[sub], in 16-byte units) and is row v % pos_per_sub of it.  plan + v * 2 * NC is its slot;
+// the parts of a column (see the modes) are tiles `part_bytes` apart.
 // All NT threads take part; each keeps the loads of IB positions in flight together so that global-memory
 // latency is overlapped.  nvpos must be a multiple of (NT / lanes-per-position) * IB.
-//   MODE TC_BF16 / TC_F16: img16 is the 16-bit image, one tile `hi`; 8 lanes x 8 channels per position.
-//   MODE TC_SPLIT: img16 is the f32 image, the blend is split into bf16 hi + lo; 16 lanes x 4 channels.
-template <int NC, int MODE, int NT, int IB = (NC >= 8 ? 2 : 4)>
-__device__ __forceinline__ void produce_tiles(uint8_t *hi, uint8_t *lo, uint32_t sub_bytes, int pos_per_sub, int nvpos,
-                                              const uint4 *__restrict__ img16, const uint32_t *chan16,
-                                              const PlanEntry *plan, int tid) {
-    constexpr int LPP = MODE == TC_SPLIT ? 16 : 8;
+//   16-bit data: 8 lanes x 8 channels per position; f32 data: 16 lanes x 4 channels.
+template <int NC, int MODE, int NT, int IB>
+__device__ __forceinline__ void produce_tiles(uint8_t *tiles, uint32_t part_bytes, uint32_t sub_bytes, int pos_per_sub,
+                                              int nvpos, const uint4 *__restrict__ img16, const uint32_t *chan16,
+                                              const uint32_t *plan, int tid) {
+    using M = Mode<MODE>;
+    using T16 = typename M::T16;
+    constexpr int LPP = M::F32 ? 16 : 8;
     constexpr int PPI = NT / LPP;
     const int part = tid & (LPP - 1);
     const int psub = tid / LPP;
     for (int v0 = 0; v0 < nvpos; v0 += PPI * IB) {
         uint4 v[IB][NC];
-        uint32_t w[IB][NC];
 #pragma unroll
         for (int i = 0; i < IB; ++i) {
             const int vp = v0 + i * PPI + psub;
             const uint4 *src = img16 + chan16[(v0 + i * PPI) / pos_per_sub] + part;
-            const PlanEntry *pe = plan + vp * NC;
+            uint32_t rows[NC];
+            load_slot_half<NC>(rows, plan + vp * 2 * NC);
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const PlanEntry e = pe[c];
-                w[i][c] = e.w;
-                v[i][c] = __ldg(src + e.row16);
-            }
+            for (int c = 0; c < NC; ++c) v[i][c] = __ldg(src + rows[c]);
         }
 #pragma unroll
         for (int i = 0; i < IB; ++i) {
             const int vp = v0 + i * PPI + psub;
             const int sub = (v0 + i * PPI) / pos_per_sub;
             const int pos = vp - sub * pos_per_sub;
-            uint8_t *dst_hi = hi + (size_t)sub * sub_bytes;
-            if constexpr (MODE != TC_SPLIT) {
-                using T16 = typename std::conditional<MODE == TC_F16, __half, __nv_bfloat16>::type;
+            uint8_t *dst = tiles + (size_t)sub * sub_bytes;
+            uint32_t w[NC];
+            load_slot_half<NC>(w, plan + vp * 2 * NC + NC);
+            if constexpr (!M::BLEND_F32) {
                 uint4 o;
-                o.x = mul2<T16>(w[i][0], v[i][0].x);
-                o.y = mul2<T16>(w[i][0], v[i][0].y);
-                o.z = mul2<T16>(w[i][0], v[i][0].z);
-                o.w = mul2<T16>(w[i][0], v[i][0].w);
+                o.x = mul2<T16>(w[0], v[i][0].x);
+                o.y = mul2<T16>(w[0], v[i][0].y);
+                o.z = mul2<T16>(w[0], v[i][0].z);
+                o.w = mul2<T16>(w[0], v[i][0].w);
 #pragma unroll
                 for (int c = 1; c < NC; ++c) {
-                    o.x = fma2<T16>(w[i][c], v[i][c].x, o.x);
-                    o.y = fma2<T16>(w[i][c], v[i][c].y, o.y);
-                    o.z = fma2<T16>(w[i][c], v[i][c].z, o.z);
-                    o.w = fma2<T16>(w[i][c], v[i][c].w, o.w);
+                    o.x = fma2<T16>(w[c], v[i][c].x, o.x);
+                    o.y = fma2<T16>(w[c], v[i][c].y, o.y);
+                    o.z = fma2<T16>(w[c], v[i][c].z, o.z);
+                    o.w = fma2<T16>(w[c], v[i][c].w, o.w);
                 }
-                *reinterpret_cast<uint4 *>(dst_hi + sw128_offset(pos, part)) = o;
+                *reinterpret_cast<uint4 *>(dst + sw128_offset(pos, part)) = o;
+            } else if constexpr (!M::F32) {
+                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float wf = __uint_as_float(w[c]);
+                    float f[8];
+                    unpack8(v[i][c], f, T16());
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[k] = fmaf(wf, f[k], acc[k]);
+                }
+                uint32_t p[4][M::COL_PARTS];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) split_pair<M::COL_PARTS, T16>(acc[2 * k], acc[2 * k + 1], p[k]);
+#pragma unroll
+                for (int q = 0; q < M::COL_PARTS; ++q)
+                    *reinterpret_cast<uint4 *>(dst + q * part_bytes + sw128_offset(pos, part)) =
+                        make_uint4(p[0][q], p[1][q], p[2][q], p[3][q]);
             } else {
-                uint8_t *dst_lo = lo + (size_t)sub * sub_bytes;
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    const float wf = __uint_as_float(w[i][c]);
+                    const float wf = __uint_as_float(w[c]);
                     acc[0] = fmaf(wf, __uint_as_float(v[i][c].x), acc[0]);
                     acc[1] = fmaf(wf, __uint_as_float(v[i][c].y), acc[1]);
                     acc[2] = fmaf(wf, __uint_as_float(v[i][c].z), acc[2]);
                     acc[3] = fmaf(wf, __uint_as_float(v[i][c].w), acc[3]);
                 }
-                // hi = bf16(acc) by truncation-free rounding, lo = bf16(acc - hi)
-                const uint32_t h01 = pack2(acc[0], acc[1], __nv_bfloat16());
-                const uint32_t h23 = pack2(acc[2], acc[3], __nv_bfloat16());
-                const float l0 = acc[0] - __uint_as_float(h01 << 16);
-                const float l1 = acc[1] - __uint_as_float(h01 & 0xffff0000u);
-                const float l2 = acc[2] - __uint_as_float(h23 << 16);
-                const float l3 = acc[3] - __uint_as_float(h23 & 0xffff0000u);
-                uint2 oh, ol;
-                oh.x = h01;
-                oh.y = h23;
-                ol.x = pack2(l0, l1, __nv_bfloat16());
-                ol.y = pack2(l2, l3, __nv_bfloat16());
+                uint32_t p01[M::COL_PARTS], p23[M::COL_PARTS];
+                split_pair<M::COL_PARTS, T16>(acc[0], acc[1], p01);
+                split_pair<M::COL_PARTS, T16>(acc[2], acc[3], p23);
                 const uint32_t off = sw128_offset(pos, part >> 1) + (uint32_t)(part & 1) * 8u;
-                *reinterpret_cast<uint2 *>(dst_hi + off) = oh;
-                *reinterpret_cast<uint2 *>(dst_lo + off) = ol;
+#pragma unroll
+                for (int q = 0; q < M::COL_PARTS; ++q)
+                    *reinterpret_cast<uint2 *>(dst + q * part_bytes + off) = make_uint2(p01[q], p23[q]);
             }
         }
     }
@@ -332,5 +384,26 @@ __device__ __forceinline__ void produce_tiles(uint8_t *hi, uint8_t *lo, uint32_t
 // entry point is unavailable or rejects the description.
 bool make_tensor_map_16bit(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
                            const uint64_t *strides_bytes /* rank-1 entries */, const uint32_t *box);
+// The maps of an operand's parts, all of one shape; unused entries repeat the first.
+inline bool make_part_maps(CUtensorMap *maps /* 3 */, const void *const *parts, int n, int rank, const uint64_t *dims,
+                           const uint64_t *strides_bytes, const uint32_t *box) {
+    for (int k = 0; k < n; ++k)
+        if (!make_tensor_map_16bit(&maps[k], parts[k], rank, dims, strides_bytes, box)) return false;
+    for (int k = n; k < 3; ++k) maps[k] = maps[0];
+    return true;
+}
+
+template <typename F>
+inline cudaError_t with_mode(int mode, F &&f) {
+    switch (mode) {
+        case TC_BF16: return f(std::integral_constant<int, TC_BF16>());
+        case TC_F16: return f(std::integral_constant<int, TC_F16>());
+        case TC_SPLIT: return f(std::integral_constant<int, TC_SPLIT>());
+        case TC_BF16_WIDE: return f(std::integral_constant<int, TC_BF16_WIDE>());
+        case TC_F16_WIDE: return f(std::integral_constant<int, TC_F16_WIDE>());
+        case TC_F32_WIDE: return f(std::integral_constant<int, TC_F32_WIDE>());
+    }
+    return cudaErrorInvalidValue;
+}
 
 }  // namespace tvdcn_b200

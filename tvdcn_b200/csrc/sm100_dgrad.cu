@@ -48,7 +48,7 @@ struct DgradParams {
     float *img_grad_cl;     // [B*S, Cs] f32, accumulated into; may be null
     float *goff;            // f32, accumulated into; may be null
     float *gmask;           // f32, accumulated into; may be null
-    int *status;
+    Status status;
     int rc;                 // reduction chunks: cdg / 64
     int tb;                 // taps per batch
     int nbatch;             // ceil(K / tb)
@@ -141,12 +141,10 @@ struct ScLayout {
 };
 __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_stages) {
     ScLayout L;
-    const int parts = mode == TC_SPLIT ? 2 : 1;
-    L.n = tb * SC_SLAB;
+        L.n = tb * SC_SLAB;
     L.col_stride = L.n + 4;                       // words; = 4 mod 32, so that the row-per-lane stores spread over the banks
     L.max_entries = TILE_POS * tb * (1 << dim);
     L.b_stage = (uint32_t)(L.n * 128);             // one 16-bit part (hi or lo) of one reduction chunk
-    (void)parts;
     L.col_buf = (uint32_t)(TILE_POS * L.col_stride * 4);
     // three arrays (pixel offset; col index | dot slot << 16; weight) of max_entries + SC_PLAN_SLACK words -- room for
     // the padding of the groups' spans and the read-ahead of the last group -- then one dot product per entry (+ a
@@ -168,12 +166,13 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
 template <int DIM, int MODE, bool COORD>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMap tmap_b_hi,
-                    const __grid_constant__ CUtensorMap tmap_b_lo) {
+                    const __grid_constant__ CUtensorMap tmap_b_lo, const __grid_constant__ CUtensorMap tmap_b_lo2) {
     constexpr int NC = 1 << DIM;
-    constexpr bool SPLIT = MODE == TC_SPLIT;
-    constexpr int PARTS = SPLIT ? 2 : 1;
+    using M = Mode<MODE>;
+    constexpr int PARTS = M::MAT_PARTS;                 // 16-bit parts of the dense tile and of the weights
+    constexpr int ACCS = MODE == TC_F32_WIDE ? 2 : 1;   // accumulators of a pass: leading / small products
     constexpr int TBM = sc_tb_max(DIM);
-    using T16 = typename std::conditional<MODE == TC_F16, __half, __nv_bfloat16>::type;
+    using T16 = typename M::T16;
     const Geo<DIM> &g = P.g;
 
     extern __shared__ uint8_t smem_raw[];
@@ -256,7 +255,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     }
     if (warp == SC_TMA_WARP && lane == 0) {
         ptx::prefetch_tmap(&tmap_b_hi);
-        if (SPLIT) ptx::prefetch_tmap(&tmap_b_lo);
+        if (PARTS > 1) ptx::prefetch_tmap(&tmap_b_lo);
+        if (PARTS > 2) ptx::prefetch_tmap(&tmap_b_lo2);
     }
     if (warp == SC_MMA_WARP) {
         ptx::tmem_alloc(tmem_slot, SC_TMEM_COLS);
@@ -369,43 +369,62 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         const int q = warp & 3, part = warp >> 2;
         const PosInfo<DIM> pa = decode_position<DIM>(g, m0 + q * 32 + lane);
         const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
-        const int64_t base = ((int64_t)pa.b * g.Cd + (int64_t)grp * g.cdg) * g.P + pa.p;
+        const int64_t base = ((int64_t)pa.b * g.Cd_r + (int64_t)grp * g.cdg_r) * g.P + pa.p;
         // two units (32 loads) in flight per thread: the tile is read once from DRAM, its latency is what counts
         const int n_units_a = g.cdg / 16;
         for (int u0 = part; u0 < n_units_a; u0 += 2 * (SC_LOAD_WARPS / 4)) {
             const int u1 = u0 + SC_LOAD_WARPS / 4;
             const bool two = u1 < n_units_a;
-            if constexpr (SPLIT) {
+            // channels past the group's end (a group is padded to a multiple of 64) are zeros
+            const bool in0 = pa.valid && u0 * 16 + 16 <= g.cdg_r, in1 = pa.valid && two && u1 * 16 + 16 <= g.cdg_r;
+            const int part0 = pa.valid ? g.cdg_r - u0 * 16 : 0, part1 = pa.valid && two ? g.cdg_r - u1 * 16 : 0;
+            const bool ragged = (g.cdg_r & 15) != 0;   // a unit of 16 channels is partly inside
+            if constexpr (M::F32) {
                 const float *src0 = reinterpret_cast<const float *>(P.dense) + base + (int64_t)(u0 * 16) * g.P;
                 const float *src1 = reinterpret_cast<const float *>(P.dense) + base + (int64_t)(u1 * 16) * g.P;
                 float v[2][16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[0][i] = pa.valid ? __ldg(src0 + (int64_t)i * g.P) : 0.f;
+                for (int i = 0; i < 16; ++i) v[0][i] = in0 ? __ldg(src0 + (int64_t)i * g.P) : 0.f;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[1][i] = (pa.valid && two) ? __ldg(src1 + (int64_t)i * g.P) : 0.f;
+                for (int i = 0; i < 16; ++i) v[1][i] = in1 ? __ldg(src1 + (int64_t)i * g.P) : 0.f;
+                if (ragged) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        if (!in0 && i < part0) v[0][i] = __ldg(src0 + (int64_t)i * g.P);
+                        if (!in1 && i < part1) v[1][i] = __ldg(src1 + (int64_t)i * g.P);
+                    }
+                }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (h == 1 && !two) break;
                     const int d0 = (h == 0 ? u0 : u1) * 16;
-                    uint32_t hi[8], lo[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        hi[i] = pack2(v[h][2 * i], v[h][2 * i + 1], __nv_bfloat16());
-                        const float l0 = v[h][2 * i] - __uint_as_float(hi[i] << 16);
-                        const float l1 = v[h][2 * i + 1] - __uint_as_float(hi[i] & 0xffff0000u);
-                        lo[i] = pack2(l0, l1, __nv_bfloat16());
+                    for (int q = 0; q < PARTS; ++q) {   // v keeps what the parts so far leave
+                        uint32_t part16[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            part16[i] = pack2(v[h][2 * i], v[h][2 * i + 1], __nv_bfloat16());
+                            v[h][2 * i] -= __uint_as_float(part16[i] << 16);
+                            v[h][2 * i + 1] -= __uint_as_float(part16[i] & 0xffff0000u);
+                        }
+                        ptx::tmem_st_32x8(t_lane + (uint32_t)(q * a_cols + d0 / 2), part16);
                     }
-                    ptx::tmem_st_32x8(t_lane + (uint32_t)(d0 / 2), hi);
-                    ptx::tmem_st_32x8(t_lane + (uint32_t)(a_cols + d0 / 2), lo);
                 }
             } else {
                 const uint16_t *src0 = reinterpret_cast<const uint16_t *>(P.dense) + base + (int64_t)(u0 * 16) * g.P;
                 const uint16_t *src1 = reinterpret_cast<const uint16_t *>(P.dense) + base + (int64_t)(u1 * 16) * g.P;
                 uint32_t v[2][16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[0][i] = pa.valid ? (uint32_t)__ldg(src0 + (int64_t)i * g.P) : 0u;
+                for (int i = 0; i < 16; ++i) v[0][i] = in0 ? (uint32_t)__ldg(src0 + (int64_t)i * g.P) : 0u;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[1][i] = (pa.valid && two) ? (uint32_t)__ldg(src1 + (int64_t)i * g.P) : 0u;
+                for (int i = 0; i < 16; ++i) v[1][i] = in1 ? (uint32_t)__ldg(src1 + (int64_t)i * g.P) : 0u;
+                if (ragged) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        if (!in0 && i < part0) v[0][i] = (uint32_t)__ldg(src0 + (int64_t)i * g.P);
+                        if (!in1 && i < part1) v[1][i] = (uint32_t)__ldg(src1 + (int64_t)i * g.P);
+                    }
+                }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (h == 1 && !two) break;
@@ -441,7 +460,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 bool good = ptx::mbar_wait(&plan_done[pb], (uint32_t)((j >> 1) & 1));
                 good = __all_sync(0xffffffffu, good);
                 if (!good) {
-                    if (lane == 0) atomicExch(P.status, 308);
+                    if (lane == 0) ptx::report(P.status, 308);
                     return false;
                 }
                 finalize(pi, row, unit0 + j, pb, ru);
@@ -462,16 +481,28 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 w_cempty += SC_CLK() - c1;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
-                    if (lane == 0) atomicExch(P.status, 301);
+                    if (lane == 0) ptx::report(P.status, 301);
                     break;
                 }
                 ptx::tc_fence_after();
                 float *dst = col + (size_t)cb * (L.col_buf / 4) + row * L.col_stride;
-                const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col0 + (uint32_t)(aq * N);
+                const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col0 + (uint32_t)(aq * ACCS * N);
                 for (int j32 = 0; j32 < N / 32; ++j32) {
                     uint32_t raw[32];
                     ptx::tmem_ld_32x32(src + (uint32_t)(j32 * 32), raw);
                     ptx::tmem_ld_wait();
+                    if constexpr (ACCS == 2) {
+                        // in two halves: the store warps have few registers
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) {
+                            uint32_t low[8];
+                            ptx::tmem_ld_32x8(src + (uint32_t)(N + j32 * 32 + h * 8), low);
+                            ptx::tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                raw[h * 8 + e] = __float_as_uint(__uint_as_float(raw[h * 8 + e]) + __uint_as_float(low[e]));
+                        }
+                    }
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         float4 v;
@@ -514,8 +545,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             // while the current four are processed.
             const int gid = (warp - SC_STORE_WARPS) * 4 + (lane >> 3);
             const int l8 = lane & 7;
-            using TI = typename std::conditional<SPLIT, float, T16>::type;
-            using RAW = typename std::conditional<SPLIT, uint4, uint2>::type;
+            using TI = typename std::conditional<M::F32, float, T16>::type;
+            using RAW = typename std::conditional<M::F32, uint4, uint2>::type;
             const TI *img = reinterpret_cast<const TI *>(P.img_cl);
             const uint32_t zrow = (uint32_t)g.B * (uint32_t)g.S * (uint32_t)g.Cs;   // what padding entries point at
             bool ok = true;
@@ -533,7 +564,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 w_col += c2 - c1;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
-                    if (lane == 0) atomicExch(P.status, 306);
+                    if (lane == 0) ptx::report(P.status, 306);
                     break;
                 }
                 const int span = (int)n_entries[pb];     // entries per group, padded: a multiple of 4
@@ -558,10 +589,10 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     }
                 };
                 auto image_values = [&](const RAW &r) -> float4 {
-                    if constexpr (SPLIT) {
+                    if constexpr (M::F32) {
                         return make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z),
                                            __uint_as_float(r.w));
-                    } else if constexpr (MODE == TC_F16) {
+                    } else if constexpr (M::HALF) {
                         const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r.x));
                         const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
                         return make_float4(a.x, a.y, b.x, b.y);
@@ -803,7 +834,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 ok = wait_all(&plan_free[pb], (uint32_t)(((j >> 1) & 1) ^ 1));
                 w_done += SC_CLK() - c0;
                 if (!ok) {
-                    if (pt == 0) atomicExch(P.status, 307);
+                    if (pt == 0) ptx::report(P.status, 307);
                     break;
                 }
             }
@@ -822,9 +853,9 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         // ------------------------------------------------------------------ MMA issue
         ptx::reg_dec<SC_REGS_ISSUE>();
         if (lane == 0) {
-            const uint32_t idesc = ptx::instr_desc_f16(MODE == TC_F16 ? 0 : 1, TILE_POS, N, 0, 0);
+            const uint32_t idesc = ptx::instr_desc_f16(M::HALF ? 0 : 1, TILE_POS, N, 0, 0);
             bool ok = ptx::mbar_wait(a_full, 0);
-            if (!ok) atomicExch(P.status, 302);
+            if (!ok) ptx::report(P.status, 302);
             ptx::tc_fence_after();
             // ring position and phase are stepped, never divided: a division by the run-time ring depth per stage
             // costs this single thread more than the stage's MMAs
@@ -838,21 +869,21 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 const bool got = ptx::mbar_wait_backoff<SC_SLEEP_NS>(&t_empty[aq], t_phase);
                 w_te += SC_CLK() - c0;
                 if (!got) {
-                    atomicExch(P.status, 303);
+                    ptx::report(P.status, 303);
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc_col0 + (uint32_t)(aq * N);
-                // f32 data: the hi and the lo part of a weight chunk are two stages of the ring; the first feeds
-                // a_hi x b_hi and a_lo x b_hi, the second a_hi x b_lo
+                const uint32_t d_tmem = tmem_base + acc_col0 + (uint32_t)(aq * ACCS * N);
+                // f32 data: the parts of a weight chunk are stages of their own; part b meets the dense parts a with
+                // a + b < PARTS (two parts: hi x hi, lo x hi; hi x lo)
                 for (int st = 0; st < RC * PARTS && ok; ++st) {
                     const int rc = st / PARTS, part = st % PARTS;
                     long long c1 = SC_CLK();
                     const bool gotb = ptx::mbar_wait(&b_full[s], b_phase);
                     w_bf += SC_CLK() - c1;
                     if (!gotb) {
-                        atomicExch(P.status, 304);
+                        ptx::report(P.status, 304);
                         ok = false;
                         break;
                     }
@@ -862,22 +893,36 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     // is 32 bytes inside the swizzled rows (+ 2), 8 TMEM columns of A
                     const uint64_t b_desc = b_desc0 + (uint64_t)((uint32_t)s * (L.b_stage >> 4));
                     const uint32_t a_hi = tmem_base + (uint32_t)(rc * 32);
-                    if (part == 0) {
-                        if (rc == 0)
-                            ptx::mma_f16_ts(d_tmem, a_hi, b_desc, idesc, 0u);
-                        else
-                            ptx::mma_f16_ts_acc(d_tmem, a_hi, b_desc, idesc);
-                        if constexpr (SPLIT) ptx::mma_f16_ts_acc(d_tmem, a_hi + (uint32_t)a_cols, b_desc, idesc);
-#pragma unroll
-                        for (int k4 = 1; k4 < 4; ++k4) {
-                            ptx::mma_f16_ts_acc(d_tmem, a_hi + (uint32_t)(k4 * 8), b_desc + (uint64_t)(2 * k4), idesc);
-                            if constexpr (SPLIT)
-                                ptx::mma_f16_ts_acc(d_tmem, a_hi + (uint32_t)(a_cols + k4 * 8), b_desc + (uint64_t)(2 * k4), idesc);
-                        }
-                    } else {
+                    // the products of one weight part with the dense parts PA0 ... PA1 - 1, into accumulator d
+                    auto products = [&](uint32_t d, auto pa0, auto pa1, bool open) {
 #pragma unroll
                         for (int k4 = 0; k4 < 4; ++k4)
-                            ptx::mma_f16_ts_acc(d_tmem, a_hi + (uint32_t)(k4 * 8), b_desc + (uint64_t)(2 * k4), idesc);
+#pragma unroll
+                            for (int pa = decltype(pa0)::value; pa < decltype(pa1)::value; ++pa) {
+                                const uint32_t a_k = a_hi + (uint32_t)(pa * a_cols + k4 * 8);
+                                if (k4 == 0 && pa == decltype(pa0)::value)
+                                    ptx::mma_f16_ts(d, a_k, b_desc, idesc, open ? 0u : 1u);
+                                else
+                                    ptx::mma_f16_ts_acc(d, a_k, b_desc + (uint64_t)(2 * k4), idesc);
+                            }
+                    };
+                    using std::integral_constant;
+                    const bool open = rc == 0;
+                    if constexpr (ACCS == 1) {
+                        if (part == 0)
+                            products(d_tmem, integral_constant<int, 0>(), integral_constant<int, PARTS>(), open);
+                        else
+                            products(d_tmem, integral_constant<int, 0>(), integral_constant<int, 1>(), false);
+                    } else {
+                        const uint32_t d_low = d_tmem + (uint32_t)N;
+                        if (part == 0) {
+                            products(d_tmem, integral_constant<int, 0>(), integral_constant<int, 1>(), open);
+                            products(d_low, integral_constant<int, 1>(), integral_constant<int, 3>(), open);
+                        } else if (part == 1) {
+                            products(d_low, integral_constant<int, 0>(), integral_constant<int, 2>(), false);
+                        } else {
+                            products(d_low, integral_constant<int, 0>(), integral_constant<int, 1>(), false);
+                        }
                     }
                     ptx::mma_commit(&b_empty[s]);
                     if (++s == BS) {
@@ -911,12 +956,12 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 for (int st = 0; st < RC * PARTS; ++st) {
                     const int rc = st / PARTS, part = st % PARTS;
                     if (!ptx::mbar_wait_backoff<SC_SLEEP_NS>(&b_empty[s], e_phase)) {
-                        atomicExch(P.status, 305);
+                        ptx::report(P.status, 305);
                         ok = false;
                         break;
                     }
                     ptx::mbar_arrive_expect_tx(&b_full[s], L.b_stage);
-                    ptx::tma_load_4d(sB + (size_t)s * L.b_stage, part == 0 ? &tmap_b_hi : &tmap_b_lo, &b_full[s], rc * 64, s0,
+                    ptx::tma_load_4d(sB + (size_t)s * L.b_stage, part == 0 ? &tmap_b_hi : (part == 1 ? &tmap_b_lo : &tmap_b_lo2), &b_full[s], rc * 64, s0,
                                      t0, grp);
                     last_s = s;
                     last_phase = e_phase ^ 1u;
@@ -953,7 +998,7 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, dim3 grid, const CUtensorM
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     LaunchScope scope("dcn_dgrad_tc", stream);
-    kern<<<grid, SC_THREADS, smem, stream>>>(P, maps[0], maps[1]);
+    kern<<<grid, SC_THREADS, smem, stream>>>(P, maps[0], maps[1], maps[2]);
     return cudaGetLastError();
 }
 
@@ -964,13 +1009,13 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, dim3 grid, const CUtensorM
 bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int *b_stages) {
     static const int tb_cap = tuning_int("TVDCN_B200_DG_TB", 4);
     static const int st_cap = tuning_int("TVDCN_B200_DG_STAGES", 4);
-    const int a_cols = (cdg / 2) * (mode == TC_SPLIT ? 2 : 1);
+    const int a_cols = (cdg / 2) * mode_mat_parts(mode);
     for (int cand = std::min(std::min(sc_tb_max(dim), tb_cap), K); cand >= 1; --cand) {
         // equal batches: the fewest batches of at most `cand` taps
         const int nb = (K + cand - 1) / cand;
         const int t = (K + nb - 1) / nb;
         const int n = t * SC_SLAB;
-        const int acc = std::min(4, (SC_TMEM_COLS - a_cols) / n);
+        const int acc = std::min(4, (SC_TMEM_COLS - a_cols) / (n * (mode == TC_F32_WIDE ? 2 : 1)));
         if (acc < 1) continue;
         for (int st = std::min(st_cap, 4); st >= 2; --st)
             if (dgrad_smem_bytes(dim, mode, t, st) <= 227 * 1024) {
@@ -983,28 +1028,22 @@ bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int 
     return false;
 }
 
-// dense: [B, Cd, P] in the problem's data type; w_kd_*: weights packed [g][tap][s'][d'] 16-bit (hi / lo);
+// dense: [B, Cd_r, P] in the problem's data type; w_parts: weights packed [g][tap][s'][d'], one 16-bit tensor per part;
 // img_cl: sampled image channels-last (needed for goff / gmask); accumulation targets are f32 and initialised by
 // the caller.
-cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense, const void *w_kd_hi,
-                                   const void *w_kd_lo, const void *img_cl, const float *offset, const float *mask,
-                                   float *img_grad_cl, float *goff, float *gmask, int *status, cudaStream_t stream) {
+cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense, void *const *w_parts,
+                                   const void *img_cl, const float *offset, const float *mask, float *img_grad_cl, float *goff, float *gmask, const Status &status, cudaStream_t stream) {
     const int cdg = h.Cd / h.groups, csg = h.Cs / h.groups;
     int tb = 0, nacc = 0, bs = 0;
     if (!dgrad_tc_config(h.dim, mode, cdg, h.K, &tb, &nacc, &bs)) return cudaErrorInvalidConfiguration;
     const int nbatch = (h.K + tb - 1) / tb;
     const long long BP = (long long)h.B * h.P;
-    CUtensorMap maps[2];
+    CUtensorMap maps[3];
     {
         const uint64_t dims[4] = {(uint64_t)cdg, (uint64_t)csg, (uint64_t)h.K, (uint64_t)h.groups};
         const uint64_t strides[3] = {(uint64_t)cdg * 2, (uint64_t)cdg * csg * 2, (uint64_t)cdg * csg * h.K * 2};
         const uint32_t box[4] = {64, (uint32_t)SC_SLAB, (uint32_t)tb, 1};
-        if (!make_tensor_map_16bit(&maps[0], w_kd_hi, 4, dims, strides, box)) return cudaErrorInvalidValue;
-        if (mode == TC_SPLIT) {
-            if (!make_tensor_map_16bit(&maps[1], w_kd_lo, 4, dims, strides, box)) return cudaErrorInvalidValue;
-        } else {
-            maps[1] = maps[0];
-        }
+        if (!make_part_maps(maps, w_parts, mode_mat_parts(mode), 4, dims, strides, box)) return cudaErrorInvalidValue;
     }
     // Share each position tile between `splits` CTAs (equal ranges of its units) when that evens out the last
     // wave: cost of a launch ~ ceil(CTAs / SMs) / splits tile-times; a split is taken only for a gain above 4 %
@@ -1041,9 +1080,14 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
         P.nacc = nacc;
         P.b_stages = bs;
         P.units_per_cta = n_units / splits;
-        if (mode == TC_BF16) return launch_dgrad_t<DIM, TC_BF16>(P, grid, maps, stream);
-        if (mode == TC_F16) return launch_dgrad_t<DIM, TC_F16>(P, grid, maps, stream);
-        return launch_dgrad_t<DIM, TC_SPLIT>(P, grid, maps, stream);
+        // 16-bit data: nothing is rounded between the MMA and the results, there is no wide mode of its own
+        switch (mode) {
+            case TC_BF16: case TC_BF16_WIDE: return launch_dgrad_t<DIM, TC_BF16>(P, grid, maps, stream);
+            case TC_F16: case TC_F16_WIDE: return launch_dgrad_t<DIM, TC_F16>(P, grid, maps, stream);
+            case TC_SPLIT: return launch_dgrad_t<DIM, TC_SPLIT>(P, grid, maps, stream);
+            case TC_F32_WIDE: return launch_dgrad_t<DIM, TC_F32_WIDE>(P, grid, maps, stream);
+        }
+        return cudaErrorInvalidValue;
     };
     if (h.dim == 1) return run(std::integral_constant<int, 1>());
     if (h.dim == 2) return run(std::integral_constant<int, 2>());

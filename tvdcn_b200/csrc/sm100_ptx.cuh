@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kernels.h"
+
 namespace tvdcn_b200 {
 namespace ptx {
 
@@ -82,6 +84,19 @@ __device__ __forceinline__ bool mbar_wait_backoff(uint64_t *bar, uint32_t parity
         __nanosleep(NS);
     }
     return false;
+}
+
+// A wait ran out: the code goes to the device word and, where there is one, straight to the host's.
+__device__ __forceinline__ void report(const Status &st, int code) {
+    atomicExch(st.device, code);
+    if (st.host != nullptr) *reinterpret_cast<volatile int *>(st.host) = code;
+}
+// One thread of a call's first kernel: what an earlier call left in the device word reaches the host.  A store, not a
+// copy: a copy would queue behind the caller's own transfers on the copy engines.
+__device__ __forceinline__ void publish(const Status &st) {
+    if (st.host == nullptr) return;
+    const int v = *reinterpret_cast<volatile int *>(st.device);
+    if (v != 0) *reinterpret_cast<volatile int *>(st.host) = v;
 }
 
 // Generic-proxy writes to shared memory (st.shared by the producer threads) must be made visible to the
@@ -185,6 +200,13 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
+}
+// 32 lanes x 8 consecutive columns
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 

@@ -34,7 +34,7 @@ struct WgradParams {
     const float *offset;
     const float *mask;
     float *gw;               // staged weight gradient [g][tap][d'][s'] f32, accumulated into
-    int *status;
+    Status status;
     int stages;
     int chunks_per_tap;      // csg / 64
     int n_sub;               // 64-column blocks per CTA
@@ -61,11 +61,11 @@ constexpr int WG_B_TILE = WG_POS * 128;          // [64 pos][64 ch] 16-bit
 
 template <int DIM, int MODE>
 __global__ void __launch_bounds__(WG_THREADS, 1)
-dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMap tmap_hi,
-                    const __grid_constant__ CUtensorMap tmap_lo) {
+dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMap tmap0,
+                    const __grid_constant__ CUtensorMap tmap1, const __grid_constant__ CUtensorMap tmap2) {
     constexpr int NC = 1 << DIM;
-    constexpr bool SPLIT = MODE == TC_SPLIT;
-    constexpr int PARTS = SPLIT ? 2 : 1;
+    using M = Mode<MODE>;
+    constexpr int CPARTS = M::COL_PARTS, MPARTS = M::MAT_PARTS;
     const Geo<DIM> &g = P.g;
 
     extern __shared__ uint8_t smem_raw[];
@@ -73,13 +73,13 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint8_t *smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const int S = P.stages;
     const int NS = P.n_sub, MT = P.m_tiles;
-    const uint32_t a_stage_bytes = (uint32_t)(MT * PARTS * WG_A_TILE);   // [m][part]
+    const uint32_t a_stage_bytes = (uint32_t)(MT * MPARTS * WG_A_TILE);   // [m][part]
     const uint32_t b_part_bytes = (uint32_t)(NS * WG_B_TILE);            // [part][sub]
-    const uint32_t b_stage_bytes = b_part_bytes * PARTS;
+    const uint32_t b_stage_bytes = b_part_bytes * CPARTS;
     uint8_t *sA = smem;
     uint8_t *sB = sA + (size_t)S * a_stage_bytes;
-    PlanEntry *plan = reinterpret_cast<PlanEntry *>(sB + (size_t)S * b_stage_bytes);   // [bufs][NS * 64][NC]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(plan + WG_PLAN_BUFS * NS * NC * WG_POS);
+    uint32_t *plan = reinterpret_cast<uint32_t *>(sB + (size_t)S * b_stage_bytes);   // slots [bufs][NS * 64][2 NC]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(plan + WG_PLAN_BUFS * NS * 2 * NC * WG_POS);
     uint64_t *full_s = bars;           // sampled tiles written
     uint64_t *full_d = bars + S;       // dense tiles landed
     uint64_t *empty = bars + 2 * S;
@@ -92,16 +92,19 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub_total = g.K * P.chunks_per_tap;                 // 64-column blocks per group
     const int kt0 = blockIdx.x * NS;                              // first column block of this CTA
-    const int y_tiles = (g.cdg + 128 * MT - 1) / (128 * MT);
+    const int y_tiles = (g.cdg_r + 128 * MT - 1) / (128 * MT);
     const int grp = blockIdx.y / y_tiles;
     const int d0 = (blockIdx.y % y_tiles) * 128 * MT;             // first dense channel within the group
     const int chunk_begin = blockIdx.z * P.chunks_per_split;
     const int chunk_end = min(chunk_begin + P.chunks_per_split, P.total_chunks);
     const int n_stages = max(chunk_end - chunk_begin, 0);
-    const uint32_t cols_used = (uint32_t)(MT * NS * 64);
+    // accumulators of the leading products, then (f32 data) as many of the small ones: see the modes
+    const uint32_t acc_cols = (uint32_t)(MT * NS * 64);
+    const uint32_t low_col = M::LOW_ACC ? acc_cols : 0u;
+    const uint32_t cols_used = acc_cols + low_col;
     uint32_t ncols = 32;
     while (ncols < cols_used) ncols <<= 1;
-    constexpr uint32_t ESZ = SPLIT ? 4 : 2;
+    constexpr uint32_t ESZ = M::F32 ? 4 : 2;
     // column blocks are ordered channel chunk outermost, tap innermost: the blocks of one CTA share an
     // image slab, which stays in L1
     auto sub_chan0 = [&](int sub) {
@@ -124,8 +127,9 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
     }
     if (threadIdx.x < 4) chan16_s[threadIdx.x] = (uint32_t)sub_chan0(min((int)threadIdx.x, NS - 1)) * ESZ / 16u;
     if (warp == WG_PRODUCER_WARPS + 1 && lane == 0) {
-        ptx::prefetch_tmap(&tmap_hi);
-        if (SPLIT) ptx::prefetch_tmap(&tmap_lo);
+        ptx::prefetch_tmap(&tmap0);
+        if (MPARTS > 1) ptx::prefetch_tmap(&tmap1);
+        if (MPARTS > 2) ptx::prefetch_tmap(&tmap2);
     }
     if (warp == WG_PRODUCER_WARPS) {
         ptx::tmem_alloc(tmem_slot, ncols);
@@ -146,18 +150,19 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
             const int s = i % S, r = i / S;
             const int pb = i % WG_PLAN_BUFS;
             if (ok && !ptx::mbar_wait(&plan_full[pb], (uint32_t)((i / WG_PLAN_BUFS) & 1))) {
-                atomicExch(P.status, 205);
+                ptx::report(P.status, 205);
                 ok = false;
             }
             if (ok && !ptx::mbar_wait(&empty[s], (uint32_t)((r & 1) ^ 1))) {
-                atomicExch(P.status, 201);
+                ptx::report(P.status, 201);
                 ok = false;
             }
             ok = __all_sync(0xffffffffu, ok);  // keep the warp converged for the __syncwarp below
             if (!ok) break;
-            uint8_t *b_hi = sB + (size_t)s * b_stage_bytes;
-            produce_tiles<NC, MODE, WG_GROUP_THREADS>(b_hi, b_hi + b_part_bytes, WG_B_TILE, WG_POS, NS * WG_POS, img16,
-                                                      chan16_s, plan + pb * NS * WG_POS * NC, tg);
+            uint8_t *b_tiles = sB + (size_t)s * b_stage_bytes;
+            produce_tiles<NC, MODE, WG_GROUP_THREADS, (NC >= 8 ? 2 : 4)>(b_tiles, b_part_bytes, WG_B_TILE, WG_POS,
+                                                                         NS * WG_POS, img16, chan16_s,
+                                                                         plan + pb * NS * WG_POS * 2 * NC, tg);
             ptx::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -169,7 +174,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
         // ------------------------------------------------------------------ epilogue: atomics into gw
         if (n_stages > 0) {
             if (ok && !ptx::mbar_wait(accum, 0)) {
-                atomicExch(P.status, 202);
+                ptx::report(P.status, 202);
                 ok = false;
             }
             ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is a whole-warp instruction
@@ -182,18 +187,25 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     uint32_t v[32];
                     ptx::tmem_ld_32x32(lane_base + (uint32_t)(cb * 32), v);
                     ptx::tmem_ld_wait();
+                    if constexpr (M::LOW_ACC) {
+                        uint32_t u[32];
+                        ptx::tmem_ld_32x32(lane_base + low_col + (uint32_t)(cb * 32), u);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]));
+                    }
                     const int m = cb / (NS * 2);
                     const int col0 = (cb % (NS * 2)) * 32;      // column within the M tile
                     const int sub = col0 / 64;
                     const int kt = kt0 + sub;
                     const int dl = d0 + m * 128 + lane_q * 32 + lane;   // dense channel within the group
-                    if (kt < sub_total && dl < g.cdg) {
+                    if (kt < sub_total && dl < g.cdg_r) {
                         const int tap = kt % g.K;
                         const int sl0 = (kt / g.K) * CHUNK_C + (col0 % 64);
                         // staged layout [g][tap][d'][s']: this thread's 32 values are 128 contiguous bytes, added
                         // with eight 16-byte reductions (the caller's [Cd, csg, K] layout would put every value in
                         // a sector of its own)
-                        float *dst = P.gw + (((int64_t)grp * g.K + tap) * g.cdg + dl) * g.csg + sl0;
+                        float *dst = P.gw + (((int64_t)grp * g.K + tap) * g.cdg_r + dl) * g.csg + sl0;
 #pragma unroll
                         for (int e = 0; e < 32; e += 4)
                             asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + e),
@@ -207,7 +219,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
     } else if (warp == WG_PRODUCER_WARPS) {
         // ------------------------------------------------------------------ MMA issue
         if (lane == 0) {
-            const uint32_t idesc = ptx::instr_desc_f16(MODE == TC_F16 ? 0 : 1, 128, NS * 64, 0, 1);
+            const uint32_t idesc = ptx::instr_desc_f16(M::HALF ? 0 : 1, 128, NS * 64, 0, 1);
             bool ok = true;
             // ring position and phase are stepped and the stage's descriptors derived from those of stage 0 by an
             // addition: bookkeeping must stay cheap next to the MMAs this single thread issues
@@ -217,7 +229,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
             uint32_t phase = 0;
             for (int i = 0; i < n_stages && ok; ++i) {
                 if (!ptx::mbar_wait(&full_s[s], phase) || !ptx::mbar_wait(&full_d[s], phase)) {
-                    atomicExch(P.status, 203);
+                    ptx::report(P.status, 203);
                     ok = false;
                     break;
                 }
@@ -226,7 +238,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 const uint64_t b_hi0 = b_desc0 + (uint64_t)((uint32_t)s * (b_stage_bytes >> 4));
                 for (int m = 0; m < MT; ++m) {
                     const uint32_t d_tmem = tmem_base + (uint32_t)(m * NS * 64);
-                    const uint64_t am = a_st + (uint64_t)((uint32_t)(m * PARTS) * (WG_A_TILE >> 4));
+                    const uint64_t am = a_st + (uint64_t)((uint32_t)(m * MPARTS) * (WG_A_TILE >> 4));
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4) {
                         // A: K-major rows of 64 positions (32 bytes per K step); B: MN-major, 16 positions = 16 rows
@@ -234,10 +246,16 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                         const uint64_t a_hi = am + 2 * k4;
                         const uint64_t b_hi = b_hi0 + 128 * k4;
                         ptx::mma_f16(d_tmem, a_hi, b_hi, idesc, (i > 0 || k4 > 0) ? 1u : 0u);
-                        if constexpr (SPLIT) {
-                            ptx::mma_f16(d_tmem, a_hi + (WG_A_TILE >> 4), b_hi, idesc, 1u);
-                            ptx::mma_f16(d_tmem, a_hi, b_hi + (b_part_bytes >> 4), idesc, 1u);
-                        }
+                        uint32_t low_on = (!M::LOW_ACC || i > 0 || k4 > 0) ? 1u : 0u;
+#pragma unroll
+                        for (int ca = 0; ca < MPARTS; ++ca)
+#pragma unroll
+                            for (int cb = 0; cb < CPARTS; ++cb)
+                                if (ca + cb > 0 && ca + cb < CPARTS) {
+                                    ptx::mma_f16(d_tmem + low_col, a_hi + (uint64_t)(ca * (WG_A_TILE >> 4)),
+                                                 b_hi + (uint64_t)((uint32_t)cb * (b_part_bytes >> 4)), idesc, low_on);
+                                    low_on = 1u;
+                                }
                     }
                 }
                 ptx::mma_commit(&empty[s]);
@@ -256,7 +274,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
             for (int i = 0; i < n_stages; ++i) {
                 const int s = i % S, r = i / S;
                 if (!ptx::mbar_wait(&empty[s], (uint32_t)((r & 1) ^ 1))) {
-                    atomicExch(P.status, 204);
+                    ptx::report(P.status, 204);
                     break;
                 }
                 const int pc = chunk_begin + i;
@@ -265,10 +283,11 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 uint8_t *a_dst = sA + (size_t)s * a_stage_bytes;
                 ptx::mbar_arrive_expect_tx(&full_d[s], a_stage_bytes);
                 for (int m = 0; m < MT; ++m) {
-                    const int dch = grp * g.cdg + d0 + m * 128;
-                    ptx::tma_load_3d(a_dst + (size_t)(m * PARTS) * WG_A_TILE, &tmap_hi, &full_d[s], p0, dch, b);
-                    if (SPLIT)
-                        ptx::tma_load_3d(a_dst + (size_t)(m * PARTS + 1) * WG_A_TILE, &tmap_lo, &full_d[s], p0, dch, b);
+                    const int dch = grp * g.cdg_r + d0 + m * 128;
+                    uint8_t *a_m = a_dst + (size_t)(m * MPARTS) * WG_A_TILE;
+                    ptx::tma_load_3d(a_m, &tmap0, &full_d[s], p0, dch, b);
+                    if (MPARTS > 1) ptx::tma_load_3d(a_m + WG_A_TILE, &tmap1, &full_d[s], p0, dch, b);
+                    if (MPARTS > 2) ptx::tma_load_3d(a_m + 2 * WG_A_TILE, &tmap2, &full_d[s], p0, dch, b);
                 }
                 issued = i + 1;
             }
@@ -330,14 +349,14 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
             bool ok = ptx::mbar_wait(&plan_empty[pb], (uint32_t)(((i / WG_PLAN_BUFS) & 1) ^ 1));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
-                if (lane == 0) atomicExch(P.status, 206);
+                if (lane == 0) ptx::report(P.status, 206);
                 break;
             }
 #pragma unroll
             for (int k = 0; k < EPT; ++k) {
                 if (e_on[k])
                     build_plan<DIM, MODE>(g, cur.pi[k], cur.rc[k], deformable, e_tap[k], row_scale,
-                                          plan + ((pb * NS) * WG_POS + t + k * WG_PLANNERS) * NC);
+                                          plan + ((pb * NS) * WG_POS + t + k * WG_PLANNERS) * 2 * NC);
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&plan_full[pb]);
@@ -350,32 +369,29 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
 }
 
 size_t wgrad_smem_bytes(int dim, int mode, int n_sub, int m_tiles, int stages) {
-    const int parts = mode == TC_SPLIT ? 2 : 1;
-    const size_t stage = (size_t)parts * (m_tiles * WG_A_TILE + n_sub * WG_B_TILE);
+    const size_t stage = (size_t)mode_mat_parts(mode) * m_tiles * WG_A_TILE + (size_t)mode_col_parts(mode) * n_sub * WG_B_TILE;
     const size_t plan = (size_t)WG_PLAN_BUFS * n_sub * (1 << dim) * WG_POS * 8;
     return 1024 + stages * stage + plan + (3 * stages + 1 + 2 * WG_PLAN_BUFS) * 8 + 16;
 }
 
 template <int DIM, int MODE>
-cudaError_t launch_wgrad_t(const WgradParams<DIM> &P, dim3 grid, const CUtensorMap &hi, const CUtensorMap &lo,
-                           cudaStream_t stream) {
+cudaError_t launch_wgrad_t(const WgradParams<DIM> &P, dim3 grid, const CUtensorMap *maps, cudaStream_t stream) {
     const size_t smem = wgrad_smem_bytes(DIM, MODE, P.n_sub, P.m_tiles, P.stages);
     auto kern = dcn_wgrad_tc_kernel<DIM, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     LaunchScope scope("dcn_wgrad_tc", stream);
-    kern<<<grid, WG_THREADS, smem, stream>>>(P, hi, lo);
+    kern<<<grid, WG_THREADS, smem, stream>>>(P, maps[0], maps[1], maps[2]);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 // Tile shape and pipeline depth; false when the shape is not covered.
-bool wgrad_tc_config(int dim, int mode, int cdg, int P, int *n_sub, int *m_tiles, int *stages) {
-    if (P % 8 != 0) return false;  // the dense tensor's row pitch must be a multiple of 16 bytes for TMA
-    const int mt = cdg > 128 ? 2 : 1;
-    int ns = mode == TC_SPLIT ? 2 : 4;
-    if (dim == 3 && mode != TC_SPLIT) ns = 4;
+bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages) {
+    // f32 data: twice the accumulators (see the modes), and two or three parts of every operand in shared memory
+    const int mt = cdg > 128 && mode != TC_F32_WIDE ? 2 : 1;
+    const int ns = mode_f32(mode) ? 2 : 4;
     int s = 0;
     static const int max_stages = tuning_int("TVDCN_B200_WG_STAGES", 2);
     for (int cand = max_stages; cand >= 2; --cand)
@@ -387,24 +403,19 @@ bool wgrad_tc_config(int dim, int mode, int cdg, int P, int *n_sub, int *m_tiles
     return true;
 }
 
-// dense_hi / dense_lo: the dense tensor [B, Cd, P] as 16-bit (the tensor itself for 16-bit data; bf16 hi
-// and lo parts of the f32 tensor in split mode).  gw must be zero-initialised f32.
-cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, const void *dense_hi, const void *dense_lo,
+// dense_parts: the dense tensor [B, Cd_r, P] as 16-bit parts (the tensor itself for 16-bit data) with rows
+// `pitch` elements apart, a multiple of 8.  gw must be zero-initialised f32 [groups][K][cdg_r][csg]; h: padded geometry.
+cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch,
                                    const void *img_cl, const float *offset, const float *mask, float *gw,
-                                   int *status, cudaStream_t stream) {
-    const int cdg = h.Cd / h.groups, csg = h.Cs / h.groups;
+                                   const Status &status, cudaStream_t stream) {
+    const int cdg = h.Cd_r / h.groups, csg = h.Cs / h.groups;
     int ns = 0, mt = 0, st = 0;
-    if (!wgrad_tc_config(h.dim, mode, cdg, h.P, &ns, &mt, &st)) return cudaErrorInvalidConfiguration;
-    CUtensorMap hi, lo;
-    const uint64_t dims[3] = {(uint64_t)h.P, (uint64_t)h.Cd, (uint64_t)h.B};
-    const uint64_t strides[2] = {(uint64_t)h.P * 2, (uint64_t)h.P * h.Cd * 2};
+    if (pitch % 8 != 0 || !wgrad_tc_config(h.dim, mode, cdg, &ns, &mt, &st)) return cudaErrorInvalidConfiguration;
+    CUtensorMap maps[3];
+    const uint64_t dims[3] = {(uint64_t)h.P, (uint64_t)h.Cd_r, (uint64_t)h.B};
+    const uint64_t strides[2] = {(uint64_t)pitch * 2, (uint64_t)pitch * h.Cd_r * 2};
     const uint32_t box[3] = {WG_POS, 128, 1};
-    if (!make_tensor_map_16bit(&hi, dense_hi, 3, dims, strides, box)) return cudaErrorInvalidValue;
-    if (mode == TC_SPLIT) {
-        if (!make_tensor_map_16bit(&lo, dense_lo, 3, dims, strides, box)) return cudaErrorInvalidValue;
-    } else {
-        lo = hi;
-    }
+    if (!make_part_maps(maps, dense_parts, mode_mat_parts(mode), 3, dims, strides, box)) return cudaErrorInvalidValue;
     const int sub_total = h.K * (csg / CHUNK_C);
     const int k_tiles = (sub_total + ns - 1) / ns;
     const int y_tiles = h.groups * ((cdg + 128 * mt - 1) / (128 * mt));
@@ -412,12 +423,13 @@ cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, const void *dense
     const int total = h.B * cpi;
     const int per_wave = std::max(1, 148 / std::max(1, k_tiles * y_tiles));
     int splits = per_wave;
-    if (mode == TC_SPLIT) {
+    if (mode_f32(mode)) {
         // The tensor core's f32 accumulation rounds toward zero, so the error of one accumulator grows linearly
         // with the number of MMAs added into it (measured: ~4e-8 of the result per MMA).  f32 data promises
-        // 1e-4: keep one CTA's chain at 56 stages (672 MMAs) by using more waves of CTAs; the partial sums
-        // meet in grad_weight through round-to-nearest f32 atomics.
-        const int max_stages = 56;
+        // 1e-4: keep one CTA's chain of leading products at 168 stages (672 MMAs; a quarter of that in the mode
+        // that keeps all 24 bits) by using more waves of CTAs; the partial sums meet in grad_weight through
+        // round-to-nearest f32 atomics.
+        const int max_stages = mode == TC_SPLIT ? 168 : 42;
         int waves = 1;
         while ((total + waves * per_wave - 1) / (waves * per_wave) > max_stages) ++waves;
         splits = waves * per_wave;
@@ -442,9 +454,7 @@ cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, const void *dense
         P.chunks_per_image = cpi;
         P.chunks_per_split = per;
         P.total_chunks = total;
-        if (mode == TC_BF16) return launch_wgrad_t<DIM, TC_BF16>(P, grid, hi, lo, stream);
-        if (mode == TC_F16) return launch_wgrad_t<DIM, TC_F16>(P, grid, hi, lo, stream);
-        return launch_wgrad_t<DIM, TC_SPLIT>(P, grid, hi, lo, stream);
+        return with_mode(mode, [&](auto m) { return launch_wgrad_t<DIM, decltype(m)::value>(P, grid, maps, stream); });
     };
     if (h.dim == 1) return run(std::integral_constant<int, 1>());
     if (h.dim == 2) return run(std::integral_constant<int, 2>());
@@ -453,18 +463,22 @@ cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, const void *dense
 }
 
 namespace {
-// staged [g][tap][d'][s'] f32 -> the caller's [Cd, csg, K] in its data type
+// staged [g][tap][d'][padded s'] f32 -> the caller's [Cd, csg, K] in its data type; a granule of `gran` sampled
+// channels sits at a multiple of gran_pad
 template <typename TO>
 __global__ void __launch_bounds__(256) unpack_weight_grad_kernel(const float *__restrict__ staged, TO *__restrict__ gw,
-                                                                 int groups, int cdg, int csg, int K) {
+                                                                 int groups, int cdg, int csg, int K, int gran,
+                                                                 int gran_pad) {
     // one block per (dense channel, 64 sampled channels): reads K rows of 64 floats, writes 64 * K contiguous values
     extern __shared__ float tile[];   // [K][65]
     const int d = blockIdx.x;                // grp * cdg + dl
     const int grp = d / cdg, dl = d % cdg;
     const int s0 = blockIdx.y * 64;
+    const int csg_pad = csg / gran * gran_pad;
     for (int i = threadIdx.x; i < K * 64; i += blockDim.x) {
-        const int tap = i / 64, sl = i % 64;
-        tile[tap * 65 + sl] = s0 + sl < csg ? staged[(((int64_t)grp * K + tap) * cdg + dl) * csg + s0 + sl] : 0.f;
+        const int tap = i / 64, sl = i % 64, s = s0 + sl;
+        const int sp = gran == gran_pad ? s : s / gran * gran_pad + s % gran;
+        tile[tap * 65 + sl] = s < csg ? staged[(((int64_t)grp * K + tap) * cdg + dl) * csg_pad + sp] : 0.f;
     }
     __syncthreads();
     TO *out = gw + ((int64_t)d * csg + s0) * K;
@@ -473,9 +487,10 @@ __global__ void __launch_bounds__(256) unpack_weight_grad_kernel(const float *__
 }
 }  // namespace
 
-cudaError_t launch_unpack_weight_grad(const float *staged, void *gw, int dtype, int groups, int cdg, int csg, int K,
-                                      cudaStream_t stream) {
-    dim3 grid((unsigned)(groups * cdg), (unsigned)((csg + 63) / 64));
+// h: padded geometry
+cudaError_t launch_unpack_weight_grad(const float *staged, void *gw, int dtype, const GeoHost &h, cudaStream_t stream) {
+    const int cdg = h.Cd_r / h.groups, csg = h.Cs_r / h.groups, K = h.K;
+    dim3 grid((unsigned)h.Cd_r, (unsigned)((csg + 63) / 64));
     const size_t smem = (size_t)K * 65 * sizeof(float);
     auto run = [&](auto kern, auto *out) -> cudaError_t {
         if (smem > 48 * 1024) {   // many taps: the tile needs the opt-in shared memory size
@@ -483,7 +498,7 @@ cudaError_t launch_unpack_weight_grad(const float *staged, void *gw, int dtype, 
             if (e != cudaSuccess) return e;
         }
         LaunchScope scope("unpack_weight_grad", stream);
-        kern<<<grid, 256, smem, stream>>>(staged, out, groups, cdg, csg, K);
+        kern<<<grid, 256, smem, stream>>>(staged, out, h.groups, cdg, csg, K, h.gran, h.gran_pad);
         return cudaGetLastError();
     };
     if (dtype == DT_F32) return run(unpack_weight_grad_kernel<float>, (float *)gw);

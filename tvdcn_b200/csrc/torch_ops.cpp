@@ -247,10 +247,10 @@ Call prepare(const Tensor &input, const Tensor &weight, const OptTensor &offset,
 
 // ---- status of the bounded waits, without a synchronisation per call --------------------------------------
 // The tensor-core kernels give up on a barrier wait that runs out and leave a code in a per-device word; their
-// outputs are then incomplete.  After every operator call a one-thread kernel, behind the call's kernels on the same
-// stream, stores a non-zero word into one mapped pinned host integer per device (a store, not a copy: a copy would
-// queue behind the caller's own transfers on the copy engines); the next operator call on that device looks at the
-// integer first and raises.  With TVDCN_B200_CHECK_STATUS=1 every call synchronises and raises itself.
+// outputs are then incomplete.  The kernels also store it into one mapped pinned host integer per device (a store, not
+// a copy: a copy would queue behind the caller's own transfers on the copy engines), and the first kernel of a call
+// stores what the device word holds already; the next operator call on that device looks at the integer first and
+// raises.  Only calls that run no tensor-core kernel launch a kernel of their own for it.  With TVDCN_B200_CHECK_STATUS=1 every call synchronises and raises itself.
 struct StatusWatch {
     int *pinned = nullptr;       // host view of the mapped pinned word
     int *pinned_dev = nullptr;   // the same word as the device addresses it
@@ -266,6 +266,7 @@ StatusWatch &status_watch(int device) {
             cudaHostGetDevicePointer(&dev_view, w.pinned, 0) == cudaSuccess) {
             *w.pinned = 0;
             w.pinned_dev = static_cast<int *>(dev_view);
+            (void)tvdcn_b200_watch_status(w.pinned_dev);
         } else {
             w.pinned = nullptr;
         }
