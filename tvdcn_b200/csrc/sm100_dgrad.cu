@@ -19,8 +19,8 @@
 //          B = weights packed [g][tap][s'][d'], one TMA box {64 d', 32 s', TB taps} per reduction chunk (ring);
 //          D = ring of accumulators in the TMEM columns behind A.
 //   plan   Four planner warps (thread = position) turn the unit's offsets / mask into one entry per in-image
-//          bilinear corner (pixel row, position, tap, weight x mask) and GROUP THE ENTRIES BY PIXEL with a
-//          shared-memory hash table (integer atomics) + prefix sum.
+//          bilinear corner (pixel row, position, tap, weight x mask) and GROUP THE ENTRIES BY PIXEL: a counting
+//          sort by pixel row modulo SC_SLOTS (shared-memory integer atomics + prefix sum).
 //   store  Four warps copy each finished accumulator TMEM -> shared memory ([128 pos][TB*32] f32).
 //   gather Twelve warps, 8 lanes per entry (4 channels each), walk equal spans of the pixel-grouped entry
 //          list: one 16-byte shared load of the entry's column values feeds both the running sum of the
@@ -76,13 +76,15 @@ constexpr int SC_REGS_WORK = 96, SC_REGS_STORE = 56, SC_REGS_ISSUE = 40;
 constexpr int SC_GROUPS = SC_GATHER_WARPS * 4;                    // 8-lane groups walking the entry list
 constexpr int SC_SLAB = 32;                                       // channels per pass
 constexpr int SC_PLAN_SLACK = SC_GROUPS * 4 + 16;
-constexpr int SC_HASH = 2048;                                     // slots; >= entries of one unit
+// Slots of the counting sort.  A tile's entries lie around its positions, so rows that share a slot are rare; where
+// they do, their entries interleave and the pixel's running sum leaves the SM more often, nothing else.
+constexpr int SC_SLOTS = 2048;
 constexpr uint32_t SC_NONE = 0xffffffffu;
 constexpr int SC_TMEM_COLS = 512;
 constexpr int SC_SLEEP_NS = 32;                                   // back-off of the long waits (64 to 512 measured equal)
 constexpr int SC_MAX_TAPS = 512;                                  // taps whose kernel coordinates a CTA tabulates
 
-// most taps per batch: 128 * tb * 2^dim entries must fit the hash table
+// most taps per batch: shared memory holds the column values and the entry lists of two batches
 __host__ __device__ constexpr int sc_tb_max(int dim) { return dim == 1 ? 4 : (dim == 2 ? 3 : 2); }
 
 // Predicated form: no branch around the reduction, and no "memory" clobber either -- nothing in this kernel reads
@@ -136,7 +138,7 @@ __device__ __forceinline__ void corner_of(const Geo<DIM> &g, const PosInfo<DIM> 
 
 // Byte offsets of the dynamic shared memory regions (after alignment to 1024).
 struct ScLayout {
-    uint32_t b_stage, col_buf, plan_buf, col, plan, keys, cnt, taps, misc, bars, total;
+    uint32_t b_stage, col_buf, plan_buf, col, plan, cnt, taps, misc, bars, total;
     int n, col_stride, max_entries;
 };
 __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_stages) {
@@ -154,8 +156,7 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
     o += (uint32_t)b_stages * L.b_stage;
     L.col = o;  o += 2 * L.col_buf;
     L.plan = o; o += 2 * L.plan_buf;
-    L.keys = o; o += SC_HASH * 4;
-    L.cnt = o;  o += SC_HASH * 4;
+    L.cnt = o;  o += SC_SLOTS * 4;
     L.taps = o; o += SC_MAX_TAPS * 3 * 2;         // kernel coordinates of every tap (int16)
     L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot
     L.bars = o; o += (uint32_t)(19 + 2 * b_stages) * 8;
@@ -185,7 +186,6 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     const uint32_t acc_col0 = (uint32_t)(a_cols * PARTS);
     uint8_t *sB = smem;
     float *col = reinterpret_cast<float *>(smem + L.col);
-    uint32_t *keys = reinterpret_cast<uint32_t *>(smem + L.keys);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(smem + L.cnt);
     uint32_t *misc = reinterpret_cast<uint32_t *>(smem + L.misc);
     uint32_t *scan_part = misc;          // [4]
@@ -700,18 +700,14 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             int t0, ogi, mgi;
             unit_groups(unit, t0, ogi, mgi);
             {
-                uint4 *k4 = reinterpret_cast<uint4 *>(keys), *c4 = reinterpret_cast<uint4 *>(cnt);
+                uint4 *c4 = reinterpret_cast<uint4 *>(cnt);
 #pragma unroll
-                for (int i = 0; i < SC_HASH / 4 / 128; ++i) {
-                    k4[pt + 128 * i] = make_uint4(SC_NONE, SC_NONE, SC_NONE, SC_NONE);
-                    c4[pt + 128 * i] = make_uint4(0u, 0u, 0u, 0u);
-                }
+                for (int i = 0; i < SC_SLOTS / 4 / 128; ++i) c4[pt + 128 * i] = make_uint4(0u, 0u, 0u, 0u);
             }
             planner_barrier();
             phase(0);
-            // pass 1: a hash slot per distinct pixel row, and the entry's rank among the entries of that row.  First
-            // probe of every entry before any retry, so that the shared-memory atomics of one thread overlap.
-            uint32_t rows[TBM * NC], slot[TBM * NC];
+            // pass 1: every entry's rank within its slot; all atomics of a thread are independent
+            uint32_t rows[TBM * NC], rank[TBM * NC];
             float wts[TBM * NC];
 #pragma unroll
             for (int t = 0; t < TBM; ++t) {
@@ -727,23 +723,9 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     wts[t * NC + c] = w * tg.mval;
                 }
             }
-            uint32_t old[TBM * NC];
 #pragma unroll
-            for (int i = 0; i < TBM * NC; ++i) {
-                slot[i] = (rows[i] * 2654435761u) >> 21;
-                old[i] = rows[i] != SC_NONE ? atomicCAS(&keys[slot[i]], SC_NONE, rows[i]) : rows[i];
-            }
-#pragma unroll
-            for (int i = 0; i < TBM * NC; ++i) {
-                if (rows[i] != SC_NONE) {
-                    uint32_t o = old[i];
-                    for (int probe = 0; probe < SC_HASH && o != SC_NONE && o != rows[i]; ++probe) {
-                        slot[i] = (slot[i] + 1) & (SC_HASH - 1);
-                        o = atomicCAS(&keys[slot[i]], SC_NONE, rows[i]);
-                    }
-                    old[i] = atomicAdd(&cnt[slot[i]], 1u);   // from here on: the entry's rank within its pixel's run
-                }
-            }
+            for (int i = 0; i < TBM * NC; ++i)
+                rank[i] = rows[i] != SC_NONE ? atomicAdd(&cnt[rows[i] & (SC_SLOTS - 1)], 1u) : 0u;
             phase(1);
             planner_barrier();
             phase(2);
@@ -786,7 +768,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             if (pt == 0) n_entries[pb] = span;
             planner_barrier();
             phase(3);
-            // pass 2: every entry goes to (start of its pixel's run) + (its rank)
+            // pass 2: every entry goes to (start of its slot) + (its rank)
             uint32_t *e_px = plan_px(pb);
             uint32_t *e_meta = plan_meta(pb);
             float *e_w = plan_w(pb);
@@ -796,7 +778,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 for (int c = 0; c < NC; ++c) {
                     const int i = t * NC + c;
                     if (rows[i] != SC_NONE) {
-                        const uint32_t at = cnt[slot[i]] + old[i];
+                        const uint32_t at = cnt[rows[i] & (SC_SLOTS - 1)] + rank[i];
                         e_px[at] = rows[i] * (uint32_t)g.Cs;
                         e_meta[at] = (colq_row + (uint32_t)(t * (SC_SLAB / 4))) | ((uint32_t)((pt * TB + t) * NC + c) << 16);
                         e_w[at] = wts[i];
