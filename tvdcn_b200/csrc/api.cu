@@ -189,6 +189,7 @@ struct TcCall {
         void *w[3];
         parts(kd ? pl.w_pack_kd : pl.w_pack, w);
         stage.pack(weight, w, g, p->dtype, mode_mat_parts(pl.mode), kd);
+        if (!kd && pl.sg_counters > 0) stage.zero(at(pl.sg_arrived), (int64_t)(pl.sg_counters * sizeof(unsigned)));
     }
     void stage_aux(const void *off, const void *msk, const void *bia) {
         const int64_t points = (int64_t)g.B * g.K * g.P;
@@ -210,7 +211,9 @@ struct TcCall {
     cudaError_t sample_gemm(void *out, cudaStream_t stream) const {
         void *w[3];
         parts(pl.w_pack, w);
-        return launch_sample_gemm_tc(g, pl.mode, at(pl.img_cl), w, offset, mask, bias, out, status, stream);
+        return launch_sample_gemm_tc(g, pl.mode, at(pl.img_cl), w, offset, mask, bias, out,
+                                     static_cast<float *>(at(pl.sg_partial)), static_cast<unsigned *>(at(pl.sg_arrived)),
+                                     status, stream);
     }
     // scatter_out (data type of the problem, [B, Cs, *img], may be null) receives the scattered image plus bias;
     // goff / gmask are zeroed f32 accumulators, may be null

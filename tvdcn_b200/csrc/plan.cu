@@ -69,6 +69,17 @@ void take_aux(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool 
     if (bias) pl.bias32 = b.take((size_t)p->out_channels * sizeof(float));
 }
 
+// buffers of the sample -> GEMM kernel besides the staged image
+void take_sample_buffers(Plan &pl, Bump &b, const GeoHost &g, int bn) {
+    take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
+    size_t partial = 0;
+    fwd_tc_workspace(g, bn, &partial, &pl.sg_counters);
+    if (partial > 0) {
+        pl.sg_partial = b.take(partial);
+        pl.sg_arrived = b.take(pl.sg_counters * sizeof(unsigned));
+    }
+}
+
 // buffers of the GEMM -> scatter kernel
 void take_scatter_buffers(Plan &pl, Bump &b, const GeoHost &g, bool scatter) {
     take_parts(pl.w_pack_kd, b, mode_mat_parts(pl.mode), packed_elems(g));
@@ -104,7 +115,7 @@ Plan plan_forward(const tvdcn_problem *p) {
         if (fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &bn, &st) && chain_ok(pl.mode, g, bn)) {
             pl.tensor = pl.tc_sg = true;
             pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);   // + one row of zeros
-            take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
+            take_sample_buffers(pl, b, g, bn);
             take_aux(pl, b, p, g, true);
         } else {
             why = "no tile configuration fits (or the f32 accumulation chain would be too long)";
@@ -138,11 +149,11 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
     want_offset = want_offset && g.og > 0;
     want_mask = want_mask && g.mg > 0;
     if (why == nullptr) {
-        int bn = 0, st = 0, ns = 0, mt = 0, gbufs = 0;
+        int bn = 0, sg_bn = 0, st = 0, ns = 0, mt = 0, gbufs = 0;
         // which primitives run on the tensor cores
         // transposed backward: grad_input is a sample -> GEMM over grad_output
-        pl.tc_sg = p->transposed && want_input && fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &bn, &st) &&
-                   chain_ok(pl.mode, g, bn);
+        pl.tc_sg = p->transposed && want_input && fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &sg_bn, &st) &&
+                   chain_ok(pl.mode, g, sg_bn);
         pl.tc_sw = want_weight && wgrad_tc_config(g.dim, pl.mode_sw, g.Cd_r / g.groups, &ns, &mt, &st);
         // conv: scatter into grad_input + coordinate gradients; transposed: coordinate gradients only
         const bool scatter = !p->transposed && want_input;
@@ -155,7 +166,7 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
             pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);
             take_aux(pl, b, p, g, false);
         }
-        if (pl.tc_sg) take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
+        if (pl.tc_sg) take_sample_buffers(pl, b, g, sg_bn);
         if (pl.tc_sw) {
             // f32 data is split into 16-bit parts; 16-bit rows are copied only where TMA cannot read them
             pl.dense_pitch = round_up(g.P, 8);

@@ -33,6 +33,7 @@ struct Plan {
     int dense_pitch = 0;
     size_t img_grad_cl = NO_BUF;   // f32 channels-last accumulator of the scatter
     size_t off32 = NO_BUF, mask32 = NO_BUF, bias32 = NO_BUF;   // 16-bit offset / mask / bias widened to f32
+    size_t sg_partial = NO_BUF, sg_arrived = NO_BUF, sg_counters = 0;   // sample -> GEMM: tiles shared between CTAs
     size_t sum_partial = NO_BUF, sum_done = NO_BUF;   // partial sums of the bias gradient and their arrival counters
 };
 
@@ -94,8 +95,9 @@ cudaError_t launch_dense_pass(const void *src, int dtype, int n_parts, void *con
 // ---- tensor-core kernels (sm100_*.cu); all take the padded geometry ---------------------------------------
 bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages);
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
-                                  const float *offset, const float *mask, const float *bias, void *out,
-                                  const Status &status, cudaStream_t stream);
+                                  const float *offset, const float *mask, const float *bias, void *out, float *partial,
+                                  unsigned *arrived, const Status &status, cudaStream_t stream);
+void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters);
 bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages);
 cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch, const void *img_cl,
                                    const float *offset, const float *mask, float *gw, const Status &status,

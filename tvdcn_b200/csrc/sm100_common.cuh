@@ -76,8 +76,9 @@ template <int DIM>
 __device__ __forceinline__ PosInfo<DIM> decode_position(const Geo<DIM> &g, long long idx) {
     PosInfo<DIM> pi;
     pi.valid = idx < g.BP;
-    pi.b = pi.valid ? (int)(idx / g.P) : 0;
-    pi.p = pi.valid ? (int)(idx % g.P) : 0;
+    const int i = pi.valid ? (int)idx : 0;             // fewer than 2^31 positions
+    pi.b = i / g.P;
+    pi.p = i - pi.b * g.P;
     decode_in_image<DIM>(g, pi);
     return pi;
 }
