@@ -121,22 +121,6 @@ struct RawCoords {
     float m;
 };
 
-template <int DIM>
-__device__ __forceinline__ RawCoords<DIM> load_coords(const Geo<DIM> &g, const PosInfo<DIM> &pi,
-                                                      const float *__restrict__ offset,
-                                                      const float *__restrict__ mask, int tap, int ogi, int mgi) {
-    RawCoords<DIM> rc;
-#pragma unroll
-    for (int a = 0; a < DIM; ++a)
-        rc.off[a] = (offset != nullptr && pi.valid)
-                        ? __ldg(offset + ((((int64_t)pi.b * g.og + ogi) * g.K + tap) * DIM + a) * (int64_t)g.P + pi.p)
-                        : 0.f;
-    rc.m = (mask != nullptr && pi.valid)
-               ? __ldg(mask + (((int64_t)pi.b * g.mg + mgi) * g.K + tap) * (int64_t)g.P + pi.p)
-               : 1.f;
-    return rc;
-}
-
 template <int MODE>
 __device__ __forceinline__ uint32_t encode_weight(float w) {
     if constexpr (Mode<MODE>::BLEND_F32) {
@@ -161,22 +145,9 @@ __device__ __forceinline__ void tap_coords(const Geo<DIM> &g, int tap, int (&tc)
     }
 }
 
-template <int DIM, int MODE>
-__device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
-                                              bool deformable, const int (&tc)[DIM], uint32_t row_scale,
-                                              uint32_t *slot);
-
-// Writes the plan slot of one position.  row_scale = Cs * element size / 16.
-template <int DIM, int MODE>
-__device__ __forceinline__ void build_plan(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
-                                           bool deformable, int tap, uint32_t row_scale, uint32_t *slot) {
-    int tc[DIM];
-    tap_coords<DIM>(g, tap, tc);
-    build_plan_at<DIM, MODE>(g, pi, rc, deformable, tc, row_scale, slot);
-}
-
-// Same, with the tap's kernel coordinates already known: the divisions by the kernel extents are a quarter of
-// the instructions of a plan entry, and a planner thread makes entries back to back.
+// Writes the plan slot of one position and tap, whose kernel coordinates are tc (the divisions by the kernel extents were
+// a quarter of the instructions of a slot, and a planner thread makes slots back to back).  row_scale = Cs * element
+// size / 16.
 template <int DIM, int MODE>
 __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
                                               bool deformable, const int (&tc)[DIM], uint32_t row_scale,

@@ -56,6 +56,8 @@ constexpr int WG_PLANNERS = WG_PLANNER_WARPS * 32;
 constexpr int WG_PLAN_BUFS = 3;
 constexpr int WG_THREADS = WG_PRODUCERS + 64 + WG_PLANNERS;
 constexpr int WG_POS = 64;                       // positions per stage
+// 64-column blocks per CTA; f32 data has twice the accumulators and several parts of every operand
+__host__ __device__ constexpr int wg_blocks(bool f32) { return f32 ? 2 : 4; }
 constexpr int WG_A_TILE = 128 * 128;             // [128 d][64 pos] 16-bit
 constexpr int WG_B_TILE = WG_POS * 128;          // [64 pos][64 ch] 16-bit
 
@@ -300,12 +302,16 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ planners
-        // entry e = (column block e / 64, position slot e % 64) of a stage; each thread fills up to two entries
-        constexpr int EPT = 4 * WG_POS / WG_PLANNERS;
+        // entry e = (column block e / 64, position slot e % 64) of a stage; each thread fills one entry (f32 data, two
+        // column blocks) or two (16-bit data, four), both of its position slot.  A planner thread runs one dependent instruction chain that paces the whole CTA, so nothing
+        // in it divides: taps are decoded once, positions are stepped by 64.
+        constexpr int EPT = wg_blocks(M::F32) * WG_POS / WG_PLANNERS;
         const int t = threadIdx.x - (WG_PRODUCERS + 64);
+        const int slot = t % WG_POS;
         const bool deformable = P.offset != nullptr;
         const uint32_t row_scale = (uint32_t)g.Cs * ESZ / 16u;
-        int e_tap[EPT], e_og[EPT], e_mg[EPT];
+        int e_tc[EPT][DIM];
+        const float *e_off[EPT], *e_mask[EPT];     // of the entry's tap and groups, at image 0, position 0
         bool e_on[EPT], e_ok[EPT];
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
@@ -313,54 +319,105 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
             const int kt = kt0 + sub;
             e_on[k] = sub < NS;
             e_ok[k] = e_on[k] && kt < sub_total;
-            e_tap[k] = e_ok[k] ? kt % g.K : 0;
+            const int tap = e_ok[k] ? kt % g.K : 0;
+            tap_coords<DIM>(g, tap, e_tc[k]);
             const int chan0 = sub_chan0(sub);
-            e_og[k] = g.og > 0 ? chan0 / g.cs_per_og : 0;
-            e_mg[k] = g.mg > 0 ? chan0 / g.cs_per_mg : 0;
+            const int ogi = g.og > 0 ? chan0 / g.cs_per_og : 0, mgi = g.mg > 0 ? chan0 / g.cs_per_mg : 0;
+            e_off[k] = P.offset != nullptr && e_ok[k] ? P.offset + (int64_t)((ogi * g.K + tap) * DIM) * g.P : nullptr;
+            e_mask[k] = P.mask != nullptr && e_ok[k] ? P.mask + (int64_t)(mgi * g.K + tap) * g.P : nullptr;
         }
-        const int slot = t % WG_POS;
-        // offsets / mask of stage i + 2 are requested while stage i is planned, so that their latency stays off
-        // the critical path
-        struct StageCoords {
-            PosInfo<DIM> pi[EPT];
-            RawCoords<DIM> rc[EPT];
-        };
-        auto fetch = [&](int i, StageCoords &sc) {
-            const int pc = chunk_begin + i;
-            const int p = (pc % P.chunks_per_image) * WG_POS + slot;
+        const int64_t off_image = (int64_t)g.og * g.K * DIM * g.P, mask_image = (int64_t)g.mg * g.K * g.P;
+        // grid coordinates of this slot in an image's first 64 positions, and of position 64
+        int slot_c[DIM], step_c[DIM];
+        auto grid_coords = [&](int p, int (&c)[DIM]) {
 #pragma unroll
-            for (int k = 0; k < EPT; ++k) {
-                sc.pi[k].valid = e_ok[k] && p < g.P;
-                sc.pi[k].b = pc / P.chunks_per_image;
-                sc.pi[k].p = sc.pi[k].valid ? p : 0;
-                decode_in_image<DIM>(g, sc.pi[k]);
-                if (e_on[k]) sc.rc[k] = load_coords<DIM>(g, sc.pi[k], P.offset, P.mask, e_tap[k], e_og[k], e_mg[k]);
+            for (int a = DIM - 1; a >= 0; --a) {
+                c[a] = a == 0 ? p : p % g.grid[a];
+                p /= g.grid[a];
             }
         };
-        StageCoords c0, c1, c2;
-        if (n_stages > 0) fetch(0, c0);
-        if (n_stages > 1) fetch(1, c1);
-        for (int i = 0; i < n_stages; ++i) {
+        grid_coords(slot, slot_c);
+        grid_coords(WG_POS, step_c);
+        struct Where {
+            int b, p, c[DIM];          // image, position, its grid coordinates
+        };
+        auto advance = [&](Where &w) {
+            w.p += WG_POS;
+            if (w.p - slot >= g.P) {   // the image's positions are through
+                ++w.b;
+                w.p = slot;
+#pragma unroll
+                for (int a = 0; a < DIM; ++a) w.c[a] = slot_c[a];
+                return;
+            }
+            int carry = 0;
+#pragma unroll
+            for (int a = DIM - 1; a >= 0; --a) {
+                w.c[a] += step_c[a] + carry;
+                carry = a > 0 && w.c[a] >= g.grid[a] ? 1 : 0;
+                if (carry) w.c[a] -= g.grid[a];
+            }
+        };
+        Where cur_w;
+        cur_w.b = chunk_begin / P.chunks_per_image;
+        cur_w.p = chunk_begin % P.chunks_per_image * WG_POS + slot;
+        grid_coords(cur_w.p, cur_w.c);
+        int fetch_b = cur_w.b, fetch_p = cur_w.p;      // of the stage whose offsets are being requested
+        // Offsets / mask of stage i + 2 are requested while stage i is planned, so that their latency stays off the
+        // critical path; the three sets rotate by name, never by assignment, which would wait for the loads.
+        struct StageCoords {
+            RawCoords<DIM> rc[EPT];
+        };
+        auto fetch = [&](StageCoords &sc) {
+            const bool in = fetch_p < g.P;
+            const int64_t off_at = fetch_b * off_image + fetch_p, mask_at = fetch_b * mask_image + fetch_p;
+#pragma unroll
+            for (int k = 0; k < EPT; ++k) {
+#pragma unroll
+                for (int a = 0; a < DIM; ++a)
+                    sc.rc[k].off[a] = in && e_off[k] != nullptr ? __ldg(e_off[k] + off_at + (int64_t)a * g.P) : 0.f;
+                sc.rc[k].m = in && e_mask[k] != nullptr ? __ldg(e_mask[k] + mask_at) : 1.f;
+            }
+            fetch_p += WG_POS;
+            if (fetch_p - slot >= g.P) {
+                ++fetch_b;
+                fetch_p = slot;
+            }
+        };
+        auto step = [&](int i, const StageCoords &cur, StageCoords &fill) -> bool {
             const int pb = i % WG_PLAN_BUFS;
-            if (i + 2 < n_stages) fetch(i + 2, c2);
-            const StageCoords cur = c0;
-            c0 = c1;
-            c1 = c2;
+            if (i + 2 < n_stages) fetch(fill);
             bool ok = ptx::mbar_wait(&plan_empty[pb], (uint32_t)(((i / WG_PLAN_BUFS) & 1) ^ 1));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 if (lane == 0) ptx::report(P.status, 206);
-                break;
+                return false;
             }
+            PosInfo<DIM> pi;
+            pi.b = cur_w.b;
+            pi.p = cur_w.p;
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) pi.base[a] = cur_w.c[a] * g.stride[a] - g.pad[a];
 #pragma unroll
             for (int k = 0; k < EPT; ++k) {
+                pi.valid = e_ok[k] && cur_w.p < g.P;
                 if (e_on[k])
-                    build_plan<DIM, MODE>(g, cur.pi[k], cur.rc[k], deformable, e_tap[k], row_scale,
-                                          plan + ((pb * NS) * WG_POS + t + k * WG_PLANNERS) * 2 * NC);
+                    build_plan_at<DIM, MODE>(g, pi, cur.rc[k], deformable, e_tc[k], row_scale,
+                                             plan + ((pb * NS) * WG_POS + t + k * WG_PLANNERS) * 2 * NC);
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&plan_full[pb]);
-        }
+            advance(cur_w);
+            return true;
+        };
+        StageCoords r0, r1, r2;
+        if (n_stages > 0) fetch(r0);
+        if (n_stages > 1) fetch(r1);
+        int i = 0;
+        bool ok = true;
+        for (; ok && i + 2 < n_stages; i += 3) ok = step(i, r0, r2) && step(i + 1, r1, r0) && step(i + 2, r2, r1);
+        if (ok && i < n_stages) ok = step(i, r0, r2);
+        if (ok && i + 1 < n_stages) ok = step(i + 1, r1, r0);
     }
 
     ptx::tc_fence_before();
@@ -391,7 +448,7 @@ cudaError_t launch_wgrad_t(const WgradParams<DIM> &P, dim3 grid, const CUtensorM
 bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages) {
     // f32 data: twice the accumulators (see the modes), and two or three parts of every operand in shared memory
     const int mt = cdg > 128 && mode != TC_F32_WIDE ? 2 : 1;
-    const int ns = mode_f32(mode) ? 2 : 4;
+    const int ns = wg_blocks(mode_f32(mode));
     int s = 0;
     static const int max_stages = tuning_int("TVDCN_B200_WG_STAGES", 2);
     for (int cand = max_stages; cand >= 2; --cand)
