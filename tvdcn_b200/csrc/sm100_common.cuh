@@ -7,7 +7,9 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -351,7 +353,41 @@ __device__ __forceinline__ void produce_tiles(uint8_t *tiles, uint32_t part_byte
     }
 }
 
+// a / b where b is often 1: a division costs a kernel's first instructions some hundred cycles
+__host__ __device__ __forceinline__ int div_often_one(int a, int b) { return b == 1 ? a : a / b; }
+
 // ---- host helpers ---------------------------------------------------------------------------------
+// Launches a kernel as a dependent of the one before it in the stream (see ptx::allow_dependents).  The kernel is granted
+// all dynamic shared memory there is once per device, not its launch's share on every launch (host time, and two threads
+// would overwrite each other's grant).
+template <auto Kern, typename... Args>
+inline cudaError_t launch_dependent(dim3 grid, unsigned block, size_t smem, cudaStream_t stream, const Args &...args) {
+    static std::atomic<uint64_t> granted{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if ((granted.load(std::memory_order_acquire) & bit) == 0) {
+        cudaFuncAttributes fa;
+        e = cudaFuncGetAttributes(&fa, Kern);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
+        if (e != cudaSuccess) return e;
+        granted.fetch_or(bit, std::memory_order_acq_rel);
+    }
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, Kern, args...);
+}
+
 // 16-bit tiled tensor map with 128-byte swizzle; dims innermost first.  Returns false when the driver
 // entry point is unavailable or rejects the description.
 bool make_tensor_map_16bit(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,

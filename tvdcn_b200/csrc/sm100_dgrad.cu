@@ -266,6 +266,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_dependency_wait();     // nothing above reads what an earlier kernel wrote
 
     // ---- pieces shared by the planners (which build a unit's entry list) and the store warps (which turn its dot
     // products into coordinate gradients); both map thread -> position of the tile
@@ -976,12 +977,10 @@ template <int DIM, int MODE>
 cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, dim3 grid, const CUtensorMap *maps, cudaStream_t stream) {
     const size_t smem = dgrad_smem_bytes(DIM, MODE, P.tb, P.b_stages);
     const bool coord = P.goff != nullptr || P.gmask != nullptr;
-    auto kern = coord ? dcn_dgrad_tc_kernel<DIM, MODE, true> : dcn_dgrad_tc_kernel<DIM, MODE, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     LaunchScope scope("dcn_dgrad_tc", stream);
-    kern<<<grid, SC_THREADS, smem, stream>>>(P, maps[0], maps[1], maps[2]);
-    return cudaGetLastError();
+    if (coord)
+        return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, true>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
+    return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, false>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
 }
 
 }  // namespace

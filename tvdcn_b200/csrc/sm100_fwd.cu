@@ -61,11 +61,11 @@ struct FwdWork {
 struct ChunkIter {
     int tap, cc, y, x;
     __device__ __forceinline__ void start(const FwdWork &w, int unit, int taps) {
-        const int tile = unit / w.n_chunks, j = unit % w.n_chunks;
-        x = tile / w.tiles_y;
-        y = tile % w.tiles_y;
-        cc = j / taps;
-        tap = j % taps;
+        const int tile = unit / w.n_chunks, j = unit - tile * w.n_chunks;
+        x = div_often_one(tile, w.tiles_y);
+        y = tile - x * w.tiles_y;
+        cc = j < taps ? 0 : j / taps;
+        tap = j - cc * taps;
     }
     // returns whether a new tile begins
     __device__ __forceinline__ bool next(int taps, int chunks, int tiles_y) {
@@ -216,6 +216,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_dependency_wait();     // nothing above reads what an earlier kernel wrote
 
     constexpr uint32_t ESZ = M::F32 ? 4 : 2;
     const uint4 *img16 = reinterpret_cast<const uint4 *>(P.img_cl);
@@ -275,8 +276,9 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
         }
     };
     // A tile's (or piece's) sums, `len` chunks of it, leave tensor memory: to the output, or to the workspace where the tile
-    // is shared -- whoever brings the last piece there adds them all.  4 * parts warps, this one being of quad `part`.
-    auto finish_piece = [&](int tile, int len, bool first_unit, int buf, int part, auto parts_c, bool last_piece, auto barrier) {
+    // is shared -- whoever brings the last piece there adds them all.  4 * parts warps, this one being of quad `part`; a warp
+    // whose wait ran out (!ok) passes the barriers with the others, which have no time limit, and does nothing else.
+    auto finish_piece = [&](bool ok, int tile, int len, bool first_unit, int buf, int part, auto parts_c, bool last_piece, auto barrier) {
         constexpr int parts = decltype(parts_c)::value;
         uint32_t *last_flag = last_flags + (last_piece ? 1 : 0);
         const int row = (warp & 3) * 32 + lane;               // position in the tile = TMEM lane
@@ -287,7 +289,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
         // this CTA's piece: in its first slot where it begins with the CTA's first unit, else in its second
         float4 *mine = shared_tile ? reinterpret_cast<float4 *>(P.partial) + ((size_t)blockIdx.x * 2 + (first_unit ? 0 : 1)) * (BN / 4) * TILE_POS
                                    : nullptr;
-        for (int cb = part; cb < BN / CW; cb += parts) {
+        for (int cb = ok ? part : BN / CW; cb < BN / CW; cb += parts) {
             float v[CW];
             uint32_t raw[CW];
             ptx::tmem_ld_32x16(t_lane + (uint32_t)(cb * CW), raw);
@@ -324,7 +326,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
                 __threadfence();
             }
             barrier();
-            if (*last_flag != 0) sum_pieces(tile, row, part, parts, std::integral_constant<int, 4>());
+            if (ok && *last_flag != 0) sum_pieces(tile, row, part, parts, std::integral_constant<int, 4>());
             barrier();
         }
     };
@@ -356,7 +358,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
             ok = __all_sync(0xffffffffu, ok);  // keep the warp converged for the __syncwarp below
             if (!ok) break;
             uint8_t *a_tiles = sA + (size_t)s * a_stage_bytes;
-            const uint32_t c16 = (uint32_t)(it.y / tiles_n * g.csg + it.cc * CHUNK_C) * ESZ / 16u;
+            const uint32_t c16 = (uint32_t)(div_often_one(it.y, tiles_n) * g.csg + it.cc * CHUNK_C) * ESZ / 16u;
             produce_tiles<NC, MODE, GROUP_THREADS, (NC >= 8 ? 2 : 4)>(a_tiles, A_TILE_BYTES, 0u, TILE_POS, TILE_POS, img16, &c16,
                                                                       plan + pbuf * TILE_POS * 2 * NC, tg);
             ptx::fence_proxy_async_smem();
@@ -371,14 +373,11 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
         const int before = last_tile - first_tile, buf = before % acc_bufs;
         ok = ok && ptx::mbar_wait(&acc_full[buf], (uint32_t)((before / acc_bufs) & 1));
         ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is a whole-warp instruction
-        if (!ok) {
-            if (lane == 0) ptx::report(P.status, 108);
-        } else {
-            ptx::tc_fence_after();
-            const int len = before == 0 ? n_local : unit0 + n_local - last_tile * n_chunks;
-            finish_piece(last_tile, len, before == 0, buf, warp >> 2, std::integral_constant<int, PRODUCER_WARPS / 4>(), true,
-                         [] { asm volatile("bar.sync 2, %0;" ::"n"(PRODUCERS) : "memory"); });
-        }
+        if (!ok && lane == 0) ptx::report(P.status, 108);
+        ptx::tc_fence_after();
+        const int len = before == 0 ? n_local : unit0 + n_local - last_tile * n_chunks;
+        finish_piece(ok, last_tile, len, before == 0, buf, warp >> 2, std::integral_constant<int, PRODUCER_WARPS / 4>(), true,
+                     [] { asm volatile("bar.sync 2, %0;" ::"n"(PRODUCERS) : "memory"); });
     } else if (warp >= EPI_WARP0 && warp < MMA_WARP) {
         // ------------------------------------------------------------------ epilogue: one thread per position
         ptx::reg_dec<FWD_REGS_EPILOGUE>();
@@ -386,14 +385,13 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
         int buf = 0;
         uint32_t phase = 0;
         for (int tile = first_tile; tile < last_tile; ++tile) {
-            ok = ptx::mbar_wait(&acc_full[buf], phase);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) {
-                if (lane == 0) ptx::report(P.status, 102);
-                break;
+            if (ok) {
+                ok = ptx::mbar_wait(&acc_full[buf], phase);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok && lane == 0) ptx::report(P.status, 102);
             }
             ptx::tc_fence_after();
-            finish_piece(tile, tile == first_tile ? (tile + 1) * n_chunks - unit0 : n_chunks, tile == first_tile, buf, 0,
+            finish_piece(ok, tile, tile == first_tile ? (tile + 1) * n_chunks - unit0 : n_chunks, tile == first_tile, buf, 0,
                          std::integral_constant<int, 1>(), false, [] { asm volatile("bar.sync 1, 128;" ::: "memory"); });
             if (++buf == acc_bufs) {
                 buf = 0;
@@ -483,7 +481,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
                 }
                 uint8_t *b_dst = sB + (size_t)s * b_stage_bytes;
                 ptx::mbar_arrive_expect_tx(&full_b[s], b_stage_bytes);
-                const int c0 = it.cc * CHUNK_C, grp = it.y / tiles_n, n0 = it.y % tiles_n * BN;
+                const int c0 = it.cc * CHUNK_C, grp = div_often_one(it.y, tiles_n), n0 = (it.y - grp * tiles_n) * BN;
                 ptx::tma_load_4d(b_dst, &tmap0, &full_b[s], c0, n0, it.tap, grp);
                 if (MPARTS > 1) ptx::tma_load_4d(b_dst + b_part_bytes, &tmap1, &full_b[s], c0, n0, it.tap, grp);
                 if (MPARTS > 2) ptx::tma_load_4d(b_dst + 2 * b_part_bytes, &tmap2, &full_b[s], c0, n0, it.tap, grp);
@@ -519,9 +517,9 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
             int ogi, mgi;
         };
         auto groups_of = [&](Cursor &c) {
-            const int chan0 = c.it.y / tiles_n * g.csg + c.it.cc * CHUNK_C;
-            c.ogi = g.og > 0 ? chan0 / g.cs_per_og : 0;
-            c.mgi = g.mg > 0 ? chan0 / g.cs_per_mg : 0;
+            const int chan0 = div_often_one(c.it.y, tiles_n) * g.csg + c.it.cc * CHUNK_C;
+            c.ogi = g.og > 1 ? chan0 / g.cs_per_og : 0;
+            c.mgi = g.mg > 1 ? chan0 / g.cs_per_mg : 0;
         };
         Cursor fetch_c;
         ChunkIter cur_c;
@@ -651,12 +649,9 @@ bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages) {
 template <int DIM, int MODE>
 cudaError_t launch_fwd_tc_t(const GeoHost &h, const FwdParams<DIM> &P, const CUtensorMap *maps, cudaStream_t stream) {
     const size_t smem = fwd_tc_smem_bytes(DIM, MODE, P.bn, P.stages);
-    auto kern = dcn_fwd_tc_kernel<DIM, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     LaunchScope scope("dcn_fwd_tc", stream);
-    kern<<<(unsigned)P.work.ctas, FWD_THREADS, smem, stream>>>(P, maps[0], maps[1], maps[2]);
-    return cudaGetLastError();
+    return launch_dependent<dcn_fwd_tc_kernel<DIM, MODE>>(dim3((unsigned)P.work.ctas), FWD_THREADS, smem, stream, P, maps[0],
+                                                          maps[1], maps[2]);
 }
 
 static bool fwd_work(const GeoHost &h, int bn, FwdWork *w) {

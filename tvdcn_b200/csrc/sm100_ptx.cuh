@@ -38,6 +38,14 @@ __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.al
 template <int N>
 __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
+// ---- programmatic dependent launch ---------------------------------------------------------------
+// The next kernel of the stream, if it was launched as a dependent, may begin once every block of this one has said so
+// (or has ended): its blocks then set up barriers and tensor memory while this kernel still works.  It touches nothing
+// that this kernel or an earlier one writes before grid_dependency_wait(), which returns when this kernel has ended and
+// its writes are visible.
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- mbarrier -----------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

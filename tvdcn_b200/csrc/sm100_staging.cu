@@ -224,6 +224,7 @@ __device__ void pitch_range(const StageJob &j, int block) {
 
 __global__ void __launch_bounds__(256) stage_kernel(const __grid_constant__ StageList list) {
     __shared__ uint32_t tile[STAGE_WORDS];
+    ptx::allow_dependents();
     if (blockIdx.x == 0 && threadIdx.x == 0) ptx::publish(list.status);
     int q = 0, first = 0;
     while (q + 1 < list.n && (int)blockIdx.x >= list.job[q].end_block) first = list.job[q++].end_block;
@@ -252,6 +253,7 @@ __global__ void __launch_bounds__(256) from_channels_last_kernel(const float *__
                                                                  int C, int c_pad, int gran, int gran_pad, int S,
                                                                  int wide) {
     __shared__ float tile[64 * 65];
+    ptx::grid_dependency_wait();
     const int c64 = c_pad / 64, s64 = (S + 63) / 64;
     const int c0 = (int)blockIdx.x % c64 * 64, s0 = (int)blockIdx.x / c64 % s64 * 64;
     const int64_t b = (int)blockIdx.x / c64 / s64;
@@ -480,9 +482,9 @@ cudaError_t launch_from_channels_last_bias(const float *src, const float *bias, 
     const int wide = h.S % 4 == 0 && aligned(dst, 16);
     LaunchScope scope("from_channels_last", stream);
     auto run = [&](auto *out) {
-        from_channels_last_kernel<<<(unsigned)blocks, 256, 0, stream>>>(src, bias, out, h.Cs_r, h.Cs, h.gran, h.gran_pad,
-                                                                        h.S, wide);
-        return cudaGetLastError();
+        using TO = typename std::remove_pointer<decltype(out)>::type;
+        return launch_dependent<from_channels_last_kernel<TO>>(dim3((unsigned)blocks), 256u, 0, stream, src, bias, out, h.Cs_r,
+                                                               h.Cs, h.gran, h.gran_pad, h.S, wide);
     };
     if (dst_dtype == DT_F32) return run((float *)dst);
     if (dst_dtype == DT_BF16) return run((__nv_bfloat16 *)dst);

@@ -141,6 +141,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_dependency_wait();     // nothing above reads what an earlier kernel wrote
 
     if (warp < WG_PRODUCER_WARPS) {
         // ------------------------------------------------------------------ producers
@@ -434,12 +435,8 @@ size_t wgrad_smem_bytes(int dim, int mode, int n_sub, int m_tiles, int stages) {
 template <int DIM, int MODE>
 cudaError_t launch_wgrad_t(const WgradParams<DIM> &P, dim3 grid, const CUtensorMap *maps, cudaStream_t stream) {
     const size_t smem = wgrad_smem_bytes(DIM, MODE, P.n_sub, P.m_tiles, P.stages);
-    auto kern = dcn_wgrad_tc_kernel<DIM, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     LaunchScope scope("dcn_wgrad_tc", stream);
-    kern<<<grid, WG_THREADS, smem, stream>>>(P, maps[0], maps[1], maps[2]);
-    return cudaGetLastError();
+    return launch_dependent<dcn_wgrad_tc_kernel<DIM, MODE>>(grid, WG_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
 }
 
 }  // namespace
@@ -528,6 +525,7 @@ __global__ void __launch_bounds__(256) unpack_weight_grad_kernel(const float *__
                                                                  int gran_pad) {
     // one block per (dense channel, 64 sampled channels): reads K rows of 64 floats, writes 64 * K contiguous values
     extern __shared__ float tile[];   // [K][65]
+    ptx::grid_dependency_wait();
     const int d = blockIdx.x;                // grp * cdg + dl
     const int grp = d / cdg, dl = d % cdg;
     const int s0 = blockIdx.y * 64;
@@ -549,18 +547,15 @@ cudaError_t launch_unpack_weight_grad(const float *staged, void *gw, int dtype, 
     const int cdg = h.Cd_r / h.groups, csg = h.Cs_r / h.groups, K = h.K;
     dim3 grid((unsigned)h.Cd_r, (unsigned)((csg + 63) / 64));
     const size_t smem = (size_t)K * 65 * sizeof(float);
-    auto run = [&](auto kern, auto *out) -> cudaError_t {
-        if (smem > 48 * 1024) {   // many taps: the tile needs the opt-in shared memory size
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-        }
+    auto run = [&](auto *out) -> cudaError_t {
+        using TO = typename std::remove_pointer<decltype(out)>::type;
         LaunchScope scope("unpack_weight_grad", stream);
-        kern<<<grid, 256, smem, stream>>>(staged, out, h.groups, cdg, csg, K, h.gran, h.gran_pad);
-        return cudaGetLastError();
+        return launch_dependent<unpack_weight_grad_kernel<TO>>(grid, 256u, smem, stream, staged, out, h.groups, cdg, csg, K, h.gran,
+                                                               h.gran_pad);
     };
-    if (dtype == DT_F32) return run(unpack_weight_grad_kernel<float>, (float *)gw);
-    if (dtype == DT_BF16) return run(unpack_weight_grad_kernel<__nv_bfloat16>, (__nv_bfloat16 *)gw);
-    if (dtype == DT_F16) return run(unpack_weight_grad_kernel<__half>, (__half *)gw);
+    if (dtype == DT_F32) return run((float *)gw);
+    if (dtype == DT_BF16) return run((__nv_bfloat16 *)gw);
+    if (dtype == DT_F16) return run((__half *)gw);
     return cudaErrorInvalidValue;
 }
 
