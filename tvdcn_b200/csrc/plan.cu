@@ -121,7 +121,12 @@ Plan plan_forward(const tvdcn_problem *p) {
             why = "no tile configuration fits (or the f32 accumulation chain would be too long)";
         }
     } else if (why == nullptr) {
-        if (dgrad_tc_config(g.dim, pl.mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st)) {
+        // One wave of SIMT blocks with one or two reduction steps is through before the three kernels of the tensor path
+        // have started up (8 -> 16 channels, 330 positions: 22 against 26 us of kernels).
+        const long long simt_blocks = ((long long)g.B * g.P + 63) / 64 * g.groups * (((long long)g.Cs_r / g.groups * g.K + 63) / 64);
+        if (pl.wide && p->engine == TVDCN_ENGINE_AUTO && g.Cd_r / g.groups <= 32 && simt_blocks <= 148) {
+            why = "so small that the SIMT kernel is faster";
+        } else if (dgrad_tc_config(g.dim, pl.mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st)) {
             pl.tensor = pl.tc_gs = true;
             take_scatter_buffers(pl, b, g, true);
             take_aux(pl, b, p, g, true);

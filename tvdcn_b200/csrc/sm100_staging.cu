@@ -46,17 +46,20 @@ __device__ void stage_image_tile(const StageJob &j, int block, uint32_t *tile) {
                 w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
             }
         } else {
+            // all loads of a thread before the first store: they are its only latency
+            const int s = s0 + 2 * lane;
+            uint32_t lo[8], hi[8];
+#pragma unroll
+            for (int pass = 0; pass < 8; ++pass) {
+                const int c = real_channel(c0 + warp * 8 + pass, j.gran, j.gran_pad);
+                const uint16_t *p = in + (int64_t)max(c, 0) * j.S + s;
+                lo[pass] = c >= 0 && s < j.S ? __ldg(p) : 0;
+                hi[pass] = c >= 0 && s + 1 < j.S ? __ldg(p + 1) : 0;
+            }
 #pragma unroll
             for (int pass = 0; pass < 8; ++pass) {
                 const int cl = warp * 8 + pass;
-                const int c = real_channel(c0 + cl, j.gran, j.gran_pad), s = s0 + 2 * lane;
-                uint32_t x = 0;
-                if (c >= 0) {
-                    const uint16_t *p = in + (int64_t)c * j.S + s;
-                    if (s < j.S) x = __ldg(p);
-                    if (s + 1 < j.S) x |= (uint32_t)__ldg(p + 1) << 16;
-                }
-                tile[(cl >> 1) * 65 + (cl & 1) * 32 + lane] = x;
+                tile[(cl >> 1) * 65 + (cl & 1) * 32 + lane] = lo[pass] | (hi[pass] << 16);
             }
         }
         __syncthreads();
@@ -84,12 +87,15 @@ __device__ void stage_image_tile(const StageJob &j, int block, uint32_t *tile) {
                 w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
             }
         } else {
+            const int sl = (warp & 1) * 32 + lane, s = s0 + sl;
+            uint32_t x[16];
 #pragma unroll
             for (int pass = 0; pass < 16; ++pass) {
-                const int cl = pass * 4 + (warp >> 1), sl = (warp & 1) * 32 + lane;
-                const int c = real_channel(c0 + cl, j.gran, j.gran_pad), s = s0 + sl;
-                tile[cl * 65 + sl] = c >= 0 && s < j.S ? __ldg(in + (int64_t)c * j.S + s) : 0u;
+                const int c = real_channel(c0 + pass * 4 + (warp >> 1), j.gran, j.gran_pad);
+                x[pass] = c >= 0 && s < j.S ? __ldg(in + (int64_t)max(c, 0) * j.S + s) : 0u;
             }
+#pragma unroll
+            for (int pass = 0; pass < 16; ++pass) tile[(pass * 4 + (warp >> 1)) * 65 + sl] = x[pass];
         }
         __syncthreads();
 #pragma unroll
