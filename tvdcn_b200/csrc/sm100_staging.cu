@@ -228,7 +228,12 @@ __device__ void pitch_range(const StageJob &j, int block) {
     }
 }
 
-__global__ void __launch_bounds__(256) stage_kernel(const __grid_constant__ StageList list) {
+// RESIDENT blocks per SM.  Copies of large images are bound by bytes in flight: eight blocks of 32 registers moved 537 MB in
+// 451 us (two calls' staging) where five of 48 took 523.  The unaligned paths keep 16 loads per thread in flight and spill
+// with 32 registers, and a launch that is resident as a whole either way gains nothing.
+constexpr int STAGE_RESIDENT = 5;             // what 48 registers allow
+template <int RESIDENT>
+__global__ void __launch_bounds__(256, RESIDENT) stage_kernel(const __grid_constant__ StageList list) {
     __shared__ uint32_t tile[STAGE_WORDS];
     ptx::allow_dependents();
     if (blockIdx.x == 0 && threadIdx.x == 0) ptx::publish(list.status);
@@ -477,7 +482,12 @@ cudaError_t Stager::launch(const Status &status, cudaStream_t stream) {
     if (list_.n == 0) return cudaSuccess;
     list_.status = status;
     LaunchScope scope("stage", stream);
-    stage_kernel<<<(unsigned)blocks_, 256, 0, stream>>>(list_);
+    bool wide = true;
+    for (int q = 0; q < list_.n; ++q) wide = wide && (list_.job[q].kind != STAGE_IMAGE || list_.job[q].wide);
+    if (wide && blocks_ > 148 * STAGE_RESIDENT)
+        stage_kernel<8><<<(unsigned)blocks_, 256, 0, stream>>>(list_);
+    else
+        stage_kernel<STAGE_RESIDENT><<<(unsigned)blocks_, 256, 0, stream>>>(list_);
     return cudaGetLastError();
 }
 
