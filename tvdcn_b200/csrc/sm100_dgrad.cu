@@ -10,12 +10,15 @@
 // (tvdcn/csrc/ops/cuda/deform_conv2d_kernel.cpp:519-598) and addmm_ + col2im of the transposed forward
 // (tvdcn/csrc/ops/cuda/deform_conv_transpose2d_kernel.cpp:333-362): the column buffer is never written.
 //
-// One CTA owns a tile of 128 grid positions and walks *units* = (64-channel chunk, batch of TB taps); every
-// unit is two *passes* over 32-channel slabs.
+// Work is cut into *units*: (tile of 128 grid positions, 64-channel chunk, batch of TB taps), ordered tile by tile.  The
+// grid has one CTA per SM (see launch_dgrad_t) and each takes an equal, contiguous range of units: nothing but a CTA's first unit waits
+// for its operands (start-up was 12 k of 36 k cycles per tile for short 1-d reductions), and the SMs finish together
+// whatever the number of tiles.  Every unit is two *passes* over 32-channel slabs.
 //   GEMM   D[128 positions (TMEM lanes) x TB*32 columns] over the dense channels of the group.
-//          A = the dense tile [128 pos][cdg], read once per CTA from the caller's [B, Cd, P] tensor (thread =
-//              position, coalesced), converted to 16-bit (f32 data: bf16 hi + lo) and kept in TENSOR MEMORY for
-//              the whole CTA (tcgen05.st; the MMA reads A from TMEM, so shared memory carries only B);
+//          A = the dense tile [128 pos][cdg], read once per tile from the caller's [B, Cd, P] tensor (thread =
+//              position, coalesced), converted to 16-bit (f32 data: bf16 parts) and kept in TENSOR MEMORY
+//              (tcgen05.st; the MMA reads A from TMEM, so shared memory carries only B); later tiles are loaded by the
+//              planner warps, idle half of the time, as soon as the old tile's last MMA is through;
 //          B = weights packed [g][tap][s'][d'], one TMA box {64 d', 32 s', TB taps} per reduction chunk (ring);
 //          D = ring of accumulators in the TMEM columns behind A.
 //   plan   Four planner warps (thread = position) turn the unit's offsets / mask into one entry per in-image
@@ -54,7 +57,9 @@ struct DgradParams {
     int nbatch;             // ceil(K / tb)
     int nacc;               // accumulators in the TMEM ring
     int b_stages;
-    int units_per_cta;      // (csg / 64) * nbatch / gridDim.z
+    int tiles_x;            // position tiles
+    int n_units;            // units per (position tile, group): (csg / 64) * nbatch
+    int total_units;
 };
 
 namespace {
@@ -98,16 +103,6 @@ __device__ __forceinline__ void red_add_v4_if(bool p, float *addr, float a, floa
         "}\n" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"((int)p));
 }
 
-// Cycle counters of one CTA in the middle of the grid, per role; compiled in only with -DTVDCN_B200_TUNING.
-#ifdef TVDCN_B200_TUNING
-__device__ long long g_dg_prof[64];
-#define SC_CLK() clock64()
-#define SC_PROF_OUT(i, v) do { if (prof_cta) g_dg_prof[i] = (v); } while (0)
-#else
-#define SC_CLK() 0ll
-#define SC_PROF_OUT(i, v) do { (void)(v); } while (0)
-#endif
-
 __device__ __forceinline__ void planner_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Sampling geometry of one (position, tap): floor and fraction per axis, mask value.
@@ -138,7 +133,7 @@ __device__ __forceinline__ void corner_of(const Geo<DIM> &g, const PosInfo<DIM> 
 
 // Byte offsets of the dynamic shared memory regions (after alignment to 1024).
 struct ScLayout {
-    uint32_t b_stage, col_buf, plan_buf, col, plan, cnt, taps, misc, bars, total;
+    uint32_t b_stage, col_buf, plan_buf, col, plan, info, pos, cnt, taps, misc, bars, total;
     int n, col_stride, max_entries;
 };
 __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_stages) {
@@ -156,12 +151,64 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
     o += (uint32_t)b_stages * L.b_stage;
     L.col = o;  o += 2 * L.col_buf;
     L.plan = o; o += 2 * L.plan_buf;
+    L.info = o; o += 2 * 16;                      // per plan buffer: first channel, first tap, offset group, mask group
+    L.pos = o;  o += 2 * TILE_POS * 8;            // and per position of the tile: image (or -1), position in it
     L.cnt = o;  o += SC_SLOTS * 4;
     L.taps = o; o += SC_MAX_TAPS * 3 * 2;         // kernel coordinates of every tap (int16)
     L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot
-    L.bars = o; o += (uint32_t)(19 + 2 * b_stages) * 8;
+    L.bars = o; o += (uint32_t)(20 + 2 * b_stages) * 8;
     L.total = o;
     return L;
+}
+
+// The units of a CTA in order.  1-d and 2-d: a CTA's tiles follow one another, so it finds its neighbourhood of the image
+// in the caches.  3-d: that neighbourhood spans planes and 148 of them do not fit L2 (contiguous ranges: 5.1 ms instead of
+// 4.4 for 8 x 64 x 16 x 56 x 56), so the CTAs take neighbouring tiles at the same time: ranges run down the columns of a matrix of
+// tiles with one column per CTA, filled row by row.
+struct UnitIter {
+    int x, grp, chunk, batch;   // position tile, group, 64-channel chunk, tap batch
+    int order;                  // the tile's place in that order
+};
+template <int DIM>
+__device__ __forceinline__ void locate_tile(const DgradParams<DIM> &P, UnitIter &u) {
+    int tile = u.order;
+    if constexpr (DIM == 3) {
+        const int tiles = P.tiles_x * P.g.groups, cols = (int)gridDim.x, rows = (tiles + cols - 1) / cols;
+        const int full = tiles - cols * (rows - 1);    // columns that have all rows
+        int c, r;
+        if (u.order < full * rows) {
+            c = u.order / rows;
+            r = u.order - c * rows;
+        } else {
+            const int o = u.order - full * rows;
+            c = o / (rows - 1);
+            r = o - c * (rows - 1);
+            c += full;
+        }
+        tile = r * cols + c;
+    }
+    u.grp = tile < P.tiles_x ? 0 : tile / P.tiles_x;
+    u.x = tile - u.grp * P.tiles_x;
+}
+template <int DIM>
+__device__ __forceinline__ UnitIter first_unit(const DgradParams<DIM> &P, int unit) {
+    UnitIter u;
+    u.order = unit / P.n_units;
+    const int r = unit - u.order * P.n_units;
+    u.chunk = r / P.nbatch;
+    u.batch = r - u.chunk * P.nbatch;
+    locate_tile(P, u);
+    return u;
+}
+// Returns whether a new tile begins.  (Behind the last unit of the launch there is none: its position stays as it is.)
+template <int DIM>
+__device__ __forceinline__ bool next_unit(const DgradParams<DIM> &P, UnitIter &u) {
+    if (++u.batch < P.nbatch) return false;
+    u.batch = 0;
+    if (++u.chunk < P.g.csg / CHUNK_C) return false;
+    u.chunk = 0;
+    if (++u.order < P.tiles_x * P.g.groups) locate_tile(P, u);
+    return true;
 }
 
 template <int DIM, int MODE, bool COORD>
@@ -193,8 +240,9 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint32_t *n_entries = misc + 6;      // [2]
     uint32_t *tmem_slot = misc + 8;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *a_full = bars;
-    uint64_t *b_full = bars + 1;
+    uint64_t *a_first = bars;            // dense tile of the CTA's first unit is in TMEM / of every later tile
+    uint64_t *a_next = bars + 1;
+    uint64_t *b_full = bars + 2;
     uint64_t *b_empty = b_full + BS;
     uint64_t *t_full = b_empty + BS;     // [4] MMA -> store warps: accumulator complete
     uint64_t *t_empty = t_full + 4;      // [4] store warps -> MMA: accumulator read out
@@ -213,23 +261,20 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     auto plan_w = [&](int pb) { return reinterpret_cast<float *>(plan_px(pb) + 2 * plan_words); };
     auto plan_dot = [&](int pb) { return reinterpret_cast<float *>(plan_px(pb) + 3 * plan_words); };
 
+    auto info_of = [&](int pb) { return reinterpret_cast<int4 *>(smem + L.info) + pb; };
+    auto pos_of = [&](int pb) { return reinterpret_cast<int2 *>(smem + L.pos) + pb * TILE_POS; };
+
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int grp = blockIdx.y;
-    const long long m0 = (long long)blockIdx.x * TILE_POS;
-    // units of this CTA: gridDim.z CTAs share one position tile and take equal ranges of its units, which evens
-    // out the last wave when the tiles do not fill the SMs a whole number of times
-    const int n_units = P.units_per_cta;
-    const int unit0 = (int)blockIdx.z * n_units;
+    // this CTA's units
+    const int unit0 = (int)((long long)P.total_units * blockIdx.x / gridDim.x);
+    const int n_units = (int)((long long)P.total_units * (blockIdx.x + 1) / gridDim.x) - unit0;
     const int n_pass = 2 * n_units;
     constexpr bool want_coord = COORD;    // grad_offset and / or grad_mask are wanted
     const bool scatter = P.img_grad_cl != nullptr;
     const bool deformable = P.offset != nullptr;
-    const bool prof_cta = blockIdx.x == gridDim.x / 2 && blockIdx.y == 0 && blockIdx.z == 0;
-    (void)prof_cta;
-    const long long clk_start = SC_CLK();
-
     if (threadIdx.x == 0) {
-        ptx::mbar_init(a_full, SC_LOAD_WARPS);
+        ptx::mbar_init(a_first, SC_LOAD_WARPS);
+        ptx::mbar_init(a_next, SC_PLAN_WARPS);
         for (int s = 0; s < BS; ++s) {
             ptx::mbar_init(&b_full[s], 1);
             ptx::mbar_init(&b_empty[s], 1);
@@ -270,21 +315,18 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
 
     // ---- pieces shared by the planners (which build a unit's entry list) and the store warps (which turn its dot
     // products into coordinate gradients); both map thread -> position of the tile
-    auto unit_groups = [&](int unit, int &t0, int &ogi, int &mgi) {
-        const int chunk = unit / P.nbatch;
-        t0 = (unit % P.nbatch) * TB;
-        const int chan0 = grp * g.csg + chunk * CHUNK_C;
-        ogi = g.og > 0 ? chan0 / g.cs_per_og : 0;
-        mgi = g.mg > 0 ? chan0 / g.cs_per_mg : 0;
+    // {first channel, first tap, offset group, mask group} of a unit
+    auto describe = [&](const UnitIter &u) {
+        const int chan0 = u.grp * g.csg + u.chunk * CHUNK_C;
+        return make_int4(chan0, u.batch * TB, g.og > 1 ? chan0 / g.cs_per_og : 0, g.mg > 1 ? chan0 / g.cs_per_mg : 0);
     };
     // offsets and mask of this position for the taps of one unit, as loaded (all loads in flight together)
     struct RawUnit {
         float off[TBM][DIM];
         float m[TBM];
     };
-    auto load_unit = [&](const PosInfo<DIM> &pi, int unit, RawUnit &ru) {
-        int t0, ogi, mgi;
-        unit_groups(unit, t0, ogi, mgi);
+    auto load_unit = [&](const PosInfo<DIM> &pi, const int4 &info, RawUnit &ru) {
+        const int t0 = info.y, ogi = info.z, mgi = info.w;
 #pragma unroll
         for (int t = 0; t < TBM; ++t) {
             const bool live = t < TB && t0 + t < g.K && pi.valid;
@@ -318,10 +360,9 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     };
 
     // combines the dot products of a finished unit into the coordinate gradients of its (position, tap)s
-    auto finalize = [&](const PosInfo<DIM> &pi, int pt, int unit, int pb, const RawUnit &ru) {
+    auto finalize = [&](const PosInfo<DIM> &pi, int pt, const int4 &info, int pb, const RawUnit &ru) {
         if (!want_coord || !pi.valid) return;
-        int t0, ogi, mgi;
-        unit_groups(unit, t0, ogi, mgi);
+        const int t0 = info.y, ogi = info.z, mgi = info.w;
         const float *dots = plan_dot(pb);
 #pragma unroll
         for (int t = 0; t < TBM; ++t) {
@@ -364,122 +405,111 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
 
 
     // ------------------------------------------------------------------ dense tile -> tensor memory
-    // Thread = position (its TMEM lane); the 16 store + gather warps split the channels in units of 16 (8 TMEM
-    // columns).
-    auto load_dense = [&]() {
-        const int q = warp & 3, part = warp >> 2;
-        const PosInfo<DIM> pa = decode_position<DIM>(g, m0 + q * 32 + lane);
+    // Thread = position (its TMEM lane); `loaders` warps per lane quarter split the channels in units of 16 (8 TMEM
+    // columns), this warp being number `part` of them.
+    auto load_dense = [&](const UnitIter &u, int part, int loaders, uint64_t *bar) {
+        constexpr int U = 2;                            // units (of 16 loads) in flight per thread
+        const int q = warp & 3;
+        const PosInfo<DIM> pa = decode_position<DIM>(g, (long long)u.x * TILE_POS + q * 32 + lane);
         const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
-        const int64_t base = ((int64_t)pa.b * g.Cd_r + (int64_t)grp * g.cdg_r) * g.P + pa.p;
-        // two units (32 loads) in flight per thread: the tile is read once from DRAM, its latency is what counts
+        const int64_t base = ((int64_t)pa.b * g.Cd_r + (int64_t)u.grp * g.cdg_r) * g.P + pa.p;
         const int n_units_a = g.cdg / 16;
-        for (int u0 = part; u0 < n_units_a; u0 += 2 * (SC_LOAD_WARPS / 4)) {
-            const int u1 = u0 + SC_LOAD_WARPS / 4;
-            const bool two = u1 < n_units_a;
-            // channels past the group's end (a group is padded to a multiple of 64) are zeros
-            const bool in0 = pa.valid && u0 * 16 + 16 <= g.cdg_r, in1 = pa.valid && two && u1 * 16 + 16 <= g.cdg_r;
-            const int part0 = pa.valid ? g.cdg_r - u0 * 16 : 0, part1 = pa.valid && two ? g.cdg_r - u1 * 16 : 0;
-            const bool ragged = (g.cdg_r & 15) != 0;   // a unit of 16 channels is partly inside
-            if constexpr (M::F32) {
-                const float *src0 = reinterpret_cast<const float *>(P.dense) + base + (int64_t)(u0 * 16) * g.P;
-                const float *src1 = reinterpret_cast<const float *>(P.dense) + base + (int64_t)(u1 * 16) * g.P;
-                float v[2][16];
+        using TD = typename std::conditional<M::F32, float, uint16_t>::type;
+        using TV = typename std::conditional<M::F32, float, uint32_t>::type;
+        const TD *dense = static_cast<const TD *>(P.dense) + base;
+        for (int u0 = part; u0 < n_units_a; u0 += U * loaders) {
+            TV v[U][16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[0][i] = in0 ? __ldg(src0 + (int64_t)i * g.P) : 0.f;
+            for (int h = 0; h < U; ++h) {
+                const int c0 = (u0 + h * loaders) * 16;
+                const int n = pa.valid ? g.cdg_r - c0 : 0;      // channels past the group's end are zeros
+                const TD *src = dense + (int64_t)c0 * g.P;
+                if (n >= 16) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[1][i] = in1 ? __ldg(src1 + (int64_t)i * g.P) : 0.f;
-                if (ragged) {
+                    for (int i = 0; i < 16; ++i) v[h][i] = (TV)__ldg(src + (int64_t)i * g.P);
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (!in0 && i < part0) v[0][i] = __ldg(src0 + (int64_t)i * g.P);
-                        if (!in1 && i < part1) v[1][i] = __ldg(src1 + (int64_t)i * g.P);
-                    }
+                    for (int i = 0; i < 16; ++i) v[h][i] = i < n ? (TV)__ldg(src + (int64_t)i * g.P) : (TV)0;
                 }
+            }
+            __syncwarp();                                       // tcgen05.st is a whole-warp instruction
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (h == 1 && !two) break;
-                    const int d0 = (h == 0 ? u0 : u1) * 16;
+            for (int h = 0; h < U; ++h) {
+                if (u0 + h * loaders >= n_units_a) break;
+                const uint32_t t_col = t_lane + (uint32_t)((u0 + h * loaders) * 8);
+                uint32_t part16[8];
+                if constexpr (M::F32) {
 #pragma unroll
-                    for (int q = 0; q < PARTS; ++q) {   // v keeps what the parts so far leave
-                        uint32_t part16[8];
+                    for (int k = 0; k < PARTS; ++k) {           // v keeps what the parts so far leave
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             part16[i] = pack2(v[h][2 * i], v[h][2 * i + 1], __nv_bfloat16());
                             v[h][2 * i] -= __uint_as_float(part16[i] << 16);
                             v[h][2 * i + 1] -= __uint_as_float(part16[i] & 0xffff0000u);
                         }
-                        ptx::tmem_st_32x8(t_lane + (uint32_t)(q * a_cols + d0 / 2), part16);
+                        ptx::tmem_st_32x8(t_col + (uint32_t)(k * a_cols), part16);
                     }
-                }
-            } else {
-                const uint16_t *src0 = reinterpret_cast<const uint16_t *>(P.dense) + base + (int64_t)(u0 * 16) * g.P;
-                const uint16_t *src1 = reinterpret_cast<const uint16_t *>(P.dense) + base + (int64_t)(u1 * 16) * g.P;
-                uint32_t v[2][16];
+                } else {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[0][i] = in0 ? (uint32_t)__ldg(src0 + (int64_t)i * g.P) : 0u;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[1][i] = in1 ? (uint32_t)__ldg(src1 + (int64_t)i * g.P) : 0u;
-                if (ragged) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (!in0 && i < part0) v[0][i] = (uint32_t)__ldg(src0 + (int64_t)i * g.P);
-                        if (!in1 && i < part1) v[1][i] = (uint32_t)__ldg(src1 + (int64_t)i * g.P);
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (h == 1 && !two) break;
-                    const int d0 = (h == 0 ? u0 : u1) * 16;
-                    uint32_t hi[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) hi[i] = v[h][2 * i] | (v[h][2 * i + 1] << 16);
-                    ptx::tmem_st_32x8(t_lane + (uint32_t)(d0 / 2), hi);
+                    for (int i = 0; i < 8; ++i) part16[i] = v[h][2 * i] | (v[h][2 * i + 1] << 16);
+                    ptx::tmem_st_32x8(t_col, part16);
                 }
             }
         }
         ptx::tmem_st_wait();
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(a_full);
-        if (threadIdx.x == 0) SC_PROF_OUT(1, SC_CLK() - clk_start);
+        if (lane == 0) ptx::mbar_arrive(bar);
     };
 
     if (warp < SC_WORK_WARPS) {
         if (warp < SC_STORE_WARPS) {
             // -------------------------------------------------------------- store warps: TMEM -> shared
-            load_dense();                      // with the launch allocation, before registers are handed over
+            load_dense(first_unit(P, unit0), warp >> 2, SC_LOAD_WARPS / 4, a_first);   // before registers are handed over
             ptx::reg_dec<SC_REGS_STORE>();
             const int q = warp;
             const int row = q * 32 + lane;
-            const PosInfo<DIM> pi = decode_position<DIM>(g, m0 + row);
             bool ok = true;
-            long long w_tfull = 0, w_cempty = 0, t_fin = 0;
+            // this thread's position in the tile of a plan buffer
+            auto position = [&](int pb) {
+                const int2 at = pos_of(pb)[row];
+                PosInfo<DIM> pi;
+                pi.valid = at.x >= 0;
+                pi.b = max(at.x, 0);
+                pi.p = at.y;
+                decode_in_image<DIM>(g, pi);
+                return pi;
+            };
+            auto wait_done = [&](int j) -> bool {
+                bool good = ptx::mbar_wait(&plan_done[j & 1], (uint32_t)((j >> 1) & 1));
+                good = __all_sync(0xffffffffu, good);
+                if (!good && lane == 0) ptx::report(P.status, 308);
+                return good;
+            };
             // The gather warps finish unit j (its dot products are complete) with pass 2 j + 1; the wait for that
             // pass' staging buffer below covers it, so the unit is turned into gradients right after the next store.
-            auto finish_unit = [&](int j, const RawUnit &ru) -> bool {
+            auto finish_unit = [&](int j, const PosInfo<DIM> &pi, const RawUnit &ru) -> bool {
                 const int pb = j & 1;
-                bool good = ptx::mbar_wait(&plan_done[pb], (uint32_t)((j >> 1) & 1));
-                good = __all_sync(0xffffffffu, good);
-                if (!good) {
-                    if (lane == 0) ptx::report(P.status, 308);
-                    return false;
-                }
-                finalize(pi, row, unit0 + j, pb, ru);
+                if (!wait_done(j)) return false;
+                finalize(pi, row, *info_of(pb), pb, ru);
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&fin_done[pb]);
                 return true;
             };
+            int aq = 0;
+            uint32_t t_phase = 0;
             for (int jp = 0; jp < n_pass && ok; ++jp) {
-                const int aq = jp % NACC, cb = jp & 1;
+                const int cb = jp & 1;
                 const bool fin_now = COORD && jp >= 3 && (jp & 1) == 1;   // pass jp - 2 closed unit (jp - 2) / 2
                 RawUnit ru_fin;
-                if (fin_now) load_unit(pi, unit0 + ((jp - 2) >> 1), ru_fin);
-                long long c0 = SC_CLK();
-                ok = ptx::mbar_wait(&t_full[aq], (uint32_t)((jp / NACC) & 1));
-                long long c1 = SC_CLK();
+                PosInfo<DIM> pi_fin;
+                if (fin_now) {     // (its plan is known here: the gather warps have released its first slab)
+                    const int pb = ((jp - 2) >> 1) & 1;
+                    pi_fin = position(pb);
+                    load_unit(pi_fin, *info_of(pb), ru_fin);
+                }
+                ok = ptx::mbar_wait(&t_full[aq], t_phase);
                 ok = ok && ptx::mbar_wait_backoff<SC_SLEEP_NS>(&col_empty[cb], (uint32_t)(((jp >> 1) & 1) ^ 1));
-                w_tfull += c1 - c0;
-                w_cempty += SC_CLK() - c1;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
                     if (lane == 0) ptx::report(P.status, 301);
@@ -520,26 +550,22 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     ptx::mbar_arrive(&t_empty[aq]);
                     ptx::mbar_arrive(&col_full[cb]);
                 }
-                if (fin_now) {
-                    long long c3 = SC_CLK();
-                    ok = finish_unit((jp - 2) >> 1, ru_fin);
-                    t_fin += SC_CLK() - c3;
+                if (++aq == NACC) {
+                    aq = 0;
+                    t_phase ^= 1u;
                 }
+                if (fin_now) ok = finish_unit((jp - 2) >> 1, pi_fin, ru_fin);
             }
-            if (COORD && ok) {   // the last unit
+            if (COORD && ok && wait_done(n_units - 1)) {   // the last unit
+                const int pb = (n_units - 1) & 1;
+                const PosInfo<DIM> pi_fin = position(pb);
                 RawUnit ru_fin;
-                load_unit(pi, unit0 + n_units - 1, ru_fin);
-                ok = finish_unit(n_units - 1, ru_fin);
-            }
-            if (threadIdx.x == 0) {
-                SC_PROF_OUT(2, w_tfull);
-                SC_PROF_OUT(3, w_cempty);
-                SC_PROF_OUT(4, SC_CLK() - clk_start);
-                SC_PROF_OUT(18, t_fin);
+                load_unit(pi_fin, *info_of(pb), ru_fin);
+                finish_unit(n_units - 1, pi_fin, ru_fin);
             }
         } else {
             // -------------------------------------------------------------- gather warps
-            if (warp < SC_LOAD_WARPS) load_dense();
+            if (warp < SC_LOAD_WARPS) load_dense(first_unit(P, unit0), warp >> 2, SC_LOAD_WARPS / 4, a_first);
             ptx::reg_inc<SC_REGS_WORK>();
             // An 8-lane group walks its span of the pixel-grouped entry list four entries at a time; lane l8 owns
             // channels 4 l8 .. 4 l8 + 3 of the slab.  The next four entries (and their image rows) are fetched
@@ -551,18 +577,10 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             const TI *img = reinterpret_cast<const TI *>(P.img_cl);
             const uint32_t zrow = (uint32_t)g.B * (uint32_t)g.S * (uint32_t)g.Cs;   // what padding entries point at
             bool ok = true;
-            long long w_plan = 0, w_col = 0, t_loop = 0, n_ent = 0;
             for (int jp = 0; jp < n_pass && ok; ++jp) {
                 const int j = jp >> 1, slab = jp & 1, pb = j & 1, cb = jp & 1;
-                const int unit = unit0 + j;
-                const int chunk = unit / P.nbatch;
-                long long c0 = SC_CLK();
                 if (slab == 0) ok = ptx::mbar_wait(&plan_full[pb], (uint32_t)((j >> 1) & 1));
-                long long c1 = SC_CLK();
                 ok = ok && ptx::mbar_wait(&col_full[cb], (uint32_t)((jp >> 1) & 1));
-                long long c2 = SC_CLK();
-                w_plan += c1 - c0;
-                w_col += c2 - c1;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
                     if (lane == 0) ptx::report(P.status, 306);
@@ -574,7 +592,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 const float4 *my_w = reinterpret_cast<const float4 *>(plan_w(pb) + gid * span);
                 float *p_dot = plan_dot(pb);
                 const float4 *colb = reinterpret_cast<const float4 *>(col + (size_t)cb * (L.col_buf / 4)) + l8;
-                const uint32_t chan = (uint32_t)(grp * g.csg + chunk * CHUNK_C + slab * SC_SLAB + l8 * 4);
+                const uint32_t chan = (uint32_t)(info_of(pb)->x + slab * SC_SLAB + l8 * 4);
                 const TI *img_c = img + chan;
                 float *gimg_c = P.img_grad_cl + chan;
 
@@ -666,15 +684,6 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     ptx::mbar_arrive(&col_empty[cb]);
                     if (slab == 1) ptx::mbar_arrive(&plan_done[pb]);
                 }
-                t_loop += SC_CLK() - c2;
-                n_ent += span;
-            }
-            if (threadIdx.x == SC_STORE_WARPS * 32) {
-                SC_PROF_OUT(8, w_plan);
-                SC_PROF_OUT(9, w_col);
-                SC_PROF_OUT(10, t_loop);
-                SC_PROF_OUT(11, n_ent);
-                SC_PROF_OUT(12, SC_CLK() - clk_start);
             }
         }
     } else if (warp < SC_MMA_WARP) {
@@ -682,7 +691,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         ptx::reg_inc<SC_REGS_WORK>();
         const int pt = threadIdx.x - SC_PLAN_WARP0 * 32;
         const int pw = warp - SC_PLAN_WARP0;
-        const PosInfo<DIM> pi = decode_position<DIM>(g, m0 + pt);
+        UnitIter u = first_unit(P, unit0);
+        PosInfo<DIM> pi = decode_position<DIM>(g, (long long)u.x * TILE_POS + pt);
         const uint32_t colq_row = (uint32_t)(pt * (L.col_stride / 4));
         const uint32_t zrow = (uint32_t)g.B * (uint32_t)g.S * (uint32_t)g.Cs;
 
@@ -694,19 +704,16 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             planner_barrier();
             return r;
         };
-        long long ph[6] = {0, 0, 0, 0, 0, 0};
-        auto build = [&](int unit, int pb, const RawUnit &ru) {
-            long long pc = SC_CLK();
-            auto phase = [&](int i) { const long long now = SC_CLK(); ph[i] += now - pc; pc = now; };
-            int t0, ogi, mgi;
-            unit_groups(unit, t0, ogi, mgi);
+        auto build = [&](const int4 &info, int pb, const RawUnit &ru) {
+            const int t0 = info.y;
+            if (pt == 0) *info_of(pb) = info;
+            pos_of(pb)[pt] = make_int2(pi.valid ? pi.b : -1, pi.p);
             {
                 uint4 *c4 = reinterpret_cast<uint4 *>(cnt);
 #pragma unroll
                 for (int i = 0; i < SC_SLOTS / 4 / 128; ++i) c4[pt + 128 * i] = make_uint4(0u, 0u, 0u, 0u);
             }
             planner_barrier();
-            phase(0);
             // pass 1: every entry's rank within its slot; all atomics of a thread are independent
             uint32_t rows[TBM * NC], rank[TBM * NC];
             float wts[TBM * NC];
@@ -727,9 +734,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
 #pragma unroll
             for (int i = 0; i < TBM * NC; ++i)
                 rank[i] = rows[i] != SC_NONE ? atomicAdd(&cnt[rows[i] & (SC_SLOTS - 1)], 1u) : 0u;
-            phase(1);
             planner_barrier();
-            phase(2);
             // exclusive prefix sum of the slot counts, in place (16 slots per thread)
             uint32_t total;
             {
@@ -768,7 +773,6 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             const uint32_t span = ((total + SC_GROUPS * 4 - 1) / (SC_GROUPS * 4)) * 4;
             if (pt == 0) n_entries[pb] = span;
             planner_barrier();
-            phase(3);
             // pass 2: every entry goes to (start of its slot) + (its rank)
             uint32_t *e_px = plan_px(pb);
             uint32_t *e_meta = plan_meta(pb);
@@ -794,64 +798,80 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 e_meta[i] = (uint32_t)L.max_entries << 16;
                 e_w[i] = 0.f;
             }
-            phase(4);
             planner_barrier();
-            phase(5);
             if (lane == 0) ptx::mbar_arrive(&plan_full[pb]);
         };
 
         bool ok = true;
-        long long w_done = 0, t_build = 0;
         // a plan buffer is free again once its unit's dots have been used (store warps), or, without coordinate
         // gradients, once the gather warps are through with it
         uint64_t *plan_free = COORD ? fin_done : plan_done;
         RawUnit ru, ru_next;
-        load_unit(pi, unit0, ru);
+        int4 info = describe(u);
+        load_unit(pi, info, ru);
         ru_next = ru;
+        bool new_tile = false;
         for (int j = 0; j < n_units && ok; ++j) {
             const int pb = j & 1;
-            // the next unit's offsets and mask travel while this unit is built
-            if (j + 1 < n_units) load_unit(pi, unit0 + j + 1, ru_next);
             if (j >= 2) {
-                long long c0 = SC_CLK();
                 ok = wait_all(&plan_free[pb], (uint32_t)(((j >> 1) & 1) ^ 1));
-                w_done += SC_CLK() - c0;
                 if (!ok) {
                     if (pt == 0) ptx::report(P.status, 307);
                     break;
                 }
             }
-            long long c2 = SC_CLK();
-            build(unit0 + j, pb, ru);
-            t_build += SC_CLK() - c2;
+            // the next unit's offsets and mask travel while this unit is built
+            UnitIter u_next = u;
+            const bool next_new = next_unit(P, u_next);
+            PosInfo<DIM> pi_next = pi;
+            if (next_new) pi_next = decode_position<DIM>(g, (long long)u_next.x * TILE_POS + pt);
+            const int4 info_next = describe(u_next);
+            if (j + 1 < n_units) load_unit(pi_next, info_next, ru_next);
+            build(info, pb, ru);
+            if (new_tile) {
+                // the dense tile is free once the MMAs of the pass before this unit are through; no pass behind it can
+                // complete before this load, so its phase is not missed
+                const int pass = 2 * j - 1;
+                ok = wait_all(&t_full[pass % NACC], (uint32_t)((pass / NACC) & 1));
+                if (!ok) {
+                    if (pt == 0) ptx::report(P.status, 309);
+                    break;
+                }
+                ptx::tc_fence_after();
+                load_dense(u, 0, 1, a_next);
+            }
             ru = ru_next;
-        }
-        if (pt == 0) {
-            SC_PROF_OUT(16, w_done);
-            SC_PROF_OUT(17, t_build);
-            SC_PROF_OUT(19, SC_CLK() - clk_start);
-            for (int i = 0; i < 6; ++i) SC_PROF_OUT(32 + i, ph[i]);
+            u = u_next;
+            pi = pi_next;
+            info = info_next;
+            new_tile = next_new;
         }
     } else if (warp == SC_MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
         ptx::reg_dec<SC_REGS_ISSUE>();
         if (lane == 0) {
             const uint32_t idesc = ptx::instr_desc_f16(M::HALF ? 0 : 1, TILE_POS, N, 0, 0);
-            bool ok = ptx::mbar_wait(a_full, 0);
-            if (!ok) ptx::report(P.status, 302);
-            ptx::tc_fence_after();
+            bool ok = true, new_tile = true;
+            UnitIter u = first_unit(P, unit0);
             // ring position and phase are stepped, never divided: a division by the run-time ring depth per stage
             // costs this single thread more than the stage's MMAs
             int s = 0, aq = 0;
-            uint32_t b_phase = 0, t_phase = 1;
+            uint32_t b_phase = 0, t_phase = 1, a_phase = 0;
             const uint64_t b_desc0 = ptx::smem_desc_sw128(ptx::smem_u32(sB), 16, 1024);
-            long long w_te = 0, w_bf = 0;
-            SC_PROF_OUT(24, SC_CLK() - clk_start);
             for (int jp = 0; jp < n_pass && ok; ++jp) {
-                long long c0 = SC_CLK();
-                const bool got = ptx::mbar_wait_backoff<SC_SLEEP_NS>(&t_empty[aq], t_phase);
-                w_te += SC_CLK() - c0;
-                if (!got) {
+                if ((jp & 1) == 0) {
+                    if (new_tile) {
+                        ok = jp == 0 ? ptx::mbar_wait(a_first, 0) : ptx::mbar_wait(a_next, a_phase);
+                        if (jp > 0) a_phase ^= 1u;
+                        if (!ok) {
+                            ptx::report(P.status, 302);
+                            break;
+                        }
+                        ptx::tc_fence_after();
+                    }
+                    new_tile = next_unit(P, u);
+                }
+                if (!ptx::mbar_wait_backoff<SC_SLEEP_NS>(&t_empty[aq], t_phase)) {
                     ptx::report(P.status, 303);
                     ok = false;
                     break;
@@ -862,10 +882,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 // a + b < PARTS (two parts: hi x hi, lo x hi; hi x lo)
                 for (int st = 0; st < RC * PARTS && ok; ++st) {
                     const int rc = st / PARTS, part = st % PARTS;
-                    long long c1 = SC_CLK();
-                    const bool gotb = ptx::mbar_wait(&b_full[s], b_phase);
-                    w_bf += SC_CLK() - c1;
-                    if (!gotb) {
+                    if (!ptx::mbar_wait(&b_full[s], b_phase)) {
                         ptx::report(P.status, 304);
                         ok = false;
                         break;
@@ -919,9 +936,6 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     t_phase ^= 1u;
                 }
             }
-            SC_PROF_OUT(25, w_te);
-            SC_PROF_OUT(26, w_bf);
-            SC_PROF_OUT(27, SC_CLK() - clk_start);
         }
         __syncwarp();
     } else if (warp == SC_TMA_WARP) {
@@ -931,11 +945,10 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             int s = 0, last_s = -1;
             uint32_t e_phase = 1, last_phase = 0;
             bool ok = true;
+            UnitIter u = first_unit(P, unit0);
             for (int jp = 0; jp < n_pass && ok; ++jp) {
-                const int unit = unit0 + (jp >> 1);
-                const int chunk = unit / P.nbatch;
-                const int t0 = (unit % P.nbatch) * TB;
-                const int s0 = chunk * CHUNK_C + (jp & 1) * SC_SLAB;
+                const int t0 = u.batch * TB, grp = u.grp;
+                const int s0 = u.chunk * CHUNK_C + (jp & 1) * SC_SLAB;
                 for (int st = 0; st < RC * PARTS; ++st) {
                     const int rc = st / PARTS, part = st % PARTS;
                     if (!ptx::mbar_wait_backoff<SC_SLEEP_NS>(&b_empty[s], e_phase)) {
@@ -954,6 +967,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     }
                 }
                 if (!ok) break;
+                if (jp & 1) next_unit(P, u);
             }
             // no copy may still be in flight when the CTA's shared memory is released
             if (last_s >= 0) ptx::mbar_wait(&b_full[last_s], last_phase);
@@ -966,7 +980,6 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == SC_MMA_WARP) ptx::tmem_dealloc(tmem_base, SC_TMEM_COLS);
-    if (threadIdx.x == 0) SC_PROF_OUT(0, SC_CLK() - clk_start);
 }
 
 size_t dgrad_smem_bytes(int dim, int mode, int tb, int b_stages) {
@@ -974,9 +987,13 @@ size_t dgrad_smem_bytes(int dim, int mode, int tb, int b_stages) {
 }
 
 template <int DIM, int MODE>
-cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, dim3 grid, const CUtensorMap *maps, cudaStream_t stream) {
+cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, cudaStream_t stream) {
     const size_t smem = dgrad_smem_bytes(DIM, MODE, P.tb, P.b_stages);
     const bool coord = P.goff != nullptr || P.gmask != nullptr;
+    // One CTA per SM, except for volumes of many tiles: 27 taps of 8 corners dwarf a CTA's start-up, and the tiles' costs
+    // differ so much that the hardware's scheduling beats equal ranges (4.19 against 4.36 ms).
+    const int tiles = P.total_units / P.n_units;
+    const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= 8 * 148 ? tiles : std::min(P.total_units, 148)));
     LaunchScope scope("dcn_dgrad_tc", stream);
     if (coord)
         return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, true>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
@@ -1026,23 +1043,9 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
         const uint32_t box[4] = {64, (uint32_t)SC_SLAB, (uint32_t)tb, 1};
         if (!make_part_maps(maps, w_parts, mode_mat_parts(mode), 4, dims, strides, box)) return cudaErrorInvalidValue;
     }
-    // Share each position tile between `splits` CTAs (equal ranges of its units) when that evens out the last
-    // wave: cost of a launch ~ ceil(CTAs / SMs) / splits tile-times; a split is taken only for a gain above 4 %
-    // (each extra CTA reloads the dense tile).
-    const long long tiles = ((BP + TILE_POS - 1) / TILE_POS) * h.groups;
-    const int n_units = (csg / CHUNK_C) * nbatch;
-    int splits = 1;
-    {
-        static const int forced = tuning_int("TVDCN_B200_DG_SPLITS", 0);
-        double best = (double)((tiles + 147) / 148);
-        for (int cand = 2; cand <= 4; ++cand) {
-            if (n_units % cand != 0) continue;
-            const double cost = (double)((tiles * cand + 147) / 148) / cand;
-            if (cost < best * 0.96) { best = cost; splits = cand; }
-        }
-        if (forced > 0 && n_units % forced == 0) splits = forced;
-    }
-    dim3 grid((unsigned)((BP + TILE_POS - 1) / TILE_POS), (unsigned)h.groups, (unsigned)splits);
+    const long long tiles_x = (BP + TILE_POS - 1) / TILE_POS;
+    const long long n_units = (long long)(csg / CHUNK_C) * nbatch, total = tiles_x * h.groups * n_units;
+    if (total > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     auto run = [&](auto dimc) -> cudaError_t {
         constexpr int DIM = decltype(dimc)::value;
         DgradParams<DIM> P;
@@ -1060,13 +1063,15 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
         P.nbatch = nbatch;
         P.nacc = nacc;
         P.b_stages = bs;
-        P.units_per_cta = n_units / splits;
+        P.tiles_x = (int)tiles_x;
+        P.n_units = (int)n_units;
+        P.total_units = (int)total;
         // 16-bit data: nothing is rounded between the MMA and the results, there is no wide mode of its own
         switch (mode) {
-            case TC_BF16: case TC_BF16_WIDE: return launch_dgrad_t<DIM, TC_BF16>(P, grid, maps, stream);
-            case TC_F16: case TC_F16_WIDE: return launch_dgrad_t<DIM, TC_F16>(P, grid, maps, stream);
-            case TC_SPLIT: return launch_dgrad_t<DIM, TC_SPLIT>(P, grid, maps, stream);
-            case TC_F32_WIDE: return launch_dgrad_t<DIM, TC_F32_WIDE>(P, grid, maps, stream);
+            case TC_BF16: case TC_BF16_WIDE: return launch_dgrad_t<DIM, TC_BF16>(P, maps, stream);
+            case TC_F16: case TC_F16_WIDE: return launch_dgrad_t<DIM, TC_F16>(P, maps, stream);
+            case TC_SPLIT: return launch_dgrad_t<DIM, TC_SPLIT>(P, maps, stream);
+            case TC_F32_WIDE: return launch_dgrad_t<DIM, TC_F32_WIDE>(P, maps, stream);
         }
         return cudaErrorInvalidValue;
     };
@@ -1075,16 +1080,5 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
     if (h.dim == 3) return run(std::integral_constant<int, 3>());
     return cudaErrorInvalidValue;
 }
-
-#ifdef TVDCN_B200_TUNING
-// tuning builds only: copies the cycle counters of the profiled CTA to the host
-extern "C" int tvdcn_b200_tuning_read_dgrad(long long *out, int n) {
-    long long host[64];
-    if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-    if (cudaMemcpyFromSymbol(host, g_dg_prof, sizeof(host)) != cudaSuccess) return -1;
-    for (int i = 0; i < n && i < 64; ++i) out[i] = host[i];
-    return 0;
-}
-#endif
 
 }  // namespace tvdcn_b200
