@@ -1,0 +1,61 @@
+"""Edges of how the tensor-core kernels share their work between CTAs: forward tiles that two CTAs sum together, CTAs that
+walk several tiles (the next dense tile is loaded under the old one), remainders of the split, volumes with one CTA per
+tile, and the line below which a padded transposed forward stays on the SIMT kernel."""
+import pytest
+import torch
+
+import cases
+from cases import Case, make_inputs, run_cabi, run_oracle
+from test_tensor_gpu import kernels_launched
+
+pytestmark = pytest.mark.gpu
+
+SPLITS = [
+    # one tile, long reduction: two CTAs share it
+    Case('one_long_tile', 2, False, 1, 256, 64, (9, 9), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 2, 1, True, 1.5),
+    # 150 tiles: two of them over a full wave, shared ranges with pieces at both ends of a CTA
+    Case('wave_plus_two', 2, False, 2, 128, 64, (98, 97), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+    # several tiles per CTA, two groups: tiles of one group follow those of the other
+    Case('many_tiles_groups', 2, False, 2, 128, 128, (120, 107), (3, 1), (1, 1), (1, 0), (1, 1), (), 2, 2, 1, True, 2.0),
+    # one tap and one chunk: a tile is a single unit everywhere
+    Case('single_units', 2, False, 1, 64, 64, (150, 141), (1, 1), (1, 1), (0, 0), (1, 1), (), 1, 1, 1, True, 1.0),
+    # dense channels that fill tensor memory (f32: one accumulator beside the dense tile)
+    Case('one_accumulator', 2, False, 1, 64, 384, (130, 150), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 0, True, 1.0),
+]
+
+
+@pytest.mark.parametrize('case', SPLITS, ids=[c.name for c in SPLITS])
+@pytest.mark.parametrize('dtype,tol', [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)], ids=['f32', 'bf16'])
+def test_split_work(case, dtype, tol):
+    x, w, off, mask, bias, go = make_inputs(case, seed=71)
+    # coordinates that f32 holds exactly: one that rounds across an integer has another derivative than in f64
+    off = (off * 64).round() / 64 + 1 / 128
+    q = lambda t, d: None if t is None else t.to(d)
+    dev = (q(x, dtype), q(w, dtype), q(off, torch.float32), q(mask, torch.float32), q(bias, torch.float32), q(go, dtype))
+    ref = run_oracle(case, *(None if t is None else t.double() for t in dev))
+    dev = [None if t is None else t.cuda() for t in dev]
+    got = run_cabi(case, *dev, engine=2)
+    cases.assert_parity(got, ref, tol, case.name)
+    # shared tiles are summed in a fixed order: the same call gives the same bits
+    assert torch.equal(got[0], run_cabi(case, *dev, engine=2)[0])
+    from tvdcn_b200 import cabi
+    assert cabi.lib().tvdcn_b200_device_status() == 0
+
+
+def test_volume_with_one_cta_per_tile():
+    """592 tiles and more of at least eight units: as many CTAs as tiles.  Too large for the CPU oracle, so the SIMT kernels,
+    which are checked against it elsewhere, stand in."""
+    case = Case('volume', 3, False, 2, 64, 64, (12, 57, 57), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0)
+    dev = [t.float().cuda() for t in make_inputs(case, seed=72)]
+    cases.assert_parity(run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1), 1e-4, case.name)
+
+
+@pytest.mark.parametrize('batch,simt', [(148, True), (149, False)], ids=['one_wave', 'more'])
+def test_small_padded_transposed_forward_stays_simt(batch, simt):
+    case = Case('tiny_T', 1, True, batch, 8, 16, (64,), (4,), (2,), (1,), (1,), (), 1, 1, 1, True, 1.5)
+    dev = [t.float() for t in make_inputs(case, seed=73)]
+    ref = run_oracle(case, *(t.double() for t in dev))
+    dev = [t.cuda() for t in dev]
+    names, got = kernels_launched(lambda: run_cabi(case, *dev))
+    assert (names.get('gemm_scatter', 0) == 1) == simt, names
+    cases.assert_parity(got, ref, 1e-5, case.name)

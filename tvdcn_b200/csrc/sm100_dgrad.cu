@@ -993,7 +993,7 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, c
     // One CTA per SM, except for volumes of many tiles: 27 taps of 8 corners dwarf a CTA's start-up, and the tiles' costs
     // differ so much that the hardware's scheduling beats equal ranges (4.19 against 4.36 ms).
     const int tiles = P.total_units / P.n_units;
-    const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= 8 * 148 ? tiles : std::min(P.total_units, 148)));
+    const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= 4 * 148 ? tiles : std::min(P.total_units, 148)));
     LaunchScope scope("dcn_dgrad_tc", stream);
     if (coord)
         return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, true>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
