@@ -662,12 +662,13 @@ static bool fwd_work(const GeoHost &h, int bn, FwdWork *w) {
     w->n_tiles = (int)(tiles_x * tiles_y);
     w->tiles_y = (int)tiles_y;
     // Sharing tiles evens out the last wave, or spreads few tiles over the chip: each SM then takes units / SMs chunks
-    // instead of whole tiles.  A shared tile costs the time of about eight chunks (its sums go through the workspace); the
-    // fewer pieces the better, so few tiles are shared by two CTAs each.
+    // instead of whole tiles.  A shared tile costs the time of about eight chunks, sixteen with 256 dense channels (its sums
+    // go through the workspace: 15 tiles of 27 chunks took 48 us shared, 30 whole); the fewer pieces the better, so few
+    // tiles are shared by two CTAs each.
     const long long sms = 148;
     const long long shared = std::min(sms, std::min(units / 3, 2LL * w->n_tiles));
     const long long whole_time = (w->n_tiles + sms - 1) / sms * w->n_chunks;
-    w->whole = w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + 8;
+    w->whole = w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + (bn > 128 ? 16 : 8);
     w->ctas = (int)(w->whole ? std::min<long long>(sms, w->n_tiles) : shared);
     const long long items = w->whole ? w->n_tiles : units;
     w->base = (int)(items / w->ctas);
