@@ -92,8 +92,10 @@ typedef struct tvdcn_problem {
  * call for the same problem and the same `input` tensor ran with last, and nothing has written to it or to `input`
  * since.  The backward call then reuses the forward call's channels-last staging of `input` (it sits at the start of
  * both workspaces) instead of staging it again.  (No counterpart in the reference, which re-reads its inputs.)
- * The caller vouches for all of that; with the flag clear the backward call stages the input itself.
- * Ignored where no staging exists (SIMT kernels, transposed operator).
+ * The caller vouches for all of that, and for passing both calls the same workspace_bytes; with the flag clear the
+ * backward call stages the input itself.
+ * Ignored where no staging exists (SIMT kernels, a forward call that took them because its workspace was too small
+ * for the tensor-core kernels, transposed operator).
  */
 #define TVDCN_FLAG_REUSE_STAGED_INPUT 1
 

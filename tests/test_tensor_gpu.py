@@ -176,6 +176,32 @@ def test_backward_reuses_the_forward_staging(dtype):
     assert L.tvdcn_b200_device_status() == 0
 
 
+def test_reuse_flag_after_a_forward_that_fell_back_to_simt():
+    """A padded shape whose forward call gets too little workspace runs on the SIMT kernels and stages nothing.  The
+    same workspace is enough for the weight gradient alone: with TVDCN_FLAG_REUSE_STAGED_INPUT that call must stage
+    the input itself instead of reading what the workspace happened to hold."""
+    from tvdcn_b200 import cabi
+    L = cabi.lib()
+    case = Case('reuse_simt', 2, False, 2, 40, 8, (20, 20), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5)
+    x, w, off, mask, bias, go = (t.float().cuda() for t in make_inputs(case, seed=6))
+    p = cases.cabi_problem(case, torch.float32)
+    p.flags = cabi.FLAG_REUSE_STAGED_INPUT
+    whole = L.tvdcn_b200_forward_workspace_bytes(ctypes.byref(p))
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    ws = torch.full((whole,), 0xff, dtype=torch.uint8, device='cuda')     # f32 NaN everywhere
+    n = whole - 256
+    out, gw = torch.full_like(go, float('nan')), torch.full_like(w, float('nan'))
+    names, _ = kernels_launched(lambda: cabi.check(L.tvdcn_b200_deform_conv_forward(
+        ctypes.byref(p), vp(x), vp(w), vp(off), vp(mask), vp(bias), vp(out), vp(ws), n, st)))
+    assert names == {'sample_gemm': 1}, names
+    names, _ = kernels_launched(lambda: cabi.check(L.tvdcn_b200_deform_conv_backward(
+        ctypes.byref(p), vp(go), vp(x), vp(w), vp(off), vp(mask), None, vp(gw), None, None, None, vp(ws), n, st)))
+    assert names.get('dcn_wgrad_tc', 0) == 1, names
+    ref = run_oracle(case, *(t.double().cpu() for t in (x, w, off, mask, bias, go)))
+    assert nerr(out, ref[0]) <= 1e-5 and nerr(gw, ref[2]) <= 1e-5
+
+
 def test_misaligned_16bit_grad_output_still_computes():
     """A contiguous bf16 grad_output whose storage offset leaves it off a 16-byte boundary cannot be read by TMA:
     the weight gradient must fall back to the SIMT kernel instead of failing the whole backward call."""

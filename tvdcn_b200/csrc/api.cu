@@ -496,11 +496,12 @@ int tvdcn_b200_deform_conv_backward_ex(const tvdcn_problem *p, const void *grad_
     TcCall tc(p, g, pl, ws);
     if (pl.tensor) {
         // The caller may vouch that the forward call's staging of `input` is still at the start of this workspace
-        // (only where the forward call for this problem stages the image at all, and at the same offset).
+        // (only where the forward call for this problem stages the image at all, and at the same offset: with a workspace
+        // too small for its plan, which may still do for this call's, it ran on the SIMT kernels and staged nothing).
         bool staged = false;
         if ((p->flags & TVDCN_FLAG_REUSE_STAGED_INPUT) && !p->transposed) {
-            const Plan fwd = plan_forward(p);
-            staged = fwd.img_cl != NO_BUF && fwd.img_cl == pl.img_cl;
+            const Plan fwd = plan_for(p, workspace_bytes, [](const tvdcn_problem *q) { return plan_forward(q); });
+            staged = fwd.img_cl != NO_BUF && fwd.img_cl == pl.img_cl && fwd.total <= workspace_bytes;
         }
         if (!staged && (pl.tc_sg || tc_sw || goff_acc || gmask_acc)) tc.stage_image(img);
         if (pl.tc_gs) tc.stage_weight(weight, true);
