@@ -139,14 +139,18 @@ int tvdcn_b200_deform_conv_forward(const tvdcn_problem *p,
  * tvdcn_b200_static_scratch_bytes() bytes (16 MiB) of device memory that every GPU which loads the library
  * holds until the process exits.  It calls no cudaMalloc / cudaFree and no allocating library routine.
  *
- *  - A problem whose forward workspace (tvdcn_b200_forward_workspace_bytes) exceeds that size is refused with
- *    TVDCN_ERR_WORKSPACE and a message that names both sizes; nothing is launched.
+ *  - The call is planned for that size: tiles that several CTAs would sum together through the workspace have one CTA
+ *    each, and shapes that the tensor-core kernels take only with padding run on the SIMT kernels, where the larger
+ *    plan does not fit.  So problems whose tvdcn_b200_forward_workspace_bytes exceeds the scratch may still run; one
+ *    that fits in no plan is refused with TVDCN_ERR_WORKSPACE and a message that names both sizes, and nothing is
+ *    launched.
  *  - The first call on each device looks up the array's device address (cudaGetSymbolAddress, with that
  *    device current).  Make that first call outside any stream capture.
  *  - All calls share the one array, and it keeps whatever the previous call left there.  The kernels
  *    rewrite everything they read from it, so consecutive calls on one stream are independent; two calls that
  *    overlap on the GPU (different streams, different threads) race on it and corrupt each other.
- *  - Results are those of tvdcn_b200_deform_conv_forward for the same problem.
+ *  - Results are those of tvdcn_b200_deform_conv_forward for the same problem, to the rounding of another order of
+ *    summation where the plans differ.
  */
 int tvdcn_b200_deform_conv_forward_static(const tvdcn_problem *p,
                                           const void *input, const void *weight,

@@ -16,6 +16,7 @@ import torch
 
 import cases
 from cases import Case, make_inputs, nerr, run_oracle
+from test_tensor_gpu import kernels_launched
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +84,30 @@ def test_static_forward_refuses_problems_larger_than_its_scratch():
     assert rc == 3  # TVDCN_ERR_WORKSPACE, before anything is launched
     msg = L.tvdcn_b200_last_error().decode()
     assert 'scratch' in msg and str(L.tvdcn_b200_static_scratch_bytes()) in msg
+
+
+@pytest.mark.parametrize('case,dtype,kernel,tol', [
+    # padded to 64 channels the image alone takes 20 MiB: the SIMT kernel, which needs nothing
+    (Case('padded', 2, False, 20, 40, 72, (64, 64), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+     torch.float32, 'sample_gemm', 1e-5),
+    # one CTA per tile: 4.4 MiB instead of the 31 MiB with the partial sums of shared tiles
+    (Case('shared_tiles', 2, False, 1, 256, 256, (67, 101), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+     torch.bfloat16, 'dcn_fwd_tc', 2e-2),
+], ids=['padded', 'shared_tiles'])
+def test_static_forward_plans_for_its_scratch(case, dtype, kernel, tol):
+    """Problems whose ordinary plan exceeds the scratch run on a plan that fits."""
+    cabi, L = _lib()
+    x, w, off, mask, bias, go = make_inputs(case, seed=74, dtype=torch.float32)
+    dev = [x.to(dtype).cuda(), w.to(dtype).cuda(), off.cuda(), mask.cuda(), bias.cuda()]
+    p = cases.cabi_problem(case, dtype, torch.float32)
+    assert L.tvdcn_b200_forward_workspace_bytes(ctypes.byref(p)) > L.tvdcn_b200_static_scratch_bytes()
+    out = torch.full(go.shape, float('nan'), dtype=dtype, device='cuda')
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    names, _ = kernels_launched(lambda: cabi.check(L.tvdcn_b200_deform_conv_forward_static(
+        ctypes.byref(p), *map(vp, dev), vp(out), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))))
+    assert names.get(kernel, 0) == 1, names
+    assert L.tvdcn_b200_device_status() == 0
+    from oracle import restate
+    args = [t.double().cpu() for t in dev]
+    ref = restate.deform_conv(*args, case.stride, case.padding, case.dilation, case.groups)
+    assert nerr(out, ref) <= tol

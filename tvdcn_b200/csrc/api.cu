@@ -343,26 +343,19 @@ static int check_ws(const Plan &pl, void *ws, size_t bytes) {
     return TVDCN_OK;
 }
 
-int tvdcn_b200_deform_conv_forward(const tvdcn_problem *p, const void *input, const void *weight,
-                                   const void *offset, const void *mask, const void *bias, void *output,
-                                   void *workspace, size_t workspace_bytes, void *cuda_stream) {
-    int rc = check_problem(p);
-    if (rc) return rc;
-    rc = check_sizes(p);
-    if (rc) return rc;
-    if (p->batch == 0) return TVDCN_OK;  // nothing to compute; empty tensors may have NULL storage
+static int check_forward_args(const tvdcn_problem *p, const void *input, const void *weight, const void *offset,
+                              const void *mask, const void *output) {
     if (input == nullptr || weight == nullptr || output == nullptr)
         return fail(TVDCN_ERR_INVALID, "input, weight and output must not be NULL");
     if ((p->offset_groups > 0) != (offset != nullptr))
         return fail(TVDCN_ERR_INVALID, "offset pointer and offset_groups disagree");
     if ((p->mask_groups > 0) != (mask != nullptr))
         return fail(TVDCN_ERR_INVALID, "mask pointer and mask_groups disagree");
-    cudaStream_t stream = (cudaStream_t)cuda_stream;
-    const Plan pl = plan_for(p, workspace_bytes, [](const tvdcn_problem *q) { return plan_forward(q); });
-    if (p->engine == TVDCN_ENGINE_TENSOR && !pl.tensor)
-        return fail(TVDCN_ERR_UNSUPPORTED, "shape not covered by the tensor-core kernels: %s", pl.why_not);
-    rc = check_ws(pl, workspace, workspace_bytes);
-    if (rc) return rc;
+    return TVDCN_OK;
+}
+
+static int run_forward(const tvdcn_problem *p, const Plan &pl, const void *input, const void *weight, const void *offset,
+                       const void *mask, const void *bias, void *output, void *workspace, cudaStream_t stream) {
     char *ws = (char *)workspace;
     const GeoHost g = make_geo_host(p);
     const int dt = p->dtype, aux = p->aux_dtype;
@@ -393,6 +386,24 @@ int tvdcn_b200_deform_conv_forward(const tvdcn_problem *p, const void *input, co
     CUDA_TRY(launch_gemm_scatter(g, dt, aux, input, weight, offset, mask, nullptr, acc, nullptr, nullptr, stream));
     if (pl.img_acc != NO_BUF) CUDA_TRY(launch_cast_from_acc(dt, acc, output, n_out, stream));
     return TVDCN_OK;
+}
+
+int tvdcn_b200_deform_conv_forward(const tvdcn_problem *p, const void *input, const void *weight,
+                                   const void *offset, const void *mask, const void *bias, void *output,
+                                   void *workspace, size_t workspace_bytes, void *cuda_stream) {
+    int rc = check_problem(p);
+    if (rc) return rc;
+    rc = check_sizes(p);
+    if (rc) return rc;
+    if (p->batch == 0) return TVDCN_OK;  // nothing to compute; empty tensors may have NULL storage
+    rc = check_forward_args(p, input, weight, offset, mask, output);
+    if (rc) return rc;
+    const Plan pl = plan_for(p, workspace_bytes, [](const tvdcn_problem *q) { return plan_forward(q); });
+    if (p->engine == TVDCN_ENGINE_TENSOR && !pl.tensor)
+        return fail(TVDCN_ERR_UNSUPPORTED, "shape not covered by the tensor-core kernels: %s", pl.why_not);
+    rc = check_ws(pl, workspace, workspace_bytes);
+    if (rc) return rc;
+    return run_forward(p, pl, input, weight, offset, mask, bias, output, workspace, (cudaStream_t)cuda_stream);
 }
 
 // Side stream of the backward pass: the scatter kernel does not depend on the weight-gradient kernel and the bias sum,
@@ -722,20 +733,29 @@ int tvdcn_b200_deform_conv_forward_static(const tvdcn_problem *p, const void *in
     if (rc) return rc;
     rc = check_sizes(p);
     if (rc) return rc;
-    const size_t need = plan_forward(p).total;
-    if (need > TVDCN_STATIC_SCRATCH_BYTES)
+    if (p->batch == 0) return TVDCN_OK;
+    rc = check_forward_args(p, input, weight, offset, mask, output);
+    if (rc) return rc;
+    // The plan is made for the scratch there is: without shared tiles where their partial sums do not fit, and on the
+    // SIMT kernels where a padded shape does not fit at all.
+    Plan pl = plan_forward(p);
+    if (pl.total > TVDCN_STATIC_SCRATCH_BYTES)
+        pl = plan_for(p, TVDCN_STATIC_SCRATCH_BYTES, [](const tvdcn_problem *q) { return plan_forward(q, false); });
+    if (p->engine == TVDCN_ENGINE_TENSOR && !pl.tensor)
+        return fail(TVDCN_ERR_UNSUPPORTED, "shape not covered by the tensor-core kernels: %s", pl.why_not);
+    if (pl.total > TVDCN_STATIC_SCRATCH_BYTES)
         return fail(TVDCN_ERR_WORKSPACE,
                     "this problem needs %zu bytes of scratch, more than the %u bytes built into the library; use "
                     "tvdcn_b200_deform_conv_forward with a workspace of your own",
-                    need, (unsigned)TVDCN_STATIC_SCRATCH_BYTES);
+                    pl.total, (unsigned)TVDCN_STATIC_SCRATCH_BYTES);
     void *scratch = nullptr;
-    if (need > 0) {
+    if (pl.total > 0) {
         const cudaError_t e = static_scratch_address(&scratch);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(static scratch)");
     }
     // The forward kernels overwrite every scratch byte they later read (staged image, packed weights) and
     // zero the scatter accumulator themselves, so nothing left by an earlier call can leak into this one.
-    return tvdcn_b200_deform_conv_forward(p, input, weight, offset, mask, bias, output, scratch, need, cuda_stream);
+    return run_forward(p, pl, input, weight, offset, mask, bias, output, scratch, (cudaStream_t)cuda_stream);
 }
 
 }  // extern "C"

@@ -69,9 +69,10 @@ void take_aux(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool 
     if (bias) pl.bias32 = b.take((size_t)p->out_channels * sizeof(float));
 }
 
-// buffers of the sample -> GEMM kernel besides the staged image
-void take_sample_buffers(Plan &pl, Bump &b, const GeoHost &g, int bn) {
+// buffers of the sample -> GEMM kernel besides the staged image (no partial sums: no tile is shared)
+void take_sample_buffers(Plan &pl, Bump &b, const GeoHost &g, int bn, bool share_tiles) {
     take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
+    if (!share_tiles) return;
     size_t partial = 0;
     fwd_tc_workspace(g, bn, &partial, &pl.sg_counters);
     if (partial > 0) {
@@ -102,7 +103,7 @@ GeoHost tc_geometry(const GeoHost &g) {
     return t;
 }
 
-Plan plan_forward(const tvdcn_problem *p) {
+Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
     Plan pl;
     const GeoHost g = tc_geometry(make_geo_host(p));
     Bump b;
@@ -115,7 +116,7 @@ Plan plan_forward(const tvdcn_problem *p) {
         if (fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &bn, &st) && chain_ok(pl.mode, g, bn)) {
             pl.tensor = pl.tc_sg = true;
             pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);   // + one row of zeros
-            take_sample_buffers(pl, b, g, bn);
+            take_sample_buffers(pl, b, g, bn, share_tiles);
             take_aux(pl, b, p, g, true);
         } else {
             why = "no tile configuration fits (or the f32 accumulation chain would be too long)";
@@ -171,7 +172,7 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
             pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);
             take_aux(pl, b, p, g, false);
         }
-        if (pl.tc_sg) take_sample_buffers(pl, b, g, sg_bn);
+        if (pl.tc_sg) take_sample_buffers(pl, b, g, sg_bn, true);
         if (pl.tc_sw) {
             // f32 data is split into 16-bit parts; 16-bit rows are copied only where TMA cannot read them
             pl.dense_pitch = round_up(g.P, 8);

@@ -39,7 +39,8 @@ struct Plan {
 
 inline size_t align_up(size_t v, size_t a = 256) { return (v + a - 1) / a * a; }
 
-Plan plan_forward(const tvdcn_problem *p);
+// share_tiles: sample -> GEMM tiles may be shared between CTAs, whose partial sums then take up to 39 MB of workspace
+Plan plan_forward(const tvdcn_problem *p, bool share_tiles = true);
 Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bool want_offset, bool want_mask);
 
 GeoHost make_geo_host(const tvdcn_problem *p);
@@ -97,7 +98,7 @@ bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages);
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
                                   const float *offset, const float *mask, const float *bias, void *out, float *partial,
                                   unsigned *arrived, const Status &status, cudaStream_t stream);
-void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters);
+void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters);   // partial sums of shared tiles
 bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages);
 cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch, const void *img_cl,
                                    const float *offset, const float *mask, float *gw, const Status &status,

@@ -654,7 +654,7 @@ cudaError_t launch_fwd_tc_t(const GeoHost &h, const FwdParams<DIM> &P, const CUt
                                                           maps[1], maps[2]);
 }
 
-static bool fwd_work(const GeoHost &h, int bn, FwdWork *w) {
+static bool fwd_work(const GeoHost &h, int bn, bool may_share, FwdWork *w) {
     const long long tiles_x = ((long long)h.B * h.P + TILE_POS - 1) / TILE_POS, tiles_y = h.groups * ((h.Cd / h.groups) / bn);
     w->n_chunks = h.K * (h.Cs / h.groups / CHUNK_C);
     const long long units = tiles_x * tiles_y * w->n_chunks;
@@ -668,7 +668,7 @@ static bool fwd_work(const GeoHost &h, int bn, FwdWork *w) {
     const long long sms = 148;
     const long long shared = std::min(sms, std::min(units / 3, 2LL * w->n_tiles));
     const long long whole_time = (w->n_tiles + sms - 1) / sms * w->n_chunks;
-    w->whole = w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + (bn > 128 ? 16 : 8);
+    w->whole = !may_share || w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + (bn > 128 ? 16 : 8);
     w->ctas = (int)(w->whole ? std::min<long long>(sms, w->n_tiles) : shared);
     const long long items = w->whole ? w->n_tiles : units;
     w->base = (int)(items / w->ctas);
@@ -680,13 +680,13 @@ static bool fwd_work(const GeoHost &h, int bn, FwdWork *w) {
 void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters) {
     FwdWork w;
     *partial_bytes = *counters = 0;
-    if (!fwd_work(h, bn, &w) || w.whole) return;
+    if (!fwd_work(h, bn, true, &w) || w.whole) return;
     *partial_bytes = (size_t)w.ctas * 2 * bn * TILE_POS * sizeof(float);
     *counters = (size_t)w.n_tiles;
 }
 
 // img_cl: channels-last sampled image in the problem's data type; w_parts: weights packed [g][tap][d'][s'], one
-// 16-bit tensor per part of the mode; h: padded geometry; partial / arrived: see fwd_tc_workspace, arrived zeroed.
+// 16-bit tensor per part of the mode; h: padded geometry; partial / arrived: see fwd_tc_workspace, arrived zeroed (partial null: every tile has one CTA).
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
                                   const float *offset, const float *mask, const float *bias, void *out, float *partial,
                                   unsigned *arrived, const Status &status, cudaStream_t stream) {
@@ -694,7 +694,7 @@ cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl
     int bn = 0, stages = 0;
     if (!fwd_tc_config(h.dim, mode, cdg, &bn, &stages)) return cudaErrorInvalidConfiguration;
     FwdWork work;
-    if (!fwd_work(h, bn, &work) || (!work.whole && partial == nullptr)) return cudaErrorInvalidConfiguration;
+    if (!fwd_work(h, bn, partial != nullptr, &work)) return cudaErrorInvalidConfiguration;
     CUtensorMap maps[3];
     const uint64_t dims[4] = {(uint64_t)csg, (uint64_t)cdg, (uint64_t)h.K, (uint64_t)h.groups};
     const uint64_t strides[3] = {(uint64_t)csg * 2, (uint64_t)csg * cdg * 2, (uint64_t)csg * cdg * h.K * 2};
