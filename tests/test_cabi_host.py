@@ -88,6 +88,39 @@ def test_workspace_sizes():
     assert L.tvdcn_b200_engine_name(ctypes.byref(p32), 0).decode() == 'simt'
 
 
+def test_problems_too_large_for_the_tensor_kernels_are_planned_on_the_simt_ones():
+    """The tensor-core launchers count their work in 32 bits and their grids in 16: a plan must not choose them beyond."""
+    L = cabi.lib()
+
+    def engine(*args, **kw):
+        return L.tvdcn_b200_engine_name(ctypes.byref(cabi.make_problem(*args, **kw)), 0).decode()
+    # sample -> GEMM: 129604 position tiles x (channels / 256) x 512 taps
+    conv = lambda cout: engine(2, False, cabi.BF16, 1, 64, cout, (4096, 4096), (16, 32), (1, 1), (0, 0), (1, 1), 1, 0, 0,
+                               aux_dtype=cabi.F32)
+    assert conv(8192) == 'tcgen05' and conv(8448) == 'simt'
+    # GEMM -> scatter: 131072 position tiles x (channels / 64) x 128 batches of four taps
+    transposed = lambda cout: engine(1, True, cabi.BF16, 1, 64, cout, (1 << 24,), (512,), (1,), ((1 << 23) - 50000,), (1,), 1,
+                                     0, 0, aux_dtype=cabi.F32)
+    assert transposed(8128) == 'tcgen05' and transposed(8192) == 'simt'
+
+    # weight gradient: a split for every 42 chunks of one image each, at most 65535; the 16-bit parts of grad_output, 3 KB
+    # per image, are what the workspace no longer holds
+    def backward_bytes(batch):
+        p = cabi.make_problem(2, False, cabi.F32, batch, 64, 64, (1, 1), (1, 1), (1, 1), (0, 0), (1, 1), 1, 0, 0)
+        return L.tvdcn_b200_backward_workspace_bytes(ctypes.byref(p))
+    assert backward_bytes(2_700_000) > 2_700_000 * 3072 and backward_bytes(3_000_000) < 3_000_000 * 3072
+
+
+@pytest.mark.parametrize('transposed', [False, True])
+@pytest.mark.parametrize('dtype', [cabi.F32, cabi.BF16])
+def test_workspace_sizes_of_an_empty_batch(transposed, dtype):
+    L = cabi.lib()
+    p = cabi.make_problem(2, transposed, dtype, 0, 64, 64, (8, 8), (3, 3), (1, 1), (1, 1), (1, 1), 1, 1, 1)
+    one = cabi.make_problem(2, transposed, dtype, 1, 64, 64, (8, 8), (3, 3), (1, 1), (1, 1), (1, 1), 1, 1, 1)
+    for size in (L.tvdcn_b200_forward_workspace_bytes, L.tvdcn_b200_backward_workspace_bytes):
+        assert 0 <= size(ctypes.byref(p)) < size(ctypes.byref(one))
+
+
 def test_null_pointer_is_an_error_not_a_crash():
     L = cabi.lib()
     p = cabi.make_problem(2, False, cabi.F32, 2, 8, 8, (8, 8), (3, 3), (1, 1), (1, 1), (1, 1), 1, 0, 0)

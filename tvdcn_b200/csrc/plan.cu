@@ -113,13 +113,13 @@ Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
     const size_t es = p->dtype == TVDCN_F32 ? 4 : 2;
     int bn = 0, st = 0, gbufs = 0;
     if (why == nullptr && !p->transposed) {
-        if (fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &bn, &st) && chain_ok(pl.mode, g, bn)) {
+        if (fwd_tc_config(g, pl.mode, &bn, &st) && chain_ok(pl.mode, g, bn)) {
             pl.tensor = pl.tc_sg = true;
             pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);   // + one row of zeros
             take_sample_buffers(pl, b, g, bn, share_tiles);
             take_aux(pl, b, p, g, true);
         } else {
-            why = "no tile configuration fits (or the f32 accumulation chain would be too long)";
+            why = "no tile configuration fits (or too many work units, or too long an f32 accumulation chain)";
         }
     } else if (why == nullptr) {
         // One wave of SIMT blocks with one or two reduction steps is through before the three kernels of the tensor path
@@ -127,12 +127,12 @@ Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
         const long long simt_blocks = ((long long)g.B * g.P + 63) / 64 * g.groups * (((long long)g.Cs_r / g.groups * g.K + 63) / 64);
         if (pl.wide && p->engine == TVDCN_ENGINE_AUTO && g.Cd_r / g.groups <= 32 && simt_blocks <= 148) {
             why = "so small that the SIMT kernel is faster";
-        } else if (dgrad_tc_config(g.dim, pl.mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st)) {
+        } else if (dgrad_tc_config(g, pl.mode, &bn, &gbufs, &st)) {
             pl.tensor = pl.tc_gs = true;
             take_scatter_buffers(pl, b, g, true);
             take_aux(pl, b, p, g, true);
         } else {
-            why = "no tile configuration fits";
+            why = "no tile configuration fits (or too many work units)";
         }
     }
     if (why != nullptr) {
@@ -158,13 +158,13 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
         int bn = 0, sg_bn = 0, st = 0, ns = 0, mt = 0, gbufs = 0;
         // which primitives run on the tensor cores
         // transposed backward: grad_input is a sample -> GEMM over grad_output
-        pl.tc_sg = p->transposed && want_input && fwd_tc_config(g.dim, pl.mode, g.Cd / g.groups, &sg_bn, &st) &&
+        pl.tc_sg = p->transposed && want_input && fwd_tc_config(g, pl.mode, &sg_bn, &st) &&
                    chain_ok(pl.mode, g, sg_bn);
-        pl.tc_sw = want_weight && wgrad_tc_config(g.dim, pl.mode_sw, g.Cd_r / g.groups, &ns, &mt, &st);
+        pl.tc_sw = want_weight && wgrad_tc_config(g, pl.mode_sw, &ns, &mt, &st);
         // conv: scatter into grad_input + coordinate gradients; transposed: coordinate gradients only
         const bool scatter = !p->transposed && want_input;
         pl.tc_gs = (scatter || want_offset || want_mask) &&
-                   dgrad_tc_config(g.dim, pl.mode, g.Cd / g.groups, g.K, &bn, &gbufs, &st);
+                   dgrad_tc_config(g, pl.mode, &bn, &gbufs, &st);
         pl.tensor = pl.tc_sg || pl.tc_sw || pl.tc_gs;
         // The staged image comes first, as in the forward plan: a backward call that is told to reuse the
         // forward call's staging (TVDCN_FLAG_REUSE_STAGED_INPUT) finds it at the same offset of the same workspace.

@@ -94,16 +94,17 @@ cudaError_t launch_dense_pass(const void *src, int dtype, int n_parts, void *con
                               float *partial, unsigned *done, void *sum_out, int sum_dtype, cudaStream_t stream);
 
 // ---- tensor-core kernels (sm100_*.cu); all take the padded geometry ---------------------------------------
-bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages);
+// A configuration is returned for every problem that the launcher below it takes, and for no other.
+bool fwd_tc_config(const GeoHost &h, int mode, int *bn, int *stages);
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
                                   const float *offset, const float *mask, const float *bias, void *out, float *partial,
                                   unsigned *arrived, const Status &status, cudaStream_t stream);
 void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters);   // partial sums of shared tiles
-bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages);
+bool wgrad_tc_config(const GeoHost &h, int mode, int *n_sub, int *m_tiles, int *stages);
 cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch, const void *img_cl,
                                    const float *offset, const float *mask, float *gw, const Status &status,
                                    cudaStream_t stream);
-bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int *b_stages);
+bool dgrad_tc_config(const GeoHost &h, int mode, int *tb, int *nacc, int *b_stages);
 cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense, void *const *w_parts,
                                    const void *img_cl, const float *offset, const float *mask, float *img_grad_cl,
                                    float *goff, float *gmask, const Status &status, cudaStream_t stream);

@@ -1002,13 +1002,24 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, c
 
 }  // namespace
 
+// Position tiles, and the units they are cut into (per tile and group, and in all); false from 2^31 units on.
+static bool dgrad_units(const GeoHost &h, int tb, int *tiles_x, int *per_tile, int *total) {
+    const long long tx = ((long long)h.B * h.P + TILE_POS - 1) / TILE_POS;
+    const long long n = (long long)(h.Cs / h.groups / CHUNK_C) * ((h.K + tb - 1) / tb), all = tx * h.groups * n;
+    if (all > 0x7fffffffLL) return false;
+    *tiles_x = (int)tx;
+    *per_tile = (int)n;
+    *total = (int)all;
+    return true;
+}
+
 // Taps per batch, accumulator ring and weight-ring depth that fit tensor memory and shared memory; false when
-// nothing fits (the dense tile of one group must fit tensor memory beside one accumulator).
-bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int *b_stages) {
+// nothing fits (the dense tile of one group must fit tensor memory beside one accumulator) or the work is too much.
+bool dgrad_tc_config(const GeoHost &h, int mode, int *tb, int *nacc, int *b_stages) {
     static const int tb_cap = tuning_int("TVDCN_B200_DG_TB", 4);
     static const int st_cap = tuning_int("TVDCN_B200_DG_STAGES", 4);
-    const int a_cols = (cdg / 2) * mode_mat_parts(mode);
-    for (int cand = std::min(std::min(sc_tb_max(dim), tb_cap), K); cand >= 1; --cand) {
+    const int K = h.K, a_cols = (h.Cd / h.groups / 2) * mode_mat_parts(mode);
+    for (int cand = std::min(std::min(sc_tb_max(h.dim), tb_cap), K); cand >= 1; --cand) {
         // equal batches: the fewest batches of at most `cand` taps
         const int nb = (K + cand - 1) / cand;
         const int t = (K + nb - 1) / nb;
@@ -1016,7 +1027,9 @@ bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int 
         const int acc = std::min(4, (SC_TMEM_COLS - a_cols) / (n * (mode == TC_F32_WIDE ? 2 : 1)));
         if (acc < 1) continue;
         for (int st = std::min(st_cap, 4); st >= 2; --st)
-            if (dgrad_smem_bytes(dim, mode, t, st) <= 227 * 1024) {
+            if (dgrad_smem_bytes(h.dim, mode, t, st) <= 227 * 1024) {
+                int tiles, per_tile, total;
+                if (!dgrad_units(h, t, &tiles, &per_tile, &total)) return false;
                 *tb = t;
                 *nacc = acc;
                 *b_stages = st;
@@ -1032,10 +1045,10 @@ bool dgrad_tc_config(int dim, int mode, int cdg, int K, int *tb, int *nacc, int 
 cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense, void *const *w_parts,
                                    const void *img_cl, const float *offset, const float *mask, float *img_grad_cl, float *goff, float *gmask, const Status &status, cudaStream_t stream) {
     const int cdg = h.Cd / h.groups, csg = h.Cs / h.groups;
-    int tb = 0, nacc = 0, bs = 0;
-    if (!dgrad_tc_config(h.dim, mode, cdg, h.K, &tb, &nacc, &bs)) return cudaErrorInvalidConfiguration;
+    int tb = 0, nacc = 0, bs = 0, tiles_x = 0, n_units = 0, total = 0;
+    if (!dgrad_tc_config(h, mode, &tb, &nacc, &bs) || !dgrad_units(h, tb, &tiles_x, &n_units, &total))
+        return cudaErrorInvalidConfiguration;
     const int nbatch = (h.K + tb - 1) / tb;
-    const long long BP = (long long)h.B * h.P;
     CUtensorMap maps[3];
     {
         const uint64_t dims[4] = {(uint64_t)cdg, (uint64_t)csg, (uint64_t)h.K, (uint64_t)h.groups};
@@ -1043,9 +1056,6 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
         const uint32_t box[4] = {64, (uint32_t)SC_SLAB, (uint32_t)tb, 1};
         if (!make_part_maps(maps, w_parts, mode_mat_parts(mode), 4, dims, strides, box)) return cudaErrorInvalidValue;
     }
-    const long long tiles_x = (BP + TILE_POS - 1) / TILE_POS;
-    const long long n_units = (long long)(csg / CHUNK_C) * nbatch, total = tiles_x * h.groups * n_units;
-    if (total > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     auto run = [&](auto dimc) -> cudaError_t {
         constexpr int DIM = decltype(dimc)::value;
         DgradParams<DIM> P;
@@ -1063,9 +1073,9 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
         P.nbatch = nbatch;
         P.nacc = nacc;
         P.b_stages = bs;
-        P.tiles_x = (int)tiles_x;
-        P.n_units = (int)n_units;
-        P.total_units = (int)total;
+        P.tiles_x = tiles_x;
+        P.n_units = n_units;
+        P.total_units = total;
         // 16-bit data: nothing is rounded between the MMA and the results, there is no wide mode of its own
         switch (mode) {
             case TC_BF16: case TC_BF16_WIDE: return launch_dgrad_t<DIM, TC_BF16>(P, maps, stream);

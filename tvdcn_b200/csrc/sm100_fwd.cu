@@ -626,34 +626,6 @@ size_t fwd_tc_smem_bytes(int dim, int mode, int bn, int stages) {
 // statically allocated shared memory of the kernel (tap table), which counts against the same 227 KB
 static size_t fwd_static_smem(int dim) { return (size_t)FWD_MAX_TAPS * dim * sizeof(int16_t) + 64; }
 
-// Picks the dense-channel tile and the pipeline depth; returns false when the shape is not covered.
-bool fwd_tc_config(int dim, int mode, int cdg, int *bn, int *stages) {
-    static const int cap_split = tuning_int("TVDCN_B200_FWD_BN_SPLIT", 256);
-    static const int max_stages = tuning_int("TVDCN_B200_FWD_STAGES", 3);
-    const int cap = mode == TC_SPLIT ? cap_split : 256;
-    // widest tile of dense channels first (the sampled tile is produced once per CTA, so a wider tile divides the
-    // sampling work), then the deepest pipeline that fits
-    int n = 0, s = 0;
-    for (int cand_n : {256, 128, 64}) {
-        if (cand_n > cap || cdg % cand_n != 0) continue;
-        for (int cand = max_stages; cand >= 2; --cand)
-            if (fwd_tc_smem_bytes(dim, mode, cand_n, cand) + fwd_static_smem(dim) <= 227 * 1024) { s = cand; break; }
-        if (s != 0) { n = cand_n; break; }
-    }
-    if (n == 0) return false;
-    *bn = n;
-    *stages = s;
-    return true;
-}
-
-template <int DIM, int MODE>
-cudaError_t launch_fwd_tc_t(const GeoHost &h, const FwdParams<DIM> &P, const CUtensorMap *maps, cudaStream_t stream) {
-    const size_t smem = fwd_tc_smem_bytes(DIM, MODE, P.bn, P.stages);
-    LaunchScope scope("dcn_fwd_tc", stream);
-    return launch_dependent<dcn_fwd_tc_kernel<DIM, MODE>>(dim3((unsigned)P.work.ctas), FWD_THREADS, smem, stream, P, maps[0],
-                                                          maps[1], maps[2]);
-}
-
 static bool fwd_work(const GeoHost &h, int bn, bool may_share, FwdWork *w) {
     const long long tiles_x = ((long long)h.B * h.P + TILE_POS - 1) / TILE_POS, tiles_y = h.groups * ((h.Cd / h.groups) / bn);
     w->n_chunks = h.K * (h.Cs / h.groups / CHUNK_C);
@@ -669,11 +641,42 @@ static bool fwd_work(const GeoHost &h, int bn, bool may_share, FwdWork *w) {
     const long long shared = std::min(sms, std::min(units / 3, 2LL * w->n_tiles));
     const long long whole_time = (w->n_tiles + sms - 1) / sms * w->n_chunks;
     w->whole = !may_share || w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + (bn > 128 ? 16 : 8);
-    w->ctas = (int)(w->whole ? std::min<long long>(sms, w->n_tiles) : shared);
+    w->ctas = (int)(w->whole ? std::max(1LL, std::min<long long>(sms, w->n_tiles)) : shared);   // 1: an empty batch, planned but not launched
     const long long items = w->whole ? w->n_tiles : units;
     w->base = (int)(items / w->ctas);
     w->extra = (int)(items % w->ctas);
     return true;
+}
+
+// Picks the dense-channel tile and the pipeline depth; returns false when the shape is not covered
+// or has 2^31 units of work or more.
+bool fwd_tc_config(const GeoHost &h, int mode, int *bn, int *stages) {
+    const int cdg = h.Cd / h.groups;
+    static const int cap_split = tuning_int("TVDCN_B200_FWD_BN_SPLIT", 256);
+    static const int max_stages = tuning_int("TVDCN_B200_FWD_STAGES", 3);
+    const int cap = mode == TC_SPLIT ? cap_split : 256;
+    // widest tile of dense channels first (the sampled tile is produced once per CTA, so a wider tile divides the
+    // sampling work), then the deepest pipeline that fits
+    int n = 0, s = 0;
+    for (int cand_n : {256, 128, 64}) {
+        if (cand_n > cap || cdg % cand_n != 0) continue;
+        for (int cand = max_stages; cand >= 2; --cand)
+            if (fwd_tc_smem_bytes(h.dim, mode, cand_n, cand) + fwd_static_smem(h.dim) <= 227 * 1024) { s = cand; break; }
+        if (s != 0) { n = cand_n; break; }
+    }
+    FwdWork work;
+    if (n == 0 || !fwd_work(h, n, false, &work)) return false;
+    *bn = n;
+    *stages = s;
+    return true;
+}
+
+template <int DIM, int MODE>
+cudaError_t launch_fwd_tc_t(const GeoHost &h, const FwdParams<DIM> &P, const CUtensorMap *maps, cudaStream_t stream) {
+    const size_t smem = fwd_tc_smem_bytes(DIM, MODE, P.bn, P.stages);
+    LaunchScope scope("dcn_fwd_tc", stream);
+    return launch_dependent<dcn_fwd_tc_kernel<DIM, MODE>>(dim3((unsigned)P.work.ctas), FWD_THREADS, smem, stream, P, maps[0],
+                                                          maps[1], maps[2]);
 }
 
 // Bytes of the partial sums and number of arrival counters that a launch needs in its workspace (0: no tile is shared).
@@ -692,7 +695,7 @@ cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl
                                   unsigned *arrived, const Status &status, cudaStream_t stream) {
     const int cdg = h.Cd / h.groups, csg = h.Cs / h.groups;
     int bn = 0, stages = 0;
-    if (!fwd_tc_config(h.dim, mode, cdg, &bn, &stages)) return cudaErrorInvalidConfiguration;
+    if (!fwd_tc_config(h, mode, &bn, &stages)) return cudaErrorInvalidConfiguration;
     FwdWork work;
     if (!fwd_work(h, bn, partial != nullptr, &work)) return cudaErrorInvalidConfiguration;
     CUtensorMap maps[3];

@@ -441,40 +441,14 @@ cudaError_t launch_wgrad_t(const WgradParams<DIM> &P, dim3 grid, const CUtensorM
 
 }  // namespace
 
-// Tile shape and pipeline depth; false when the shape is not covered.
-bool wgrad_tc_config(int dim, int mode, int cdg, int *n_sub, int *m_tiles, int *stages) {
-    // f32 data: twice the accumulators (see the modes), and two or three parts of every operand in shared memory
-    const int mt = cdg > 128 && mode != TC_F32_WIDE ? 2 : 1;
-    const int ns = wg_blocks(mode_f32(mode));
-    int s = 0;
-    static const int max_stages = tuning_int("TVDCN_B200_WG_STAGES", 2);
-    for (int cand = max_stages; cand >= 2; --cand)
-        if (wgrad_smem_bytes(dim, mode, ns, mt, cand) <= 227 * 1024) { s = cand; break; }
-    if (s == 0) return false;
-    *n_sub = ns;
-    *m_tiles = mt;
-    *stages = s;
-    return true;
-}
+static int wgrad_chunks_per_image(const GeoHost &h) { return (h.P + WG_POS - 1) / WG_POS; }
 
-// dense_parts: the dense tensor [B, Cd_r, P] as 16-bit parts (the tensor itself for 16-bit data) with rows
-// `pitch` elements apart, a multiple of 8.  gw must be zero-initialised f32 [groups][K][cdg_r][csg]; h: padded geometry.
-cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch,
-                                   const void *img_cl, const float *offset, const float *mask, float *gw,
-                                   const Status &status, cudaStream_t stream) {
-    const int cdg = h.Cd_r / h.groups, csg = h.Cs / h.groups;
-    int ns = 0, mt = 0, st = 0;
-    if (pitch % 8 != 0 || !wgrad_tc_config(h.dim, mode, cdg, &ns, &mt, &st)) return cudaErrorInvalidConfiguration;
-    CUtensorMap maps[3];
-    const uint64_t dims[3] = {(uint64_t)h.P, (uint64_t)h.Cd_r, (uint64_t)h.B};
-    const uint64_t strides[2] = {(uint64_t)pitch * 2, (uint64_t)pitch * h.Cd_r * 2};
-    const uint32_t box[3] = {WG_POS, 128, 1};
-    if (!make_part_maps(maps, dense_parts, mode_mat_parts(mode), 3, dims, strides, box)) return cudaErrorInvalidValue;
-    const int sub_total = h.K * (csg / CHUNK_C);
+// The grid, and the 64-position chunks that each of its z slices reduces; false when a grid dimension is out of range.
+static bool wgrad_grid(const GeoHost &h, int mode, int ns, int mt, dim3 *grid, int *chunks_per_split) {
+    const int sub_total = h.K * (h.Cs / h.groups / CHUNK_C), cdg = h.Cd_r / h.groups;
     const int k_tiles = (sub_total + ns - 1) / ns;
     const int y_tiles = h.groups * ((cdg + 128 * mt - 1) / (128 * mt));
-    const int cpi = (h.P + WG_POS - 1) / WG_POS;
-    const int total = h.B * cpi;
+    const int total = std::max(1, h.B * wgrad_chunks_per_image(h));   // 1: an empty batch, planned but not launched
     const int per_wave = std::max(1, 148 / std::max(1, k_tiles * y_tiles));
     int splits = per_wave;
     if (mode_f32(mode)) {
@@ -491,7 +465,45 @@ cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dens
     splits = std::min(splits, total);
     const int per = (total + splits - 1) / splits;
     splits = (total + per - 1) / per;
-    dim3 grid((unsigned)k_tiles, (unsigned)y_tiles, (unsigned)splits);
+    if (y_tiles > 65535 || splits > 65535) return false;
+    *grid = dim3((unsigned)k_tiles, (unsigned)y_tiles, (unsigned)splits);
+    *chunks_per_split = per;
+    return true;
+}
+
+// Tile shape and pipeline depth; false when the shape is not covered or the grid too large.
+bool wgrad_tc_config(const GeoHost &h, int mode, int *n_sub, int *m_tiles, int *stages) {
+    const int cdg = h.Cd_r / h.groups;
+    // f32 data: twice the accumulators (see the modes), and two or three parts of every operand in shared memory
+    const int mt = cdg > 128 && mode != TC_F32_WIDE ? 2 : 1;
+    const int ns = wg_blocks(mode_f32(mode));
+    int s = 0;
+    static const int max_stages = tuning_int("TVDCN_B200_WG_STAGES", 2);
+    for (int cand = max_stages; cand >= 2; --cand)
+        if (wgrad_smem_bytes(h.dim, mode, ns, mt, cand) <= 227 * 1024) { s = cand; break; }
+    dim3 grid;
+    int per = 0;
+    if (s == 0 || !wgrad_grid(h, mode, ns, mt, &grid, &per)) return false;
+    *n_sub = ns;
+    *m_tiles = mt;
+    *stages = s;
+    return true;
+}
+
+// dense_parts: the dense tensor [B, Cd_r, P] as 16-bit parts (the tensor itself for 16-bit data) with rows
+// `pitch` elements apart, a multiple of 8.  gw must be zero-initialised f32 [groups][K][cdg_r][csg]; h: padded geometry.
+cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch,
+                                   const void *img_cl, const float *offset, const float *mask, float *gw,
+                                   const Status &status, cudaStream_t stream) {
+    int ns = 0, mt = 0, st = 0, per = 0;
+    dim3 grid;
+    if (pitch % 8 != 0 || !wgrad_tc_config(h, mode, &ns, &mt, &st) || !wgrad_grid(h, mode, ns, mt, &grid, &per))
+        return cudaErrorInvalidConfiguration;
+    CUtensorMap maps[3];
+    const uint64_t dims[3] = {(uint64_t)h.P, (uint64_t)h.Cd_r, (uint64_t)h.B};
+    const uint64_t strides[2] = {(uint64_t)pitch * 2, (uint64_t)pitch * h.Cd_r * 2};
+    const uint32_t box[3] = {WG_POS, 128, 1};
+    if (!make_part_maps(maps, dense_parts, mode_mat_parts(mode), 3, dims, strides, box)) return cudaErrorInvalidValue;
     auto run = [&](auto dimc) -> cudaError_t {
         constexpr int DIM = decltype(dimc)::value;
         WgradParams<DIM> P;
@@ -502,12 +514,12 @@ cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dens
         P.gw = gw;
         P.status = status;
         P.stages = st;
-        P.chunks_per_tap = csg / CHUNK_C;
+        P.chunks_per_tap = h.Cs / h.groups / CHUNK_C;
         P.n_sub = ns;
         P.m_tiles = mt;
-        P.chunks_per_image = cpi;
+        P.chunks_per_image = wgrad_chunks_per_image(h);
         P.chunks_per_split = per;
-        P.total_chunks = total;
+        P.total_chunks = h.B * wgrad_chunks_per_image(h);
         return with_mode(mode, [&](auto m) { return launch_wgrad_t<DIM, decltype(m)::value>(P, grid, maps, stream); });
     };
     if (h.dim == 1) return run(std::integral_constant<int, 1>());
