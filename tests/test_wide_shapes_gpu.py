@@ -48,3 +48,37 @@ def test_padded_and_widened_shapes(case, dtype, aux, tol):
     cases.assert_parity(got, ref, tol, case.name)
     from tvdcn_b200 import cabi
     assert cabi.lib().tvdcn_b200_device_status() == 0
+
+
+@pytest.mark.parametrize('scales', [
+    # image, mask, weight, grad_output, bias: columns up to 16 x 60000, past f16's 65504 ...
+    (15000., 16., 1e-3, 1e-3, 100.),
+    # ... and columns near 1e-6, whose second part lies below f16's smallest step
+    (1e-3, 1e-3, 1000., 100., 1e-3),
+], ids=['large_columns', 'small_columns'])
+@pytest.mark.parametrize('aux', [torch.float16, torch.float32], ids=['aux16', 'aux32'])
+@pytest.mark.parametrize('case', [
+    Case('padded', 2, False, 2, 40, 72, (17, 19), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+    Case('groups', 2, False, 2, 48, 80, (8, 9), (3, 2), (1, 1), (1, 0), (1, 2), (), 2, 3, 2, True, 1.5),
+    # with f32 offsets only the weight gradient of this one is wide (an odd extent)
+    Case('odd_extent', 2, False, 2, 64, 64, (7, 9), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+    Case('transposed', 2, True, 2, 24, 40, (9, 10), (4, 4), (2, 2), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+], ids=lambda c: c.name)
+def test_f16_columns_outside_the_range_of_f16(case, aux, scales):
+    """The columns of the wide f16 mode are scaled into the range of their f16 parts: sums of large and of small ones are
+    as exact as those of the SIMT kernels, which keep columns in f32 (half a unit of the f16 results)."""
+    if case.name == 'odd_extent' and aux == torch.float32:
+        pytest.skip('its forward keeps columns in f16, as the reference does')
+    x, w, off, mask, bias, go = make_inputs(case, seed=62)
+    sx, sm, sw, sg, sb = scales
+    x, w, go = x.clamp(-4, 4), w * w.shape[1] ** 0.5, go.clamp(-3, 3)
+    if case.transposed:   # the sampled image is grad_output, whose sum has to fit f16 as well
+        x, go, sm = x * sg, go * sx / 100, sm * 100
+    else:
+        x, go = x * sx, go * sg
+    dev = (x.half(), (w * sw).half(), off.to(aux), (mask * sm).to(aux), (bias * sb).to(aux), go.half())
+    ref = run_oracle(case, *(t.double() for t in dev))
+    assert all(float(r.abs().max()) < 65504 for r in ref), [float(r.abs().max()) for r in ref]
+    names, got = kernels_launched(lambda: run_cabi(case, *(t.cuda() for t in dev), engine=2))
+    assert not {'sample_gemm', 'gemm_scatter', 'sample_wgrad'} & set(names), names
+    cases.assert_parity(got, ref, 6e-4, case.name)

@@ -184,7 +184,9 @@ struct TcCall {
     void parts(const size_t (&buf)[3], void *(&out)[3]) const {
         for (int q = 0; q < 3; ++q) out[q] = at(buf[q]);
     }
-    void stage_image(const void *img) { stage.image(img, at(pl.img_cl), g, p->dtype == TVDCN_F32 ? 4 : 2); }
+    void stage_image(const void *img) {
+        stage.image(img, at(pl.img_cl), g, p->dtype == TVDCN_F32 ? 4 : 2, static_cast<unsigned *>(at(pl.img_max)));
+    }
     void stage_weight(const void *weight, bool kd) {
         void *w[3];
         parts(kd ? pl.w_pack_kd : pl.w_pack, w);
@@ -193,14 +195,19 @@ struct TcCall {
     }
     void stage_aux(const void *off, const void *msk, const void *bia) {
         const int64_t points = (int64_t)g.B * g.K * g.P;
-        auto widen = [&](const void *src, size_t buf, int64_t n) -> const float * {
+        auto widen = [&](const void *src, size_t buf, int64_t n, unsigned *maxima = nullptr) -> const float * {
             if (src == nullptr || buf == NO_BUF) return static_cast<const float *>(src);
-            stage.widen(src, at(buf), p->aux_dtype, n);
+            stage.widen(src, at(buf), p->aux_dtype, n, maxima);
             return static_cast<const float *>(at(buf));
         };
         offset = widen(off, pl.off32, points * g.og * g.dim);
-        mask = widen(msk, pl.mask32, points * g.mg);
+        unsigned *maxima = static_cast<unsigned *>(at(pl.mask_max));
+        mask = widen(msk, pl.mask32, points * g.mg, maxima);
+        if (msk != nullptr && msk == mask && maxima != nullptr) stage.max_abs(msk, maxima, points * g.mg);
         bias = widen(bia, pl.bias32, p->out_channels);
+    }
+    ColumnRange range() const {
+        return {static_cast<unsigned *>(at(pl.img_max)), static_cast<unsigned *>(at(pl.mask_max)), pl.n_img_max, pl.n_mask_max};
     }
     cudaError_t prepare(cudaStream_t stream) {
         cudaError_t e = current_status(&status);
@@ -211,7 +218,7 @@ struct TcCall {
     cudaError_t sample_gemm(void *out, cudaStream_t stream) const {
         void *w[3];
         parts(pl.w_pack, w);
-        return launch_sample_gemm_tc(g, pl.mode, at(pl.img_cl), w, offset, mask, bias, out,
+        return launch_sample_gemm_tc(g, pl.mode, at(pl.img_cl), w, offset, mask, bias, range(), out,
                                      static_cast<float *>(at(pl.sg_partial)), static_cast<unsigned *>(at(pl.sg_arrived)),
                                      status, stream);
     }
@@ -252,7 +259,7 @@ struct TcCall {
         }
         float *acc = static_cast<float *>(at(pl.gw_acc));
         if (e == cudaSuccess)
-            e = launch_sample_wgrad_tc(g, pl.mode_sw, d, pitch, at(pl.img_cl), offset, mask, acc, status, stream);
+            e = launch_sample_wgrad_tc(g, pl.mode_sw, d, pitch, at(pl.img_cl), offset, mask, range(), acc, status, stream);
         if (e == cudaSuccess) e = launch_unpack_weight_grad(acc, grad_weight, p->dtype, g, stream);
         return e;
     }

@@ -69,6 +69,19 @@ void take_aux(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool 
     if (bias) pl.bias32 = b.take((size_t)p->out_channels * sizeof(float));
 }
 
+// The staged sampled image comes first in both plans, and the maxima of its blocks next: a backward call that is told to
+// reuse the forward call's staging (TVDCN_FLAG_REUSE_STAGED_INPUT) finds them at the same offsets of the same workspace.
+// So the forward call takes the maxima also where only the weight gradient needs them (rows that TMA cannot read).
+void take_image(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g) {
+    pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * (p->dtype == TVDCN_F32 ? 4 : 2));   // + one row of zeros
+    if (p->dtype != TVDCN_F16 || !(pl.wide || g.P % 8 != 0)) return;
+    pl.n_img_max = (int)Stager::image_blocks(g);
+    pl.img_max = b.take((size_t)pl.n_img_max * sizeof(unsigned));
+    if (g.mg == 0) return;
+    pl.n_mask_max = (int)Stager::widen_blocks((int64_t)g.B * g.mg * g.K * g.P);
+    pl.mask_max = b.take((size_t)pl.n_mask_max * sizeof(unsigned));
+}
+
 // buffers of the sample -> GEMM kernel besides the staged image (no partial sums: no tile is shared)
 void take_sample_buffers(Plan &pl, Bump &b, const GeoHost &g, int bn, bool share_tiles) {
     take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
@@ -110,12 +123,11 @@ Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
     const char *why = tc_common(p, g);
     pl.wide = !unpadded(p, g);
     pl.mode = mode_of(p->dtype, pl.wide);
-    const size_t es = p->dtype == TVDCN_F32 ? 4 : 2;
     int bn = 0, st = 0, gbufs = 0;
     if (why == nullptr && !p->transposed) {
         if (fwd_tc_config(g, pl.mode, &bn, &st) && chain_ok(pl.mode, g, bn)) {
             pl.tensor = pl.tc_sg = true;
-            pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);   // + one row of zeros
+            take_image(pl, b, p, g);
             take_sample_buffers(pl, b, g, bn, share_tiles);
             take_aux(pl, b, p, g, true);
         } else {
@@ -151,7 +163,6 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
     pl.wide = !unpadded(p, g);
     pl.mode = mode_of(p->dtype, pl.wide);
     pl.mode_sw = mode_of(p->dtype, pl.wide || g.P % 8 != 0);
-    const size_t es = p->dtype == TVDCN_F32 ? 4 : 2;
     want_offset = want_offset && g.og > 0;
     want_mask = want_mask && g.mg > 0;
     if (why == nullptr) {
@@ -166,10 +177,8 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
         pl.tc_gs = (scatter || want_offset || want_mask) &&
                    dgrad_tc_config(g, pl.mode, &bn, &gbufs, &st);
         pl.tensor = pl.tc_sg || pl.tc_sw || pl.tc_gs;
-        // The staged image comes first, as in the forward plan: a backward call that is told to reuse the
-        // forward call's staging (TVDCN_FLAG_REUSE_STAGED_INPUT) finds it at the same offset of the same workspace.
         if (pl.tensor) {
-            pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * es);
+            take_image(pl, b, p, g);
             take_aux(pl, b, p, g, false);
         }
         if (pl.tc_sg) take_sample_buffers(pl, b, g, sg_bn, true);

@@ -32,6 +32,8 @@ struct Plan {
     size_t dense[3] = {NO_BUF, NO_BUF, NO_BUF};       // dense tensor, rows dense_pitch apart (absent: the caller's own)
     int dense_pitch = 0;
     size_t img_grad_cl = NO_BUF;   // f32 channels-last accumulator of the scatter
+    size_t img_max = NO_BUF, mask_max = NO_BUF;   // see ColumnRange: maxima of the image's and the mask's blocks
+    int n_img_max = 0, n_mask_max = 0;
     size_t off32 = NO_BUF, mask32 = NO_BUF, bias32 = NO_BUF;   // 16-bit offset / mask / bias widened to f32
     size_t sg_partial = NO_BUF, sg_arrived = NO_BUF, sg_counters = 0;   // sample -> GEMM: tiles shared between CTAs
     size_t sum_partial = NO_BUF, sum_done = NO_BUF;   // partial sums of the bias gradient and their arrival counters
@@ -51,9 +53,10 @@ int cuda_fail(cudaError_t e, const char *what);
 GeoHost tc_geometry(const GeoHost &g);
 
 // ---- staging (sm100_staging.cu) ------------------------------------------------------------------------
-enum : int { STAGE_IMAGE, STAGE_PACK, STAGE_ZERO, STAGE_WIDEN, STAGE_PITCH };
+enum : int { STAGE_IMAGE, STAGE_PACK, STAGE_ZERO, STAGE_WIDEN, STAGE_PITCH, STAGE_MAX };
 struct StageJob {
     const void *src;
+    // part: STAGE_PACK: one tensor per part; STAGE_IMAGE (f16), STAGE_WIDEN (may be null), STAGE_MAX: [0] = the blocks' maxima
     void *dst, *part[3];
     int64_t n;
     int kind, end_block;           // the job's blocks end before this one
@@ -69,11 +72,15 @@ struct StageList {
 // Collects the preparations of one call and runs them as one launch.
 class Stager {
    public:
-    void image(const void *src, void *dst, const GeoHost &h, int elem_bytes);   // + the row of zeros behind it
+    // + the row of zeros behind it; maxima (f16, may be null): image_blocks values
+    void image(const void *src, void *dst, const GeoHost &h, int elem_bytes, unsigned *maxima);
+    static int64_t image_blocks(const GeoHost &h) { return (int64_t)h.B * ((h.S + 63) / 64) * (h.Cs / 64); }
     void pack(const void *weight, void *const *parts, const GeoHost &h, int dtype, int n_parts, bool kd);
     void zero(void *dst, int64_t bytes);                                        // bytes: a multiple of 4
-    void widen(const void *src, void *dst, int dtype, int64_t n);               // 16-bit -> f32
+    void widen(const void *src, void *dst, int dtype, int64_t n, unsigned *maxima = nullptr);   // 16-bit -> f32
+    static int64_t widen_blocks(int64_t n);
     void pitch(const void *src, void *dst, int64_t rows, int P, int pitch);     // 16-bit rows, `pitch` apart
+    void max_abs(const void *src, unsigned *maxima, int64_t n);                 // f32, widen_blocks values
     cudaError_t launch(const Status &status, cudaStream_t stream);
     bool empty() const { return list_.n == 0; }
 
@@ -97,13 +104,13 @@ cudaError_t launch_dense_pass(const void *src, int dtype, int n_parts, void *con
 // A configuration is returned for every problem that the launcher below it takes, and for no other.
 bool fwd_tc_config(const GeoHost &h, int mode, int *bn, int *stages);
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
-                                  const float *offset, const float *mask, const float *bias, void *out, float *partial,
-                                  unsigned *arrived, const Status &status, cudaStream_t stream);
+                                  const float *offset, const float *mask, const float *bias, const ColumnRange &range,
+                                  void *out, float *partial, unsigned *arrived, const Status &status, cudaStream_t stream);
 void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters);   // partial sums of shared tiles
 bool wgrad_tc_config(const GeoHost &h, int mode, int *n_sub, int *m_tiles, int *stages);
 cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch, const void *img_cl,
-                                   const float *offset, const float *mask, float *gw, const Status &status,
-                                   cudaStream_t stream);
+                                   const float *offset, const float *mask, const ColumnRange &range, float *gw,
+                                   const Status &status, cudaStream_t stream);
 bool dgrad_tc_config(const GeoHost &h, int mode, int *tb, int *nacc, int *b_stages);
 cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense, void *const *w_parts,
                                    const void *img_cl, const float *offset, const float *mask, float *img_grad_cl,

@@ -123,6 +123,46 @@ struct RawCoords {
     float m;
 };
 
+// The power of two of a ColumnRange, 2^15 / (bounds of the two maxima); the 128 planner threads, thread t among them,
+// take part and all get it.  It is the planners' work because they have the loads of their first coordinates to wait for
+// meanwhile.  part: 8 words of shared memory; BAR: a named barrier of theirs.
+template <int BAR>
+__device__ __forceinline__ float column_scale(const ColumnRange &r, int t, uint32_t *part) {
+    constexpr int U = 4;
+    uint32_t m[2] = {0u, 0u};
+    for (int i0 = t; i0 < max(r.n_img, r.n_mask); i0 += 128 * U) {
+        uint32_t a[U], b[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int i = i0 + 128 * k;
+            a[k] = i < r.n_img ? __ldg(r.img + i) : 0u;
+            b[k] = i < r.n_mask ? __ldg(r.mask + i) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            m[0] = max(m[0], a[k]);
+            m[1] = max(m[1], b[k]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        m[q] = __reduce_max_sync(0xffffffffu, m[q]);
+        if ((t & 31) == 0) part[q * 4 + (t >> 5)] = m[q];
+    }
+    asm volatile("bar.sync %0, 128;" ::"n"(BAR) : "memory");
+    int e = 15;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const uint32_t v = max(max(part[q * 4], part[q * 4 + 1]), max(part[q * 4 + 2], part[q * 4 + 3]));
+        // a normal value is below 2^(biased exponent - 126); zero and subnormals: as if 1, they need no factor
+        if (v >= 0x00800000u) e -= (int)(v >> 23) - 126;
+    }
+    return __uint_as_float((uint32_t)(127 + min(max(e, -120), 120)) << 23);
+}
+__device__ __forceinline__ float inverse_of_power_of_two(float v) {
+    return __uint_as_float((254u << 23) - __float_as_uint(v));
+}
+
 template <int MODE>
 __device__ __forceinline__ uint32_t encode_weight(float w) {
     if constexpr (Mode<MODE>::BLEND_F32) {
@@ -149,11 +189,11 @@ __device__ __forceinline__ void tap_coords(const Geo<DIM> &g, int tap, int (&tc)
 
 // Writes the plan slot of one position and tap, whose kernel coordinates are tc (the divisions by the kernel extents were
 // a quarter of the instructions of a slot, and a planner thread makes slots back to back).  row_scale = Cs * element
-// size / 16.
+// size / 16; weight_scale: see ColumnRange.
 template <int DIM, int MODE>
 __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<DIM> &pi, const RawCoords<DIM> &rc,
                                               bool deformable, const int (&tc)[DIM], uint32_t row_scale,
-                                              uint32_t *slot) {
+                                              uint32_t *slot, float weight_scale = 1.f) {
     constexpr int NC = 1 << DIM;
     int fl[DIM];
     float fr[DIM];
@@ -175,7 +215,7 @@ __device__ __forceinline__ void build_plan_at(const Geo<DIM> &g, const PosInfo<D
     for (int c = 0; c < NC; ++c) {
         bool ok = pi.valid && (deformable || c == 0);
         int flat = 0;
-        float w = rc.m;
+        float w = MODE == TC_F16_WIDE ? rc.m * weight_scale : rc.m;
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
             const int bit = (c >> (DIM - 1 - a)) & 1;

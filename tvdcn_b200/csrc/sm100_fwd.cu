@@ -88,6 +88,7 @@ struct FwdParams {
     const float *offset;    // may be null
     const float *mask;      // may be null
     const float *bias;      // may be null
+    ColumnRange range;      // TC_F16_WIDE
     void *out;              // [B, Cd, P], data type of the problem
     Status status;
     float *partial;         // partial sums of shared tiles: two [bn / 4][128] float4 per CTA (null: no tile is shared)
@@ -164,6 +165,8 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
 #pragma unroll
         for (int a = 0; a < DIM; ++a) tap_tab[tp * DIM + a] = (int16_t)tc[a];
     }
+    // TC_F16_WIDE: the factor of the sums, written by the planners before their first plan and read behind a tile's last MMA
+    __shared__ float out_scale;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_n = g.cdg / BN, chunks = g.csg / CHUNK_C;
     const FwdWork &W = P.work;
@@ -223,13 +226,18 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
 
     constexpr int CW = 16;                            // dense channels the epilogue handles at a time
     // n consecutive dense channels of one position, from channel col0 of the tile
-    auto store_block = [&](const PosInfo<DIM> &pi, int y, const auto &v, int col0) {
+    auto store_block = [&](const PosInfo<DIM> &pi, int y, auto &v, int col0) {
         constexpr int N = sizeof(v) / sizeof(float);
         if (!pi.valid) return;
         const int grp = y / tiles_n, dl0 = y % tiles_n * BN + col0;      // first dense channel within the group
         const int d0 = grp * g.cdg_r + dl0, n = min(N, g.cdg_r - dl0);
         using TO = typename std::conditional<M::F32, float, T16>::type;
         TO *out = static_cast<TO *>(P.out) + ((int64_t)pi.b * g.Cd_r + d0) * (int64_t)g.P + pi.p;
+        if constexpr (MODE == TC_F16_WIDE) {
+            const float factor = out_scale;
+#pragma unroll
+            for (int e = 0; e < N; ++e) v[e] *= factor;
+        }
         if (n == N) {
 #pragma unroll
             for (int e = 0; e < N; ++e) {
@@ -270,7 +278,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
             }
 #pragma unroll
             for (int k = 0; k < QN; ++k) {
-                const float f[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
+                float f[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
                 store_block(pi, tile % W.tiles_y, f, (q + k * step) * 4);
             }
         }
@@ -548,6 +556,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
         // Plans chunk i from `cur` and requests the coordinates of chunk i + 2 into `fill`.  The three coordinate
         // sets rotate by name (the loop below is unrolled by three), never by assignment: copying a set whose loads
         // are still in flight would wait for them and put their latency back on the critical path.
+        float col_scale = 1.f;
         auto step = [&](int i, const RawCoords<DIM> &cur, RawCoords<DIM> &fill) -> bool {
             const int pbuf = i % PLAN_BUFS;
             if (i + 2 < n_local) fetch(fill);
@@ -561,7 +570,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
             int tc[DIM];
 #pragma unroll
             for (int a = 0; a < DIM; ++a) tc[a] = tap_tab[cur_c.tap * DIM + a];
-            build_plan_at<DIM, MODE>(g, pi, cur, deformable, tc, row_scale, slot);
+            build_plan_at<DIM, MODE>(g, pi, cur, deformable, tc, row_scale, slot, col_scale);
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&plan_full[pbuf]);
             const int x = cur_c.x;
@@ -572,6 +581,11 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
         RawCoords<DIM> r0, r1, r2;
         if (n_local > 0) fetch(r0);
         if (n_local > 1) fetch(r1);
+        if constexpr (MODE == TC_F16_WIDE) {
+            __shared__ uint32_t scale_part[8];
+            col_scale = column_scale<3>(P.range, t, scale_part);
+            if (t == 0) out_scale = inverse_of_power_of_two(col_scale);
+        }
         int i = 0;
         bool ok = true;
         for (; ok && i + 2 < n_local; i += 3) ok = step(i, r0, r2) && step(i + 1, r1, r0) && step(i + 2, r2, r1);
@@ -624,7 +638,7 @@ size_t fwd_tc_smem_bytes(int dim, int mode, int bn, int stages) {
 }
 
 // statically allocated shared memory of the kernel (tap table), which counts against the same 227 KB
-static size_t fwd_static_smem(int dim) { return (size_t)FWD_MAX_TAPS * dim * sizeof(int16_t) + 64; }
+static size_t fwd_static_smem(int dim) { return (size_t)FWD_MAX_TAPS * dim * sizeof(int16_t) + 128; }
 
 static bool fwd_work(const GeoHost &h, int bn, bool may_share, FwdWork *w) {
     const long long tiles_x = ((long long)h.B * h.P + TILE_POS - 1) / TILE_POS, tiles_y = h.groups * ((h.Cd / h.groups) / bn);
@@ -691,8 +705,8 @@ void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *c
 // img_cl: channels-last sampled image in the problem's data type; w_parts: weights packed [g][tap][d'][s'], one
 // 16-bit tensor per part of the mode; h: padded geometry; partial / arrived: see fwd_tc_workspace, arrived zeroed (partial null: every tile has one CTA).
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
-                                  const float *offset, const float *mask, const float *bias, void *out, float *partial,
-                                  unsigned *arrived, const Status &status, cudaStream_t stream) {
+                                  const float *offset, const float *mask, const float *bias, const ColumnRange &range,
+                                  void *out, float *partial, unsigned *arrived, const Status &status, cudaStream_t stream) {
     const int cdg = h.Cd / h.groups, csg = h.Cs / h.groups;
     int bn = 0, stages = 0;
     if (!fwd_tc_config(h, mode, &bn, &stages)) return cudaErrorInvalidConfiguration;
@@ -711,6 +725,7 @@ cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl
         P.offset = offset;
         P.mask = mask;
         P.bias = bias;
+        P.range = range;
         P.out = out;
         P.status = status;
         P.bn = bn;

@@ -23,9 +23,34 @@ __device__ __forceinline__ int real_channel(int cp, int gran, int gran_pad) {
 // widened to f32, ...).  As launches of their own they cost more than their work on small calls (1.5-2 us of device
 // time and about as much of host time each), so they are jobs of one kernel: a block finds its job by its index.
 
+// Largest finite magnitude of a block's values, as float bits, whose order is that of the magnitudes.
+__device__ __forceinline__ uint32_t finite_magnitude(float v) {
+    const uint32_t m = __float_as_uint(v) & 0x7fffffffu;
+    return m < 0x7f800000u ? m : 0u;
+}
+__device__ void store_block_max(uint32_t m, const StageJob &j, int block) {
+    __shared__ uint32_t part[8];
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = max(m, part[w]);
+        static_cast<unsigned *>(j.part[0])[block] = m;
+    }
+}
+// the same of two pairs of f16 values, as pairs of f16 bits
+__device__ __forceinline__ uint32_t max_finite_f16x2(uint32_t m, uint32_t w) {
+    w &= 0x7fff7fffu;
+    return __vmaxu2(m, w & __vcmpltu2(w, 0x7c007c00u));
+}
+__device__ __forceinline__ uint32_t f16x2_to_magnitude(uint32_t m) {
+    return __float_as_uint(__half2float(__ushort_as_half((unsigned short)max(m & 0xffffu, m >> 16))));
+}
+
 // Image [B, C, S] -> [B, S, Cpad], one 64 x 64 tile per block.  16-bit tiles are held as words of two neighbouring
 // positions, the words of a channel pair 32 words apart and pairs 65 apart, 32-bit tiles in rows of 65: the
 // transposing accesses are free of bank conflicts.
+template <bool MAXIMA>
 __device__ void stage_image_tile(const StageJob &j, int block, uint32_t *tile) {
     const int C64 = j.c_pad / 64, S64 = (j.S + 63) / 64;
     const int c0 = block % C64 * 64, s0 = block / C64 % S64 * 64;
@@ -64,14 +89,17 @@ __device__ void stage_image_tile(const StageJob &j, int block, uint32_t *tile) {
         }
         __syncthreads();
         const int c = c0 + 2 * lane;
+        uint32_t largest = 0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int s2 = warp * 4 + i;
             const uint32_t a = tile[lane * 65 + s2], bb = tile[lane * 65 + 32 + s2];
+            if constexpr (MAXIMA) largest = max_finite_f16x2(max_finite_f16x2(largest, a), bb);
             const int s = s0 + 2 * s2;
             if (s < j.S) out[((int64_t)s * j.c_pad + c) >> 1] = __byte_perm(a, bb, 0x5410);
             if (s + 1 < j.S) out[((int64_t)(s + 1) * j.c_pad + c) >> 1] = __byte_perm(a, bb, 0x7632);
         }
+        if constexpr (MAXIMA) store_block_max(f16x2_to_magnitude(largest), j, block);
     } else {
         const uint32_t *in = static_cast<const uint32_t *>(j.src) + b * j.C * (int64_t)j.S;
         uint32_t *out = static_cast<uint32_t *>(j.dst) + b * j.S * (int64_t)j.c_pad;
@@ -200,12 +228,31 @@ __device__ void zero_range(const StageJob &j, int block) {
 }
 
 constexpr int WIDEN_ELEMS = 256 * 8;          // per block
+template <bool MAXIMA>
 __device__ void widen_range(const StageJob &j, int block) {
     const int64_t end = min(j.n, ((int64_t)block + 1) * WIDEN_ELEMS);
     float *out = static_cast<float *>(j.dst);
-    for (int64_t i = (int64_t)block * WIDEN_ELEMS + threadIdx.x; i < end; i += 256)
-        out[i] = j.dtype == DT_F16 ? __half2float(__ldg(static_cast<const __half *>(j.src) + i))
-                                   : __bfloat162float(__ldg(static_cast<const __nv_bfloat16 *>(j.src) + i));
+    uint32_t largest = 0;
+    for (int64_t i = (int64_t)block * WIDEN_ELEMS + threadIdx.x; i < end; i += 256) {
+        const float v = j.dtype == DT_F16 ? __half2float(__ldg(static_cast<const __half *>(j.src) + i))
+                                          : __bfloat162float(__ldg(static_cast<const __nv_bfloat16 *>(j.src) + i));
+        out[i] = v;
+        if constexpr (MAXIMA) largest = max(largest, finite_magnitude(v));
+    }
+    if constexpr (MAXIMA)
+        if (j.part[0] != nullptr) store_block_max(largest, j, block);
+}
+// The maxima alone, of f32 values.
+__device__ void max_range(const StageJob &j, int block) {
+    const int64_t first = (int64_t)block * WIDEN_ELEMS + threadIdx.x;
+    float v[WIDEN_ELEMS / 256];               // all loads in flight together
+#pragma unroll
+    for (int k = 0; k < WIDEN_ELEMS / 256; ++k)
+        v[k] = first + k * 256 < j.n ? __ldg(static_cast<const float *>(j.src) + first + k * 256) : 0.f;
+    uint32_t largest = 0;
+#pragma unroll
+    for (int k = 0; k < WIDEN_ELEMS / 256; ++k) largest = max(largest, finite_magnitude(v[k]));
+    store_block_max(largest, j, block);
 }
 
 // Rows of S 16-bit values -> rows c_pad apart (a multiple of 8), so that TMA can read them.
@@ -232,7 +279,8 @@ __device__ void pitch_range(const StageJob &j, int block) {
 // 451 us (two calls' staging) where five of 48 took 523.  The unaligned paths keep 16 loads per thread in flight and spill
 // with 32 registers, and a launch that is resident as a whole either way gains nothing.
 constexpr int STAGE_RESIDENT = 5;             // what 48 registers allow
-template <int RESIDENT>
+// MAXIMA: with the jobs that take maxima (a branch in the image path of every call cost 1 us of a 154 us training step).
+template <int RESIDENT, bool MAXIMA>
 __global__ void __launch_bounds__(256, RESIDENT) stage_kernel(const __grid_constant__ StageList list) {
     __shared__ uint32_t tile[STAGE_WORDS];
     ptx::allow_dependents();
@@ -242,7 +290,7 @@ __global__ void __launch_bounds__(256, RESIDENT) stage_kernel(const __grid_const
     const StageJob &j = list.job[q];
     const int block = (int)blockIdx.x - first;
     switch (j.kind) {
-        case STAGE_IMAGE: stage_image_tile(j, block, tile); break;
+        case STAGE_IMAGE: stage_image_tile<MAXIMA>(j, block, tile); break;
         case STAGE_PACK: {
             float *f = reinterpret_cast<float *>(tile);
             if (j.dtype == DT_F32) pack_weight_tile<float>(j, block, f);
@@ -251,8 +299,11 @@ __global__ void __launch_bounds__(256, RESIDENT) stage_kernel(const __grid_const
             break;
         }
         case STAGE_ZERO: zero_range(j, block); break;
-        case STAGE_WIDEN: widen_range(j, block); break;
+        case STAGE_WIDEN: widen_range<MAXIMA>(j, block); break;
         case STAGE_PITCH: pitch_range(j, block); break;
+        case STAGE_MAX:
+            if constexpr (MAXIMA) max_range(j, block);
+            break;
     }
 }
 
@@ -426,10 +477,10 @@ StageJob *Stager::add(int kind, int64_t blocks) {
 
 static bool aligned(const void *p, size_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; }
 
-void Stager::image(const void *src, void *dst, const GeoHost &h, int elem_bytes) {
-    StageJob *j = add(STAGE_IMAGE, (int64_t)h.B * ((h.S + 63) / 64) * (h.Cs / 64));
+void Stager::image(const void *src, void *dst, const GeoHost &h, int elem_bytes, unsigned *maxima) {
+    StageJob *j = add(STAGE_IMAGE, image_blocks(h));
     if (j == nullptr) return;
-    j->src = src; j->dst = dst;
+    j->src = src; j->dst = dst; j->part[0] = maxima;
     j->C = h.Cs_r; j->c_pad = h.Cs; j->gran = h.gran; j->gran_pad = h.gran_pad;
     j->S = h.S;
     j->elem_bytes = elem_bytes;
@@ -461,11 +512,20 @@ void Stager::zero(void *dst, int64_t bytes) {
     j->wide = aligned(dst, 16);
 }
 
-void Stager::widen(const void *src, void *dst, int dtype, int64_t n) {
-    StageJob *j = add(STAGE_WIDEN, (n + WIDEN_ELEMS - 1) / WIDEN_ELEMS);
+int64_t Stager::widen_blocks(int64_t n) { return (n + WIDEN_ELEMS - 1) / WIDEN_ELEMS; }
+
+void Stager::widen(const void *src, void *dst, int dtype, int64_t n, unsigned *maxima) {
+    StageJob *j = add(STAGE_WIDEN, widen_blocks(n));
     if (j == nullptr) return;
-    j->src = src; j->dst = dst;
+    j->src = src; j->dst = dst; j->part[0] = maxima;
     j->dtype = dtype;
+    j->n = n;
+}
+
+void Stager::max_abs(const void *src, unsigned *maxima, int64_t n) {
+    StageJob *j = add(STAGE_MAX, widen_blocks(n));
+    if (j == nullptr) return;
+    j->src = src; j->part[0] = maxima;
     j->n = n;
 }
 
@@ -482,12 +542,16 @@ cudaError_t Stager::launch(const Status &status, cudaStream_t stream) {
     if (list_.n == 0) return cudaSuccess;
     list_.status = status;
     LaunchScope scope("stage", stream);
-    bool wide = true;
-    for (int q = 0; q < list_.n; ++q) wide = wide && (list_.job[q].kind != STAGE_IMAGE || list_.job[q].wide);
-    if (wide && blocks_ > 148 * STAGE_RESIDENT)
-        stage_kernel<8><<<(unsigned)blocks_, 256, 0, stream>>>(list_);
-    else
-        stage_kernel<STAGE_RESIDENT><<<(unsigned)blocks_, 256, 0, stream>>>(list_);
+    bool wide = true, maxima = false;
+    for (int q = 0; q < list_.n; ++q) {
+        const StageJob &j = list_.job[q];
+        wide = wide && (j.kind != STAGE_IMAGE || j.wide);
+        maxima = maxima || (j.kind != STAGE_PACK && j.part[0] != nullptr);
+    }
+    const bool eight = wide && blocks_ > 148 * STAGE_RESIDENT;
+    auto *kernel = eight ? (maxima ? stage_kernel<8, true> : stage_kernel<8, false>)
+                         : (maxima ? stage_kernel<STAGE_RESIDENT, true> : stage_kernel<STAGE_RESIDENT, false>);
+    kernel<<<(unsigned)blocks_, 256, 0, stream>>>(list_);
     return cudaGetLastError();
 }
 

@@ -33,6 +33,7 @@ struct WgradParams {
     const void *img_cl;
     const float *offset;
     const float *mask;
+    ColumnRange range;       // TC_F16_WIDE
     float *gw;               // staged weight gradient [g][tap][d'][s'] f32, accumulated into
     Status status;
     int stages;
@@ -90,6 +91,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint64_t *plan_empty = plan_full + WG_PLAN_BUFS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(plan_empty + WG_PLAN_BUFS);
     __shared__ uint32_t chan16_s[4];
+    __shared__ float out_scale;        // TC_F16_WIDE: the factor of the sums, written by the planners before their first plan
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub_total = g.K * P.chunks_per_tap;                 // 64-column blocks per group
@@ -196,6 +198,11 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                         ptx::tmem_ld_wait();
 #pragma unroll
                         for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]));
+                    }
+                    if constexpr (MODE == TC_F16_WIDE) {
+                        const float factor = out_scale;
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * factor);
                     }
                     const int m = cb / (NS * 2);
                     const int col0 = (cb % (NS * 2)) * 32;      // column within the M tile
@@ -385,6 +392,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 fetch_p = slot;
             }
         };
+        float col_scale = 1.f;
         auto step = [&](int i, const StageCoords &cur, StageCoords &fill) -> bool {
             const int pb = i % WG_PLAN_BUFS;
             if (i + 2 < n_stages) fetch(fill);
@@ -404,7 +412,7 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 pi.valid = e_ok[k] && cur_w.p < g.P;
                 if (e_on[k])
                     build_plan_at<DIM, MODE>(g, pi, cur.rc[k], deformable, e_tc[k], row_scale,
-                                             plan + ((pb * NS) * WG_POS + t + k * WG_PLANNERS) * 2 * NC);
+                                             plan + ((pb * NS) * WG_POS + t + k * WG_PLANNERS) * 2 * NC, col_scale);
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&plan_full[pb]);
@@ -414,6 +422,11 @@ dcn_wgrad_tc_kernel(const WgradParams<DIM> P, const __grid_constant__ CUtensorMa
         StageCoords r0, r1, r2;
         if (n_stages > 0) fetch(r0);
         if (n_stages > 1) fetch(r1);
+        if constexpr (MODE == TC_F16_WIDE) {
+            __shared__ uint32_t scale_part[8];
+            col_scale = column_scale<1>(P.range, t, scale_part);
+            if (t == 0) out_scale = inverse_of_power_of_two(col_scale);
+        }
         int i = 0;
         bool ok = true;
         for (; ok && i + 2 < n_stages; i += 3) ok = step(i, r0, r2) && step(i + 1, r1, r0) && step(i + 2, r2, r1);
@@ -493,8 +506,8 @@ bool wgrad_tc_config(const GeoHost &h, int mode, int *n_sub, int *m_tiles, int *
 // dense_parts: the dense tensor [B, Cd_r, P] as 16-bit parts (the tensor itself for 16-bit data) with rows
 // `pitch` elements apart, a multiple of 8.  gw must be zero-initialised f32 [groups][K][cdg_r][csg]; h: padded geometry.
 cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch,
-                                   const void *img_cl, const float *offset, const float *mask, float *gw,
-                                   const Status &status, cudaStream_t stream) {
+                                   const void *img_cl, const float *offset, const float *mask, const ColumnRange &range,
+                                   float *gw, const Status &status, cudaStream_t stream) {
     int ns = 0, mt = 0, st = 0, per = 0;
     dim3 grid;
     if (pitch % 8 != 0 || !wgrad_tc_config(h, mode, &ns, &mt, &st) || !wgrad_grid(h, mode, ns, mt, &grid, &per))
@@ -511,6 +524,7 @@ cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dens
         P.img_cl = img_cl;
         P.offset = offset;
         P.mask = mask;
+        P.range = range;
         P.gw = gw;
         P.status = status;
         P.stages = st;
