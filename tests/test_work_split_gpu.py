@@ -42,6 +42,16 @@ def test_split_work(case, dtype, tol):
     assert cabi.lib().tvdcn_b200_device_status() == 0
 
 
+def test_dense_tile_is_reloaded_behind_the_last_mma_on_it():
+    """384 dense channels of f32 leave tensor memory for one accumulator, 153 tiles give a few CTAs two: the second dense
+    tile may overwrite the first only behind its last MMA, whatever the timing of the call."""
+    case = SPLITS[-1]
+    dev = [None if t is None else t.float().cuda() for t in make_inputs(case, seed=75)]
+    ref = run_cabi(case, *dev, engine=1)
+    for _ in range(25):
+        cases.assert_parity(run_cabi(case, *dev, engine=2)[:2], ref[:2], 1e-4, case.name)
+
+
 def test_volume_with_one_cta_per_tile():
     """592 tiles and more of at least eight units: as many CTAs as tiles.  Too large for the CPU oracle, so the SIMT kernels,
     which are checked against it elsewhere, stand in."""

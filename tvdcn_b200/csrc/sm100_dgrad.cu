@@ -156,7 +156,7 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
     L.cnt = o;  o += SC_SLOTS * 4;
     L.taps = o; o += SC_MAX_TAPS * 3 * 2;         // kernel coordinates of every tap (int16)
     L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot
-    L.bars = o; o += (uint32_t)(20 + 2 * b_stages) * 8;
+    L.bars = o; o += (uint32_t)(21 + 2 * b_stages) * 8;
     L.total = o;
     return L;
 }
@@ -251,6 +251,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint64_t *plan_full = col_empty + 2; // [2] planners -> gather warps
     uint64_t *plan_done = plan_full + 2; // [2] gather warps -> whoever turns the unit's dots into gradients / planners
     uint64_t *fin_done = plan_done + 2;  // [2] store warps -> planners: the unit's dots have been used
+    uint64_t *a_free = fin_done + 2;     // MMA -> planners: the last MMA on the dense tile is through
     int16_t *tap_tab = reinterpret_cast<int16_t *>(smem + L.taps);
     // Entry e of the pixel-grouped list sits at word e of each array; a group's span is a multiple of four entries, so
     // that a batch of four is one 16-byte read per array (each 8-lane group is a quarter-warp phase of its own: the
@@ -275,6 +276,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     if (threadIdx.x == 0) {
         ptx::mbar_init(a_first, SC_LOAD_WARPS);
         ptx::mbar_init(a_next, SC_PLAN_WARPS);
+        ptx::mbar_init(a_free, 1);
         for (int s = 0; s < BS; ++s) {
             ptx::mbar_init(&b_full[s], 1);
             ptx::mbar_init(&b_empty[s], 1);
@@ -811,6 +813,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         load_unit(pi, info, ru);
         ru_next = ru;
         bool new_tile = false;
+        uint32_t free_phase = 0;
         for (int j = 0; j < n_units && ok; ++j) {
             const int pb = j & 1;
             if (j >= 2) {
@@ -829,10 +832,11 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             if (j + 1 < n_units) load_unit(pi_next, info_next, ru_next);
             build(info, pb, ru);
             if (new_tile) {
-                // the dense tile is free once the MMAs of the pass before this unit are through; no pass behind it can
-                // complete before this load, so its phase is not missed
-                const int pass = 2 * j - 1;
-                ok = wait_all(&t_full[pass % NACC], (uint32_t)((pass / NACC) & 1));
+                // One phase of a_free per tile, and the next one cannot complete before this load: neither an earlier
+                // phase nor a later one is taken for it.  (The barriers of the accumulators do not serve: with a single
+                // accumulator the pass two before looks like the one before this unit.)
+                ok = wait_all(a_free, free_phase);
+                free_phase ^= 1u;
                 if (!ok) {
                     if (pt == 0) ptx::report(P.status, 309);
                     break;
@@ -931,6 +935,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     }
                 }
                 if (ok) ptx::mma_commit(&t_full[aq]);
+                // the tile's last pass, and another tile follows
+                if (ok && (jp & 1) && new_tile && jp + 1 < n_pass) ptx::mma_commit(a_free);
                 if (++aq == NACC) {
                     aq = 0;
                     t_phase ^= 1u;
