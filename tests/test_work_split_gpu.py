@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import cases
-from cases import Case, make_inputs, run_cabi, run_oracle
+from cases import Case, make_inputs, nerr, run_cabi, run_oracle
 from test_tensor_gpu import kernels_launched
 
 pytestmark = pytest.mark.gpu
@@ -50,6 +50,20 @@ def test_dense_tile_is_reloaded_behind_the_last_mma_on_it():
     ref = run_cabi(case, *dev, engine=1)
     for _ in range(25):
         cases.assert_parity(run_cabi(case, *dev, engine=2)[:2], ref[:2], 1e-4, case.name)
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16], ids=['f32', 'bf16'])
+def test_last_tile_of_a_cta_is_read_behind_its_last_mma(dtype):
+    """One tap and one chunk: a CTA's second tile is sampled while the first is summed, and its result may be read only
+    when its own sums are complete, whatever the timing: the same bits from every call."""
+    case = Case('two_units', 2, False, 4, 64, 64, (150, 41), (1, 1), (1, 1), (0, 0), (1, 1), (), 1, 1, 1, True, 1.0)
+    dev = [t.float().cuda() for t in make_inputs(case, seed=76)]
+    dev = [dev[0].to(dtype), dev[1].to(dtype), *dev[2:5], dev[5].to(dtype)]
+    ref = run_cabi(case, *dev, engine=1)[0]
+    first = run_cabi(case, *dev, engine=2)[0]
+    assert nerr(first, ref) <= (1e-4 if dtype == torch.float32 else 2e-2)
+    for _ in range(25):
+        assert torch.equal(run_cabi(case, *dev, engine=2)[0], first)
 
 
 def test_volume_with_one_cta_per_tile():

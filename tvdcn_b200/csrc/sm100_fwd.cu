@@ -152,7 +152,8 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
     uint64_t *empty = bars + 2 * S;
     uint64_t *acc_full = bars + 3 * S;      // [2] MMA -> epilogue: a tile's (or a piece's) sums are complete
     uint64_t *acc_empty = acc_full + 2;     // [2] epilogue -> MMA
-    uint64_t *plan_full = acc_empty + 2;
+    uint64_t *acc_last = acc_empty + 2;     // MMA -> producers: the sums of the CTA's last piece are complete
+    uint64_t *plan_full = acc_last + 1;
     uint64_t *plan_empty = plan_full + PLAN_BUFS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(plan_empty + PLAN_BUFS);
     uint32_t *last_flags = tmem_slot + 1;     // [2] epilogue warps, producers: this CTA brought the last piece
@@ -200,6 +201,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
             ptx::mbar_init(&acc_full[b], 1);
             ptx::mbar_init(&acc_empty[b], EPI_WARPS);
         }
+        ptx::mbar_init(acc_last, 1);
         for (int b = 0; b < PLAN_BUFS; ++b) {
             ptx::mbar_init(&plan_full[b], PLANNER_WARPS);
             ptx::mbar_init(&plan_empty[b], GROUP_WARPS);
@@ -379,7 +381,8 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
             for (int k = 0; k < PGROUPS; ++k) it.next(g.K, chunks, W.tiles_y);
         }
         const int before = last_tile - first_tile, buf = before % acc_bufs;
-        ok = ok && ptx::mbar_wait(&acc_full[buf], (uint32_t)((before / acc_bufs) & 1));
+        // (a barrier of its own: tiles of one chunk are made faster than summed, and two pieces before acc_full looks alike)
+        ok = ok && ptx::mbar_wait(acc_last, 0);
         ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is a whole-warp instruction
         if (!ok && lane == 0) ptx::report(P.status, 108);
         ptx::tc_fence_after();
@@ -460,7 +463,7 @@ dcn_fwd_tc_kernel(const FwdParams<DIM> P, const __grid_constant__ CUtensorMap tm
                 if (++acc_i == NACC) acc_i = 0;
                 ++j;
                 if (--left == 0) {                            // the piece is complete
-                    ptx::mma_commit(&acc_full[buf]);
+                    ptx::mma_commit(i + 1 < n_local ? &acc_full[buf] : acc_last);
                     j = 0;
                     acc_i = 0;
                     left = min(n_chunks, n_local - i - 1);
@@ -634,7 +637,7 @@ int tuning_int(const char *name, int fallback) {
 size_t fwd_tc_smem_bytes(int dim, int mode, int bn, int stages) {
     const size_t stage = (size_t)A_TILE_BYTES * mode_col_parts(mode) + (size_t)bn * 128 * mode_mat_parts(mode);
     const size_t plan = (size_t)PLAN_BUFS * (1 << dim) * TILE_POS * 8;
-    return 1024 + stages * stage + plan + (3 * stages + 4 + 2 * PLAN_BUFS) * 8 + 16;
+    return 1024 + stages * stage + plan + (3 * stages + 5 + 2 * PLAN_BUFS) * 8 + 16;
 }
 
 // statically allocated shared memory of the kernel (tap table), which counts against the same 227 KB
