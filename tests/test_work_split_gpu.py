@@ -13,6 +13,8 @@ pytestmark = pytest.mark.gpu
 SPLITS = [
     # one tile, long reduction: two CTAs share it
     Case('one_long_tile', 2, False, 1, 256, 64, (9, 9), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 2, 1, True, 1.5),
+    # three tiles of 27 chunks: two CTAs each, whose halves differ by a chunk
+    Case('odd_halves', 2, False, 1, 192, 256, (17, 19), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
     # 150 tiles: two of them over a full wave, shared ranges with pieces at both ends of a CTA
     Case('wave_plus_two', 2, False, 2, 128, 64, (98, 97), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
     # several tiles per CTA, two groups: tiles of one group follow those of the other

@@ -87,7 +87,7 @@ void take_sample_buffers(Plan &pl, Bump &b, const GeoHost &g, int bn, bool share
     take_parts(pl.w_pack, b, mode_mat_parts(pl.mode), packed_elems(g));
     if (!share_tiles) return;
     size_t partial = 0;
-    fwd_tc_workspace(g, bn, &partial, &pl.sg_counters);
+    fwd_tc_workspace(g, pl.mode, bn, &partial, &pl.sg_counters);
     if (partial > 0) {
         pl.sg_partial = b.take(partial);
         pl.sg_arrived = b.take(pl.sg_counters * sizeof(unsigned));

@@ -106,7 +106,7 @@ bool fwd_tc_config(const GeoHost &h, int mode, int *bn, int *stages);
 cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl, void *const *w_parts,
                                   const float *offset, const float *mask, const float *bias, const ColumnRange &range,
                                   void *out, float *partial, unsigned *arrived, const Status &status, cudaStream_t stream);
-void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters);   // partial sums of shared tiles
+void fwd_tc_workspace(const GeoHost &h, int mode, int bn, size_t *partial_bytes, size_t *counters);   // partial sums of shared tiles
 bool wgrad_tc_config(const GeoHost &h, int mode, int *n_sub, int *m_tiles, int *stages);
 cudaError_t launch_sample_wgrad_tc(const GeoHost &h, int mode, void *const *dense_parts, int pitch, const void *img_cl,
                                    const float *offset, const float *mask, const ColumnRange &range, float *gw,

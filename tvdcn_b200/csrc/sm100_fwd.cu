@@ -14,7 +14,7 @@
 // Work is cut into chunk-sized units ordered tile by tile; the grid has at most one CTA per SM and each takes an equal,
 // contiguous range of units.  So a CTA runs through its tiles without starting over (2048 tiles x 8 groups of 5 chunks
 // were 16384 CTAs whose start-up and epilogue outlasted their main loops), the SMs finish together where the tiles make
-// 5.3 waves, and a handful of tiles with long reductions is spread over the whole chip.  A tile that several CTAs share
+// 5.3 waves, and a handful of tiles with long reductions is spread over the chip, two CTAs to a tile.  A tile that several CTAs share
 // is summed from partial results in the workspace by whichever of them arrives last, in a fixed order; nobody waits.
 //
 // Warp roles (896 threads): warps 0-15 producers, 16-19 planners, 20-23 epilogue, 24 MMA issue + TMEM owner, 25 TMA,
@@ -36,11 +36,13 @@ struct FwdWork {
     int n_chunks;           // units per tile: taps x 64-channel chunks
     int ctas;
     int whole;              // no tile is shared
-    int base, extra;        // CTA c has `base` units (whole: tiles), the first `extra` CTAs one more
+    int halves;             // every tile is shared by two CTAs, 2 t and 2 t + 1
+    int base, extra;        // else CTA c has `base` units (whole: tiles), the first `extra` CTAs one more
 
     // First unit of CTA c.  A piece of one chunk is not worth its trip through the workspace: it stays with its neighbour.
     // (32-bit arithmetic: every role of every CTA starts with it.)
     __host__ __device__ int bound(int c) const {
+        if (halves) return (c >> 1) * n_chunks + ((c & 1) ? (n_chunks + 1) / 2 : 0);
         const int b = c * base + (c < extra ? c : extra);
         if (whole) return b * n_chunks;
         const int r = b % n_chunks;
@@ -48,6 +50,10 @@ struct FwdWork {
     }
     // the CTA that has a unit
     __host__ __device__ int owner(int unit) const {
+        if (halves) {
+            const int t = unit / n_chunks;
+            return 2 * t + (unit - t * n_chunks >= (n_chunks + 1) / 2 ? 1 : 0);
+        }
         const int wide = extra * (base + 1);
         int c = unit < wide ? unit / (base + 1) : extra + (unit - wide) / base;
         if (c + 1 < ctas && bound(c + 1) <= unit) ++c;     // the neighbour's, after its bound was moved by one
@@ -643,7 +649,7 @@ size_t fwd_tc_smem_bytes(int dim, int mode, int bn, int stages) {
 // statically allocated shared memory of the kernel (tap table), which counts against the same 227 KB
 static size_t fwd_static_smem(int dim) { return (size_t)FWD_MAX_TAPS * dim * sizeof(int16_t) + 128; }
 
-static bool fwd_work(const GeoHost &h, int bn, bool may_share, FwdWork *w) {
+static bool fwd_work(const GeoHost &h, int mode, int bn, bool may_share, FwdWork *w) {
     const long long tiles_x = ((long long)h.B * h.P + TILE_POS - 1) / TILE_POS, tiles_y = h.groups * ((h.Cd / h.groups) / bn);
     w->n_chunks = h.K * (h.Cs / h.groups / CHUNK_C);
     const long long units = tiles_x * tiles_y * w->n_chunks;
@@ -651,13 +657,23 @@ static bool fwd_work(const GeoHost &h, int bn, bool may_share, FwdWork *w) {
     w->n_tiles = (int)(tiles_x * tiles_y);
     w->tiles_y = (int)tiles_y;
     // Sharing tiles evens out the last wave, or spreads few tiles over the chip: each SM then takes units / SMs chunks
-    // instead of whole tiles.  A shared tile costs the time of about eight chunks, sixteen with 256 dense channels (its sums
-    // go through the workspace: 15 tiles of 27 chunks took 48 us shared, 30 whole); the fewer pieces the better, so few
-    // tiles are shared by two CTAs each.
+    // instead of whole tiles.  What it costs, in chunks: a piece of 128 x bn sums goes to the workspace, and whoever comes last
+    // reads all of a tile's.  Two CTAs per tile (`halves`) end with their only piece, which their 16 producer warps take out
+    // together; in equal ranges of units most CTAs also begin with the rest of a tile, which falls to the four epilogue
+    // warps.  (Halves cut by equal ranges drift against the tiles where their chunks are odd: 37 tiles of 27 chunks of 256
+    // bf16 channels took 56 us, cut exactly 38, whole 39.)  A chunk of f32 data takes twice the time, so it counts half.
+    // Fitted to 1700 calls of 1 to 600 tiles of 4 to 72 chunks, each timed both ways: these lines lose 0.1 % against the better
+    // side on average and 10 % at worst (8 chunks for all, 16 with 256 channels: 1.0 % and 28 %).  Microseconds, whole /
+    // shared, 37 tiles of 36 chunks of 64, 128, 256 channels: bf16 43 / 33, 45 / 37, 46 / 41; f32 67 / 45, 73 / 51, 80 / 59; 150
+    // tiles of 36 chunks: bf16 74 / 54, 77 / 58, 78 / 67; f32 124 / 80, 129 / 91, 157 / 117.
+    constexpr int HALVES[2][3] = {{6, 6, 11}, {3, 3, 5}}, RANGES[2][3] = {{7, 12, 22}, {4, 5, 11}};   // [f32][64, 128, 256 channels]
     const long long sms = 148;
     const long long shared = std::min(sms, std::min(units / 3, 2LL * w->n_tiles));
+    const bool two_each = shared == 2LL * w->n_tiles;
+    const int cost = (two_each ? HALVES : RANGES)[mode_f32(mode)][bn / 128];
     const long long whole_time = (w->n_tiles + sms - 1) / sms * w->n_chunks;
-    w->whole = !may_share || w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + (bn > 128 ? 16 : 8);
+    w->whole = !may_share || w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + cost;
+    w->halves = !w->whole && two_each;
     w->ctas = (int)(w->whole ? std::max(1LL, std::min<long long>(sms, w->n_tiles)) : shared);   // 1: an empty batch, planned but not launched
     const long long items = w->whole ? w->n_tiles : units;
     w->base = (int)(items / w->ctas);
@@ -682,7 +698,7 @@ bool fwd_tc_config(const GeoHost &h, int mode, int *bn, int *stages) {
         if (s != 0) { n = cand_n; break; }
     }
     FwdWork work;
-    if (n == 0 || !fwd_work(h, n, false, &work)) return false;
+    if (n == 0 || !fwd_work(h, mode, n, false, &work)) return false;
     *bn = n;
     *stages = s;
     return true;
@@ -697,10 +713,10 @@ cudaError_t launch_fwd_tc_t(const GeoHost &h, const FwdParams<DIM> &P, const CUt
 }
 
 // Bytes of the partial sums and number of arrival counters that a launch needs in its workspace (0: no tile is shared).
-void fwd_tc_workspace(const GeoHost &h, int bn, size_t *partial_bytes, size_t *counters) {
+void fwd_tc_workspace(const GeoHost &h, int mode, int bn, size_t *partial_bytes, size_t *counters) {
     FwdWork w;
     *partial_bytes = *counters = 0;
-    if (!fwd_work(h, bn, true, &w) || w.whole) return;
+    if (!fwd_work(h, mode, bn, true, &w) || w.whole) return;
     *partial_bytes = (size_t)w.ctas * 2 * bn * TILE_POS * sizeof(float);
     *counters = (size_t)w.n_tiles;
 }
@@ -714,7 +730,7 @@ cudaError_t launch_sample_gemm_tc(const GeoHost &h, int mode, const void *img_cl
     int bn = 0, stages = 0;
     if (!fwd_tc_config(h, mode, &bn, &stages)) return cudaErrorInvalidConfiguration;
     FwdWork work;
-    if (!fwd_work(h, bn, partial != nullptr, &work)) return cudaErrorInvalidConfiguration;
+    if (!fwd_work(h, mode, bn, partial != nullptr, &work)) return cudaErrorInvalidConfiguration;
     CUtensorMap maps[3];
     const uint64_t dims[4] = {(uint64_t)csg, (uint64_t)cdg, (uint64_t)h.K, (uint64_t)h.groups};
     const uint64_t strides[3] = {(uint64_t)csg * 2, (uint64_t)csg * cdg * 2, (uint64_t)csg * cdg * h.K * 2};
