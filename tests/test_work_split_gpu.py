@@ -76,6 +76,15 @@ def test_volume_with_one_cta_per_tile():
     cases.assert_parity(run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1), 1e-4, case.name)
 
 
+@pytest.mark.parametrize('width', [58, 60], ids=['ranges', 'one_per_tile'])
+def test_volume_of_16_bit_data_around_its_line(width):
+    """290 and 300 tiles: 16-bit volumes have one CTA per tile from 296 on."""
+    case = Case('volume16', 3, False, 1, 64, 64, (16, 40, width), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0)
+    x, w, off, mask, bias, go = (t.float().cuda() for t in make_inputs(case, seed=77))
+    dev = [x.bfloat16(), w.bfloat16(), off, mask, bias, go.bfloat16()]
+    cases.assert_parity(run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1), 2e-2, case.name)
+
+
 @pytest.mark.parametrize('batch,simt', [(148, True), (149, False)], ids=['one_wave', 'more'])
 def test_small_padded_transposed_forward_stays_simt(batch, simt):
     case = Case('tiny_T', 1, True, batch, 8, 16, (64,), (4,), (2,), (1,), (1,), (), 1, 1, 1, True, 1.5)

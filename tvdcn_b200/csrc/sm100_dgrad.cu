@@ -997,9 +997,13 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, c
     const size_t smem = dgrad_smem_bytes(DIM, MODE, P.tb, P.b_stages);
     const bool coord = P.goff != nullptr || P.gmask != nullptr;
     // One CTA per SM, except for volumes of many tiles: 27 taps of 8 corners dwarf a CTA's start-up, and the tiles' costs
-    // differ so much that the hardware's scheduling beats equal ranges (4.19 against 4.36 ms).
-    const int tiles = P.total_units / P.n_units;
-    const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= 4 * 148 ? tiles : std::min(P.total_units, 148)));
+    // differ so much that the hardware's scheduling beats equal ranges.  Backward calls, us, ranges / one CTA per tile: 16-bit
+    // data gain from two tiles per SM on (216 tiles 400 / 410, 296 491 / 486, 440 761 / 705, 1032 1723 / 1638, at worst 3.5 % lost at
+    // 392 tiles), f32 data, with its longer loads of a dense tile, from some ten on (440 817 / 826, 1036 1848 / 1895, 3136 6089 / 5798,
+    // 4096 8900 / 8039; between 3 and 10 per SM either side wins 4 % at most, so the line is at four).  Eight taps have too
+    // few units per tile (2651 tiles 1362 / 1402).
+    const int tiles = P.total_units / P.n_units, many = (Mode<MODE>::F32 ? 4 : 2) * 148;
+    const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= many ? tiles : std::min(P.total_units, 148)));
     LaunchScope scope("dcn_dgrad_tc", stream);
     if (coord)
         return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, true>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
