@@ -812,8 +812,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         int4 info = describe(u);
         load_unit(pi, info, ru);
         ru_next = ru;
-        bool new_tile = false;
-        uint32_t free_phase = 0;
+        uint32_t reload = 0;     // bit 0: the unit begins a new tile; bit 1: the phase of a_free (one register, they are short)
         for (int j = 0; j < n_units && ok; ++j) {
             const int pb = j & 1;
             if (j >= 2) {
@@ -831,12 +830,12 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             const int4 info_next = describe(u_next);
             if (j + 1 < n_units) load_unit(pi_next, info_next, ru_next);
             build(info, pb, ru);
-            if (new_tile) {
+            if (reload & 1u) {
                 // One phase of a_free per tile, and the next one cannot complete before this load: neither an earlier
                 // phase nor a later one is taken for it.  (The barriers of the accumulators do not serve: with a single
                 // accumulator the pass two before looks like the one before this unit.)
-                ok = wait_all(a_free, free_phase);
-                free_phase ^= 1u;
+                ok = wait_all(a_free, reload >> 1);
+                reload ^= 2u;
                 if (!ok) {
                     if (pt == 0) ptx::report(P.status, 309);
                     break;
@@ -848,7 +847,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             u = u_next;
             pi = pi_next;
             info = info_next;
-            new_tile = next_new;
+            reload = (reload & 2u) | (next_new ? 1u : 0u);
         }
     } else if (warp == SC_MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
