@@ -111,6 +111,41 @@ def test_problems_too_large_for_the_tensor_kernels_are_planned_on_the_simt_ones(
     assert backward_bytes(2_700_000) > 2_700_000 * 3072 and backward_bytes(3_000_000) < 3_000_000 * 3072
 
 
+@pytest.mark.parametrize('dim,transposed,dtype,cin,cout,positions,taps,backward,engine', [
+    # one tap: up to 16 of 64 sampled channels, up to 64 dense ones
+    (2, False, 'F32', 16, 64, 1024, 1, 0, 'simt'), (2, False, 'BF16', 16, 16, 1024, 1, 0, 'simt'),
+    (2, False, 'F32', 17, 16, 1024, 1, 0, 'tcgen05'), (2, False, 'F32', 16, 72, 1024, 1, 0, 'tcgen05'),
+    (2, False, 'F32', 16, 64, 1024, 9, 0, 'tcgen05'), (2, False, 'F32', 16, 64, 1024, 1, 1, 'tcgen05'),
+    # 1-d f32: 8 and 9 channels; backward only above 32768 positions
+    (1, False, 'F32', 9, 32, 1024, 5, 0, 'simt'), (1, False, 'F32', 10, 32, 1024, 5, 0, 'tcgen05'),
+    (1, False, 'F32', 8, 40, 1024, 5, 0, 'tcgen05'), (1, False, 'BF16', 8, 8, 1024, 5, 0, 'tcgen05'),
+    (1, False, 'F32', 8, 8, 32768, 5, 1, 'tcgen05'), (1, False, 'F32', 8, 8, 32769, 5, 1, 'simt'),
+    # transposed forward: 8 to 10 sampled channels above 4096 (f32) or 65536 positions
+    (2, True, 'F32', 8, 10, 4096, 16, 0, 'tcgen05'), (2, True, 'F32', 8, 10, 4225, 16, 0, 'simt'),
+    (2, True, 'F32', 8, 11, 4225, 16, 0, 'tcgen05'), (2, True, 'F32', 72, 8, 4225, 16, 0, 'tcgen05'),
+    (2, True, 'BF16', 8, 8, 65536, 16, 0, 'tcgen05'), (2, True, 'BF16', 8, 8, 66049, 16, 0, 'simt'),
+    (2, True, 'F32', 8, 9, 33124, 16, 1, 'simt'), (2, True, 'F32', 8, 10, 33124, 16, 1, 'tcgen05'),
+    (1, True, 'F32', 8, 8, 40000, 4, 1, 'tcgen05'),
+    # transposed 1-d f32 forward within one wave of SIMT blocks
+    (1, True, 'F32', 16, 16, 64 * 148, 4, 0, 'simt'), (1, True, 'F32', 16, 16, 64 * 148 + 1, 4, 0, 'tcgen05'),
+    (1, True, 'F32', 17, 16, 330, 4, 0, 'tcgen05'), (1, True, 'BF16', 8, 16, 330, 4, 0, 'tcgen05'),
+    (2, True, 'F32', 8, 16, 324, 16, 0, 'tcgen05'),
+    # fewer than eight channels: never; not padded at all: always on the tensor cores
+    (2, False, 'F32', 7, 64, 1024, 9, 0, 'simt'), (1, True, 'F32', 64, 64, 64, 4, 0, 'tcgen05'),
+])
+def test_lines_between_the_engines(dim, transposed, dtype, cin, cout, positions, taps, backward, engine):
+    L = cabi.lib()
+    side = positions if dim == 1 else round(positions ** 0.5)
+    k = taps if dim == 1 else round(taps ** 0.5)
+    stride, pad = (2, (k - 2) // 2) if transposed else (1, k // 2)
+    p = cabi.make_problem(dim, transposed, getattr(cabi, dtype), 1, cin, cout, (side,) * dim, (k,) * dim, (stride,) * dim,
+                          (pad,) * dim, (1,) * dim, 1, 1, 1, aux_dtype=cabi.F32)
+    assert L.tvdcn_b200_engine_name(ctypes.byref(p), backward).decode() == engine
+    if engine == 'simt' and min(cin, cout) >= 8:    # asked for, the tensor cores still take it
+        p.engine = cabi.ENGINE_TENSOR
+        assert L.tvdcn_b200_engine_name(ctypes.byref(p), backward).decode() == 'tcgen05'
+
+
 @pytest.mark.parametrize('transposed', [False, True])
 @pytest.mark.parametrize('dtype', [cabi.F32, cabi.BF16])
 def test_workspace_sizes_of_an_empty_batch(transposed, dtype):

@@ -14,7 +14,10 @@ struct Bump {
         return at;
     }
 };
-// A granule of channels padded by more than this runs on the SIMT kernels.
+// A granule of channels padded by more than this runs on the SIMT kernels.  A tensor-core kernel's time does not depend on how
+// much of the 64 channels is real, a SIMT kernel's is proportional to it.  SIMT / tensor us at 4 x 128 x 128, 3 x 3 (f32; bf16),
+// forward and backward: 4 channels 45 / 75, 171 / 241; 43 / 57, 176 / 203.  8 channels 74 / 76, 303 / 240; 70 / 58, 315 / 203.
+// 12 channels 105 / 76, 343 / 240; 99 / 58, 357 / 203.
 constexpr int MAX_CHANNEL_PADDING = 8;
 bool is16(int dt) { return dt == DT_F16 || dt == DT_BF16; }
 
@@ -44,6 +47,32 @@ int mode_of(int dtype, bool wide) {
     if (dtype == DT_F32) return wide ? TC_F32_WIDE : TC_SPLIT;
     if (dtype == DT_F16) return wide ? TC_F16_WIDE : TC_F16;
     return wide ? TC_BF16_WIDE : TC_BF16;
+}
+
+// Calls that the tensor-core kernels take but the SIMT kernels finish sooner.  Figures: SIMT / tensor us, one granule.
+bool simt_is_faster(const tvdcn_problem *p, const GeoHost &g, bool backward) {
+    const int gran = g.gran, pad = g.gran_pad, cdg = g.Cd_r / g.groups;
+    const long long n = (long long)g.B * g.P * (g.Cs_r / gran);     // positions of all granules
+    const bool f32 = p->dtype == TVDCN_F32;
+    if (backward)
+        // 8 channels, f32.  1-d: 32000 positions 103 / 80, 120000 207 / 242, 400000 581 / 765, but 8 -> 64 channels 799 / 748; transposed
+        // 2-d: 32400 267 / 263, 65536 448 / 526, 262144 1753 / 2184, 3-d: 102400 4561 / 5203, but 1-d 480000 956 / 840.  10 channels:
+        // 720 / 773, 608 / 526.
+        return f32 && pad > 7 * gran && n > 32768 && (p->transposed ? g.dim > 1 && cdg <= 64 : g.dim == 1 && cdg <= 32);
+    if (!p->transposed)
+        // One tap, 102400 positions: f32 16 channels 32 / 39, 24 channels 49 / 41; bf16 31 / 33, 47 / 35; 8 -> 64 channels 35 / 39, 8 -> 128
+        // 60 / 59.  f32, 1-d, five taps: 8 channels 23 / 31 at 32000 positions, 785 / 867 at 1.6 million, 10 channels 29 / 31 and
+        // 971 / 869, 8 -> 64 channels at 400000 238 / 222.
+        return (g.K == 1 && pad >= 4 * gran && cdg <= 64) || (f32 && g.dim == 1 && pad > 7 * gran && cdg <= 32);
+    // The transposed forward has the widest accumulator to zero, scatter into and turn back.  2-d, 4 x 4 taps, 8 channels: f32
+    // 1000 positions 20 / 20, 5000 29 / 33, 65536 173 / 201, 262144 632 / 930; bf16 5000 31 / 31, 65536 179 / 191, 262144 644 / 921;
+    // 10 channels, bf16: 65536 224 / 190, 131044 427 / 383, 262144 829 / 921; 11 channels: 939 / 919.
+    if (pad > 6 * gran && cdg <= 64 && n > (f32 ? 4096 : 65536)) return true;
+    // f32, 1-d, up to one wave of SIMT blocks of one or two reduction steps (four taps, 330 positions, 8 -> 16 channels 16.4 / 18.5,
+    // 16 -> 16 18.4 / 18.4; 8 -> 16, 9400 positions 18.4 / 20.5): they are through before the tensor path's three kernels
+    // have started up.  16-bit data, whose SIMT sums are converted by a kernel of their own, 18.5 / 16.4; 2-d, 16 taps, 22.5 / 20.5.
+    const long long blocks = ((long long)g.B * g.P + 63) / 64 * g.groups * (((long long)g.Cs_r / g.groups * g.K + 63) / 64);
+    return f32 && g.dim == 1 && cdg <= 16 && blocks <= 148 && pad != gran;
 }
 
 // f32 data on the tensor cores: one accumulator may take about 2400 MMAs before the round-toward-zero error of
@@ -121,6 +150,7 @@ Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
     const GeoHost g = tc_geometry(make_geo_host(p));
     Bump b;
     const char *why = tc_common(p, g);
+    if (why == nullptr && p->engine == TVDCN_ENGINE_AUTO && simt_is_faster(p, g, false)) why = "the SIMT kernels are faster";
     pl.wide = !unpadded(p, g);
     pl.mode = mode_of(p->dtype, pl.wide);
     int bn = 0, st = 0, gbufs = 0;
@@ -134,12 +164,7 @@ Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
             why = "no tile configuration fits (or too many work units, or too long an f32 accumulation chain)";
         }
     } else if (why == nullptr) {
-        // One wave of SIMT blocks with one or two reduction steps is through before the three kernels of the tensor path
-        // have started up (8 -> 16 channels, 330 positions: 22 against 26 us of kernels).
-        const long long simt_blocks = ((long long)g.B * g.P + 63) / 64 * g.groups * (((long long)g.Cs_r / g.groups * g.K + 63) / 64);
-        if (pl.wide && p->engine == TVDCN_ENGINE_AUTO && g.Cd_r / g.groups <= 32 && simt_blocks <= 148) {
-            why = "so small that the SIMT kernel is faster";
-        } else if (dgrad_tc_config(g, pl.mode, &bn, &gbufs, &st)) {
+        if (dgrad_tc_config(g, pl.mode, &bn, &gbufs, &st)) {
             pl.tensor = pl.tc_gs = true;
             take_scatter_buffers(pl, b, g, true);
             take_aux(pl, b, p, g, true);
@@ -160,6 +185,7 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
     const GeoHost g = tc_geometry(make_geo_host(p));
     Bump b;
     const char *why = tc_common(p, g);
+    if (why == nullptr && p->engine == TVDCN_ENGINE_AUTO && simt_is_faster(p, g, true)) why = "the SIMT kernels are faster";
     pl.wide = !unpadded(p, g);
     pl.mode = mode_of(p->dtype, pl.wide);
     pl.mode_sw = mode_of(p->dtype, pl.wide || g.P % 8 != 0);
