@@ -2,6 +2,10 @@
 64, 16-bit offset / mask / bias, rows of the dense tensor that TMA cannot read (spatial extent off the multiples of 8).
 They must run there (ENGINE_TENSOR) and keep the precision of f32 columns: the tolerances are far inside those of the
 unpadded shapes (f32 data) or half a unit of the 16-bit results."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -48,6 +52,44 @@ def test_padded_and_widened_shapes(case, dtype, aux, tol):
     cases.assert_parity(got, ref, tol, case.name)
     from tvdcn_b200 import cabi
     assert cabi.lib().tvdcn_b200_device_status() == 0
+
+
+def test_padded_call_without_room_for_its_workspace_runs_on_the_simt_kernels():
+    """8 channels are padded to 64: the workspace of the tensor-core kernels is many times the tensors, and a program that
+    has no room for it must not fail for that.  A shape that needs no padding still raises.  In a process of its own, whose
+    allocator holds nothing else."""
+    run = subprocess.run([sys.executable, '-c', 'import test_wide_shapes_gpu as t; t.padded_call_without_room()'],
+                         cwd=os.path.dirname(__file__), capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-3000:]
+
+
+def padded_call_without_room():
+    from tvdcn_b200 import ops
+    dev = lambda *s: torch.randn(*s, device='cuda')
+    leaves = [dev(4, 8, 512, 512), dev(8, 8, 3, 3), dev(4, 18, 512, 512), torch.rand(4, 9, 512, 512, device='cuda'), dev(8)]
+    for t in leaves:
+        t.requires_grad_(True)
+    plain = [dev(4, 64, 512, 512), dev(64, 64, 3, 3), dev(4, 18, 128, 128)]     # workspace 268 MB, output 17 MB
+    grad = dev(4, 8, 512, 512)
+
+    def step():
+        out = ops.deform_conv2d(*leaves, padding=1)
+        return (out.detach(), *torch.autograd.grad(out, leaves, grad))
+    names, want = kernels_launched(step)
+    assert names.get('dcn_fwd_tc', 0) == 1 and names.get('dcn_dgrad_tc', 0) == 1, names
+    want = [t.cpu() for t in want]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    room = torch.cuda.memory_reserved() + (240 << 20)     # outputs and gradients 190 MB, workspaces 268 and 590 MB
+    try:
+        torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+        names, got = kernels_launched(step)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            ops.deform_conv2d(*plain, stride=4, padding=1)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert names.get('sample_gemm', 0) == 1 and names.get('gemm_scatter', 0) == 1 and names.get('sample_wgrad', 0) == 1, names
+    cases.assert_parity(got, want, 2e-5)
 
 
 @pytest.mark.parametrize('scales', [

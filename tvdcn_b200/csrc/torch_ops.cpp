@@ -307,8 +307,27 @@ void watch_this_call(int device, cudaStream_t stream) {
     if (w.pinned != nullptr) (void)tvdcn_b200_publish_status(w.pinned_dev, stream);
 }
 
-Tensor make_workspace(size_t bytes, const Tensor &like) {
-    return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));
+// Runs a call with its workspace.  Shapes that the tensor-core kernels take only with padding need several times their
+// tensors' memory, where the SIMT kernels need little or none: a program that has no room for the former gets the latter
+// (the C ABI takes them for such a shape when it is given less workspace).  run(workspace, bytes) returns the call's status.
+template <typename Run>
+int with_workspace(const tvdcn_problem &prob, size_t (*bytes_of)(const tvdcn_problem *), const Tensor &like, Run &&run) {
+    auto attempt = [&](size_t bytes, const Tensor &ws) { return run(bytes > 0 ? ws.data_ptr() : nullptr, bytes); };
+    auto allocate = [&](size_t bytes) { return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)); };
+    const size_t bytes = bytes_of(&prob);
+    Tensor ws;
+    try {
+        ws = allocate(bytes);
+    } catch (const c10::OutOfMemoryError &) {
+        tvdcn_problem simt = prob;
+        simt.engine = TVDCN_ENGINE_SIMT;
+        const size_t less = bytes_of(&simt);
+        if (less >= bytes) throw;
+        const int rc = attempt(less, allocate(less));
+        if (rc == TVDCN_ERR_WORKSPACE) throw;    // not such a shape: nothing was launched
+        return rc;
+    }
+    return attempt(bytes, ws);
 }
 
 const void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -323,12 +342,11 @@ Tensor forward_cuda_impl(const Tensor &input, const Tensor &weight, const OptTen
     std::vector<int64_t> shape{c.prob.batch, c.prob.out_channels};
     for (int a = 0; a < D; ++a) shape.push_back(c.prob.out_size[a]);
     Tensor out = at::empty(shape, c.input.options());
-    const size_t wsb = tvdcn_b200_forward_workspace_bytes(&c.prob);
-    Tensor ws = make_workspace(wsb, c.input);
     auto stream = at::cuda::getCurrentCUDAStream();
-    const int rc = tvdcn_b200_deform_conv_forward(&c.prob, ptr(c.input), ptr(c.weight), ptr(c.offset), ptr(c.mask),
-                                                  ptr(c.bias), out.data_ptr(), wsb ? ws.data_ptr() : nullptr, wsb,
-                                                  stream.stream());
+    const int rc = with_workspace(c.prob, tvdcn_b200_forward_workspace_bytes, c.input, [&](void *ws, size_t bytes) {
+        return tvdcn_b200_deform_conv_forward(&c.prob, ptr(c.input), ptr(c.weight), ptr(c.offset), ptr(c.mask), ptr(c.bias),
+                                              out.data_ptr(), ws, bytes, stream.stream());
+    });
     TORCH_CHECK(rc == TVDCN_OK, op_name<D, TR>(), ": ", tvdcn_b200_last_error());
     watch_this_call(input.device().index(), stream.stream());
     if (c.unbatched) out = out.squeeze(0);
@@ -357,14 +375,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> backward_cuda_impl(
     Tensor g_offset = c.offset.defined() ? at::empty_like(c.offset) : Tensor();
     Tensor g_mask = c.mask.defined() ? at::empty_like(c.mask) : Tensor();
     Tensor g_bias = c.bias.defined() ? at::empty_like(c.bias) : Tensor();
-    const size_t wsb = tvdcn_b200_backward_workspace_bytes(&c.prob);
-    Tensor ws = make_workspace(wsb, c.input);
     auto stream = at::cuda::getCurrentCUDAStream();
-    const int rc = tvdcn_b200_deform_conv_backward(
-        &c.prob, g.data_ptr(), ptr(c.input), ptr(c.weight), ptr(c.offset), ptr(c.mask), g_input.data_ptr(),
-        g_weight.data_ptr(), g_offset.defined() ? g_offset.data_ptr() : nullptr,
-        g_mask.defined() ? g_mask.data_ptr() : nullptr, g_bias.defined() ? g_bias.data_ptr() : nullptr,
-        wsb ? ws.data_ptr() : nullptr, wsb, stream.stream());
+    auto grad_ptr = [](const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; };
+    const int rc = with_workspace(c.prob, tvdcn_b200_backward_workspace_bytes, c.input, [&](void *ws, size_t bytes) {
+        return tvdcn_b200_deform_conv_backward(&c.prob, g.data_ptr(), ptr(c.input), ptr(c.weight), ptr(c.offset),
+                                               ptr(c.mask), grad_ptr(g_input), grad_ptr(g_weight), grad_ptr(g_offset),
+                                               grad_ptr(g_mask), grad_ptr(g_bias), ws, bytes, stream.stream());
+    });
     TORCH_CHECK(rc == TVDCN_OK, "_", op_name<D, TR>(), "_backward: ", tvdcn_b200_last_error());
     watch_this_call(input.device().index(), stream.stream());
     if (c.unbatched) {
