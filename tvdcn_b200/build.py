@@ -45,7 +45,6 @@ def build_cuda_library(verbose: bool = False, force: bool = False) -> Path:
     headers = sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh")) + sorted(INCLUDE.glob("*.h"))
     OBJ.mkdir(exist_ok=True)
     flags = list(NVCC_FLAGS) + (["-Xptxas", "-v"] if verbose else [])
-    flags += os.environ.get("TVDCN_B200_NVCC_FLAGS", "").split()   # extra flags for experiments
     jobs = []
     for src in cu:
         obj = OBJ / (src.stem + ".o")

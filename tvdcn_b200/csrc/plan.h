@@ -116,8 +116,6 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
                                    const void *img_cl, const float *offset, const float *mask, float *img_grad_cl,
                                    float *goff, float *gmask, const Status &status, cudaStream_t stream);
 
-int tuning_int(const char *name, int fallback);
-
 // Address of the per-device status word the tensor-core kernels report failed bounded waits in.
 int *device_status_word();
 

@@ -1025,17 +1025,15 @@ static bool dgrad_units(const GeoHost &h, int tb, int *tiles_x, int *per_tile, i
 // Taps per batch, accumulator ring and weight-ring depth that fit tensor memory and shared memory; false when
 // nothing fits (the dense tile of one group must fit tensor memory beside one accumulator) or the work is too much.
 bool dgrad_tc_config(const GeoHost &h, int mode, int *tb, int *nacc, int *b_stages) {
-    static const int tb_cap = tuning_int("TVDCN_B200_DG_TB", 4);
-    static const int st_cap = tuning_int("TVDCN_B200_DG_STAGES", 4);
     const int K = h.K, a_cols = (h.Cd / h.groups / 2) * mode_mat_parts(mode);
-    for (int cand = std::min(std::min(sc_tb_max(h.dim), tb_cap), K); cand >= 1; --cand) {
+    for (int cand = std::min(sc_tb_max(h.dim), K); cand >= 1; --cand) {
         // equal batches: the fewest batches of at most `cand` taps
         const int nb = (K + cand - 1) / cand;
         const int t = (K + nb - 1) / nb;
         const int n = t * SC_SLAB;
         const int acc = std::min(4, (SC_TMEM_COLS - a_cols) / (n * (mode == TC_F32_WIDE ? 2 : 1)));
         if (acc < 1) continue;
-        for (int st = std::min(st_cap, 4); st >= 2; --st)
+        for (int st = 4; st >= 2; --st)
             if (dgrad_smem_bytes(h.dim, mode, t, st) <= 227 * 1024) {
                 int tiles, per_tile, total;
                 if (!dgrad_units(h, t, &tiles, &per_tile, &total)) return false;

@@ -21,8 +21,6 @@
 // 26-27 idle.  The planners turn sampling coordinates into plan entries a few chunks ahead; the epilogue of a tile runs
 // under the main loop of the next one where tensor memory holds two sets of accumulators.
 #include <algorithm>
-#include <cstdio>
-#include <cstdlib>
 #include <type_traits>
 
 #include "plan.h"
@@ -631,14 +629,6 @@ bool make_tensor_map_16bit(CUtensorMap *map, const void *base, int rank, const u
     return rc == CUDA_SUCCESS;
 }
 
-// Tuning knob read from the environment (experiments only; the defaults are what is measured and reported).
-int tuning_int(const char *name, int fallback) {
-    const char *v = getenv(name);
-    if (v == nullptr || *v == 0) return fallback;
-    const int x = atoi(v);
-    return x > 0 ? x : fallback;
-}
-
 // ---- launcher -----------------------------------------------------------------------------------------
 size_t fwd_tc_smem_bytes(int dim, int mode, int bn, int stages) {
     const size_t stage = (size_t)A_TILE_BYTES * mode_col_parts(mode) + (size_t)bn * 128 * mode_mat_parts(mode);
@@ -685,15 +675,12 @@ static bool fwd_work(const GeoHost &h, int mode, int bn, bool may_share, FwdWork
 // or has 2^31 units of work or more.
 bool fwd_tc_config(const GeoHost &h, int mode, int *bn, int *stages) {
     const int cdg = h.Cd / h.groups;
-    static const int cap_split = tuning_int("TVDCN_B200_FWD_BN_SPLIT", 256);
-    static const int max_stages = tuning_int("TVDCN_B200_FWD_STAGES", 3);
-    const int cap = mode == TC_SPLIT ? cap_split : 256;
     // widest tile of dense channels first (the sampled tile is produced once per CTA, so a wider tile divides the
     // sampling work), then the deepest pipeline that fits
     int n = 0, s = 0;
     for (int cand_n : {256, 128, 64}) {
-        if (cand_n > cap || cdg % cand_n != 0) continue;
-        for (int cand = max_stages; cand >= 2; --cand)
+        if (cdg % cand_n != 0) continue;
+        for (int cand : {3, 2})
             if (fwd_tc_smem_bytes(h.dim, mode, cand_n, cand) + fwd_static_smem(h.dim) <= 227 * 1024) { s = cand; break; }
         if (s != 0) { n = cand_n; break; }
     }

@@ -490,16 +490,13 @@ bool wgrad_tc_config(const GeoHost &h, int mode, int *n_sub, int *m_tiles, int *
     // f32 data: twice the accumulators (see the modes), and two or three parts of every operand in shared memory
     const int mt = cdg > 128 && mode != TC_F32_WIDE ? 2 : 1;
     const int ns = wg_blocks(mode_f32(mode));
-    int s = 0;
-    static const int max_stages = tuning_int("TVDCN_B200_WG_STAGES", 2);
-    for (int cand = max_stages; cand >= 2; --cand)
-        if (wgrad_smem_bytes(h.dim, mode, ns, mt, cand) <= 227 * 1024) { s = cand; break; }
+    constexpr int STAGES = 2;
     dim3 grid;
     int per = 0;
-    if (s == 0 || !wgrad_grid(h, mode, ns, mt, &grid, &per)) return false;
+    if (wgrad_smem_bytes(h.dim, mode, ns, mt, STAGES) > 227 * 1024 || !wgrad_grid(h, mode, ns, mt, &grid, &per)) return false;
     *n_sub = ns;
     *m_tiles = mt;
-    *stages = s;
+    *stages = STAGES;
     return true;
 }
 
