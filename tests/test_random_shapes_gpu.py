@@ -1,6 +1,6 @@
 """Seeded random sweep over shapes: ragged extents, strides, dilations, groups, offset / mask groups, with and
 without offset / mask / bias, conv and transposed, 1d-3d.  Half of the draws have 64-channel multiples per group
-(tensor-core kernels, f32 split and bf16), the other half arbitrary channel counts (SIMT kernels, f32 and f64).
+(tensor-core kernels, f32 split and bf16), the other half fewer than eight channels (SIMT kernels, f32 and f64).
 
 Checker: the restated oracle in f64 on the CPU (itself pinned to the reference).  Tolerances as everywhere:
 1e-4 for f32 / f64 data, 2e-2 for bf16 data (normalised max error, f32 offset / mask / bias).
@@ -50,8 +50,8 @@ def draw_case(rng: random.Random, idx: int, tensor: bool) -> Case:
         padding = tuple(min(p, d * (k - 1)) for p, k, d in zip(padding, kernel, dilation))
         opad = tuple(rng.randint(0, max(s, d) - 1) for s, d in zip(stride, dilation))
     batch = rng.randint(1, 3)
-    # (positions per image are left ragged on purpose: the tensor-core weight gradient needs a multiple of 8 and
-    # hands the other shapes to the SIMT kernel, so both engines meet inside one backward call)
+    # (positions per image are left ragged on purpose: rows off the multiples of 8 are copied for the weight gradient's
+    # TMA loads, and its columns are then kept in more parts than those of the other kernels of the same call)
     return Case(f'rand{idx}', dim, transposed, batch, cin, cout, in_size, kernel, stride, padding, dilation, opad,
                 groups, og, mg, rng.random() < 0.7, rng.choice([0.5, 1.5, 3.0]))
 

@@ -87,9 +87,7 @@ def test_forward_backward_all_tensor(case, dtype, tol):
     names, got = kernels_launched(lambda: cases.run_cabi(case, *(None if t is None else t.cuda() for t in dev)))
     assert names.get('dcn_fwd_tc', 0) == 1 and names.get('dcn_dgrad_tc', 0) == 1, names
     assert 'sample_gemm' not in names and 'gemm_scatter' not in names, names
-    import math
-    if math.prod(case.out_size) % 8 == 0:  # row pitch of grad_output must be TMA-loadable
-        assert names.get('dcn_wgrad_tc', 0) == 1 and 'sample_wgrad' not in names, names
+    assert names.get('dcn_wgrad_tc', 0) == 1 and 'sample_wgrad' not in names, names
     cases.assert_parity(got, ref, tol, case.name)
     from tvdcn_b200 import cabi
     assert cabi.lib().tvdcn_b200_device_status() == 0
@@ -140,7 +138,7 @@ def test_non_finite_pixel_does_not_leak_through_out_of_image_corners(dtype):
 @pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16], ids=['f32split', 'bf16'])
 def test_backward_reuses_the_forward_staging(dtype):
     """TVDCN_FLAG_REUSE_STAGED_INPUT: a backward call on the forward call's workspace gives the same gradients as
-    one that stages the input itself, with one launch less."""
+    one that stages the input itself, without reading the input."""
     from tvdcn_b200 import cabi
     L = cabi.lib()
     case = Case('reuse', 2, False, 3, 128, 64, (9, 10), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 2, 1, True, 1.5)
@@ -155,9 +153,9 @@ def test_backward_reuses_the_forward_staging(dtype):
     st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     out = torch.empty(case.batch, case.out_channels, *case.out_size, dtype=dtype, device='cuda')
 
-    def backward(prob):
+    def backward(prob, inp=x):
         g = [torch.full_like(t, float('nan')) for t in (x, w, off, mask, bias)]
-        cabi.check(L.tvdcn_b200_deform_conv_backward(ctypes.byref(prob), vp(go), vp(x), vp(w), vp(off), vp(mask),
+        cabi.check(L.tvdcn_b200_deform_conv_backward(ctypes.byref(prob), vp(go), vp(inp), vp(w), vp(off), vp(mask),
                                                      vp(g[0]), vp(g[1]), vp(g[2]), vp(g[3]), vp(g[4]), vp(ws), n, st))
         return g
 
@@ -165,9 +163,9 @@ def test_backward_reuses_the_forward_staging(dtype):
     ws.fill_(0xff)                           # nothing useful left in the workspace
     cabi.check(L.tvdcn_b200_deform_conv_forward(ctypes.byref(p), vp(x), vp(w), vp(off), vp(mask), vp(bias), vp(out),
                                                 vp(ws), n, st))
-    names, got = kernels_launched(lambda: backward(q))
-    # the input staging was reused, and grad_output is read in the caller's layout: nothing is re-laid out
-    assert names.get('to_channels_last', 0) == 0, names
+    # an input of NaNs in the place of the staged one is never looked at: the staging was reused
+    names, got = kernels_launched(lambda: backward(q, torch.full_like(x, float('nan'))))
+    assert names.get('dcn_wgrad_tc', 0) == 1 and names.get('dcn_dgrad_tc', 0) == 1, names
     # same arithmetic, but the f32 atomics land in another order: a bf16 result may round the other way
     tol = 1e-5 if dtype == torch.float32 else 4e-3
     for a, b in zip(got, base):

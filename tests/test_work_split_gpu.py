@@ -1,6 +1,8 @@
 """Edges of how the tensor-core kernels share their work between CTAs: forward tiles that two CTAs sum together, CTAs that
 walk several tiles (the next dense tile is loaded under the old one), remainders of the split, volumes with one CTA per
 tile, and the line below which a padded transposed forward stays on the SIMT kernel."""
+import threading
+
 import pytest
 import torch
 
@@ -66,6 +68,31 @@ def test_last_tile_of_a_cta_is_read_behind_its_last_mma(dtype):
     assert nerr(first, ref) <= (1e-4 if dtype == torch.float32 else 2e-2)
     for _ in range(25):
         assert torch.equal(run_cabi(case, *dev, engine=2)[0], first)
+
+
+def test_shared_tiles_of_calls_that_overlap():
+    """Two host threads on two streams through tiles that CTAs share: partial sums and arrival counters are each call's own,
+    so every call gives the bits of the same call alone."""
+    from tvdcn_b200 import ops
+    jobs = []
+    for case in (SPLITS[0], SPLITS[1]):      # one tile of 36 chunks; three of 27
+        x, w, off, mask, bias, _ = (t.float().cuda() for t in make_inputs(case, seed=78))
+        jobs.append((torch.cuda.Stream(), lambda a=(x, w, off, mask, bias): ops.deform_conv2d(*a, padding=1)))
+    want = [job() for _, job in jobs]
+    torch.cuda.synchronize()
+    results = [[], []]
+
+    def work(i):
+        with torch.cuda.stream(jobs[i][0]):
+            results[i] = [jobs[i][1]() for _ in range(40)]
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for one, many in zip(want, results):
+        assert len(many) == 40 and all(torch.equal(one, r) for r in many)
 
 
 def test_volume_with_one_cta_per_tile():
