@@ -44,7 +44,7 @@ typedef enum tvdcn_status {
 
 /* Which implementation may be chosen for the GEMM-shaped parts. */
 typedef enum tvdcn_engine {
-    TVDCN_ENGINE_AUTO = 0,     /* tensor-core (tcgen05) kernels where the shape allows, else SIMT */
+    TVDCN_ENGINE_AUTO = 0,     /* tensor-core (tcgen05) kernels where they are faster, else SIMT    */
     TVDCN_ENGINE_SIMT = 1,     /* force the generic SIMT kernels (any shape, any dtype)            */
     TVDCN_ENGINE_TENSOR = 2    /* require the tensor-core kernels; TVDCN_ERR_UNSUPPORTED otherwise */
 } tvdcn_engine;
@@ -175,9 +175,9 @@ size_t tvdcn_b200_static_scratch_bytes(void);
  * gradient pointer skips that gradient.  grad_bias has out_channels elements.
  *
  * Streams: everything is ordered by cuda_stream.  When the tensor-core kernels run, the weight gradient and the
- * bias sum are queued on a second, library-owned stream that forks from cuda_stream and joins it again before
- * the call returns (event waits only, nothing blocks the host); work queued on cuda_stream after the call sees
- * all results.  The library creates that stream and its two events once per host thread and device, on the
+ * bias sum are queued on cuda_stream itself, and the other gradients beside them on a second, library-owned stream that
+ * forks from cuda_stream and joins it again before the call returns (event waits only, nothing blocks the host); work
+ * queued on cuda_stream after the call sees all results.  The library creates that stream and its two events once per host thread and device, on the
  * first such call (make it outside any stream capture).  TVDCN_B200_OVERLAP=0 in the environment keeps all
  * kernels on cuda_stream.
  */
@@ -191,8 +191,8 @@ int tvdcn_b200_deform_conv_backward(const tvdcn_problem *p,
                                     void *cuda_stream);
 
 /* The same call with one more argument for data-parallel training: `weight_grad_ready`, a cudaEvent_t the caller
- * owns (or NULL), is recorded as soon as grad_weight and grad_bias hold their final values -- on the library's
- * second stream when it is in use, well before the input / offset / mask gradients are done -- so that the
+ * owns (or NULL), is recorded on cuda_stream as soon as grad_weight and grad_bias hold their final values -- where the
+ * library's second stream is in use, well before the input / offset / mask gradients are done there -- so that the
  * all-reduce of the weight gradients can start under the rest of the backward pass.  No counterpart in the
  * reference (its backward, tvdcn/csrc/ops/cuda/deform_conv2d_kernel.cpp:387-642, has no streams and no
  * multi-GPU path). */
