@@ -331,23 +331,23 @@ def known_traffic(kernel: str, config: int, mode: str):
     under profiles/; None where no capture exists.  The figures are for the configuration's full batch on one GPU."""
     table = {
         # config 2: full-size launches (profiles/config2_tensor_kernels.md)
-        'dcn_fwd_tc/cfg2/bf16': 85.16e6 + 20.91e6,
-        'dcn_dgrad_tc/cfg2/bf16': 330.5e6 + 102.6e6,
-        'dcn_wgrad_tc/cfg2/bf16': 137.7e6 + 3.81e6,
-        'dcn_fwd_tc/cfg2/fp32': 137.8e6 + 64.83e6,
-        'dcn_dgrad_tc/cfg2/fp32': 487.1e6 + 116.9e6,
-        'dcn_wgrad_tc/cfg2/fp32': 243.0e6 + 7.46e6,
+        'dcn_fwd_tc/cfg2/bf16': 118.6e6 + 49.6e6,
+        'dcn_dgrad_tc/cfg2/bf16': 446.8e6 + 234.9e6,
+        'dcn_wgrad_tc/cfg2/bf16': 137.7e6 + 3.88e6,
+        'dcn_fwd_tc/cfg2/fp32': 220.4e6 + 99.5e6,
+        'dcn_dgrad_tc/cfg2/fp32': 768.0e6 + 281.1e6,
+        'dcn_wgrad_tc/cfg2/fp32': 250.7e6 + 5.93e6,
         # configs 3-5: captured on a cut batch (profiles/config3_config4_config5_tensor_kernels.md) and scaled to
         # the full batch by the images processed -- tiles are independent, traffic grows in proportion
-        'dcn_fwd_tc/cfg3/fp32': (73.8e6 + 29.55e6) * 8,
-        'dcn_dgrad_tc/cfg3/fp32': (214.6e6 + 44.33e6) * 8,
-        'dcn_wgrad_tc/cfg3/fp32': (141.5e6 + 4.76e6) * 8,
-        'dcn_fwd_tc/cfg4/fp32': (70.56e6 + 7.59e6) * 4,
-        'dcn_dgrad_tc/cfg4/fp32': (229.9e6 + 61.28e6) * 4,
-        'dcn_wgrad_tc/cfg4/fp32': (95.28e6 + 3.93e6) * 4,
-        'dcn_fwd_tc/cfg5/fp32': (40.98e6 + 0.15e6) * 4,
-        'dcn_dgrad_tc/cfg5/fp32': (58.56e6 + 0.50e6 + 63.9e6 + 1.27e6) / 2 * 4,   # two launches per step, mean
-        'dcn_wgrad_tc/cfg5/fp32': (57.76e6 + 0.70e6) * 4,
+        'dcn_fwd_tc/cfg3/fp32': (75.54e6 + 26.47e6) * 8,
+        'dcn_dgrad_tc/cfg3/fp32': (223.1e6 + 45.46e6) * 8,
+        'dcn_wgrad_tc/cfg3/fp32': (141.0e6 + 3.73e6) * 8,
+        'dcn_fwd_tc/cfg4/fp32': (72.93e6 + 13.54e6) * 4,
+        'dcn_dgrad_tc/cfg4/fp32': (164.9e6 + 35.47e6) * 4,
+        'dcn_wgrad_tc/cfg4/fp32': (96.05e6 + 5.36e6) * 4,
+        'dcn_fwd_tc/cfg5/fp32': (41.01e6 + 0.17e6) * 4,
+        'dcn_dgrad_tc/cfg5/fp32': (58.24e6 + 0.10e6 + 63.64e6 + 1.11e6) / 2 * 4,   # two launches per step, mean
+        'dcn_wgrad_tc/cfg5/fp32': (57.75e6 + 0.61e6) * 4,
     }
     return table.get(f'{kernel}/cfg{config}/{mode}')
 
