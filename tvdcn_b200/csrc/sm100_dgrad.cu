@@ -155,7 +155,7 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
     L.pos = o;  o += 2 * TILE_POS * 8;            // and per position of the tile: image (or -1), position in it
     L.cnt = o;  o += SC_SLOTS * 4;
     L.taps = o; o += SC_MAX_TAPS * 3 * 2;         // kernel coordinates of every tap (int16)
-    L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot
+    L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot, reloads
     L.bars = o; o += (uint32_t)(21 + 2 * b_stages) * 8;
     L.total = o;
     return L;
@@ -239,6 +239,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint32_t *wait_flag = misc + 4;
     uint32_t *n_entries = misc + 6;      // [2]
     uint32_t *tmem_slot = misc + 8;
+    uint32_t *reloads = misc + 9;        // f32 data: dense tiles behind the first that the planners have loaded
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
     uint64_t *a_first = bars;            // dense tile of the CTA's first unit is in TMEM / of every later tile
     uint64_t *a_next = bars + 1;
@@ -277,6 +278,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         ptx::mbar_init(a_first, SC_LOAD_WARPS);
         ptx::mbar_init(a_next, SC_PLAN_WARPS);
         ptx::mbar_init(a_free, 1);
+        *reloads = 0u;
         for (int s = 0; s < BS; ++s) {
             ptx::mbar_init(&b_full[s], 1);
             ptx::mbar_init(&b_empty[s], 1);
@@ -834,9 +836,22 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 // One phase of a_free per tile, and the next one cannot complete before this load: neither an earlier
                 // phase nor a later one is taken for it.  (The barriers of the accumulators do not serve: with a single
                 // accumulator the pass two before looks like the one before this unit.)
-                // (The phase from the tile's order: kept in a register it costs the f32 volume kernel 1 %, packed into new_tile the
-                // 16-bit 2-d kernel 7 %.)
-                ok = wait_all(a_free, (uint32_t)((u.order - unit0 / P.n_units - 1) & 1));
+                // (The planners are short of registers.  The phase in one of its own cost the f32 volume kernel 1 %; from the tile's
+                // order it costs 16-bit data nothing, but the f32 transposed forward 2 %; counted in shared memory f32 data nothing,
+                // 16-bit 2-d 7 %.)
+                if (pt == 0) {
+                    uint32_t before;            // tiles this CTA has reloaded
+                    if constexpr (M::F32) {
+                        before = *reloads;
+                        *reloads = before + 1u;
+                    } else {
+                        before = (uint32_t)(u.order - unit0 / P.n_units - 1);
+                    }
+                    *wait_flag = ptx::mbar_wait_backoff<SC_SLEEP_NS>(a_free, before & 1u) ? 1u : 0u;
+                }
+                planner_barrier();
+                ok = *wait_flag != 0u;
+                planner_barrier();
                 if (!ok) {
                     if (pt == 0) ptx::report(P.status, 309);
                     break;
