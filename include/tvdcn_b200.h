@@ -95,7 +95,7 @@ typedef struct tvdcn_problem {
  * The caller vouches for all of that, and for passing both calls the same workspace_bytes; with the flag clear the
  * backward call stages the input itself.
  * Ignored where no staging exists (SIMT kernels, a forward call that took them because its workspace was too small
- * for the tensor-core kernels, transposed operator).
+ * for the tensor-core kernels, transposed operator) or lacks something (f16, a grid off the multiples of 8).
  */
 #define TVDCN_FLAG_REUSE_STAGED_INPUT 1
 

@@ -174,6 +174,32 @@ def test_backward_reuses_the_forward_staging(dtype):
     assert L.tvdcn_b200_device_status() == 0
 
 
+@pytest.mark.parametrize('case', [
+    # only the weight gradient is wide (63 positions): the forward call leaves no maxima of the image
+    Case('reuse_f16_odd', 2, False, 2, 64, 64, (7, 9), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+    # both calls are wide
+    Case('reuse_f16_wide', 2, False, 2, 40, 64, (8, 8), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.5),
+], ids=lambda c: c.name)
+def test_reuse_flag_with_f16_data(case):
+    from tvdcn_b200 import cabi
+    L = cabi.lib()
+    x, w, off, mask, bias, go = make_inputs(case, seed=7, dtype=torch.float32)
+    x, w, off, mask, bias, go = (t.cuda() for t in ((x * 1000).half(), w.half(), off, mask * 100, bias, (go / 1000).half()))
+    p = cases.cabi_problem(case, torch.float16, torch.float32)
+    p.flags = cabi.FLAG_REUSE_STAGED_INPUT
+    n = max(L.tvdcn_b200_forward_workspace_bytes(ctypes.byref(p)), L.tvdcn_b200_backward_workspace_bytes(ctypes.byref(p)))
+    ws = torch.full((n,), 0x7b, dtype=torch.uint8, device='cuda')
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    out, gw = torch.full_like(go, float('nan')), torch.full_like(w, float('nan'))
+    cabi.check(L.tvdcn_b200_deform_conv_forward(ctypes.byref(p), vp(x), vp(w), vp(off), vp(mask), vp(bias), vp(out),
+                                                vp(ws), n, st))
+    cabi.check(L.tvdcn_b200_deform_conv_backward(ctypes.byref(p), vp(go), vp(x), vp(w), vp(off), vp(mask), None, vp(gw),
+                                                 None, None, None, vp(ws), n, st))
+    ref = run_oracle(case, *(t.double().cpu() for t in (x, w, off, mask, bias, go)))
+    assert nerr(gw, ref[2]) <= 6e-4
+
+
 def test_reuse_flag_after_a_forward_that_fell_back_to_simt():
     """A padded shape whose forward call gets too little workspace runs on the SIMT kernels and stages nothing.  The
     same workspace is enough for the weight gradient alone: with TVDCN_FLAG_REUSE_STAGED_INPUT that call must stage

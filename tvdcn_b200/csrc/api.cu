@@ -515,11 +515,13 @@ int tvdcn_b200_deform_conv_backward_ex(const tvdcn_problem *p, const void *grad_
     if (pl.tensor) {
         // The caller may vouch that the forward call's staging of `input` is still at the start of this workspace
         // (only where the forward call for this problem stages the image at all, and at the same offset: with a workspace
-        // too small for its plan, which may still do for this call's, it ran on the SIMT kernels and staged nothing).
+        // too small for its plan, which may still do for this call's, it ran on the SIMT kernels and staged nothing; and f16 rows that
+        // TMA cannot read make the weight gradient alone wide, whose maxima the forward call had no use for).
         bool staged = false;
         if ((p->flags & TVDCN_FLAG_REUSE_STAGED_INPUT) && !p->transposed) {
             const Plan fwd = plan_for(p, workspace_bytes, [](const tvdcn_problem *q) { return plan_forward(q); });
-            staged = fwd.img_cl != NO_BUF && fwd.img_cl == pl.img_cl && fwd.total <= workspace_bytes;
+            staged = fwd.img_cl != NO_BUF && fwd.img_cl == pl.img_cl && fwd.total <= workspace_bytes &&
+                     (pl.img_max == NO_BUF || pl.img_max == fwd.img_max);
         }
         if (!staged && (pl.tc_sg || tc_sw || goff_acc || gmask_acc)) tc.stage_image(img);
         if (pl.tc_gs) tc.stage_weight(weight, true);

@@ -98,12 +98,12 @@ void take_aux(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool 
     if (bias) pl.bias32 = b.take((size_t)p->out_channels * sizeof(float));
 }
 
-// The staged sampled image comes first in both plans, and the maxima of its blocks next: a backward call that is told to
-// reuse the forward call's staging (TVDCN_FLAG_REUSE_STAGED_INPUT) finds them at the same offsets of the same workspace.
-// So the forward call takes the maxima also where only the weight gradient needs them (rows that TMA cannot read).
-void take_image(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g) {
+// The staged sampled image comes first in both plans, and the maxima of its blocks (maxima: a kernel of the call has the
+// wide f16 mode) next: a backward call that is told to reuse the forward call's staging (TVDCN_FLAG_REUSE_STAGED_INPUT)
+// finds them at the same offsets of the same workspace.
+void take_image(Plan &pl, Bump &b, const tvdcn_problem *p, const GeoHost &g, bool maxima) {
     pl.img_cl = b.take(((size_t)g.B * g.S + 1) * g.Cs * (p->dtype == TVDCN_F32 ? 4 : 2));   // + one row of zeros
-    if (p->dtype != TVDCN_F16 || !(pl.wide || g.P % 8 != 0)) return;
+    if (!maxima) return;
     pl.n_img_max = (int)Stager::image_blocks(g);
     pl.img_max = b.take((size_t)pl.n_img_max * sizeof(unsigned));
     if (g.mg == 0) return;
@@ -157,7 +157,7 @@ Plan plan_forward(const tvdcn_problem *p, bool share_tiles) {
     if (why == nullptr && !p->transposed) {
         if (fwd_tc_config(g, pl.mode, &bn, &st) && chain_ok(pl.mode, g, bn)) {
             pl.tensor = pl.tc_sg = true;
-            take_image(pl, b, p, g);
+            take_image(pl, b, p, g, pl.mode == TC_F16_WIDE);
             take_sample_buffers(pl, b, g, bn, share_tiles);
             take_aux(pl, b, p, g, true);
         } else {
@@ -204,7 +204,7 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
                    dgrad_tc_config(g, pl.mode, &bn, &gbufs, &st);
         pl.tensor = pl.tc_sg || pl.tc_sw || pl.tc_gs;
         if (pl.tensor) {
-            take_image(pl, b, p, g);
+            take_image(pl, b, p, g, (pl.tc_sg && pl.mode == TC_F16_WIDE) || (pl.tc_sw && pl.mode_sw == TC_F16_WIDE));
             take_aux(pl, b, p, g, false);
         }
         if (pl.tc_sg) take_sample_buffers(pl, b, g, sg_bn, true);
