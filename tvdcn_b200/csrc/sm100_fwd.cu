@@ -660,7 +660,11 @@ static bool fwd_work(const GeoHost &h, int mode, int bn, bool may_share, FwdWork
     const long long sms = 148;
     const long long shared = std::min(sms, std::min(units / 3, 2LL * w->n_tiles));
     const bool two_each = shared == 2LL * w->n_tiles;
-    const int cost = (two_each ? HALVES : RANGES)[mode_f32(mode)][bn / 128];
+    int cost = (two_each ? HALVES : RANGES)[mode_f32(mode)][bn / 128];
+    // Beyond five tiles per SM the last wave is a small part, and CTAs that are out of step with one another lose something in
+    // every tile: 1050 tiles of 27 chunks, whole / shared: bf16 219 / 211 (64 channels), 227 / 223, 237 / 239 (256); f32 377 / 364, 475 / 509,
+    // 625 / 641; of 9 chunks (a gain of 8): bf16 84 / 91, 93 / 100, 120 / 127, f32 140 / 137, 160 / 160, 201 / 205.
+    if (w->n_tiles > 5 * sms) cost = bn == 256 || (mode_f32(mode) && bn == 128) ? 1 << 20 : std::max(cost, 10);
     const long long whole_time = (w->n_tiles + sms - 1) / sms * w->n_chunks;
     w->whole = !may_share || w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + cost;
     w->halves = !w->whole && two_each;
