@@ -34,24 +34,20 @@ struct FwdWork {
     int n_chunks;           // units per tile: taps x 64-channel chunks
     int ctas;
     int whole;              // no tile is shared
-    int halves;             // every tile is shared by two CTAs, 2 t and 2 t + 1
-    int base, extra;        // else CTA c has `base` units (whole: tiles), the first `extra` CTAs one more
+    int halves;             // every tile of an odd number of chunks is shared by two CTAs, 2 t (one chunk more) and 2 t + 1
+    int base, extra;        // CTA c has `base` units (whole: tiles), the first `extra` CTAs (halves: the even ones) one more
 
     // First unit of CTA c.  A piece of one chunk is not worth its trip through the workspace: it stays with its neighbour.
     // (32-bit arithmetic: every role of every CTA starts with it.)
     __host__ __device__ int bound(int c) const {
-        if (halves) return (c >> 1) * n_chunks + ((c & 1) ? (n_chunks + 1) / 2 : 0);
-        const int b = c * base + (c < extra ? c : extra);
+        const int b = c * base + (halves ? (c + 1) >> 1 : (c < extra ? c : extra));
         if (whole) return b * n_chunks;
         const int r = b % n_chunks;
         return r == 1 ? b - 1 : (r == n_chunks - 1 ? b + 1 : b);
     }
     // the CTA that has a unit
     __host__ __device__ int owner(int unit) const {
-        if (halves) {
-            const int t = unit / n_chunks;
-            return 2 * t + (unit - t * n_chunks >= (n_chunks + 1) / 2 ? 1 : 0);
-        }
+        if (halves) return 2 * unit / n_chunks;
         const int wide = extra * (base + 1);
         int c = unit < wide ? unit / (base + 1) : extra + (unit - wide) / base;
         if (c + 1 < ctas && bound(c + 1) <= unit) ++c;     // the neighbour's, after its bound was moved by one
@@ -667,7 +663,7 @@ static bool fwd_work(const GeoHost &h, int mode, int bn, bool may_share, FwdWork
     if (w->n_tiles > 5 * sms) cost = bn == 256 || (mode_f32(mode) && bn == 128) ? 1 << 20 : std::max(cost, 10);
     const long long whole_time = (w->n_tiles + sms - 1) / sms * w->n_chunks;
     w->whole = !may_share || w->n_chunks < 3 || shared < 2 || whole_time <= (units + shared - 1) / std::max(shared, 1LL) + cost;
-    w->halves = !w->whole && two_each;
+    w->halves = !w->whole && two_each && w->n_chunks % 2 != 0;       // (an even number is halved by equal ranges)
     w->ctas = (int)(w->whole ? std::max(1LL, std::min<long long>(sms, w->n_tiles)) : shared);   // 1: an empty batch, planned but not launched
     const long long items = w->whole ? w->n_tiles : units;
     w->base = (int)(items / w->ctas);
