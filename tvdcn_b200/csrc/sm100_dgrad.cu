@@ -13,25 +13,34 @@
 // Work is cut into *units*: (tile of 128 grid positions, 64-channel chunk, batch of TB taps), ordered tile by tile.  The
 // grid has one CTA per SM (see launch_dgrad_t) and each takes an equal, contiguous range of units: nothing but a CTA's first unit waits
 // for its operands (start-up was 12 k of 36 k cycles per tile for short 1-d reductions), and the SMs finish together
-// whatever the number of tiles.  Every unit is two *passes* over 32-channel slabs.
-//   GEMM   D[128 positions (TMEM lanes) x TB*32 columns] over the dense channels of the group.
+// whatever the number of tiles.
+//   GEMM   D[128 positions (TMEM lanes) x TB*32 columns] over the dense channels of the group, two of them (slabs of 32
+//          channels) per unit.
 //          A = the dense tile [128 pos][cdg], read once per tile from the caller's [B, Cd, P] tensor (thread =
 //              position, coalesced), converted to 16-bit (f32 data: bf16 parts) and kept in TENSOR MEMORY
 //              (tcgen05.st; the MMA reads A from TMEM, so shared memory carries only B); later tiles are loaded by the
-//              planner warps, idle half of the time, as soon as the old tile's last MMA is through;
+//              finishing warps as soon as the old tile's last MMA is through;
 //          B = weights packed [g][tap][s'][d'], one TMA box {64 d', 32 s', TB taps} per reduction chunk (ring);
-//          D = ring of accumulators in the TMEM columns behind A.
-//   plan   Four planner warps (thread = position) turn the unit's offsets / mask into one entry per in-image
-//          bilinear corner (pixel row, position, tap, weight x mask) and GROUP THE ENTRIES BY PIXEL: a counting
-//          sort by pixel row modulo SC_SLOTS (shared-memory integer atomics + prefix sum).
-//   store  Four warps copy each finished accumulator TMEM -> shared memory ([128 pos][TB*32] f32).
-//   gather Twelve warps, 8 lanes per entry (4 channels each), walk equal spans of the pixel-grouped entry
-//          list: one 16-byte shared load of the entry's column values feeds both the running sum of the
-//          pixel (one red.global.add.v4.f32 per lane leaves the SM when the pixel changes, instead of one per
-//          corner) and the dot product <col, image row of the pixel> that the coordinate gradients need.
-//          The dots of a unit's entries are finally combined per (position, tap) by the planner threads.
+//          D = a ring of up to four accumulators in the TMEM columns behind A.
+//   plan   Four planner warps (thread = position) turn the unit's offsets / mask into one entry per PAIR of bilinear corners
+//          that are neighbours along the image's last axis (rows of the even and of the odd one, their weights x mask) and GROUP
+//          THE ENTRIES BY PIXEL: a counting sort by the left pixel modulo SC_SLOTS (shared-memory integer atomics + prefix sum).
+//   gather Twelve warps copy the unit's columns TMEM -> shared memory ([128 pos][TB*64] f32); then 8 lanes per entry (8 channels
+//          each) walk equal spans of the pixel-grouped entry list.  An entry's column values are read once for both of its pixels:
+//          they go into the running sums of the even and of the odd pixel (which leave the SM as red.global.add.v4.f32 when the
+//          pixel changes, instead of once per corner), and into the dot products <col, image row of the pixel> that the
+//          coordinate gradients need.  The image rows stay in registers while the pixel does.
+//   finish Four warps turn the dots of a unit into grad_offset / grad_mask, and load dense tiles.
 //
-// Warp roles (768 threads): 0-3 store, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
+// What bounds it: the gather loop, by issue slots, instruction fetch and the latency of its shared-memory reads in about equal parts
+// (45-50 % of issue slots, 50 % of the load/store data pipe; its twelve warps are few because each needs 100 registers).  Hence the
+// form of the loop: two entries per iteration and no more (a loop of four, 6 KB of code beside the planners' and finishers' straight
+// lines, took 574 instead of 551 us at 128 x 256 x 28 x 28 bf16, 4 groups of offsets), columns and entries read ahead, one
+// branch per flush.  Before, one entry per corner, 4 channels per lane and the columns staged in two halves: 799 us there, 850 f32,
+// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 554, 691, 1162, 3197.  (16 gather warps have
+// no registers to read columns ahead: 586 us, and 768 with the spills of trying.)
+//
+// Warp roles (768 threads): 0-3 finish, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
 // (they complete the last warpgroup for the register hand-over).
 #include <algorithm>
 #include <type_traits>
@@ -64,10 +73,10 @@ struct DgradParams {
 
 namespace {
 
-constexpr int SC_STORE_WARPS = 4;
+constexpr int SC_FINISH_WARPS = 4;
 constexpr int SC_GATHER_WARPS = 12;
-constexpr int SC_WORK_WARPS = SC_STORE_WARPS + SC_GATHER_WARPS;
-constexpr int SC_LOAD_WARPS = 16;                                 // the first 16 of them load the dense tile first
+constexpr int SC_WORK_WARPS = SC_FINISH_WARPS + SC_GATHER_WARPS;
+constexpr int SC_LOAD_WARPS = 16;                                 // these load the first dense tile
 constexpr int SC_PLAN_WARP0 = SC_WORK_WARPS;
 constexpr int SC_PLAN_WARPS = 4;                                  // one planner thread per tile position
 constexpr int SC_MMA_WARP = SC_PLAN_WARP0 + SC_PLAN_WARPS;
@@ -75,16 +84,22 @@ constexpr int SC_TMA_WARP = SC_MMA_WARP + 1;
 constexpr int SC_THREADS = (SC_TMA_WARP + 3) * 32;                // two idle warps complete the last warpgroup
 static_assert(SC_THREADS == 768, "six warpgroups");
 // Registers per thread after the warpgroups have rebalanced them (launch: 80 each for 6 warpgroups = 480 x 128):
-// the three gather warpgroups and the planners take 96, the store warps keep 56, the MMA / TMA warpgroup 40:
-// 4 x 96 + 56 + 40 = 480.
-constexpr int SC_REGS_WORK = 96, SC_REGS_STORE = 56, SC_REGS_ISSUE = 40;
+// 3 x 104 (gather) + 72 (planners) + 64 (finish) + 32 (MMA / TMA) = 480.
+constexpr int SC_REGS_LAUNCH = 65536 / SC_THREADS / 8 * 8;
+constexpr int SC_REGS_GATHER = 104, SC_REGS_PLAN = 72, SC_REGS_FINISH = 64, SC_REGS_ISSUE = 32;
+static_assert(SC_GATHER_WARPS * SC_REGS_GATHER + SC_PLAN_WARPS * SC_REGS_PLAN + SC_FINISH_WARPS * SC_REGS_FINISH + 4 * SC_REGS_ISSUE <=
+                  SC_THREADS / 32 * SC_REGS_LAUNCH, "an increase beyond the launch's registers waits for ever");
+template <int N>
+__device__ __forceinline__ void take_registers() {
+    if constexpr (N >= SC_REGS_LAUNCH) ptx::reg_inc<N>();
+    else ptx::reg_dec<N>();
+}
 constexpr int SC_GROUPS = SC_GATHER_WARPS * 4;                    // 8-lane groups walking the entry list
 constexpr int SC_SLAB = 32;                                       // channels per pass
-constexpr int SC_PLAN_SLACK = SC_GROUPS * 4 + 16;
+constexpr int SC_PLAN_SLACK = SC_GROUPS * 2 + 8;                  // padding of the spans to a multiple of two; read-ahead
 // Slots of the counting sort.  A tile's entries lie around its positions, so rows that share a slot are rare; where
 // they do, their entries interleave and the pixel's running sum leaves the SM more often, nothing else.
-constexpr int SC_SLOTS = 2048;
-constexpr uint32_t SC_NONE = 0xffffffffu;
+constexpr int SC_SLOTS = 2048, SC_SLOT_WORDS = SC_SLOTS + SC_SLOTS / 32 * 4;
 constexpr int SC_TMEM_COLS = 512;
 constexpr int SC_SLEEP_NS = 32;                                   // back-off of the long waits (64 to 512 measured equal)
 constexpr int SC_MAX_TAPS = 512;                                  // taps whose kernel coordinates a CTA tabulates
@@ -92,15 +107,65 @@ constexpr int SC_MAX_TAPS = 512;                                  // taps whose 
 // most taps per batch: shared memory holds the column values and the entry lists of two batches
 __host__ __device__ constexpr int sc_tb_max(int dim) { return dim == 1 ? 4 : (dim == 2 ? 3 : 2); }
 
-// Predicated form: no branch around the reduction, and no "memory" clobber either -- nothing in this kernel reads
-// what the reduction writes, and the shared-memory loads around it must stay free to move.
-__device__ __forceinline__ void red_add_v4_if(bool p, float *addr, float a, float b, float c, float d) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred q;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n\t"
-        "}\n" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"((int)p));
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+template <int SIZE>
+__device__ __forceinline__ uint64_t row_at(uint64_t base, uint32_t px) {
+    uint64_t r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(px), "n"(SIZE), "l"(base));
+    return r;
+}
+
+// Where px != cur: adds the sums `v` (4 + 4 channels, 32 apart) to the row at `addr` and starts them anew.  One branch for all of
+// it: the compiler wraps every predicated reduction in a branch of its own.  No "memory" clobber: nothing in this kernel reads
+// what the reductions write, and the shared-memory loads around them must stay free to move.
+__device__ __forceinline__ void flush_sums(uint32_t px, uint32_t cur, uint64_t addr, float (&v)[8]) {
+    if (px != cur) {
+        asm volatile(
+            "red.global.add.v4.f32 [%8], {%0, %1, %2, %3};\n\t"
+            "red.global.add.v4.f32 [%8 + 128], {%4, %5, %6, %7};\n\t"
+            ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "l"(addr));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = 0.f;
+    }
+}
+// Where px != was: loads 4 + 4 channels, 32 apart, of 16-bit (4 words) or f32 (8 words) data.
+template <int IW>
+__device__ __forceinline__ void load_row(uint32_t px, uint32_t was, uint32_t (&v)[IW], uint64_t addr) {
+    if constexpr (IW == 4)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred q;\n\t"
+            "setp.ne.u32 q, %5, %6;\n\t"
+            "@q ld.global.nc.v2.u32 {%0, %1}, [%4];\n\t"
+            "@q ld.global.nc.v2.u32 {%2, %3}, [%4 + 64];\n\t"
+            "}\n" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]) : "l"(addr), "r"(px), "r"(was));
+    else
+        asm volatile(
+            "{\n\t"
+            ".reg .pred q;\n\t"
+            "setp.ne.u32 q, %9, %10;\n\t"
+            "@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%8];\n\t"
+            "@q ld.global.nc.v4.u32 {%4, %5, %6, %7}, [%8 + 128];\n\t"
+            "}\n" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+            : "l"(addr), "r"(px), "r"(was));
 }
 
 __device__ __forceinline__ void planner_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
@@ -131,32 +196,61 @@ __device__ __forceinline__ void corner_of(const Geo<DIM> &g, const PosInfo<DIM> 
     row = (uint32_t)(pi.b * g.S + flat);
 }
 
+// Pair q of the 2^(DIM - 1) pairs of corners that are neighbours along the last axis: pixel row of the left one (of the
+// place left of the image where only the right one lies in it), which of the two are in the image, their weights.  key: the
+// left one's place where every image row begins with one place more, which keeps pairs across the edges apart from others.
+template <int DIM>
+__device__ __forceinline__ void pair_of(const Geo<DIM> &g, const PosInfo<DIM> &pi, const TapGeometry<DIM> &tg,
+                                        bool deformable, int q, uint32_t &left, uint32_t &key, bool &ok_l, bool &ok_r, float &w_l,
+                                        float &w_r) {
+    bool ok = deformable || q == 0;
+    int flat = 0;
+    float w = 1.f;
+#pragma unroll
+    for (int a = 0; a < DIM - 1; ++a) {
+        const int bit = (q >> (DIM - 2 - a)) & 1;
+        const int i = (int)((unsigned)tg.fl[a] + (unsigned)bit);
+        ok = ok && ((unsigned)i < (unsigned)g.img[a]);
+        flat = flat * g.img[a] + i;
+        w *= bit ? tg.fr[a] : (1.f - tg.fr[a]);
+    }
+    const unsigned i = (unsigned)tg.fl[DIM - 1];
+    ok_l = ok && i < (unsigned)g.img[DIM - 1];
+    ok_r = ok && deformable && i + 1u < (unsigned)g.img[DIM - 1];
+    unsigned row = (unsigned)pi.b;
+#pragma unroll
+    for (int a = 0; a < DIM - 1; ++a) row *= (unsigned)g.img[a];
+    row += (unsigned)flat;
+    left = row * (unsigned)g.img[DIM - 1] + i;
+    key = left + row + 1u;
+    w_l = w * (1.f - tg.fr[DIM - 1]);
+    w_r = w * tg.fr[DIM - 1];
+}
+
 // Byte offsets of the dynamic shared memory regions (after alignment to 1024).
 struct ScLayout {
-    uint32_t b_stage, col_buf, plan_buf, col, plan, info, pos, cnt, taps, misc, bars, total;
+    uint32_t b_stage, plan_buf, col, plan, info, pos, cnt, taps, misc, bars, total;
     int n, col_stride, max_entries;
 };
 __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_stages) {
     ScLayout L;
         L.n = tb * SC_SLAB;
-    L.col_stride = L.n + 4;                       // words; = 4 mod 32, so that the row-per-lane stores spread over the banks
-    L.max_entries = TILE_POS * tb * (1 << dim);
+    L.col_stride = 2 * L.n + 4;                   // words; = 4 mod 32, so that the row-per-lane stores spread over the banks
+    L.max_entries = TILE_POS * tb << (dim - 1);
     L.b_stage = (uint32_t)(L.n * 128);             // one 16-bit part (hi or lo) of one reduction chunk
-    L.col_buf = (uint32_t)(TILE_POS * L.col_stride * 4);
-    // three arrays (pixel offset; col index | dot slot << 16; weight) of max_entries + SC_PLAN_SLACK words -- room for
-    // the padding of the groups' spans and the read-ahead of the last group -- then one dot product per entry (+ a
-    // slot for the padding entries)
-    L.plan_buf = (uint32_t)(3 * (L.max_entries + SC_PLAN_SLACK) * 4 + (L.max_entries + 4) * 4);
+    // per entry {pixel offset even, odd, weight even, odd} and a word (col index | dot slot << 16), with room for the padding
+    // of the groups' spans and the read-ahead of the last group; then two dot products per entry (+ two for the padding entries)
+    L.plan_buf = (uint32_t)((L.max_entries + SC_PLAN_SLACK) * 20 + (2 * L.max_entries + 4) * 4);
     uint32_t o = 0;
     o += (uint32_t)b_stages * L.b_stage;
-    L.col = o;  o += 2 * L.col_buf;
+    L.col = o;  o += (uint32_t)(TILE_POS * L.col_stride * 4);
     L.plan = o; o += 2 * L.plan_buf;
-    L.info = o; o += 2 * 16;                      // per plan buffer: first channel, first tap, offset group, mask group
-    L.pos = o;  o += 2 * TILE_POS * 8;            // and per position of the tile: image (or -1), position in it
-    L.cnt = o;  o += SC_SLOTS * 4;
+    L.info = o; o += 4 * 16;                      // of four units: first channel, first tap, offset group, mask group
+    L.pos = o;  o += 4 * TILE_POS * 8;            // and per position of the tile: image (or -1), position in it
+    L.cnt = o;  o += SC_SLOT_WORDS * 4;
     L.taps = o; o += SC_MAX_TAPS * 3 * 2;         // kernel coordinates of every tap (int16)
     L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot, reloads
-    L.bars = o; o += (uint32_t)(21 + 2 * b_stages) * 8;
+    L.bars = o; o += (uint32_t)(18 + 2 * b_stages) * 8;
     L.total = o;
     return L;
 }
@@ -211,11 +305,15 @@ __device__ __forceinline__ bool next_unit(const DgradParams<DIM> &P, UnitIter &u
     return true;
 }
 
-template <int DIM, int MODE, bool COORD>
+// what is wanted: the scattered image, the coordinate gradients (grad_offset and / or grad_mask), both
+enum { SC_SCATTER = 1, SC_COORD = 2 };
+
+template <int DIM, int MODE, int WANT>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMap tmap_b_hi,
                     const __grid_constant__ CUtensorMap tmap_b_lo, const __grid_constant__ CUtensorMap tmap_b_lo2) {
-    constexpr int NC = 1 << DIM;
+    constexpr bool SCATTER = (WANT & SC_SCATTER) != 0, COORD = (WANT & SC_COORD) != 0;
+    constexpr int NC = 1 << DIM, NP = NC / 2;           // corners of a cell, pairs of them
     using M = Mode<MODE>;
     constexpr int PARTS = M::MAT_PARTS;                 // 16-bit parts of the dense tile and of the weights
     constexpr int ACCS = MODE == TC_F32_WIDE ? 2 : 1;   // accumulators of a pass: leading / small products
@@ -239,60 +337,51 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint32_t *wait_flag = misc + 4;
     uint32_t *n_entries = misc + 6;      // [2]
     uint32_t *tmem_slot = misc + 8;
-    uint32_t *reloads = misc + 9;        // f32 data: dense tiles behind the first that the planners have loaded
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
     uint64_t *a_first = bars;            // dense tile of the CTA's first unit is in TMEM / of every later tile
     uint64_t *a_next = bars + 1;
     uint64_t *b_full = bars + 2;
     uint64_t *b_empty = b_full + BS;
-    uint64_t *t_full = b_empty + BS;     // [4] MMA -> store warps: accumulator complete
-    uint64_t *t_empty = t_full + 4;      // [4] store warps -> MMA: accumulator read out
-    uint64_t *col_full = t_empty + 4;    // [2] store warps -> gather warps
-    uint64_t *col_empty = col_full + 2;  // [2] gather warps -> store warps
-    uint64_t *plan_full = col_empty + 2; // [2] planners -> gather warps
-    uint64_t *plan_done = plan_full + 2; // [2] gather warps -> whoever turns the unit's dots into gradients / planners
-    uint64_t *fin_done = plan_done + 2;  // [2] store warps -> planners: the unit's dots have been used
+    uint64_t *t_full = b_empty + BS;     // [4] MMA -> gather warps: accumulator complete
+    uint64_t *t_empty = t_full + 4;      // [4] gather warps -> MMA: accumulator read out
+    uint64_t *col_full = t_empty + 4;    // gather warps: the unit's columns are in shared memory
+    uint64_t *plan_full = col_full + 1;  // [2] planners -> gather warps
+    uint64_t *plan_done = plan_full + 2; // [2] gather warps -> themselves, finishing warps, planners: through with the unit's columns and entries
+    uint64_t *fin_done = plan_done + 2;  // [2] finishing warps -> gather warps: the dots of the unit have been used
     uint64_t *a_free = fin_done + 2;     // MMA -> planners: the last MMA on the dense tile is through
     int16_t *tap_tab = reinterpret_cast<int16_t *>(smem + L.taps);
-    // Entry e of the pixel-grouped list sits at word e of each array; a group's span is a multiple of four entries, so
-    // that a batch of four is one 16-byte read per array (each 8-lane group is a quarter-warp phase of its own: the
-    // four groups of a warp never meet in one bank access).
     const int plan_words = L.max_entries + SC_PLAN_SLACK;
-    auto plan_px = [&](int pb) { return reinterpret_cast<uint32_t *>(smem + L.plan + (size_t)pb * L.plan_buf); };
-    auto plan_meta = [&](int pb) { return plan_px(pb) + plan_words; };
-    auto plan_w = [&](int pb) { return reinterpret_cast<float *>(plan_px(pb) + 2 * plan_words); };
-    auto plan_dot = [&](int pb) { return reinterpret_cast<float *>(plan_px(pb) + 3 * plan_words); };
+    auto plan_ent = [&](int pb) { return reinterpret_cast<uint4 *>(smem + L.plan + (size_t)pb * L.plan_buf); };
+    auto plan_meta = [&](int pb) { return reinterpret_cast<uint32_t *>(plan_ent(pb) + plan_words); };
+    auto plan_dot = [&](int pb) { return reinterpret_cast<float *>(plan_meta(pb) + plan_words); };
 
-    auto info_of = [&](int pb) { return reinterpret_cast<int4 *>(smem + L.info) + pb; };
-    auto pos_of = [&](int pb) { return reinterpret_cast<int2 *>(smem + L.pos) + pb * TILE_POS; };
+    // of unit j: what its finalisation reads outlives its plan
+    auto info_of = [&](int j) { return reinterpret_cast<int4 *>(smem + L.info) + (j & 3); };
+    auto pos_of = [&](int j) { return reinterpret_cast<int2 *>(smem + L.pos) + (j & 3) * TILE_POS; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // this CTA's units
     const int unit0 = (int)((long long)P.total_units * blockIdx.x / gridDim.x);
     const int n_units = (int)((long long)P.total_units * (blockIdx.x + 1) / gridDim.x) - unit0;
     const int n_pass = 2 * n_units;
-    constexpr bool want_coord = COORD;    // grad_offset and / or grad_mask are wanted
-    const bool scatter = P.img_grad_cl != nullptr;
     const bool deformable = P.offset != nullptr;
     if (threadIdx.x == 0) {
         ptx::mbar_init(a_first, SC_LOAD_WARPS);
-        ptx::mbar_init(a_next, SC_PLAN_WARPS);
+        ptx::mbar_init(a_next, SC_FINISH_WARPS);
         ptx::mbar_init(a_free, 1);
-        *reloads = 0u;
         for (int s = 0; s < BS; ++s) {
             ptx::mbar_init(&b_full[s], 1);
             ptx::mbar_init(&b_empty[s], 1);
         }
         for (int q = 0; q < 4; ++q) {
             ptx::mbar_init(&t_full[q], 1);
-            ptx::mbar_init(&t_empty[q], SC_STORE_WARPS);
+            ptx::mbar_init(&t_empty[q], SC_GATHER_WARPS);
         }
+        ptx::mbar_init(col_full, SC_GATHER_WARPS);
         for (int i = 0; i < 2; ++i) {
-            ptx::mbar_init(&col_full[i], SC_STORE_WARPS);
-            ptx::mbar_init(&col_empty[i], SC_GATHER_WARPS);
             ptx::mbar_init(&plan_full[i], SC_PLAN_WARPS);
             ptx::mbar_init(&plan_done[i], SC_GATHER_WARPS);
-            ptx::mbar_init(&fin_done[i], SC_STORE_WARPS);
+            ptx::mbar_init(&fin_done[i], SC_FINISH_WARPS);
         }
         ptx::fence_mbar_init();
     }
@@ -317,7 +406,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     const uint32_t tmem_base = *tmem_slot;
     ptx::grid_dependency_wait();     // nothing above reads what an earlier kernel wrote
 
-    // ---- pieces shared by the planners (which build a unit's entry list) and the store warps (which turn its dot
+    // ---- pieces shared by the planners (which build a unit's entry list) and the finishing warps (which turn its dot
     // products into coordinate gradients); both map thread -> position of the tile
     // {first channel, first tap, offset group, mask group} of a unit
     auto describe = [&](const UnitIter &u) {
@@ -363,9 +452,10 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         return tg;
     };
 
-    // combines the dot products of a finished unit into the coordinate gradients of its (position, tap)s
+    // combines the dot products of a finished unit (an entry has two: even pixel row, odd one) into the coordinate gradients of its
+    // (position, tap)s
     auto finalize = [&](const PosInfo<DIM> &pi, int pt, const int4 &info, int pb, const RawUnit &ru) {
-        if (!want_coord || !pi.valid) return;
+        if (!COORD || !pi.valid) return;
         const int t0 = info.y, ogi = info.z, mgi = info.w;
         const float *dots = plan_dot(pb);
 #pragma unroll
@@ -383,7 +473,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     float w;
                     corner_of<DIM>(g, pi, tg, deformable, c, okc, row, w);
                     if (okc) {
-                        const float d = dots[(pt * TB + t) * NC + c];
+                        const float d = dots[(pt * TB + t) * NC + (c & ~1) + (int)(row & 1u)];
                         gm = fmaf(w, d, gm);
 #pragma unroll
                         for (int a = 0; a < DIM; ++a) {
@@ -467,16 +557,14 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     };
 
     if (warp < SC_WORK_WARPS) {
-        if (warp < SC_STORE_WARPS) {
-            // -------------------------------------------------------------- store warps: TMEM -> shared
+        if (warp < SC_FINISH_WARPS) {
+            // -------------------------------------------------------------- finishing warps: coordinate gradients, dense tiles
             load_dense(first_unit(P, unit0), warp >> 2, SC_LOAD_WARPS / 4, a_first);   // before registers are handed over
-            ptx::reg_dec<SC_REGS_STORE>();
-            const int q = warp;
-            const int row = q * 32 + lane;
-            bool ok = true;
-            // this thread's position in the tile of a plan buffer
-            auto position = [&](int pb) {
-                const int2 at = pos_of(pb)[row];
+            take_registers<SC_REGS_FINISH>();
+            const int row = warp * 32 + lane;
+            // this thread's position in the tile of unit j
+            auto position = [&](int j) {
+                const int2 at = pos_of(j)[row];
                 PosInfo<DIM> pi;
                 pi.valid = at.x >= 0;
                 pi.b = max(at.x, 0);
@@ -484,172 +572,183 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 decode_in_image<DIM>(g, pi);
                 return pi;
             };
-            auto wait_done = [&](int j) -> bool {
-                bool good = ptx::mbar_wait(&plan_done[j & 1], (uint32_t)((j >> 1) & 1));
+            // The gather warps are through with unit j: its dot products become gradients.
+            auto finish_unit = [&](int j) -> bool {
+                bool good = ptx::mbar_wait_backoff<SC_SLEEP_NS>(&plan_done[j & 1], (uint32_t)((j >> 1) & 1));
                 good = __all_sync(0xffffffffu, good);
-                if (!good && lane == 0) ptx::report(P.status, 308);
-                return good;
-            };
-            // The gather warps finish unit j (its dot products are complete) with pass 2 j + 1; the wait for that
-            // pass' staging buffer below covers it, so the unit is turned into gradients right after the next store.
-            auto finish_unit = [&](int j, const PosInfo<DIM> &pi, const RawUnit &ru) -> bool {
-                const int pb = j & 1;
-                if (!wait_done(j)) return false;
-                finalize(pi, row, *info_of(pb), pb, ru);
+                if (!good) {
+                    if (lane == 0) ptx::report(P.status, 308);
+                    return false;
+                }
+                const PosInfo<DIM> pi = position(j);
+                RawUnit ru;
+                load_unit(pi, *info_of(j), ru);
+                finalize(pi, row, *info_of(j), j & 1, ru);
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&fin_done[pb]);
+                if (lane == 0) ptx::mbar_arrive(&fin_done[j & 1]);
                 return true;
             };
-            int aq = 0;
-            uint32_t t_phase = 0;
-            for (int jp = 0; jp < n_pass && ok; ++jp) {
-                const int cb = jp & 1;
-                const bool fin_now = COORD && jp >= 3 && (jp & 1) == 1;   // pass jp - 2 closed unit (jp - 2) / 2
-                RawUnit ru_fin;
-                PosInfo<DIM> pi_fin;
-                if (fin_now) {     // (its plan is known here: the gather warps have released its first slab)
-                    const int pb = ((jp - 2) >> 1) & 1;
-                    pi_fin = position(pb);
-                    load_unit(pi_fin, *info_of(pb), ru_fin);
-                }
-                ok = ptx::mbar_wait(&t_full[aq], t_phase);
-                ok = ok && ptx::mbar_wait_backoff<SC_SLEEP_NS>(&col_empty[cb], (uint32_t)(((jp >> 1) & 1) ^ 1));
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) {
-                    if (lane == 0) ptx::report(P.status, 301);
-                    break;
-                }
-                ptx::tc_fence_after();
-                float *dst = col + (size_t)cb * (L.col_buf / 4) + row * L.col_stride;
-                const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col0 + (uint32_t)(aq * ACCS * N);
-                for (int j32 = 0; j32 < N / 32; ++j32) {
-                    uint32_t raw[32];
-                    ptx::tmem_ld_32x32(src + (uint32_t)(j32 * 32), raw);
-                    ptx::tmem_ld_wait();
-                    if constexpr (ACCS == 2) {
-                        // in two halves: the store warps have few registers
-#pragma unroll
-                        for (int h = 0; h < 4; ++h) {
-                            uint32_t low[8];
-                            ptx::tmem_ld_32x8(src + (uint32_t)(N + j32 * 32 + h * 8), low);
-                            ptx::tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                raw[h * 8 + e] = __float_as_uint(__uint_as_float(raw[h * 8 + e]) + __uint_as_float(low[e]));
-                        }
+            // The next tile is loaded as soon as the old one's last MMA is through.  With four accumulators the MMAs run two units ahead of the
+            // gather warps, with two one unit: while those walk unit j, that moment comes for tiles that end with unit j + lead.
+            const int lead = NACC >= 4 ? 2 : (NACC >= 2 ? 1 : 0);
+            int next_tile = P.n_units - unit0 % P.n_units;       // first unit of the next tile to be loaded
+            UnitIter u = first_unit(P, unit0);
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int j = 0; j < n_units && ok; ++j) {
+                if (COORD && j > 0) ok = finish_unit(j - 1);
+                for (; ok && next_tile < n_units && next_tile - 1 - lead <= j; next_tile += P.n_units) {
+                    ok = ptx::mbar_wait_backoff<SC_SLEEP_NS>(a_free, phase);
+                    phase ^= 1u;
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) {
+                        if (lane == 0) ptx::report(P.status, 309);
+                        break;
                     }
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float4 v;
-                        v.x = __uint_as_float(raw[4 * i]);
-                        v.y = __uint_as_float(raw[4 * i + 1]);
-                        v.z = __uint_as_float(raw[4 * i + 2]);
-                        v.w = __uint_as_float(raw[4 * i + 3]);
-                        *reinterpret_cast<float4 *>(dst + j32 * 32 + i * 4) = v;
-                    }
+                    ptx::tc_fence_after();
+                    ++u.order;
+                    locate_tile(P, u);
+                    load_dense(u, 0, 1, a_next);
                 }
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    ptx::mbar_arrive(&t_empty[aq]);
-                    ptx::mbar_arrive(&col_full[cb]);
-                }
-                if (++aq == NACC) {
-                    aq = 0;
-                    t_phase ^= 1u;
-                }
-                if (fin_now) ok = finish_unit((jp - 2) >> 1, pi_fin, ru_fin);
             }
-            if (COORD && ok && wait_done(n_units - 1)) {   // the last unit
-                const int pb = (n_units - 1) & 1;
-                const PosInfo<DIM> pi_fin = position(pb);
-                RawUnit ru_fin;
-                load_unit(pi_fin, *info_of(pb), ru_fin);
-                finish_unit(n_units - 1, pi_fin, ru_fin);
-            }
+            if (COORD && ok) finish_unit(n_units - 1);   // the last unit
         } else {
             // -------------------------------------------------------------- gather warps
             if (warp < SC_LOAD_WARPS) load_dense(first_unit(P, unit0), warp >> 2, SC_LOAD_WARPS / 4, a_first);
-            ptx::reg_inc<SC_REGS_WORK>();
-            // An 8-lane group walks its span of the pixel-grouped entry list four entries at a time; lane l8 owns
-            // channels 4 l8 .. 4 l8 + 3 of the slab.  The next four entries (and their image rows) are fetched
-            // while the current four are processed.
-            const int gid = (warp - SC_STORE_WARPS) * 4 + (lane >> 3);
+            take_registers<SC_REGS_GATHER>();
+            // An 8-lane group walks its span of the pixel-grouped entry list; lane l8 owns channels 4 l8 .. 4 l8 + 3 and
+            // 32 + 4 l8 .. of the chunk, so that the 8 lanes' 16-byte accesses to columns and sums are contiguous.  An entry is a
+            // pair of neighbouring pixels, so it reads its column values once for both; the one with the even row number adds into the
+            // sums `ev`, the other into `od`, each with a pixel of its own that changes every second step along an image row.
+            const int gid = (warp - SC_FINISH_WARPS) * 4 + (lane >> 3);
             const int l8 = lane & 7;
             using TI = typename std::conditional<M::F32, float, T16>::type;
-            using RAW = typename std::conditional<M::F32, uint4, uint2>::type;
-            const TI *img = reinterpret_cast<const TI *>(P.img_cl);
-            const uint32_t zrow = (uint32_t)g.B * (uint32_t)g.S * (uint32_t)g.Cs;   // what padding entries point at
+            constexpr int IW = M::F32 ? 8 : 4;              // words of an image row per lane
+            struct Rows {
+                uint32_t ev[IW], od[IW];
+            };
+            // Columns of a unit, TMEM -> shared: a warp reads the lanes of its quarter, the warps of a quarter share the columns out in
+            // blocks of 16.
+            const int q = warp & 3, part = (warp - SC_FINISH_WARPS) >> 2;
+            float *col_row = col + (q * 32 + lane) * L.col_stride;
+            int aq = 0;
+            uint32_t t_phase = 0;
             bool ok = true;
-            for (int jp = 0; jp < n_pass && ok; ++jp) {
-                const int j = jp >> 1, slab = jp & 1, pb = j & 1, cb = jp & 1;
-                if (slab == 0) ok = ptx::mbar_wait(&plan_full[pb], (uint32_t)((j >> 1) & 1));
-                ok = ok && ptx::mbar_wait(&col_full[cb], (uint32_t)((jp >> 1) & 1));
+            for (int j = 0; j < n_units && ok; ++j) {
+                const int pb = j & 1;
+                if (j > 0) ok = ptx::mbar_wait(&plan_done[pb ^ 1], (uint32_t)(((j - 1) >> 1) & 1));   // the columns of the unit before have been used
+                for (int slab = 0; slab < 2; ++slab) {
+                    ok = ok && ptx::mbar_wait(&t_full[aq], t_phase);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) {
+                        if (lane == 0) ptx::report(P.status, 301);
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col0 + (uint32_t)(aq * ACCS * N);
+                    for (int blk = part; blk < 2 * TB; blk += SC_GATHER_WARPS / 4) {
+                        uint32_t raw[16];
+                        ptx::tmem_ld_32x16(src + (uint32_t)(blk * 16), raw);
+                        ptx::tmem_ld_wait();
+                        if constexpr (ACCS == 2) {
+                            uint32_t low[16];
+                            ptx::tmem_ld_32x16(src + (uint32_t)(N + blk * 16), low);
+                            ptx::tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 16; ++e)
+                                raw[e] = __float_as_uint(__uint_as_float(raw[e]) + __uint_as_float(low[e]));
+                        }
+                        float *dst = col_row + (blk >> 1) * CHUNK_C + slab * SC_SLAB + (blk & 1) * 16;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            *reinterpret_cast<uint4 *>(dst + 4 * e) =
+                                make_uint4(raw[4 * e], raw[4 * e + 1], raw[4 * e + 2], raw[4 * e + 3]);
+                    }
+                    ptx::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(&t_empty[aq]);
+                    if (++aq == NACC) {
+                        aq = 0;
+                        t_phase ^= 1u;
+                    }
+                }
+                if (!ok) break;
+                if (lane == 0) ptx::mbar_arrive(col_full);
+                ok = ptx::mbar_wait(&plan_full[pb], (uint32_t)((j >> 1) & 1));
+                if (COORD && j >= 2) ok = ok && ptx::mbar_wait(&fin_done[pb], (uint32_t)(((j >> 1) & 1) ^ 1));
+                ok = ok && ptx::mbar_wait(col_full, (uint32_t)(j & 1));
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) {
                     if (lane == 0) ptx::report(P.status, 306);
                     break;
                 }
-                const int span = (int)n_entries[pb];     // entries per group, padded: a multiple of 4
-                const uint4 *my_px = reinterpret_cast<const uint4 *>(plan_px(pb) + gid * span);
-                const uint4 *my_meta = reinterpret_cast<const uint4 *>(plan_meta(pb) + gid * span);
-                const float4 *my_w = reinterpret_cast<const float4 *>(plan_w(pb) + gid * span);
+                const int span = (int)n_entries[pb];     // entries per group, padded: a multiple of 2
+                const uint4 *my_ent = plan_ent(pb) + gid * span;
+                const uint2 *my_meta = reinterpret_cast<const uint2 *>(plan_meta(pb) + gid * span);
                 float *p_dot = plan_dot(pb);
-                const float4 *colb = reinterpret_cast<const float4 *>(col + (size_t)cb * (L.col_buf / 4)) + l8;
-                const uint32_t chan = (uint32_t)(info_of(pb)->x + slab * SC_SLAB + l8 * 4);
-                const TI *img_c = img + chan;
-                float *gimg_c = P.img_grad_cl + chan;
+                const float4 *colb = reinterpret_cast<const float4 *>(col) + l8;
+                const uint32_t chan = (uint32_t)(info_of(j)->x + l8 * 4);
+                // opaque: the compiler would take the sums of base, channel and row apart and add six times
+                uint64_t img_c = reinterpret_cast<uint64_t>(reinterpret_cast<const TI *>(P.img_cl) + chan);
+                uint64_t gimg_c = reinterpret_cast<uint64_t>(P.img_grad_cl + chan);
+                asm volatile("" : "+l"(img_c), "+l"(gimg_c));
 
-                uint32_t cur = zrow;
-                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                // pixel offsets of the four entries at `at`, and (for the coordinate gradients) their image rows
-                auto fetch_rows = [&](uint32_t (&px)[4], RAW (&R)[4], int at) {
-                    const uint4 p4 = my_px[at >> 2];
-                    px[0] = p4.x; px[1] = p4.y; px[2] = p4.z; px[3] = p4.w;
+                float ev[8], od[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) ev[k] = od[k] = 0.f;
+                auto fetch_rows = [&](Rows &rows, const uint4 &e, uint32_t was_ev, uint32_t was_od) {
                     if constexpr (COORD) {
-#pragma unroll
-                        for (int s = 0; s < 4; ++s) R[s] = __ldg(reinterpret_cast<const RAW *>(img_c + px[s]));
+                        load_row<IW>(e.x, was_ev, rows.ev, row_at<sizeof(TI)>(img_c, e.x));
+                        load_row<IW>(e.y, was_od, rows.od, row_at<sizeof(TI)>(img_c, e.y));
                     }
                 };
-                auto image_values = [&](const RAW &r) -> float4 {
-                    if constexpr (M::F32) {
-                        return make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z),
-                                           __uint_as_float(r.w));
-                    } else if constexpr (M::HALF) {
-                        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r.x));
-                        const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
-                        return make_float4(a.x, a.y, b.x, b.y);
-                    } else {
-                        return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u),
-                                           __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
-                    }
-                };
-                auto process = [&](int at, const uint32_t (&pxs)[4], const RAW (&R)[4]) {
-                    const uint4 m4 = my_meta[at >> 2];
-                    const float4 w4 = my_w[at >> 2];
-                    const uint32_t meta[4] = {m4.x, m4.y, m4.z, m4.w};
-                    const float wt[4] = {w4.x, w4.y, w4.z, w4.w};
-                    float d[4];
+                // this lane's share of <column, image row>
+                auto dot = [&](const uint64_t (&c)[4], const uint32_t (&row)[IW]) -> float {
+                    uint64_t d = 0;
 #pragma unroll
-                    for (int s = 0; s < 4; ++s) {
-                        const uint32_t px = pxs[s];
-                        const bool change = px != cur;
-                        red_add_v4_if(change && scatter, gimg_c + cur, acc.x, acc.y, acc.z, acc.w);
-                        cur = px;
-                        const float4 c4 = colb[meta[s] & 0xffffu];
-                        const float w = wt[s];
-                        acc.x = fmaf(w, c4.x, change ? 0.f : acc.x);
-                        acc.y = fmaf(w, c4.y, change ? 0.f : acc.y);
-                        acc.z = fmaf(w, c4.z, change ? 0.f : acc.z);
-                        acc.w = fmaf(w, c4.w, change ? 0.f : acc.w);
-                        if constexpr (COORD) {
-                            const float4 iv = image_values(R[s]);
-                            d[s] = fmaf(c4.x, iv.x, fmaf(c4.y, iv.y, fmaf(c4.z, iv.z, c4.w * iv.w)));
+                    for (int k = 0; k < 4; ++k) {
+                        uint64_t iv;
+                        if constexpr (M::F32) {
+                            iv = pack_f32x2(__uint_as_float(row[2 * k]), __uint_as_float(row[2 * k + 1]));
+                        } else if constexpr (M::HALF) {
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&row[k]));
+                            iv = pack_f32x2(f.x, f.y);
+                        } else {
+                            iv = pack_f32x2(__uint_as_float(row[k] << 16), __uint_as_float(row[k] & 0xffff0000u));
                         }
+                        d = k == 0 ? mul_f32x2(c[k], iv) : fma_f32x2(c[k], iv, d);
                     }
+                    return __uint_as_float((uint32_t)d) + __uint_as_float((uint32_t)(d >> 32));
+                };
+                // adds weight x column to the sums, which were those of pixel `cur` and are now those of px
+                auto add = [&](float (&sum)[8], uint32_t px, uint32_t cur, float w, const uint64_t (&c)[4]) {
+                    flush_sums(px, cur, row_at<4>(gimg_c, cur), sum);
+                    const uint64_t ww = pack_f32x2(w, w);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) unpack_f32x2(fma_f32x2(ww, c[k], pack_f32x2(sum[2 * k], sum[2 * k + 1])), sum[2 * k], sum[2 * k + 1]);
+                };
+                // One entry, the one before it being `prev`; its image rows are in `rows`, which then receives those of `next`.
+                auto load_columns = [&](uint64_t (&c)[4], uint32_t meta) {
+                    const float4 a = colb[meta & 0xffffu], b = colb[(meta & 0xffffu) + 8];
+                    c[0] = pack_f32x2(a.x, a.y);
+                    c[1] = pack_f32x2(a.z, a.w);
+                    c[2] = pack_f32x2(b.x, b.y);
+                    c[3] = pack_f32x2(b.z, b.w);
+                };
+                auto step = [&](const uint4 &prev, const uint4 &e, const uint64_t (&c)[4], Rows &rows, const uint4 &next, float &d_ev, float &d_od) {
                     if constexpr (COORD) {
-                        // sums over the 8 lanes of the four dots at once: after the exchanges lane (b2 b1 b0) holds
-                        // the dot of entry 2 b2 + b1
+                        d_ev = dot(c, rows.ev);
+                        d_od = dot(c, rows.od);
+                    }
+                    fetch_rows(rows, next, e.x, e.y);
+                    if constexpr (SCATTER) {
+                        add(ev, e.x, prev.x, __uint_as_float(e.z), c);
+                        add(od, e.y, prev.y, __uint_as_float(e.w), c);
+                    }
+                };
+                // sums over the 8 lanes of the four dots of two entries at once: after the exchanges lane (b2 b1 b0) holds dot 2 b2 + b1
+                auto reduce = [&](const float (&d)[4], uint32_t m0, uint32_t m1) {
+                    if constexpr (COORD) {
                         const bool h4 = (l8 & 4) != 0, h2 = (l8 & 2) != 0;
                         float k0 = h4 ? d[2] : d[0], k1 = h4 ? d[3] : d[1];
                         k0 += __shfl_xor_sync(0xffffffffu, h4 ? d[0] : d[2], 4);
@@ -657,49 +756,60 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                         float k = h2 ? k1 : k0;
                         k += __shfl_xor_sync(0xffffffffu, h2 ? k0 : k1, 2);
                         k += __shfl_xor_sync(0xffffffffu, k, 1);
-                        if ((l8 & 1) == 0) {
-                            const uint32_t m = h4 ? (h2 ? meta[3] : meta[2]) : (h2 ? meta[1] : meta[0]);
-                            float *slot = p_dot + (m >> 16);
-                            *slot = slab == 0 ? k : *slot + k;
-                        }
+                        if ((l8 & 1) == 0) p_dot[((h4 ? m1 : m0) >> 16) + (h2 ? 1 : 0)] = k;
                     }
                 };
-                RAW Ra[4], Rb[4];
-                uint32_t Pa[4], Pb[4];
                 if (span > 0) {
-                    fetch_rows(Pa, Ra, 0);
-                    // The running pixel starts as the first entry's: no flush before anything was summed.  Padding
-                    // entries (pixel offset zrow) only follow real ones, so inside the loop a flush never has
-                    // cur == zrow; the one after the loop may.
-                    cur = Pa[0];
-                }
-                for (int it = 0; it < span; it += 8) {
-                    // the fetch one batch ahead may run up to 8 entries past the span: still inside the list's slack
-                    fetch_rows(Pb, Rb, it + 4);
-                    process(it, Pa, Ra);
-                    if (it + 4 < span) {
-                        fetch_rows(Pa, Ra, it + 8);
-                        process(it + 4, Pb, Rb);
+                    uint4 A = my_ent[0], B = my_ent[1], C, D;
+                    // image rows: f32 data has registers for one entry's, 16-bit data for two
+                    Rows ra, rb;
+                    Rows &rn = M::F32 ? ra : rb;
+                    fetch_rows(ra, A, ~A.x, ~A.y);
+                    if constexpr (!M::F32) fetch_rows(rb, B, ~B.x, ~B.y);
+                    uint4 last = A;     // the running pixels start as the first entry's: no flush before anything was summed
+                    // Entries are read two ahead, their columns one, past the end of the span: still inside the list's slack.
+                    uint64_t ca[4], cb[4];
+                    uint2 m = my_meta[0];
+                    load_columns(ca, m.x);
+#pragma unroll 1
+                    for (int it = 0; it < span; it += 2) {
+                        float d[4];
+                        const uint2 m2 = my_meta[(it >> 1) + 1];
+                        C = my_ent[it + 2];
+                        load_columns(cb, m.y);
+                        step(last, A, ca, ra, M::F32 ? B : C, d[0], d[1]);
+                        D = my_ent[it + 3];
+                        load_columns(ca, m2.x);
+                        step(A, B, cb, rn, M::F32 ? C : D, d[2], d[3]);
+                        reduce(d, m.x, m.y);
+                        last = B;
+                        A = C;
+                        B = D;
+                        m = m2;
+                    }
+                    if constexpr (SCATTER) {
+                        flush_sums(~last.x, last.x, row_at<4>(gimg_c, last.x), ev);
+                        flush_sums(~last.y, last.y, row_at<4>(gimg_c, last.y), od);
                     }
                 }
-                red_add_v4_if(cur != zrow && scatter, gimg_c + cur, acc.x, acc.y, acc.z, acc.w);
                 __syncwarp();
-                if (lane == 0) {
-                    ptx::mbar_arrive(&col_empty[cb]);
-                    if (slab == 1) ptx::mbar_arrive(&plan_done[pb]);
-                }
+                if (lane == 0) ptx::mbar_arrive(&plan_done[pb]);
             }
         }
     } else if (warp < SC_MMA_WARP) {
         // ------------------------------------------------------------------ planners
-        ptx::reg_inc<SC_REGS_WORK>();
+        take_registers<SC_REGS_PLAN>();
         const int pt = threadIdx.x - SC_PLAN_WARP0 * 32;
         const int pw = warp - SC_PLAN_WARP0;
         UnitIter u = first_unit(P, unit0);
         PosInfo<DIM> pi = decode_position<DIM>(g, (long long)u.x * TILE_POS + pt);
         const uint32_t colq_row = (uint32_t)(pt * (L.col_stride / 4));
-        const uint32_t zrow = (uint32_t)g.B * (uint32_t)g.S * (uint32_t)g.Cs;
+        // Pixels outside the image: one of a few rows behind it, whose sums nobody reads (and whose image row may hold anything: nobody
+        // reads the dot product with it either).
+        const uint32_t waste = ((uint32_t)g.B * (uint32_t)g.S + (blockIdx.x % SCATTER_WASTE_ROWS)) * (uint32_t)g.Cs;
 
+        // four words of padding behind every 32: a thread's 16 slots then meet those of its seven neighbours in no bank
+        auto word_of = [](uint32_t slot) { return slot + (slot >> 5) * 4u; };
         // one thread waits, all learn the result: the named barrier must always see all 128 threads
         auto wait_all = [&](uint64_t *bar, uint32_t parity) -> bool {
             if (pt == 0) *wait_flag = ptx::mbar_wait_backoff<SC_SLEEP_NS>(bar, parity) ? 1u : 0u;
@@ -708,43 +818,45 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             planner_barrier();
             return r;
         };
-        auto build = [&](const int4 &info, int pb, const RawUnit &ru) {
-            const int t0 = info.y;
-            if (pt == 0) *info_of(pb) = info;
-            pos_of(pb)[pt] = make_int2(pi.valid ? pi.b : -1, pi.p);
+        auto build = [&](const int4 &info, int j, const RawUnit &ru) {
+            const int t0 = info.y, pb = j & 1;
+            if (pt == 0) *info_of(j) = info;
+            pos_of(j)[pt] = make_int2(pi.valid ? pi.b : -1, pi.p);
             {
-                uint4 *c4 = reinterpret_cast<uint4 *>(cnt);
+                uint4 *c4 = reinterpret_cast<uint4 *>(cnt + word_of(pt * 16));
 #pragma unroll
-                for (int i = 0; i < SC_SLOTS / 4 / 128; ++i) c4[pt + 128 * i] = make_uint4(0u, 0u, 0u, 0u);
+                for (int i = 0; i < 4; ++i) c4[i] = make_uint4(0u, 0u, 0u, 0u);
             }
             planner_barrier();
             // pass 1: every entry's rank within its slot; all atomics of a thread are independent
-            uint32_t rows[TBM * NC], rank[TBM * NC];
-            float wts[TBM * NC];
+            uint32_t left[TBM * NP];
+            uint32_t slot[TBM * NP];                        // slot, then (12 bits up) the rank in it; two top bits: left, right pixel in the image
+            float wl[TBM * NP], wr[TBM * NP];
 #pragma unroll
             for (int t = 0; t < TBM; ++t) {
                 const bool live = t < TB && t0 + t < g.K && pi.valid;
                 const TapGeometry<DIM> tg = geometry(pi, ru, t, t0 + t);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    bool okc;
-                    uint32_t row;
-                    float w;
-                    corner_of<DIM>(g, pi, tg, deformable, c, okc, row, w);
-                    rows[t * NC + c] = (live && okc) ? row : SC_NONE;
-                    wts[t * NC + c] = w * tg.mval;
+                for (int q = 0; q < NP; ++q) {
+                    const int i = t * NP + q;
+                    bool okl, okr;
+                    uint32_t key;
+                    pair_of<DIM>(g, pi, tg, deformable, q, left[i], key, okl, okr, wl[i], wr[i]);
+                    wl[i] *= tg.mval;
+                    wr[i] *= tg.mval;
+                    slot[i] = (key & (SC_SLOTS - 1)) | ((live && okl) ? 1u << 30 : 0u) | ((live && okr) ? 1u << 31 : 0u);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < TBM * NC; ++i)
-                rank[i] = rows[i] != SC_NONE ? atomicAdd(&cnt[rows[i] & (SC_SLOTS - 1)], 1u) : 0u;
+            for (int i = 0; i < TBM * NP; ++i)
+                if ((slot[i] >> 30) != 0u) slot[i] |= atomicAdd(&cnt[word_of(slot[i] & (SC_SLOTS - 1))], 1u) << 12;
             planner_barrier();
             // exclusive prefix sum of the slot counts, in place (16 slots per thread)
             uint32_t total;
             {
                 uint32_t v[16];
                 uint32_t s = 0;
-                const uint4 *c4 = reinterpret_cast<const uint4 *>(cnt + pt * 16);
+                uint4 *c4 = reinterpret_cast<uint4 *>(cnt + word_of(pt * 16));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint4 x = c4[i];
@@ -768,57 +880,56 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     total += part;
                 }
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    cnt[pt * 16 + i] = run;
-                    run += v[i];
+                for (int i = 0; i < 16; i += 4) {
+                    const uint32_t a = run + v[i], b = a + v[i + 1], c = b + v[i + 2];
+                    c4[i >> 2] = make_uint4(run, a, b, c);
+                    run = c + v[i + 3];
                 }
             }
-            // entries per gather group: a multiple of 4; the list is padded with entries that add nothing
-            const uint32_t span = ((total + SC_GROUPS * 4 - 1) / (SC_GROUPS * 4)) * 4;
+            // entries per gather group: a multiple of 2; the list is padded with entries that add nothing
+            const uint32_t span = ((total + SC_GROUPS * 2 - 1) / (SC_GROUPS * 2)) * 2;
             if (pt == 0) n_entries[pb] = span;
             planner_barrier();
             // pass 2: every entry goes to (start of its slot) + (its rank)
-            uint32_t *e_px = plan_px(pb);
+            uint4 *ent = plan_ent(pb);
             uint32_t *e_meta = plan_meta(pb);
-            float *e_w = plan_w(pb);
 #pragma unroll
             for (int t = 0; t < TBM; ++t) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int i = t * NC + c;
-                    if (rows[i] != SC_NONE) {
-                        const uint32_t at = cnt[rows[i] & (SC_SLOTS - 1)] + rank[i];
-                        e_px[at] = rows[i] * (uint32_t)g.Cs;
-                        e_meta[at] = (colq_row + (uint32_t)(t * (SC_SLAB / 4))) | ((uint32_t)((pt * TB + t) * NC + c) << 16);
-                        e_w[at] = wts[i];
+                for (int q = 0; q < NP; ++q) {
+                    const int i = t * NP + q;
+                    const uint32_t both = slot[i] >> 30;
+                    if (both != 0u) {
+                        const uint32_t at = cnt[word_of(slot[i] & (SC_SLOTS - 1))] + (slot[i] >> 12 & 0xfffu);
+                        const uint32_t pl = (both & 1u) ? left[i] * (uint32_t)g.Cs : waste;
+                        const uint32_t pr = (both & 2u) ? (left[i] + 1u) * (uint32_t)g.Cs : waste;
+                        const bool odd = (left[i] & 1u) != 0u;
+                        const uint32_t a = __float_as_uint(wl[i]), b = __float_as_uint(wr[i]);
+                        ent[at] = odd ? make_uint4(pr, pl, b, a) : make_uint4(pl, pr, a, b);
+                        e_meta[at] = (colq_row + (uint32_t)(t * (CHUNK_C / 4))) | ((uint32_t)((pt * TB + t) * NC + 2 * q) << 16);
                     }
                 }
             }
             // padding entries up to the end of the last span and the words the read-ahead of the last group touches:
-            // all point at the row of zeros and add nothing
-            const uint32_t n_words = span * SC_GROUPS + 8;
+            // all point at the row of waste
+            const uint32_t n_words = span * SC_GROUPS + 4;
             for (uint32_t i = total + pt; i < n_words; i += 128) {
-                e_px[i] = zrow;
-                e_meta[i] = (uint32_t)L.max_entries << 16;
-                e_w[i] = 0.f;
+                ent[i] = make_uint4(waste, waste, 0u, 0u);
+                e_meta[i] = (uint32_t)(2 * L.max_entries) << 16;
             }
             planner_barrier();
             if (lane == 0) ptx::mbar_arrive(&plan_full[pb]);
         };
 
         bool ok = true;
-        // a plan buffer is free again once its unit's dots have been used (store warps), or, without coordinate
-        // gradients, once the gather warps are through with it
-        uint64_t *plan_free = COORD ? fin_done : plan_done;
         RawUnit ru, ru_next;
         int4 info = describe(u);
         load_unit(pi, info, ru);
         ru_next = ru;
-        bool new_tile = false;
         for (int j = 0; j < n_units && ok; ++j) {
             const int pb = j & 1;
             if (j >= 2) {
-                ok = wait_all(&plan_free[pb], (uint32_t)(((j >> 1) & 1) ^ 1));
+                ok = wait_all(&plan_done[pb], (uint32_t)(((j >> 1) & 1) ^ 1));
                 if (!ok) {
                     if (pt == 0) ptx::report(P.status, 307);
                     break;
@@ -831,43 +942,15 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             if (next_new) pi_next = decode_position<DIM>(g, (long long)u_next.x * TILE_POS + pt);
             const int4 info_next = describe(u_next);
             if (j + 1 < n_units) load_unit(pi_next, info_next, ru_next);
-            build(info, pb, ru);
-            if (new_tile) {
-                // One phase of a_free per tile, and the next one cannot complete before this load: neither an earlier
-                // phase nor a later one is taken for it.  (The barriers of the accumulators do not serve: with a single
-                // accumulator the pass two before looks like the one before this unit.)
-                // (The planners are short of registers.  The phase in one of its own cost the f32 volume kernel 1 %; from the tile's
-                // order it costs 16-bit data nothing, but the f32 transposed forward 2 %; counted in shared memory f32 data nothing,
-                // 16-bit 2-d 7 %.)
-                if (pt == 0) {
-                    uint32_t before;            // tiles this CTA has reloaded
-                    if constexpr (M::F32) {
-                        before = *reloads;
-                        *reloads = before + 1u;
-                    } else {
-                        before = (uint32_t)(u.order - unit0 / P.n_units - 1);
-                    }
-                    *wait_flag = ptx::mbar_wait_backoff<SC_SLEEP_NS>(a_free, before & 1u) ? 1u : 0u;
-                }
-                planner_barrier();
-                ok = *wait_flag != 0u;
-                planner_barrier();
-                if (!ok) {
-                    if (pt == 0) ptx::report(P.status, 309);
-                    break;
-                }
-                ptx::tc_fence_after();
-                load_dense(u, 0, 1, a_next);
-            }
+            build(info, j, ru);
             ru = ru_next;
             u = u_next;
             pi = pi_next;
             info = info_next;
-            new_tile = next_new;
         }
     } else if (warp == SC_MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
-        ptx::reg_dec<SC_REGS_ISSUE>();
+        take_registers<SC_REGS_ISSUE>();
         if (lane == 0) {
             const uint32_t idesc = ptx::instr_desc_f16(M::HALF ? 0 : 1, TILE_POS, N, 0, 0);
             bool ok = true, new_tile = true;
@@ -961,7 +1044,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         __syncwarp();
     } else if (warp == SC_TMA_WARP) {
         // ------------------------------------------------------------------ TMA: weight ring
-        ptx::reg_dec<SC_REGS_ISSUE>();
+        take_registers<SC_REGS_ISSUE>();
         if (lane == 0) {
             int s = 0, last_s = -1;
             uint32_t e_phase = 1, last_phase = 0;
@@ -995,7 +1078,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         }
         __syncwarp();
     } else {
-        ptx::reg_dec<SC_REGS_ISSUE>();   // the two idle warps of the last warpgroup
+        take_registers<SC_REGS_ISSUE>();   // the two idle warps of the last warpgroup
     }
 
     ptx::tc_fence_before();
@@ -1020,9 +1103,13 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, c
     const int tiles = P.total_units / P.n_units, many = (Mode<MODE>::F32 ? 4 : 2) * 148;
     const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= many ? tiles : std::min(P.total_units, 148)));
     LaunchScope scope("dcn_dgrad_tc", stream);
-    if (coord)
-        return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, true>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
-    return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, false>>(grid, SC_THREADS, smem, stream, P, maps[0], maps[1], maps[2]);
+    auto run = [&](auto want) {
+        return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, decltype(want)::value>>(grid, SC_THREADS, smem, stream, P, maps[0],
+                                                                                       maps[1], maps[2]);
+    };
+    if (!coord) return run(std::integral_constant<int, SC_SCATTER>());
+    if (P.img_grad_cl == nullptr) return run(std::integral_constant<int, SC_COORD>());
+    return run(std::integral_constant<int, SC_SCATTER | SC_COORD>());
 }
 
 }  // namespace
