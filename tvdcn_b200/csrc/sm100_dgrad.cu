@@ -37,7 +37,7 @@
 // form of the loop: two entries per iteration and no more (a loop of four, 6 KB of code beside the planners' and finishers' straight
 // lines, took 574 instead of 551 us at 128 x 256 x 28 x 28 bf16, 4 groups of offsets), columns and entries read ahead, one
 // branch per flush.  Before, one entry per corner, 4 channels per lane and the columns staged in two halves: 799 us there, 850 f32,
-// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 554, 691, 1162, 3197.  (16 gather warps have
+// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 678, 1162, 3150.  (16 gather warps have
 // no registers to read columns ahead: 586 us, and 768 with the spills of trying.)
 //
 // Warp roles (768 threads): 0-3 finish, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
@@ -178,24 +178,6 @@ struct TapGeometry {
     float mval;
 };
 
-// corner c of the 2^DIM cell: in the image?, pixel row of the channels-last image, interpolation weight
-template <int DIM>
-__device__ __forceinline__ void corner_of(const Geo<DIM> &g, const PosInfo<DIM> &pi, const TapGeometry<DIM> &tg,
-                                          bool deformable, int c, bool &ok, uint32_t &row, float &w) {
-    ok = deformable || c == 0;
-    int flat = 0;
-    w = 1.f;
-#pragma unroll
-    for (int a = 0; a < DIM; ++a) {
-        const int bit = (c >> (DIM - 1 - a)) & 1;
-        const int i = (int)((unsigned)tg.fl[a] + (unsigned)bit);
-        ok = ok && ((unsigned)i < (unsigned)g.img[a]);
-        flat = flat * g.img[a] + i;
-        w *= bit ? tg.fr[a] : (1.f - tg.fr[a]);
-    }
-    row = (uint32_t)(pi.b * g.S + flat);
-}
-
 // Pair q of the 2^(DIM - 1) pairs of corners that are neighbours along the last axis: pixel row of the left one (of the
 // place left of the image where only the right one lies in it), which of the two are in the image, their weights.  key: the
 // left one's place where every image row begins with one place more, which keeps pairs across the edges apart from others.
@@ -248,7 +230,7 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
     L.info = o; o += 4 * 16;                      // of four units: first channel, first tap, offset group, mask group
     L.pos = o;  o += 4 * TILE_POS * 8;            // and per position of the tile: image (or -1), position in it
     L.cnt = o;  o += SC_SLOT_WORDS * 4;
-    L.taps = o; o += SC_MAX_TAPS * 3 * 2;         // kernel coordinates of every tap (int16)
+    L.taps = o; o += SC_MAX_TAPS * 4;             // kernel coordinates of every tap, ten bits per axis
     L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot, reloads
     L.bars = o; o += (uint32_t)(18 + 2 * b_stages) * 8;
     L.total = o;
@@ -349,7 +331,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint64_t *plan_done = plan_full + 2; // [2] gather warps -> themselves, finishing warps, planners: through with the unit's columns and entries
     uint64_t *fin_done = plan_done + 2;  // [2] finishing warps -> gather warps: the dots of the unit have been used
     uint64_t *a_free = fin_done + 2;     // MMA -> planners: the last MMA on the dense tile is through
-    int16_t *tap_tab = reinterpret_cast<int16_t *>(smem + L.taps);
+    uint32_t *tap_tab = reinterpret_cast<uint32_t *>(smem + L.taps);
     const int plan_words = L.max_entries + SC_PLAN_SLACK;
     auto plan_ent = [&](int pb) { return reinterpret_cast<uint4 *>(smem + L.plan + (size_t)pb * L.plan_buf); };
     auto plan_meta = [&](int pb) { return reinterpret_cast<uint32_t *>(plan_ent(pb) + plan_words); };
@@ -389,7 +371,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         int tc[DIM];
         tap_coords<DIM>(g, tp, tc);
 #pragma unroll
-        for (int a = 0; a < DIM; ++a) tap_tab[tp * DIM + a] = (int16_t)tc[a];
+        for (int a = 1; a < DIM; ++a) tc[0] |= tc[a] << (10 * a);
+        tap_tab[tp] = (uint32_t)tc[0];
     }
     if (warp == SC_TMA_WARP && lane == 0) {
         ptx::prefetch_tmap(&tmap_b_hi);
@@ -418,26 +401,29 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         float off[TBM][DIM];
         float m[TBM];
     };
+    // (This and the gradients below run once per unit beside the gather loop, which is short of issue slots and instruction cache: one
+    // pointer and strides, no address from scratch, one body for all taps.  Half the code it was: 554 -> 543 us at 128 x 256 x 28 x 28.)
     auto load_unit = [&](const PosInfo<DIM> &pi, const int4 &info, RawUnit &ru) {
-        const int t0 = info.y, ogi = info.z, mgi = info.w;
+        const int n = pi.valid ? min(TB, g.K - info.y) : 0;
+        const float *po = P.offset + (((int64_t)pi.b * g.og + info.z) * g.K + info.y) * DIM * (int64_t)g.P + pi.p;
+        const float *pm = P.mask + (((int64_t)pi.b * g.mg + info.w) * g.K + info.y) * (int64_t)g.P + pi.p;
 #pragma unroll
         for (int t = 0; t < TBM; ++t) {
-            const bool live = t < TB && t0 + t < g.K && pi.valid;
 #pragma unroll
-            for (int a = 0; a < DIM; ++a)
-                ru.off[t][a] = (live && P.offset != nullptr)
-                                   ? __ldg(P.offset + ((((int64_t)pi.b * g.og + ogi) * g.K + t0 + t) * DIM + a) * (int64_t)g.P + pi.p)
-                                   : 0.f;
-            ru.m[t] = (live && P.mask != nullptr)
-                          ? __ldg(P.mask + (((int64_t)pi.b * g.mg + mgi) * g.K + t0 + t) * (int64_t)g.P + pi.p)
-                          : 1.f;
+            for (int a = 0; a < DIM; ++a) {
+                ru.off[t][a] = (t < n && deformable) ? __ldg(po) : 0.f;
+                po += g.P;
+            }
+            ru.m[t] = (t < n && P.mask != nullptr) ? __ldg(pm) : 1.f;
+            pm += g.P;
         }
     };
     auto geometry = [&](const PosInfo<DIM> &pi, const RawUnit &ru, int t, int tap) -> TapGeometry<DIM> {
         TapGeometry<DIM> tg;
+        const uint32_t tc = tap_tab[tap];
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
-            const int base = pi.base[a] + (int)tap_tab[tap * DIM + a] * g.dil[a];
+            const int base = pi.base[a] + (int)(tc >> (10 * a) & 1023u) * g.dil[a];
             if (deformable) {
                 const float pos = (float)base + ru.off[t][a];
                 const float f = floorf(pos);
@@ -455,48 +441,59 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     // combines the dot products of a finished unit (an entry has two: even pixel row, odd one) into the coordinate gradients of its
     // (position, tap)s
     auto finalize = [&](const PosInfo<DIM> &pi, int pt, const int4 &info, int pb, const RawUnit &ru) {
-        if (!COORD || !pi.valid) return;
-        const int t0 = info.y, ogi = info.z, mgi = info.w;
-        const float *dots = plan_dot(pb);
+        const int n = pi.valid ? min(TB, g.K - info.y) : 0;
+        float *po = P.goff + (((int64_t)pi.b * g.og + info.z) * g.K + info.y) * DIM * (int64_t)g.P + pi.p;
+        float *pm = P.gmask + (((int64_t)pi.b * g.mg + info.w) * g.K + info.y) * (int64_t)g.P + pi.p;
+        const float2 *dots = reinterpret_cast<const float2 *>(plan_dot(pb)) + pt * TB * NP;
+#pragma unroll 1
+        for (int t = 0; t < n; ++t) {
+            RawUnit one;                                     // (a loop, not TBM copies of its body: the registers are picked by selects)
 #pragma unroll
-        for (int t = 0; t < TBM; ++t) {
-            if (t < TB && t0 + t < g.K) {
-                const int tap = t0 + t;
-                const TapGeometry<DIM> tg = geometry(pi, ru, t, tap);
-                float gm = 0.f, go[DIM];
+            for (int k = 0; k < TBM; ++k) {
+                if (k == 0 || k == t) {
 #pragma unroll
-                for (int a = 0; a < DIM; ++a) go[a] = 0.f;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    bool okc;
-                    uint32_t row;
-                    float w;
-                    corner_of<DIM>(g, pi, tg, deformable, c, okc, row, w);
-                    if (okc) {
-                        const float d = dots[(pt * TB + t) * NC + (c & ~1) + (int)(row & 1u)];
-                        gm = fmaf(w, d, gm);
-#pragma unroll
-                        for (int a = 0; a < DIM; ++a) {
-                            float dw = ((c >> (DIM - 1 - a)) & 1) ? 1.f : -1.f;
-#pragma unroll
-                            for (int a2 = 0; a2 < DIM; ++a2)
-                                if (a2 != a) dw *= ((c >> (DIM - 1 - a2)) & 1) ? tg.fr[a2] : (1.f - tg.fr[a2]);
-                            go[a] = fmaf(dw, d, go[a]);
-                        }
-                    }
+                    for (int a = 0; a < DIM; ++a) one.off[0][a] = ru.off[k][a];
+                    one.m[0] = ru.m[k];
                 }
-                if (P.goff != nullptr) {
-#pragma unroll
-                    for (int a = 0; a < DIM; ++a)
-                        atomicAdd(P.goff + ((((int64_t)pi.b * g.og + ogi) * g.K + tap) * DIM + a) * (int64_t)g.P + pi.p,
-                                  tg.mval * go[a]);
-                }
-                if (P.gmask != nullptr)
-                    atomicAdd(P.gmask + (((int64_t)pi.b * g.mg + mgi) * g.K + tap) * (int64_t)g.P + pi.p, gm);
             }
+            const TapGeometry<DIM> tg = geometry(pi, one, 0, info.y + t);
+            // the dots at the corners of the cell, then contracted axis by axis, the last one first: with the weights, and with (-1, 1) for
+            // the axis whose derivative it is
+            float val[NC], der[DIM][NC];
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                uint32_t left, key;
+                bool okl, okr;
+                float wl, wr;
+                pair_of<DIM>(g, pi, tg, deformable, q, left, key, okl, okr, wl, wr);
+                const float2 e = dots[q];
+                const bool odd = (left & 1u) != 0u;
+                val[2 * q] = okl ? (odd ? e.y : e.x) : 0.f;
+                val[2 * q + 1] = okr ? (odd ? e.x : e.y) : 0.f;
+            }
+            dots += NP;
+#pragma unroll
+            for (int a = DIM - 1; a >= 0; --a) {
+                const float f = tg.fr[a], f1 = 1.f - f;
+#pragma unroll
+                for (int i = 0; i < (1 << a); ++i) {
+                    der[a][i] = val[2 * i + 1] - val[2 * i];
+                    val[i] = fmaf(f, val[2 * i + 1], f1 * val[2 * i]);
+#pragma unroll
+                    for (int a2 = a + 1; a2 < DIM; ++a2) der[a2][i] = fmaf(f, der[a2][2 * i + 1], f1 * der[a2][2 * i]);
+                }
+            }
+            if (P.goff != nullptr) {
+#pragma unroll
+                for (int a = 0; a < DIM; ++a) {
+                    atomicAdd(po, tg.mval * der[a][0]);
+                    po += g.P;
+                }
+            }
+            if (P.gmask != nullptr) atomicAdd(pm, val[0]);
+            pm += g.P;
         }
     };
-
 
     // ------------------------------------------------------------------ dense tile -> tensor memory
     // Thread = position (its TMEM lane); `loaders` warps per lane quarter split the channels in units of 16 (8 TMEM
@@ -620,7 +617,9 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             // 32 + 4 l8 .. of the chunk, so that the 8 lanes' 16-byte accesses to columns and sums are contiguous.  An entry is a
             // pair of neighbouring pixels, so it reads its column values once for both; the one with the even row number adds into the
             // sums `ev`, the other into `od`, each with a pixel of its own that changes every second step along an image row.
-            const int gid = (warp - SC_FINISH_WARPS) * 4 + (lane >> 3);
+            // (A warp's four spans lie a quarter of the list apart: at its ends, where the pixels have few entries, every entry costs a flush,
+            // and a warp with such spans only is the one that all wait for: 543 -> 531 us, f32 709 -> 678.)
+            const int gid = (lane >> 3) * SC_GATHER_WARPS + warp - SC_FINISH_WARPS;
             const int l8 = lane & 7;
             using TI = typename std::conditional<M::F32, float, T16>::type;
             constexpr int IW = M::F32 ? 8 : 4;              // words of an image row per lane
