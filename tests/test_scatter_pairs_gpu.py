@@ -21,6 +21,8 @@ EDGES = [
     Case('length_one', 1, False, 5, 64, 128, (1,), (3,), (1,), (1,), (1,), (), 1, 1, 1, True, 1.0),
     Case('thin_volume', 3, False, 1, 64, 64, (4, 5, 1), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0),
     Case('odd_volume', 3, False, 1, 64, 64, (3, 7, 9), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 2.0),
+    # volumes are taken in blocks of 4 x 4 x 8 positions: several tiles, blocks cut off on every side
+    Case('cut_blocks', 3, False, 2, 64, 64, (6, 9, 19), (3, 2, 3), (1, 1, 2), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.5),
     Case('scattered_output', 2, True, 2, 64, 64, (9, 7), (4, 4), (2, 2), (1, 1), (1, 1), (0, 0), 1, 1, 1, True, 2.0),
 ]
 

@@ -37,7 +37,7 @@
 // form of the loop: two entries per iteration and no more (a loop of four, 6 KB of code beside the planners' and finishers' straight
 // lines, took 574 instead of 551 us at 128 x 256 x 28 x 28 bf16, 4 groups of offsets), columns and entries read ahead, one
 // branch per flush.  Before, one entry per corner, 4 channels per lane and the columns staged in two halves: 799 us there, 850 f32,
-// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 678, 1162, 3150.  (16 gather warps have
+// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 678, 1162, 2820.  (16 gather warps have
 // no registers to read columns ahead: 586 us, and 768 with the spills of trying.)
 //
 // Warp roles (768 threads): 0-3 finish, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
@@ -69,6 +69,7 @@ struct DgradParams {
     int tiles_x;            // position tiles
     int n_units;            // units per (position tile, group): (csg / 64) * nbatch
     int total_units;
+    int block[DIM];         // volumes: the grid is taken in blocks of this extent (the last of a row, strip or slab may be smaller)
 };
 
 namespace {
@@ -178,9 +179,55 @@ struct TapGeometry {
     float mval;
 };
 
+// Position number idx of the launch: images one after the other; volumes in blocks of 4 x 4 x 8, each row by row.  A tile of whole
+// rows of a volume has many pixels around it, and the more there are, the fewer entries share one: blocks take 8 x 64 x 16 x 56 x 56 f32
+// (offsets of sigma 1) from 3150 to 2820 us, 4 x 64 x 16 x 40 x 40 from 787 to 744 (sigma 0.5) and 949 to 842 (3), 128 x 6 x 60 x 90 bf16
+// from 533 to 398.  (8 x 16 in 2-d gains 10 % on images 160 wide and nothing on those below 100, and its arithmetic in the
+// planners cost narrow ones up to 5 %.)
+template <int DIM>
+__device__ __forceinline__ PosInfo<DIM> decode_blocked(const DgradParams<DIM> &P, long long idx) {
+    const Geo<DIM> &g = P.g;
+    if constexpr (DIM < 3) {
+        return decode_position<DIM>(g, idx);
+    } else {
+        PosInfo<DIM> pi;
+        pi.valid = idx < g.BP;
+        const int i = pi.valid ? (int)idx : 0;             // fewer than 2^31 positions
+        pi.b = i / g.P;
+        int r = i - pi.b * g.P;
+        int first[DIM], ext[DIM], size = g.P;              // size: positions of what is being cut (image, slab, strip)
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+            const int line = size / g.grid[a] ;            // positions per unit of length along this axis
+            const int blk = r / (line * P.block[a]);
+            first[a] = blk * P.block[a];
+            ext[a] = min(P.block[a], g.grid[a] - first[a]);
+            r -= line * first[a];
+            size = line * ext[a];
+        }
+        int c[DIM];
+#pragma unroll
+        for (int a = DIM - 1; a > 0; --a) {
+            const int q = r / ext[a];
+            c[a] = first[a] + r - q * ext[a];
+            r = q;
+        }
+        c[0] = first[0] + r;
+        pi.p = 0;
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+            pi.p = pi.p * g.grid[a] + c[a];
+            pi.base[a] = c[a] * g.stride[a] - g.pad[a];
+        }
+        return pi;
+    }
+}
+
 // Pair q of the 2^(DIM - 1) pairs of corners that are neighbours along the last axis: pixel row of the left one (of the
 // place left of the image where only the right one lies in it), which of the two are in the image, their weights.  key: the
-// left one's place where every image row begins with one place more, which keeps pairs across the edges apart from others.
+// left one's slot in the counting sort: its place where every row begins with one place more (which keeps pairs across an edge
+// apart from others), modulo the slots; in volumes, whose planes would meet there, some bits of each coordinate, as many as a
+// tile reaches.
 template <int DIM>
 __device__ __forceinline__ void pair_of(const Geo<DIM> &g, const PosInfo<DIM> &pi, const TapGeometry<DIM> &tg,
                                         bool deformable, int q, uint32_t &left, uint32_t &key, bool &ok_l, bool &ok_r, float &w_l,
@@ -188,10 +235,13 @@ __device__ __forceinline__ void pair_of(const Geo<DIM> &g, const PosInfo<DIM> &p
     bool ok = deformable || q == 0;
     int flat = 0;
     float w = 1.f;
+    unsigned row_y = 0, row_z = 0;
 #pragma unroll
     for (int a = 0; a < DIM - 1; ++a) {
         const int bit = (q >> (DIM - 2 - a)) & 1;
         const int i = (int)((unsigned)tg.fl[a] + (unsigned)bit);
+        row_z = row_y;
+        row_y = (unsigned)i;
         ok = ok && ((unsigned)i < (unsigned)g.img[a]);
         flat = flat * g.img[a] + i;
         w *= bit ? tg.fr[a] : (1.f - tg.fr[a]);
@@ -204,7 +254,9 @@ __device__ __forceinline__ void pair_of(const Geo<DIM> &g, const PosInfo<DIM> &p
     for (int a = 0; a < DIM - 1; ++a) row *= (unsigned)g.img[a];
     row += (unsigned)flat;
     left = row * (unsigned)g.img[DIM - 1] + i;
-    key = left + row + 1u;
+    if constexpr (DIM < 3) key = left + row + 1u;
+    else key = ((i + 1u) & 15u) | (row_y & 15u) << 4 | ((unsigned)pi.b * (unsigned)g.img[0] + row_z & 7u) << 8;
+    key &= SC_SLOTS - 1;
     w_l = w * (1.f - tg.fr[DIM - 1]);
     w_r = w * tg.fr[DIM - 1];
 }
@@ -501,7 +553,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     auto load_dense = [&](const UnitIter &u, int part, int loaders, uint64_t *bar) {
         constexpr int U = 2;                            // units (of 16 loads) in flight per thread
         const int q = warp & 3;
-        const PosInfo<DIM> pa = decode_position<DIM>(g, (long long)u.x * TILE_POS + q * 32 + lane);
+        const PosInfo<DIM> pa = decode_blocked<DIM>(P, (long long)u.x * TILE_POS + q * 32 + lane);
         const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
         const int64_t base = ((int64_t)pa.b * g.Cd_r + (int64_t)u.grp * g.cdg_r) * g.P + pa.p;
         const int n_units_a = g.cdg / 16;
@@ -801,7 +853,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         const int pt = threadIdx.x - SC_PLAN_WARP0 * 32;
         const int pw = warp - SC_PLAN_WARP0;
         UnitIter u = first_unit(P, unit0);
-        PosInfo<DIM> pi = decode_position<DIM>(g, (long long)u.x * TILE_POS + pt);
+        PosInfo<DIM> pi = decode_blocked<DIM>(P, (long long)u.x * TILE_POS + pt);
         const uint32_t colq_row = (uint32_t)(pt * (L.col_stride / 4));
         // Pixels outside the image: one of a few rows behind it, whose sums nobody reads (and whose image row may hold anything: nobody
         // reads the dot product with it either).
@@ -843,7 +895,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     pair_of<DIM>(g, pi, tg, deformable, q, left[i], key, okl, okr, wl[i], wr[i]);
                     wl[i] *= tg.mval;
                     wr[i] *= tg.mval;
-                    slot[i] = (key & (SC_SLOTS - 1)) | ((live && okl) ? 1u << 30 : 0u) | ((live && okr) ? 1u << 31 : 0u);
+                    slot[i] = key | ((live && okl) ? 1u << 30 : 0u) | ((live && okr) ? 1u << 31 : 0u);
                 }
             }
 #pragma unroll
@@ -938,7 +990,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             UnitIter u_next = u;
             const bool next_new = next_unit(P, u_next);
             PosInfo<DIM> pi_next = pi;
-            if (next_new) pi_next = decode_position<DIM>(g, (long long)u_next.x * TILE_POS + pt);
+            if (next_new) pi_next = decode_blocked<DIM>(P, (long long)u_next.x * TILE_POS + pt);
             const int4 info_next = describe(u_next);
             if (j + 1 < n_units) load_unit(pi_next, info_next, ru_next);
             build(info, j, ru);
@@ -1185,6 +1237,7 @@ cudaError_t launch_gemm_scatter_tc(const GeoHost &h, int mode, const void *dense
         P.tiles_x = tiles_x;
         P.n_units = n_units;
         P.total_units = total;
+        for (int a = 0; a < DIM; ++a) P.block[a] = std::min(h.grid[a], a == DIM - 1 ? 8 : 4);
         // 16-bit data: nothing is rounded between the MMA and the results, there is no wide mode of its own
         switch (mode) {
             case TC_BF16: case TC_BF16_WIDE: return launch_dgrad_t<DIM, TC_BF16>(P, maps, stream);
