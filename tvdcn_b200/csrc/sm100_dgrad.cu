@@ -37,7 +37,7 @@
 // form of the loop: two entries per iteration and no more (a loop of four, 6 KB of code beside the planners' and finishers' straight
 // lines, took 574 instead of 551 us at 128 x 256 x 28 x 28 bf16, 4 groups of offsets), columns and entries read ahead, one
 // branch per flush.  Before, one entry per corner, 4 channels per lane and the columns staged in two halves: 799 us there, 850 f32,
-// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 678, 1162, 2820.  (16 gather warps have
+// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 678, 1162, 2644.  (16 gather warps have
 // no registers to read columns ahead: 586 us, and 768 with the spills of trying.)
 //
 // Warp roles (768 threads): 0-3 finish, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
@@ -105,8 +105,9 @@ constexpr int SC_TMEM_COLS = 512;
 constexpr int SC_SLEEP_NS = 32;                                   // back-off of the long waits (64 to 512 measured equal)
 constexpr int SC_MAX_TAPS = 512;                                  // taps whose kernel coordinates a CTA tabulates
 
-// most taps per batch: shared memory holds the column values and the entry lists of two batches
-__host__ __device__ constexpr int sc_tb_max(int dim) { return dim == 1 ? 4 : (dim == 2 ? 3 : 2); }
+// most taps per batch: shared memory holds the columns of one batch and the entry lists of two (volumes: three taps leave
+// room for two stages of weights, and still gain over two taps with four: 8 x 64 x 16 x 56 x 56 f32 2822 -> 2644 us)
+__host__ __device__ constexpr int sc_tb_max(int dim) { return dim == 1 ? 4 : 3; }
 
 __device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
     uint64_t r;
@@ -880,21 +881,23 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             }
             planner_barrier();
             // pass 1: every entry's rank within its slot; all atomics of a thread are independent
-            uint32_t left[TBM * NP];
+            constexpr bool AGAIN = TBM * NP > 8;            // pass 2 works pixels and weights out again: there are no registers to keep them
+            constexpr int KEPT = AGAIN ? 1 : TBM * NP;
+            uint32_t left[KEPT];
             uint32_t slot[TBM * NP];                        // slot, then (12 bits up) the rank in it; two top bits: left, right pixel in the image
-            float wl[TBM * NP], wr[TBM * NP];
+            float wl[KEPT], wr[KEPT];
 #pragma unroll
             for (int t = 0; t < TBM; ++t) {
                 const bool live = t < TB && t0 + t < g.K && pi.valid;
                 const TapGeometry<DIM> tg = geometry(pi, ru, t, t0 + t);
 #pragma unroll
                 for (int q = 0; q < NP; ++q) {
-                    const int i = t * NP + q;
+                    const int i = t * NP + q, k = AGAIN ? 0 : i;
                     bool okl, okr;
                     uint32_t key;
-                    pair_of<DIM>(g, pi, tg, deformable, q, left[i], key, okl, okr, wl[i], wr[i]);
-                    wl[i] *= tg.mval;
-                    wr[i] *= tg.mval;
+                    pair_of<DIM>(g, pi, tg, deformable, q, left[k], key, okl, okr, wl[k], wr[k]);
+                    wl[k] *= tg.mval;
+                    wr[k] *= tg.mval;
                     slot[i] = key | ((live && okl) ? 1u << 30 : 0u) | ((live && okr) ? 1u << 31 : 0u);
                 }
             }
@@ -946,16 +949,25 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             uint32_t *e_meta = plan_meta(pb);
 #pragma unroll
             for (int t = 0; t < TBM; ++t) {
+                TapGeometry<DIM> tg;
+                if constexpr (AGAIN) tg = geometry(pi, ru, t, t0 + t);
 #pragma unroll
                 for (int q = 0; q < NP; ++q) {
-                    const int i = t * NP + q;
+                    const int i = t * NP + q, k = AGAIN ? 0 : i;
                     const uint32_t both = slot[i] >> 30;
                     if (both != 0u) {
+                        if constexpr (AGAIN) {
+                            bool okl, okr;
+                            uint32_t key;
+                            pair_of<DIM>(g, pi, tg, deformable, q, left[0], key, okl, okr, wl[0], wr[0]);
+                            wl[0] *= tg.mval;
+                            wr[0] *= tg.mval;
+                        }
                         const uint32_t at = cnt[word_of(slot[i] & (SC_SLOTS - 1))] + (slot[i] >> 12 & 0xfffu);
-                        const uint32_t pl = (both & 1u) ? left[i] * (uint32_t)g.Cs : waste;
-                        const uint32_t pr = (both & 2u) ? (left[i] + 1u) * (uint32_t)g.Cs : waste;
-                        const bool odd = (left[i] & 1u) != 0u;
-                        const uint32_t a = __float_as_uint(wl[i]), b = __float_as_uint(wr[i]);
+                        const uint32_t pl = (both & 1u) ? left[k] * (uint32_t)g.Cs : waste;
+                        const uint32_t pr = (both & 2u) ? (left[k] + 1u) * (uint32_t)g.Cs : waste;
+                        const bool odd = (left[k] & 1u) != 0u;
+                        const uint32_t a = __float_as_uint(wl[k]), b = __float_as_uint(wr[k]);
                         ent[at] = odd ? make_uint4(pr, pl, b, a) : make_uint4(pl, pr, a, b);
                         e_meta[at] = (colq_row + (uint32_t)(t * (CHUNK_C / 4))) | ((uint32_t)((pt * TB + t) * NC + 2 * q) << 16);
                     }
