@@ -81,3 +81,13 @@ def test_infinite_gradient_stays_with_its_pixels():
         hit = lambda t: (~torch.isfinite(t)).any(dim=1)
         assert hit(ref).any() and not hit(ref).all()
         assert torch.equal(hit(got), hit(ref))
+
+
+@pytest.mark.parametrize('length', [1466, 1494], ids=['ranges', 'cta_per_tile'])
+def test_volumes_around_the_line(length):
+    """f32 volumes have one CTA per tile from 1480 tiles on."""
+    case = Case('volume', 3, False, 1, 64, 64, (2, 8, 8 * length), (1, 1, 2), (1, 1, 1), (0, 0, 0), (1, 1, 1), (), 1, 1, 1, True, 1.0)
+    _, dev = _device_inputs(case, torch.float32, 84)
+    got, ref = run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1)
+    for a, r in zip((got[1], got[3], got[4]), (ref[1], ref[3], ref[4])):
+        assert cases.nerr(a, r) <= 1e-4

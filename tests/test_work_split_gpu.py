@@ -105,7 +105,7 @@ def test_volume_with_one_cta_per_tile():
 
 @pytest.mark.parametrize('width', [58, 60], ids=['ranges', 'one_per_tile'])
 def test_volume_of_16_bit_data_around_its_line(width):
-    """290 and 300 tiles: 16-bit volumes have one CTA per tile from 296 on."""
+    """290 and 300 tiles: around two tiles per SM."""
     case = Case('volume16', 3, False, 1, 64, 64, (16, 40, width), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0)
     x, w, off, mask, bias, go = (t.float().cuda() for t in make_inputs(case, seed=77))
     dev = [x.bfloat16(), w.bfloat16(), off, mask, bias, go.bfloat16()]

@@ -383,7 +383,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     uint64_t *plan_full = col_full + 1;  // [2] planners -> gather warps
     uint64_t *plan_done = plan_full + 2; // [2] gather warps -> themselves, finishing warps, planners: through with the unit's columns and entries
     uint64_t *fin_done = plan_done + 2;  // [2] finishing warps -> gather warps: the dots of the unit have been used
-    uint64_t *a_free = fin_done + 2;     // MMA -> planners: the last MMA on the dense tile is through
+    uint64_t *a_free = fin_done + 2;     // MMA -> finishing warps: the last MMA on the dense tile is through
     uint32_t *tap_tab = reinterpret_cast<uint32_t *>(smem + L.taps);
     const int plan_words = L.max_entries + SC_PLAN_SLACK;
     auto plan_ent = [&](int pb) { return reinterpret_cast<uint4 *>(smem + L.plan + (size_t)pb * L.plan_buf); };
@@ -1157,14 +1157,12 @@ template <int DIM, int MODE>
 cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, cudaStream_t stream) {
     const size_t smem = dgrad_smem_bytes(DIM, MODE, P.tb, P.b_stages);
     const bool coord = P.goff != nullptr || P.gmask != nullptr;
-    // One CTA per SM, except for volumes of many tiles: 27 taps of 8 corners dwarf a CTA's start-up, and the tiles' costs
-    // differ so much that the hardware's scheduling beats equal ranges.  Backward calls, us, ranges / one CTA per tile: 16-bit
-    // data gain from two tiles per SM on (216 tiles 400 / 410, 296 491 / 486, 440 761 / 705, 1032 1723 / 1638, at worst 3.5 % lost at
-    // 392 tiles), f32 data, with its longer loads of a dense tile, from some ten on (440 817 / 826, 1036 1848 / 1895, 3136 6089 / 5798,
-    // 4096 8900 / 8039; between 3 and 10 per SM either side wins 4 % at most, so the line is at four).  Eight taps have too
-    // few units per tile (2651 tiles 1362 / 1402).
-    const int tiles = P.total_units / P.n_units, many = (Mode<MODE>::F32 ? 4 : 2) * 148;
-    const dim3 grid((unsigned)(DIM == 3 && P.n_units >= 8 && tiles >= many ? tiles : std::min(P.total_units, 148)));
+    // One CTA per SM, except for f32 volumes of many tiles, whose costs differ so much that the hardware's scheduling beats equal
+    // ranges.  Backward kernel of 64 channels, 27 taps, us, ranges / one CTA per tile: f32 392 tiles 334 / 363, 784 674 / 713, 1568
+    // 1389 / 1351, 3136 2734 / 2643, so the line is at ten per SM; 16-bit data, with its shorter start-up but also shorter tiles, 200
+    // tiles 173 / 220, 784 588 / 664, 3136 2300 / 2433.  8 taps, 2744 tiles: f32 1918 / 1714, 16-bit 1510 / 1466.
+    const int tiles = P.total_units / P.n_units;
+    const dim3 grid((unsigned)(DIM == 3 && Mode<MODE>::F32 && tiles >= 10 * 148 ? tiles : std::min(P.total_units, 148)));
     LaunchScope scope("dcn_dgrad_tc", stream);
     auto run = [&](auto want) {
         return launch_dependent<dcn_dgrad_tc_kernel<DIM, MODE, decltype(want)::value>>(grid, SC_THREADS, smem, stream, P, maps[0],
