@@ -331,23 +331,23 @@ def known_traffic(kernel: str, config: int, mode: str):
     under profiles/; None where no capture exists.  The figures are for the configuration's full batch on one GPU."""
     table = {
         # config 2: full-size launches (profiles/config2_tensor_kernels.md)
-        'dcn_fwd_tc/cfg2/bf16': 118.6e6 + 49.6e6,
-        'dcn_dgrad_tc/cfg2/bf16': 446.8e6 + 234.9e6,
-        'dcn_wgrad_tc/cfg2/bf16': 137.7e6 + 3.88e6,
-        'dcn_fwd_tc/cfg2/fp32': 220.4e6 + 99.5e6,
-        'dcn_dgrad_tc/cfg2/fp32': 768.0e6 + 281.1e6,
-        'dcn_wgrad_tc/cfg2/fp32': 250.7e6 + 5.93e6,
+        'dcn_fwd_tc/cfg2/bf16': 98.1e6 + 21.5e6,
+        'dcn_dgrad_tc/cfg2/bf16': 427.2e6 + 219.8e6,
+        'dcn_wgrad_tc/cfg2/bf16': 137.7e6 + 3.62e6,
+        'dcn_fwd_tc/cfg2/fp32': 206.4e6 + 74.7e6,
+        'dcn_dgrad_tc/cfg2/fp32': 767.7e6 + 281.5e6,
+        'dcn_wgrad_tc/cfg2/fp32': 250.8e6 + 6.04e6,
         # configs 3-5: captured on a cut batch (profiles/config3_config4_config5_tensor_kernels.md) and scaled to
         # the full batch by the images processed -- tiles are independent, traffic grows in proportion
-        'dcn_fwd_tc/cfg3/fp32': (75.54e6 + 26.47e6) * 8,
-        'dcn_dgrad_tc/cfg3/fp32': (223.1e6 + 45.46e6) * 8,
-        'dcn_wgrad_tc/cfg3/fp32': (141.0e6 + 3.73e6) * 8,
-        'dcn_fwd_tc/cfg4/fp32': (72.93e6 + 13.54e6) * 4,
-        'dcn_dgrad_tc/cfg4/fp32': (164.9e6 + 35.47e6) * 4,
-        'dcn_wgrad_tc/cfg4/fp32': (96.05e6 + 5.36e6) * 4,
-        'dcn_fwd_tc/cfg5/fp32': (41.01e6 + 0.17e6) * 4,
-        'dcn_dgrad_tc/cfg5/fp32': (58.24e6 + 0.10e6 + 63.64e6 + 1.11e6) / 2 * 4,   # two launches per step, mean
-        'dcn_wgrad_tc/cfg5/fp32': (57.75e6 + 0.61e6) * 4,
+        'dcn_fwd_tc/cfg3/fp32': (75.52e6 + 27.14e6) * 8,
+        'dcn_dgrad_tc/cfg3/fp32': (222.9e6 + 44.69e6) * 8,
+        'dcn_wgrad_tc/cfg3/fp32': (141.0e6 + 4.24e6) * 8,
+        'dcn_fwd_tc/cfg4/fp32': (72.92e6 + 11.68e6) * 4,
+        'dcn_dgrad_tc/cfg4/fp32': (255.6e6 + 59.92e6) * 4,
+        'dcn_wgrad_tc/cfg4/fp32': (95.95e6 + 4.61e6) * 4,
+        'dcn_fwd_tc/cfg5/fp32': (41.01e6 + 0.16e6) * 4,
+        'dcn_dgrad_tc/cfg5/fp32': (57.79e6 + 0.03e6 + 63.18e6 + 2.08e6) / 2 * 4,   # two launches per step, mean
+        'dcn_wgrad_tc/cfg5/fp32': (57.75e6 + 0.65e6) * 4,
     }
     return table.get(f'{kernel}/cfg{config}/{mode}')
 
