@@ -91,3 +91,32 @@ def test_volumes_around_the_line(length):
     got, ref = run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1)
     for a, r in zip((got[1], got[3], got[4]), (ref[1], ref[3], ref[4])):
         assert cases.nerr(a, r) <= 1e-4
+
+
+ODD_OFFSETS = [
+    Case('odd_offsets_1d', 1, False, 2, 64, 64, (70,), (3,), (1,), (1,), (1,), (), 1, 1, 1, True, 1.0),
+    Case('odd_offsets_2d', 2, False, 2, 64, 64, (9, 11), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.0),
+    Case('odd_offsets_3d', 3, False, 1, 64, 64, (4, 5, 7), (3, 2, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0),
+    Case('odd_offsets_T', 2, True, 2, 64, 64, (6, 7), (4, 4), (2, 2), (1, 1), (1, 1), (0, 0), 1, 1, 1, True, 1.0),
+]
+
+
+@pytest.mark.parametrize('value', [float('inf'), float('-inf'), 1e30, float('nan')], ids=['inf', 'minus_inf', 'huge', 'nan'])
+@pytest.mark.parametrize('case', ODD_OFFSETS, ids=[c.name for c in ODD_OFFSETS])
+@pytest.mark.parametrize('dtype,aux,tol', [(torch.float32, torch.float32, 1e-4), (torch.bfloat16, torch.float32, 2e-2),
+                                           (torch.float16, torch.float16, 5e-3)], ids=['f32', 'bf16', 'f16'])
+def test_offsets_that_are_not_finite(case, dtype, aux, tol, value):
+    """A cell outside of the image, however far, has no gradients; a NaN offset's are those of the SIMT kernels, value by value."""
+    _, dev = _device_inputs(case, dtype, 85)
+    dev = [t.to(aux) if i in (2, 3, 4) else t for i, t in enumerate(dev)]
+    off = dev[2].flatten(2)
+    for axis in range(case.dim):     # some positions of every (tap, axis), each axis at positions of its own
+        off[:, axis::case.dim, axis::case.dim + 2] = value
+    got, ref = run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1)
+    if value == value:
+        assert all(torch.isfinite(r).all() for r in ref)
+        cases.assert_parity(got, ref, tol, case.name)
+    for i in (3, 4) if case.transposed else (1, 3, 4):
+        finite = torch.isfinite(ref[i])
+        assert torch.equal(torch.isfinite(got[i]), finite), cases.NAMES[i]
+        assert cases.nerr(torch.where(finite, got[i], 0), torch.where(finite, ref[i], 0)) <= tol, cases.NAMES[i]

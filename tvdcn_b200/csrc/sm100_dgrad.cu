@@ -513,6 +513,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
             // the dots at the corners of the cell, then contracted axis by axis, the last one first: with the weights, and with (-1, 1) for
             // the axis whose derivative it is
             float val[NC], der[DIM][NC];
+            bool inside = false;
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
                 uint32_t left, key;
@@ -521,6 +522,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 pair_of<DIM>(g, pi, tg, deformable, q, left, key, okl, okr, wl, wr);
                 const float2 e = dots[q];
                 const bool odd = (left & 1u) != 0u;
+                inside = inside || okl || okr;
                 val[2 * q] = okl ? (odd ? e.y : e.x) : 0.f;
                 val[2 * q + 1] = okr ? (odd ? e.x : e.y) : 0.f;
             }
@@ -536,14 +538,15 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     for (int a2 = a + 1; a2 < DIM; ++a2) der[a2][i] = fmaf(f, der[a2][2 * i + 1], f1 * der[a2][2 * i]);
                 }
             }
+            // A cell outside of the image has no gradients, whatever its fractions are: those of an infinite offset are NaN.
             if (P.goff != nullptr) {
 #pragma unroll
                 for (int a = 0; a < DIM; ++a) {
-                    atomicAdd(po, tg.mval * der[a][0]);
+                    atomicAdd(po, tg.mval * (inside ? der[a][0] : 0.f));
                     po += g.P;
                 }
             }
-            if (P.gmask != nullptr) atomicAdd(pm, val[0]);
+            if (P.gmask != nullptr) atomicAdd(pm, inside ? val[0] : 0.f);
             pm += g.P;
         }
     };
