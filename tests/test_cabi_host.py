@@ -146,6 +146,15 @@ def test_lines_between_the_engines(dim, transposed, dtype, cin, cout, positions,
         assert L.tvdcn_b200_engine_name(ctypes.byref(p), backward).decode() == 'tcgen05'
 
 
+def test_transposed_forward_needs_its_accumulator_and_weights_only():
+    """Packed weights and the f32 accumulator of the output, nothing behind them: exactly the scratch that is built in."""
+    L = cabi.lib()
+    L.tvdcn_b200_static_scratch_bytes.restype = ctypes.c_size_t
+    p = cabi.make_problem(2, True, cabi.F32, 1, 64, 64, (126, 128), (4, 4), (2, 2), (1, 1), (1, 1), 1, 1, 1)
+    need = 2 * 64 * 64 * 16 * 2 + 252 * 256 * 64 * 4
+    assert L.tvdcn_b200_forward_workspace_bytes(ctypes.byref(p)) == need == L.tvdcn_b200_static_scratch_bytes()
+
+
 @pytest.mark.parametrize('transposed', [False, True])
 @pytest.mark.parametrize('dtype', [cabi.F32, cabi.BF16])
 def test_workspace_sizes_of_an_empty_batch(transposed, dtype):

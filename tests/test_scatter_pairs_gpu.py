@@ -83,6 +83,43 @@ def test_infinite_gradient_stays_with_its_pixels():
         assert torch.equal(hit(got), hit(ref))
 
 
+LONE = [   # entries that lack a pixel: without offsets all of them, and at every edge of a narrow image
+    Case('lone_1d', 1, False, 2, 64, 64, (37,), (3,), (1,), (1,), (1,), (), 1, 0, 1, True, 0.0),
+    Case('lone_2d', 2, False, 2, 64, 64, (6, 7), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 0, 1, True, 0.0),
+    Case('lone_3d', 3, False, 2, 64, 64, (3, 4, 5), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 0, 1, True, 0.0),
+    Case('single_pixels', 1, False, 5, 64, 64, (1,), (3,), (1,), (1,), (1,), (), 1, 1, 1, True, 1.0),
+    Case('single_pixel', 2, False, 1, 64, 64, (1, 1), (3, 3), (1, 1), (1, 1), (1, 1), (), 1, 1, 1, True, 1.0),
+    Case('one_wide_volume', 3, False, 1, 64, 64, (4, 3, 1), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0),
+    Case('lone_T', 2, True, 2, 64, 64, (5, 4), (4, 4), (2, 2), (1, 1), (1, 1), (0, 0), 1, 0, 1, True, 0.0),
+]
+
+
+@pytest.mark.parametrize('case', LONE, ids=[c.name for c in LONE])
+@pytest.mark.parametrize('dtype,tol', [(torch.float32, 1e-4), (torch.bfloat16, 2e-2)], ids=['f32', 'bf16'])
+def test_lone_pixels(case, dtype, tol):
+    host, dev = _device_inputs(case, dtype, 86)
+    ref = run_oracle(case, *(None if t is None else t.double() for t in host))
+    cases.assert_parity(run_cabi(case, *dev, engine=2), ref, tol, case.name)
+
+
+@pytest.mark.parametrize('case', LONE, ids=[c.name for c in LONE])
+@pytest.mark.parametrize('at', [0, -1], ids=['first', 'last'])
+@pytest.mark.parametrize('what', ['gradient', 'mask'])
+def test_lone_pixels_take_nothing_that_is_not_finite(case, at, what):
+    """What an infinite gradient (in the transposed forward call: input) or a mask that is NaN reaches, and no neighbour of it.  The
+    mask's bits are all ones."""
+    _, dev = _device_inputs(case, torch.float32, 87)
+    dense = 0 if case.transposed else 5
+    if what == 'gradient':
+        dev[dense].flatten(2)[0 if at == 0 else -1, :, at] = float('inf')
+    else:
+        dev[3].view(torch.int32).flatten(2)[0 if at == 0 else -1, :, at] = -1
+    got, ref = run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1)
+    i = 0 if case.transposed else 1
+    hit = lambda t: (~torch.isfinite(t)).any(dim=1)
+    assert hit(ref[i]).any() and torch.equal(hit(got[i]), hit(ref[i]))
+
+
 @pytest.mark.parametrize('length', [1466, 1494], ids=['ranges', 'cta_per_tile'])
 def test_volumes_around_the_line(length):
     """f32 volumes have one CTA per tile from 1480 tiles on."""

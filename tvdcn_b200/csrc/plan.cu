@@ -13,7 +13,6 @@ struct Bump {
         off = align_up(off + bytes);
         return at;
     }
-    void reach(size_t end) { off = std::max(off, align_up(end)); }
 };
 // A granule of channels padded by more than this runs on the SIMT kernels.  A tensor-core kernel's time does not depend on how
 // much of the 64 channels is real, a SIMT kernel's is proportional to it.  SIMT / tensor us at 4 x 128 x 128, 3 x 3 (f32; bf16),
@@ -127,7 +126,7 @@ void take_sample_buffers(Plan &pl, Bump &b, const GeoHost &g, int bn, bool share
 // buffers of the GEMM -> scatter kernel
 void take_scatter_buffers(Plan &pl, Bump &b, const GeoHost &g, bool scatter) {
     take_parts(pl.w_pack_kd, b, mode_mat_parts(pl.mode), packed_elems(g));
-    if (scatter) pl.img_grad_cl = b.take(((size_t)g.B * g.S + SCATTER_WASTE_ROWS) * g.Cs * sizeof(float));
+    if (scatter) pl.img_grad_cl = b.take((size_t)g.B * g.S * g.Cs * sizeof(float));
 }
 }  // namespace
 
@@ -215,11 +214,7 @@ Plan plan_backward(const tvdcn_problem *p, bool want_input, bool want_weight, bo
             const int parts = p->dtype == TVDCN_F32 ? mode_mat_parts(pl.mode_sw) : (g.P % 8 != 0 ? 1 : 0);
             take_parts(pl.dense, b, parts, (size_t)g.B * g.Cd_r * pl.dense_pitch);
         }
-        if (pl.tc_gs) {
-            take_scatter_buffers(pl, b, g, scatter);
-            // the kernel also reads (and ignores) as many image rows behind the image: whatever lies there, but in the workspace
-            b.reach(pl.img_cl + ((size_t)g.B * g.S + SCATTER_WASTE_ROWS) * g.Cs * (p->dtype == TVDCN_F32 ? 4 : 2));
-        }
+        if (pl.tc_gs) take_scatter_buffers(pl, b, g, scatter);
         if (!pl.tensor) pl.why_not = "no tensor-core kernel covers the requested gradients for this shape";
     } else {
         pl.why_not = why;

@@ -10,7 +10,6 @@
 namespace tvdcn_b200 {
 
 constexpr size_t NO_BUF = (size_t)-1;
-constexpr int SCATTER_WASTE_ROWS = 16;   // rows behind the scattered image that take what falls outside of it (several: they are hot)
 
 struct Plan {
     bool tensor = false;           // at least one primitive runs on the tensor-core (tcgen05) kernels
@@ -32,7 +31,7 @@ struct Plan {
     size_t w_pack_kd[3] = {NO_BUF, NO_BUF, NO_BUF};   // weights packed [g][tap][s'][d']
     size_t dense[3] = {NO_BUF, NO_BUF, NO_BUF};       // dense tensor, rows dense_pitch apart (absent: the caller's own)
     int dense_pitch = 0;
-    size_t img_grad_cl = NO_BUF;   // f32 channels-last accumulator of the scatter, and SCATTER_WASTE_ROWS rows that nobody reads
+    size_t img_grad_cl = NO_BUF;   // f32 channels-last accumulator of the scatter
     size_t img_max = NO_BUF, mask_max = NO_BUF;   // see ColumnRange: maxima of the image's and the mask's blocks
     int n_img_max = 0, n_mask_max = 0;
     size_t off32 = NO_BUF, mask32 = NO_BUF, bias32 = NO_BUF;   // 16-bit offset / mask / bias widened to f32

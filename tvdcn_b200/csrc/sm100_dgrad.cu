@@ -148,6 +148,20 @@ __device__ __forceinline__ void flush_sums(uint32_t px, uint32_t cur, uint64_t a
         for (int k = 0; k < 8; ++k) v[k] = 0.f;
     }
 }
+// Weight of what adds nothing to its pixel: one outside of the image, or an entry that pads the list.  The former's pixel offset is that
+// of the place next to its real neighbour in memory, an ordinary pixel, so that running sums go on under it.  (With rows of waste
+// behind the image every such entry cost a flush, and in calls without offsets each entry lacks a pixel: backward kernel 64 x 64 x 56 x
+// 56 f32 502 us, now 205; 2 x 64 x 16 x 56 x 56 860, now 371; 128 x 256 x 28 x 28 bf16 with offsets 527, now 533.)  No product of two floats has
+// these bits (a NaN result is 0x7fffffff).  A weight of zero would not do: zero times an infinite column is NaN.
+constexpr uint32_t SC_NO_WEIGHT = 0xffffffffu;
+// sum += weight x column.  A branch: predicated multiply-adds take 580 instead of 551 us at 128 x 256 x 28 x 28 bf16.
+__device__ __forceinline__ void add_weighted(float (&sum)[8], uint32_t weight, const uint64_t (&c)[4]) {
+    if (weight != SC_NO_WEIGHT) {
+        const uint64_t ww = pack_f32x2(__uint_as_float(weight), __uint_as_float(weight));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) unpack_f32x2(fma_f32x2(ww, c[k], pack_f32x2(sum[2 * k], sum[2 * k + 1])), sum[2 * k], sum[2 * k + 1]);
+    }
+}
 // Where px != was: loads 4 + 4 channels, 32 apart, of 16-bit (4 words) or f32 (8 words) data.
 template <int IW>
 __device__ __forceinline__ void load_row(uint32_t px, uint32_t was, uint32_t (&v)[IW], uint64_t addr) {
@@ -776,11 +790,9 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     return __uint_as_float((uint32_t)d) + __uint_as_float((uint32_t)(d >> 32));
                 };
                 // adds weight x column to the sums, which were those of pixel `cur` and are now those of px
-                auto add = [&](float (&sum)[8], uint32_t px, uint32_t cur, float w, const uint64_t (&c)[4]) {
+                auto add = [&](float (&sum)[8], uint32_t px, uint32_t cur, uint32_t w, const uint64_t (&c)[4]) {
                     flush_sums(px, cur, row_at<4>(gimg_c, cur), sum);
-                    const uint64_t ww = pack_f32x2(w, w);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) unpack_f32x2(fma_f32x2(ww, c[k], pack_f32x2(sum[2 * k], sum[2 * k + 1])), sum[2 * k], sum[2 * k + 1]);
+                    add_weighted(sum, w, c);
                 };
                 // One entry, the one before it being `prev`; its image rows are in `rows`, which then receives those of `next`.
                 auto load_columns = [&](uint64_t (&c)[4], uint32_t meta) {
@@ -797,8 +809,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     }
                     fetch_rows(rows, next, e.x, e.y);
                     if constexpr (SCATTER) {
-                        add(ev, e.x, prev.x, __uint_as_float(e.z), c);
-                        add(od, e.y, prev.y, __uint_as_float(e.w), c);
+                        add(ev, e.x, prev.x, e.z, c);
+                        add(od, e.y, prev.y, e.w, c);
                     }
                 };
                 // sums over the 8 lanes of the four dots of two entries at once: after the exchanges lane (b2 b1 b0) holds dot 2 b2 + b1
@@ -859,9 +871,8 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
         UnitIter u = first_unit(P, unit0);
         PosInfo<DIM> pi = decode_blocked<DIM>(P, (long long)u.x * TILE_POS + pt);
         const uint32_t colq_row = (uint32_t)(pt * (L.col_stride / 4));
-        // Pixels outside the image: one of a few rows behind it, whose sums nobody reads (and whose image row may hold anything: nobody
-        // reads the dot product with it either).
-        const uint32_t waste = ((uint32_t)g.B * (uint32_t)g.S + (blockIdx.x % SCATTER_WASTE_ROWS)) * (uint32_t)g.Cs;
+        const uint32_t pixels = (uint32_t)g.B * (uint32_t)g.S;
+        const uint32_t padding = blockIdx.x % pixels * (uint32_t)g.Cs;   // where entries that pad the list add nothing: not one row for all
 
         // four words of padding behind every 32: a thread's 16 slots then meet those of its seven neighbours in no bank
         auto word_of = [](uint32_t slot) { return slot + (slot >> 5) * 4u; };
@@ -967,20 +978,21 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                             wr[0] *= tg.mval;
                         }
                         const uint32_t at = cnt[word_of(slot[i] & (SC_SLOTS - 1))] + (slot[i] >> 12 & 0xfffu);
-                        const uint32_t pl = (both & 1u) ? left[k] * (uint32_t)g.Cs : waste;
-                        const uint32_t pr = (both & 2u) ? (left[k] + 1u) * (uint32_t)g.Cs : waste;
+                        // (not behind the last pixel nor, where left is -1, before the first)
+                        const uint32_t pl = min(left[k], left[k] + 1u) * (uint32_t)g.Cs;
+                        const uint32_t pr = min(left[k] + 1u, pixels - 1u) * (uint32_t)g.Cs;
                         const bool odd = (left[k] & 1u) != 0u;
-                        const uint32_t a = __float_as_uint(wl[k]), b = __float_as_uint(wr[k]);
+                        const uint32_t a = (both & 1u) ? __float_as_uint(wl[k]) : SC_NO_WEIGHT;
+                        const uint32_t b = (both & 2u) ? __float_as_uint(wr[k]) : SC_NO_WEIGHT;
                         ent[at] = odd ? make_uint4(pr, pl, b, a) : make_uint4(pl, pr, a, b);
                         e_meta[at] = (colq_row + (uint32_t)(t * (CHUNK_C / 4))) | ((uint32_t)((pt * TB + t) * NC + 2 * q) << 16);
                     }
                 }
             }
-            // padding entries up to the end of the last span and the words the read-ahead of the last group touches:
-            // all point at the row of waste
+            // padding entries up to the end of the last span and the words the read-ahead of the last group touches
             const uint32_t n_words = span * SC_GROUPS + 4;
             for (uint32_t i = total + pt; i < n_words; i += 128) {
-                ent[i] = make_uint4(waste, waste, 0u, 0u);
+                ent[i] = make_uint4(padding, padding, SC_NO_WEIGHT, SC_NO_WEIGHT);
                 e_meta[i] = (uint32_t)(2 * L.max_entries) << 16;
             }
             planner_barrier();
