@@ -157,3 +157,13 @@ def test_offsets_that_are_not_finite(case, dtype, aux, tol, value):
         finite = torch.isfinite(ref[i])
         assert torch.equal(torch.isfinite(got[i]), finite), cases.NAMES[i]
         assert cases.nerr(torch.where(finite, got[i], 0), torch.where(finite, ref[i], 0)) <= tol, cases.NAMES[i]
+
+
+@pytest.mark.parametrize('case', ODD_OFFSETS, ids=[c.name for c in ODD_OFFSETS])
+def test_infinite_mask_of_a_cell_outside(case):
+    """Its product with the zeros of a cell outside of the image is NaN, on both engines."""
+    _, dev = _device_inputs(case, torch.float32, 88)
+    dev[2].flatten(2)[:, 0, 3] = 1e30
+    dev[3].flatten(2)[:, 0, 3] = float('inf')
+    got, ref = run_cabi(case, *dev, engine=2)[3], run_cabi(case, *dev, engine=1)[3]
+    assert torch.isnan(ref).any() and torch.equal(torch.isfinite(got), torch.isfinite(ref))

@@ -151,7 +151,7 @@ __device__ __forceinline__ void flush_sums(uint32_t px, uint32_t cur, uint64_t a
 // Weight of what adds nothing to its pixel: one outside of the image, or an entry that pads the list.  The former's pixel offset is that
 // of the place next to its real neighbour in memory, an ordinary pixel, so that running sums go on under it.  (With rows of waste
 // behind the image every such entry cost a flush, and in calls without offsets each entry lacks a pixel: backward kernel 64 x 64 x 56 x
-// 56 f32 502 us, now 205; 2 x 64 x 16 x 56 x 56 860, now 371; 128 x 256 x 28 x 28 bf16 with offsets 527, now 533.)  No product of two floats has
+// 56 f32 525 us, now 205; 2 x 64 x 16 x 56 x 56 818, now 359; with offsets 128 x 256 x 28 x 28 f32 662, now 670, bf16 527, now 525.)  No product of two floats has
 // these bits (a NaN result is 0x7fffffff).  A weight of zero would not do: zero times an infinite column is NaN.
 constexpr uint32_t SC_NO_WEIGHT = 0xffffffffu;
 // sum += weight x column.  A branch: predicated multiply-adds take 580 instead of 551 us at 128 x 256 x 28 x 28 bf16.
@@ -524,10 +524,25 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 }
             }
             const TapGeometry<DIM> tg = geometry(pi, one, 0, info.y + t);
+            // A cell outside of the image has no gradients, whatever its fractions are: those of an infinite offset are NaN.  (Left out
+            // here: selects at the end of the body cost 128 x 256 x 28 x 28 bf16 547 instead of 525 us, 8 x 64 x 160 x 160 301 instead of 271.)
+            bool inside = true;
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) inside = inside && (unsigned)tg.fl[a] + 1u <= (unsigned)g.img[a];
+            if (!inside) {
+                if (P.goff != nullptr) {
+                    const float none = tg.mval * 0.f;            // (but an infinite mask's product with them is NaN)
+#pragma unroll
+                    for (int a = 0; a < DIM; ++a) atomicAdd(po + (int64_t)a * g.P, none);
+                    po += DIM * (int64_t)g.P;
+                }
+                dots += NP;
+                pm += g.P;
+                continue;
+            }
             // the dots at the corners of the cell, then contracted axis by axis, the last one first: with the weights, and with (-1, 1) for
             // the axis whose derivative it is
             float val[NC], der[DIM][NC];
-            bool inside = false;
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
                 uint32_t left, key;
@@ -536,7 +551,6 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                 pair_of<DIM>(g, pi, tg, deformable, q, left, key, okl, okr, wl, wr);
                 const float2 e = dots[q];
                 const bool odd = (left & 1u) != 0u;
-                inside = inside || okl || okr;
                 val[2 * q] = okl ? (odd ? e.y : e.x) : 0.f;
                 val[2 * q + 1] = okr ? (odd ? e.x : e.y) : 0.f;
             }
@@ -552,15 +566,14 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     for (int a2 = a + 1; a2 < DIM; ++a2) der[a2][i] = fmaf(f, der[a2][2 * i + 1], f1 * der[a2][2 * i]);
                 }
             }
-            // A cell outside of the image has no gradients, whatever its fractions are: those of an infinite offset are NaN.
             if (P.goff != nullptr) {
 #pragma unroll
                 for (int a = 0; a < DIM; ++a) {
-                    atomicAdd(po, tg.mval * (inside ? der[a][0] : 0.f));
+                    atomicAdd(po, tg.mval * der[a][0]);
                     po += g.P;
                 }
             }
-            if (P.gmask != nullptr) atomicAdd(pm, inside ? val[0] : 0.f);
+            if (P.gmask != nullptr) atomicAdd(pm, val[0]);
             pm += g.P;
         }
     };
