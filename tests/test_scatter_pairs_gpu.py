@@ -120,9 +120,9 @@ def test_lone_pixels_take_nothing_that_is_not_finite(case, at, what):
     assert hit(ref[i]).any() and torch.equal(hit(got[i]), hit(ref[i]))
 
 
-@pytest.mark.parametrize('length', [1466, 1494], ids=['ranges', 'cta_per_tile'])
-def test_volumes_around_the_line(length):
-    """f32 volumes have one CTA per tile from 1480 tiles on."""
+@pytest.mark.parametrize('length', [1466, 1494], ids=['1466_tiles', '1494_tiles'])
+def test_volumes_of_one_unit_per_tile(length):
+    """f32, around ten tiles per SM: every unit begins a tile."""
     case = Case('volume', 3, False, 1, 64, 64, (2, 8, 8 * length), (1, 1, 2), (1, 1, 1), (0, 0, 0), (1, 1, 1), (), 1, 1, 1, True, 1.0)
     _, dev = _device_inputs(case, torch.float32, 84)
     got, ref = run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1)

@@ -1,6 +1,7 @@
 """Edges of how the tensor-core kernels share their work between CTAs: forward tiles that two CTAs sum together, CTAs that
 walk several tiles (the next dense tile is loaded under the old one), remainders of the split, volumes with one CTA per
 tile, and the line below which a padded transposed forward stays on the SIMT kernel."""
+import json
 import threading
 
 import pytest
@@ -95,17 +96,36 @@ def test_shared_tiles_of_calls_that_overlap():
         assert len(many) == 40 and all(torch.equal(one, r) for r in many)
 
 
-def test_volume_with_one_cta_per_tile():
-    """592 tiles and more of at least eight units: as many CTAs as tiles.  Too large for the CPU oracle, so the SIMT kernels,
-    which are checked against it elsewhere, stand in."""
-    case = Case('volume', 3, False, 2, 64, 64, (12, 57, 57), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0)
+def scatter_grids(fn, path):
+    """Runs fn() under the profiler; returns (numbers of CTAs of the scatter kernel's launches, fn's result)."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        out = fn()
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(path))
+    events = json.loads(path.read_text())['traceEvents']
+    return [e['args']['grid'][0] for e in events if 'dcn_dgrad_tc' in e.get('name', '') and 'grid' in e.get('args', {})], out
+
+
+@pytest.mark.parametrize('width,kernel,ctas', [
+    (59, (3, 3, 3), 148), (60, (3, 3, 3), 1487),      # 1463 and 1487 tiles of nine units
+    (60, (1, 2, 3), 148), (60, (1, 7, 1), 1487),      # two and three units per tile
+], ids=['few_tiles', 'many_tiles', 'two_units', 'three_units'])
+def test_volume_with_one_cta_per_tile(width, kernel, ctas, tmp_path):
+    """f32: as many CTAs as tiles from 1480 tiles of at least three units on, else one per SM.  Too large for the CPU oracle, so the
+    SIMT kernels, which are checked against it elsewhere, stand in."""
+    pad = tuple(k // 2 for k in kernel)
+    extent = tuple(n + k - 1 - 2 * p for n, k, p in zip((26, 61, width), kernel, pad))     # of the input: 26 x 61 x width positions
+    case = Case('volume', 3, False, 2, 64, 64, extent, kernel, (1, 1, 1), pad, (1, 1, 1), (), 1, 1, 1, True, 1.0)
     dev = [t.float().cuda() for t in make_inputs(case, seed=72)]
-    cases.assert_parity(run_cabi(case, *dev, engine=2), run_cabi(case, *dev, engine=1), 1e-4, case.name)
+    grids, got = scatter_grids(lambda: run_cabi(case, *dev, engine=2), tmp_path / 'trace.json')
+    assert grids == [ctas]
+    cases.assert_parity(got, run_cabi(case, *dev, engine=1), 1e-4, case.name)
 
 
-@pytest.mark.parametrize('width', [58, 60], ids=['ranges', 'one_per_tile'])
-def test_volume_of_16_bit_data_around_its_line(width):
-    """290 and 300 tiles: around two tiles per SM."""
+@pytest.mark.parametrize('width', [58, 60], ids=['290_tiles', '300_tiles'])
+def test_volume_of_16_bit_data(width):
+    """Around two tiles per SM."""
     case = Case('volume16', 3, False, 1, 64, 64, (16, 40, width), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), (), 1, 1, 1, True, 1.0)
     x, w, off, mask, bias, go = (t.float().cuda() for t in make_inputs(case, seed=77))
     dev = [x.bfloat16(), w.bfloat16(), off, mask, bias, go.bfloat16()]
