@@ -37,7 +37,7 @@
 // form of the loop: two entries per iteration and no more (a loop of four, 6 KB of code beside the planners' and finishers' straight
 // lines, took 574 instead of 551 us at 128 x 256 x 28 x 28 bf16, 4 groups of offsets), columns and entries read ahead, one
 // branch per flush.  Before, one entry per corner, 4 channels per lane and the columns staged in two halves: 799 us there, 850 f32,
-// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 678, 1162, 2644.  (16 gather warps have
+// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 525, 670, 1177, 2728.  (16 gather warps have
 // no registers to read columns ahead: 586 us, and 768 with the spills of trying.)
 //
 // Warp roles (768 threads): 0-3 finish, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
@@ -213,7 +213,7 @@ __device__ __forceinline__ PosInfo<DIM> decode_blocked(const DgradParams<DIM> &P
         int first[DIM], ext[DIM], size = g.P;              // size: positions of what is being cut (image, slab, strip)
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
-            const int line = size / g.grid[a] ;            // positions per unit of length along this axis
+            const int line = size / g.grid[a];            // positions per unit of length along this axis
             const int blk = r / (line * P.block[a]);
             first[a] = blk * P.block[a];
             ext[a] = min(P.block[a], g.grid[a] - first[a]);
@@ -281,9 +281,9 @@ struct ScLayout {
     uint32_t b_stage, plan_buf, col, plan, info, pos, cnt, taps, misc, bars, total;
     int n, col_stride, max_entries;
 };
-__host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_stages) {
+__host__ __device__ inline ScLayout sc_layout(int dim, int tb, int b_stages) {
     ScLayout L;
-        L.n = tb * SC_SLAB;
+    L.n = tb * SC_SLAB;
     L.col_stride = 2 * L.n + 4;                   // words; = 4 mod 32, so that the row-per-lane stores spread over the banks
     L.max_entries = TILE_POS * tb << (dim - 1);
     L.b_stage = (uint32_t)(L.n * 128);             // one 16-bit part (hi or lo) of one reduction chunk
@@ -298,16 +298,16 @@ __host__ __device__ inline ScLayout sc_layout(int dim, int mode, int tb, int b_s
     L.pos = o;  o += 4 * TILE_POS * 8;            // and per position of the tile: image (or -1), position in it
     L.cnt = o;  o += SC_SLOT_WORDS * 4;
     L.taps = o; o += SC_MAX_TAPS * 4;             // kernel coordinates of every tap, ten bits per axis
-    L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot, reloads
+    L.misc = o; o += 64;                          // scan partial sums [4], wait flag, entry counts [2], TMEM slot
     L.bars = o; o += (uint32_t)(18 + 2 * b_stages) * 8;
     L.total = o;
     return L;
 }
 
 // The units of a CTA in order.  1-d and 2-d: a CTA's tiles follow one another, so it finds its neighbourhood of the image
-// in the caches.  3-d: that neighbourhood spans planes and 148 of them do not fit L2 (contiguous ranges: 5.1 ms instead of
-// 4.4 for 8 x 64 x 16 x 56 x 56), so the CTAs take neighbouring tiles at the same time: ranges run down the columns of a matrix of
-// tiles with one column per CTA, filled row by row.
+// in the caches.  3-d: that neighbourhood spans planes and 148 of them do not fit L2 (tiles one after the other: 8 x 64 x 16 x 56 x 56
+// bf16 2573 instead of 2289 us, 2 x 64 x 16 x 56 x 56 f32 732 instead of 695), so the CTAs take neighbouring tiles at the same time: ranges
+// run down the columns of a matrix of tiles with one column per CTA, filled row by row.  (One CTA per tile: the same order.)
 struct UnitIter {
     int x, grp, chunk, batch;   // position tile, group, 64-channel chunk, tap batch
     int order;                  // the tile's place in that order
@@ -374,7 +374,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     // align by offset, not by integer round-trip, so that the compiler keeps these as shared-memory pointers
     uint8_t *smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const int RC = P.rc, TB = P.tb, BS = P.b_stages, NACC = P.nacc;
-    const ScLayout L = sc_layout(DIM, MODE, TB, BS);
+    const ScLayout L = sc_layout(DIM, TB, BS);
     const int N = L.n;
     const int a_cols = g.cdg / 2;                       // TMEM columns of one 16-bit copy of the dense tile
     const uint32_t acc_col0 = (uint32_t)(a_cols * PARTS);
@@ -1177,13 +1177,13 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
     if (warp == SC_MMA_WARP) ptx::tmem_dealloc(tmem_base, SC_TMEM_COLS);
 }
 
-size_t dgrad_smem_bytes(int dim, int mode, int tb, int b_stages) {
-    return 1024 + sc_layout(dim, mode, tb, b_stages).total;
+size_t dgrad_smem_bytes(int dim, int tb, int b_stages) {
+    return 1024 + sc_layout(dim, tb, b_stages).total;
 }
 
 template <int DIM, int MODE>
 cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, cudaStream_t stream) {
-    const size_t smem = dgrad_smem_bytes(DIM, MODE, P.tb, P.b_stages);
+    const size_t smem = dgrad_smem_bytes(DIM, P.tb, P.b_stages);
     const bool coord = P.goff != nullptr || P.gmask != nullptr;
     // One CTA per SM, except for f32 volumes of many tiles, whose costs differ so much that the hardware's scheduling beats equal
     // ranges, once a tile has units enough to outweigh a CTA's start-up.  64 channels, us, ranges / one CTA per tile.  Backward kernel, f32,
@@ -1230,7 +1230,7 @@ bool dgrad_tc_config(const GeoHost &h, int mode, int *tb, int *nacc, int *b_stag
         const int acc = std::min(4, (SC_TMEM_COLS - a_cols) / (n * (mode == TC_F32_WIDE ? 2 : 1)));
         if (acc < 1) continue;
         for (int st = 4; st >= 2; --st)
-            if (dgrad_smem_bytes(h.dim, mode, t, st) <= 227 * 1024) {
+            if (dgrad_smem_bytes(h.dim, t, st) <= 227 * 1024) {
                 int tiles, per_tile, total;
                 if (!dgrad_units(h, t, &tiles, &per_tile, &total)) return false;
                 *tb = t;
