@@ -37,7 +37,7 @@
 // form of the loop: two entries per iteration and no more (a loop of four, 6 KB of code beside the planners' and finishers' straight
 // lines, took 574 instead of 551 us at 128 x 256 x 28 x 28 bf16, 4 groups of offsets), columns and entries read ahead, one
 // branch per flush.  Before, one entry per corner, 4 channels per lane and the columns staged in two halves: 799 us there, 850 f32,
-// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 525, 670, 1177, 2728.  (16 gather warps have
+// 64 x 512 x 4096 1-d f32 1907, 8 x 64 x 16 x 56 x 56 3-d f32 4147; now 531, 670, 1165, 2589.  (16 gather warps have
 // no registers to read columns ahead: 586 us, and 768 with the spills of trying.)
 //
 // Warp roles (768 threads): 0-3 finish, 4-15 gather, 16-19 planners, 20 MMA issue + TMEM owner, 21 TMA, 22-23 idle
@@ -151,16 +151,14 @@ __device__ __forceinline__ void flush_sums(uint32_t px, uint32_t cur, uint64_t a
 // Weight of what adds nothing to its pixel: one outside of the image, or an entry that pads the list.  The former's pixel offset is that
 // of the place next to its real neighbour in memory, an ordinary pixel, so that running sums go on under it.  (With rows of waste
 // behind the image every such entry cost a flush, and in calls without offsets each entry lacks a pixel: backward kernel 64 x 64 x 56 x
-// 56 f32 525 us, now 205; 2 x 64 x 16 x 56 x 56 818, now 359; with offsets 128 x 256 x 28 x 28 f32 662, now 670, bf16 527, now 525.)  No product of two floats has
+// 56 f32 525 us, now 207; 2 x 64 x 16 x 56 x 56 818, now 355; with offsets 128 x 256 x 28 x 28 f32 662, now 670, bf16 527, now 531.)  No product of two floats has
 // these bits (a NaN result is 0x7fffffff).  A weight of zero would not do: zero times an infinite column is NaN.
 constexpr uint32_t SC_NO_WEIGHT = 0xffffffffu;
-// sum += weight x column.  A branch: predicated multiply-adds take 580 instead of 551 us at 128 x 256 x 28 x 28 bf16.
+// sum += weight x column
 __device__ __forceinline__ void add_weighted(float (&sum)[8], uint32_t weight, const uint64_t (&c)[4]) {
-    if (weight != SC_NO_WEIGHT) {
-        const uint64_t ww = pack_f32x2(__uint_as_float(weight), __uint_as_float(weight));
+    const uint64_t ww = pack_f32x2(__uint_as_float(weight), __uint_as_float(weight));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) unpack_f32x2(fma_f32x2(ww, c[k], pack_f32x2(sum[2 * k], sum[2 * k + 1])), sum[2 * k], sum[2 * k + 1]);
-    }
+    for (int k = 0; k < 4; ++k) unpack_f32x2(fma_f32x2(ww, c[k], pack_f32x2(sum[2 * k], sum[2 * k + 1])), sum[2 * k], sum[2 * k + 1]);
 }
 // Where px != was: loads 4 + 4 channels, 32 apart, of 16-bit (4 words) or f32 (8 words) data.
 template <int IW>
@@ -523,23 +521,15 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     one.m[0] = ru.m[k];
                 }
             }
-            const TapGeometry<DIM> tg = geometry(pi, one, 0, info.y + t);
-            // A cell outside of the image has no gradients, whatever its fractions are: those of an infinite offset are NaN.  (Left out
-            // here: selects at the end of the body cost 128 x 256 x 28 x 28 bf16 547 instead of 525 us, 8 x 64 x 160 x 160 301 instead of 271.)
+            TapGeometry<DIM> tg = geometry(pi, one, 0, info.y + t);
+            // A cell outside of the image has no gradients, whatever its fractions are: those of an infinite offset are NaN.  (Us, 128 x 256 x 28 x
+            // 28 bf16 / 8 x 64 x 160 x 160 bf16 / 4 x 64 x 16 x 56 x 56 coordinate gradients f32: selects of the results, behind the contraction, 547 /
+            // 301 / 1026; leaving the body here 527 / 271 / 1053; selects of the fractions 531 / 275 / 1020.)
             bool inside = true;
 #pragma unroll
             for (int a = 0; a < DIM; ++a) inside = inside && (unsigned)tg.fl[a] + 1u <= (unsigned)g.img[a];
-            if (!inside) {
-                if (P.goff != nullptr) {
-                    const float none = tg.mval * 0.f;            // (but an infinite mask's product with them is NaN)
 #pragma unroll
-                    for (int a = 0; a < DIM; ++a) atomicAdd(po + (int64_t)a * g.P, none);
-                    po += DIM * (int64_t)g.P;
-                }
-                dots += NP;
-                pm += g.P;
-                continue;
-            }
+            for (int a = 0; a < DIM; ++a) tg.fr[a] = inside ? tg.fr[a] : 0.f;
             // the dots at the corners of the cell, then contracted axis by axis, the last one first: with the weights, and with (-1, 1) for
             // the axis whose derivative it is
             float val[NC], der[DIM][NC];
@@ -802,10 +792,26 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                     }
                     return __uint_as_float((uint32_t)d) + __uint_as_float((uint32_t)(d >> 32));
                 };
-                // adds weight x column to the sums, which were those of pixel `cur` and are now those of px
-                auto add = [&](float (&sum)[8], uint32_t px, uint32_t cur, uint32_t w, const uint64_t (&c)[4]) {
-                    flush_sums(px, cur, row_at<4>(gimg_c, cur), sum);
-                    add_weighted(sum, w, c);
+                // Adds weight x column to the sums, which were those of the pixels of `prev` and are now those of e's.  The test of the weights, us:
+                // f32 data, one branch for entries that have both pixels, 8 x 64 x 16 x 56 x 56 2629, 128 x 256 x 28 x 28 676; a branch for each
+                // pixel 2737, 680; bf16 2406, 576 and 2306, 531 (predicated multiply-adds 2456, 580).
+                auto add = [&](const uint4 &prev, const uint4 &e, const uint64_t (&c)[4]) {
+                    if constexpr (M::F32) {
+                        flush_sums(e.x, prev.x, row_at<4>(gimg_c, prev.x), ev);
+                        flush_sums(e.y, prev.y, row_at<4>(gimg_c, prev.y), od);
+                        if (max(e.z, e.w) != SC_NO_WEIGHT) {
+                            add_weighted(ev, e.z, c);
+                            add_weighted(od, e.w, c);
+                        } else {
+                            if (e.z != SC_NO_WEIGHT) add_weighted(ev, e.z, c);
+                            if (e.w != SC_NO_WEIGHT) add_weighted(od, e.w, c);
+                        }
+                    } else {
+                        flush_sums(e.x, prev.x, row_at<4>(gimg_c, prev.x), ev);
+                        if (e.z != SC_NO_WEIGHT) add_weighted(ev, e.z, c);
+                        flush_sums(e.y, prev.y, row_at<4>(gimg_c, prev.y), od);
+                        if (e.w != SC_NO_WEIGHT) add_weighted(od, e.w, c);
+                    }
                 };
                 // One entry, the one before it being `prev`; its image rows are in `rows`, which then receives those of `next`.
                 auto load_columns = [&](uint64_t (&c)[4], uint32_t meta) {
@@ -821,10 +827,7 @@ dcn_dgrad_tc_kernel(const DgradParams<DIM> P, const __grid_constant__ CUtensorMa
                         d_od = dot(c, rows.od);
                     }
                     fetch_rows(rows, next, e.x, e.y);
-                    if constexpr (SCATTER) {
-                        add(ev, e.x, prev.x, e.z, c);
-                        add(od, e.y, prev.y, e.w, c);
-                    }
+                    if constexpr (SCATTER) add(prev, e, c);
                 };
                 // sums over the 8 lanes of the four dots of two entries at once: after the exchanges lane (b2 b1 b0) holds dot 2 b2 + b1
                 auto reduce = [&](const float (&d)[4], uint32_t m0, uint32_t m1) {
