@@ -326,30 +326,32 @@ def peaks():
     return {'hbm_gbs': 6650.0, 'tflops_burst': 1590.0, 'tflops_sustained': 1400.0, 'source': 'fallback'}
 
 
-def known_traffic(kernel: str, config: int, mode: str):
-    """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from the ncu captures summarised
-    under profiles/; None where no capture exists.  The figures are for the configuration's full batch on one GPU."""
+def known_traffic(kernel: str, config: int, mode: str, batch: int, full_batch: int):
+    """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) for `batch` images on one GPU, from the ncu captures
+    summarised under profiles/; None where no capture has the form of the launch."""
     table = {
-        # config 2: full-size launches (profiles/config2_tensor_kernels.md)
-        'dcn_fwd_tc/cfg2/bf16': 98.1e6 + 21.5e6,
-        'dcn_dgrad_tc/cfg2/bf16': 427.2e6 + 219.8e6,
-        'dcn_wgrad_tc/cfg2/bf16': 137.7e6 + 3.62e6,
-        'dcn_fwd_tc/cfg2/fp32': 206.4e6 + 74.7e6,
-        'dcn_dgrad_tc/cfg2/fp32': 767.7e6 + 281.5e6,
-        'dcn_wgrad_tc/cfg2/fp32': 250.8e6 + 6.04e6,
-        # configs 3-5: captured on a cut batch (profiles/config3_config4_config5_tensor_kernels.md) and scaled to
-        # the full batch by the images processed -- tiles are independent, traffic grows in proportion
-        'dcn_fwd_tc/cfg3/fp32': (75.52e6 + 27.14e6) * 8,
-        'dcn_dgrad_tc/cfg3/fp32': (222.9e6 + 44.69e6) * 8,
-        'dcn_wgrad_tc/cfg3/fp32': (141.0e6 + 4.24e6) * 8,
-        'dcn_fwd_tc/cfg4/fp32': (72.92e6 + 11.68e6) * 4,
-        'dcn_dgrad_tc/cfg4/fp32': (255.6e6 + 59.92e6) * 4,
-        'dcn_wgrad_tc/cfg4/fp32': (95.95e6 + 4.61e6) * 4,
-        'dcn_fwd_tc/cfg5/fp32': (41.01e6 + 0.16e6) * 4,
-        'dcn_dgrad_tc/cfg5/fp32': (57.79e6 + 0.03e6 + 63.18e6 + 2.08e6) / 2 * 4,   # two launches per step, mean
-        'dcn_wgrad_tc/cfg5/fp32': (57.75e6 + 0.65e6) * 4,
+        # config 2: full-size launches
+        'dcn_fwd_tc/cfg2/bf16': 98.1e6 + 23.0e6,
+        'dcn_dgrad_tc/cfg2/bf16': 428.5e6 + 221.7e6,
+        'dcn_wgrad_tc/cfg2/bf16': 137.7e6 + 3.51e6,
+        'dcn_fwd_tc/cfg2/fp32': 204.4e6 + 74.7e6,
+        'dcn_dgrad_tc/cfg2/fp32': 772.5e6 + 283.5e6,
+        'dcn_wgrad_tc/cfg2/fp32': 250.8e6 + 5.90e6,
+        # configs 3-5: captured on a cut batch and scaled to the full one by the images processed
+        'dcn_fwd_tc/cfg3/fp32': (75.55e6 + 26.95e6) * 8,
+        'dcn_dgrad_tc/cfg3/fp32': (222.1e6 + 43.75e6) * 8,
+        'dcn_wgrad_tc/cfg3/fp32': (141.0e6 + 6.46e6) * 8,
+        'dcn_fwd_tc/cfg4/fp32': (143.8e6 + 40.00e6) * 2,
+        'dcn_dgrad_tc/cfg4/fp32': (328.7e6 + 107.0e6) * 2,
+        'dcn_wgrad_tc/cfg4/fp32': (195.9e6 + 5.91e6) * 2,
+        'dcn_fwd_tc/cfg5/fp32': (41.01e6 + 0.93e6) * 4,
+        'dcn_dgrad_tc/cfg5/fp32': (57.78e6 + 0.14e6 + 63.29e6 + 1.87e6) / 2 * 4,   # two launches per step, mean
+        'dcn_wgrad_tc/cfg5/fp32': (57.75e6 + 0.74e6) * 4,
     }
-    return table.get(f'{kernel}/cfg{config}/{mode}')
+    if kernel == 'dcn_dgrad_tc' and config == 4 and batch < 4:
+        return None   # below 1480 tiles: ranges of tiles, in another order than the captured launch's one CTA per tile
+    traffic = table.get(f'{kernel}/cfg{config}/{mode}')
+    return None if traffic is None else traffic * batch / full_batch
 
 
 class DeviceStep:
@@ -615,9 +617,7 @@ def dominant_roofline(cfg: Config, kernels: dict, batch: int, config_index: int,
         return None
     dom = max(kernels, key=lambda k: kernels[k]['ms_per_step'])
     ms = kernels[dom]['ms_per_launch']
-    traffic = known_traffic(dom, config_index, mode)
-    if traffic is not None:
-        traffic *= batch / cfg.batch      # the captures are for the whole batch; traffic grows with the images
+    traffic = known_traffic(dom, config_index, mode, batch, cfg.batch)
     if cfg.bound == 'tensor' and dom in gemm_like:
         ach = cfg.flops_per_pass(batch) / (ms / 1e3) / 1e12
         # a kernel of about a millisecond timed by events between other kernels: the burst figure is the denominator
