@@ -1190,11 +1190,11 @@ cudaError_t launch_dgrad_t(const DgradParams<DIM> &P, const CUtensorMap *maps, c
     const bool coord = P.goff != nullptr || P.gmask != nullptr;
     // One CTA per SM, except for f32 volumes of many tiles, whose costs differ so much that the hardware's scheduling beats equal
     // ranges, once a tile has units enough to outweigh a CTA's start-up.  64 channels, us, ranges / one CTA per tile.  Backward kernel, f32,
-    // 27 taps (nine units): 392 tiles 334 / 363, 784 674 / 713, 1568 1429 / 1393, 2352 2056 / 2046, 256 dense channels 1568 1605 / 1516; 18
-    // taps 6272 3788 / 3694, the transposed one 3188 / 2992; 8 taps (three units) 1568 476 / 474, 2352 721 / 760, 6272 1916 / 1980, transposed with
-    // stride 2 2744 1055 / 961; 6 taps (two) 1568 381 / 433, 2352 599 / 639; 1 tap 127 / 209, 177 / 300.  So the lines are at ten tiles per SM
-    // and three units.  The scatter alone: 8 taps 1568 277 / 338, with stride 2 2744 889 / 766, 6 taps 1568 213 / 275, 1 tap 99 / 152.  16-bit data,
-    // with its shorter start-up but also shorter tiles: 27 taps 784 588 / 664, 3136 2300 / 2433, 8 taps 2744 1510 / 1466.
+    // 27 taps (nine units): 392 tiles 328 / 355, 784 668 / 701, 1568 1388 / 1330, 3136 2769 / 2597; 18 taps (six) 1568 871 / 904, 6272 3783 /
+    // 3531, the transposed one 3164 / 2924; 8 taps (three) 1568 480 / 502, 2352 723 / 742, 6272 1934 / 1931, transposed with stride 2 2744
+    // 1039 / 951; 6 taps (two) 1568 383 / 418, 2352 611 / 617; one tap 132 / 205, 179 / 293.  So the lines are at ten tiles per SM and three
+    // units.  The scatter alone: 27 taps 1568 744 / 822, 8 taps 277 / 344, but with stride 2 2744 887 / 768; 6 taps 1568 209 / 279, one tap 99 / 154.
+    // 16-bit data, with its shorter start-up but also shorter tiles: 27 taps 784 601 / 678, 3136 2348 / 2479, 8 taps 2744 662 / 758.
     const int tiles = P.total_units / P.n_units;
     const bool one_per_tile = DIM == 3 && Mode<MODE>::F32 && P.n_units >= 3 && tiles >= 10 * 148;
     const dim3 grid((unsigned)(one_per_tile ? tiles : std::min(P.total_units, 148)));
